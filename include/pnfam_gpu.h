@@ -227,8 +227,9 @@ int pnfam_gpu_calc_hamiltonian(pnfam_ctx_t* ctx,
 
 /*
  * The same field evaluation in the arithmetic of the mixed form's increment
- * evaluations: densities and fields in FP32, the field projection on the
- * tensor cores as 3xTF32 products (about FP32 accuracy).  No counterpart in
+ * evaluations: densities, fields and projection in FP32 (a basis of z x radial
+ * products: direction by direction; any other basis: on the tensor cores as
+ * 3xTF32 products, about FP32 accuracy).  No counterpart in
  * the reference.  Inputs and outputs as for pnfam_gpu_calc_hamiltonian.
  */
 int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* ctx,

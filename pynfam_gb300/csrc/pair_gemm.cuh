@@ -332,19 +332,20 @@ __global__ void __launch_bounds__(PG_THREADS, 1) k_pg_gemm(const PGProb* __restr
 // ---------------------------------------------------------------------------
 struct PGFold { int dens[12]; };
 
-__device__ __forceinline__ void accC(float (&acc)[2 * ND], int k, float re, float im) {
+template <class T>
+__device__ __forceinline__ void accC(T (&acc)[2 * ND], int k, T re, T im) {
   acc[2 * k] += re;
   acc[2 * k + 1] += im;
 }
 
 // same-spin class (row spin = column spin = sg): the terms of dens_same with the row
 // sums W_q(r, b) times phi_q'(b, r) summed over the columns, i.e. C(q, q')
-__device__ __forceinline__ void fold_same(float (&acc)[2 * ND], const float (&Cr)[16], const float (&Ci)[16],
-                                          float sg) {
-  const float h5 = 0.5f;
+template <class T>
+__device__ __forceinline__ void fold_same(T (&acc)[2 * ND], const T (&Cr)[16], const T (&Ci)[16], T sg) {
+  const T h5 = T(0.5);
 #define CR(i, j) Cr[(i) * 4 + (j)]
 #define CI(i, j) Ci[(i) * 4 + (j)]
-  float xr, xi;
+  T xr, xi;
   xr = CR(0, 0); xi = CI(0, 0);
   accC(acc, D_RHO, xr, xi);
   accC(acc, D_SZ, sg * xr, sg * xi);
@@ -363,23 +364,23 @@ __device__ __forceinline__ void fold_same(float (&acc)[2 * ND], const float (&Cr
   accC(acc, D_GS, sg * (CR(0, 3) + CR(3, 0)), sg * (CI(0, 3) + CI(3, 0)));
   accC(acc, D_FR, h5 * sg * (CR(1, 3) + CR(3, 1)), h5 * sg * (CI(1, 3) + CI(3, 1)));
   {
-    const float ar = h5 * sg * (CR(2, 3) - CR(3, 2)), ai = h5 * sg * (CI(2, 3) - CI(3, 2));
+    const T ar = h5 * sg * (CR(2, 3) - CR(3, 2)), ai = h5 * sg * (CI(2, 3) - CI(3, 2));
     accC(acc, D_FP, -ai, ar);
   }
   accC(acc, D_FZ, sg * CR(3, 3), sg * CI(3, 3));
 }
 
 // opposite-spin class: the terms of dens_opp (sig = +1 when the column is spin down)
-__device__ __forceinline__ void fold_opp(float (&acc)[2 * ND], const float (&Cr)[16], const float (&Ci)[16],
-                                         float sig) {
-  const float h5 = 0.5f;
-  float xr, xi;
+template <class T>
+__device__ __forceinline__ void fold_opp(T (&acc)[2 * ND], const T (&Cr)[16], const T (&Ci)[16], T sig) {
+  const T h5 = T(0.5);
+  T xr, xi;
   accC(acc, D_GS, sig * (CR(0, 2) - CR(2, 0)) + (CR(0, 1) + CR(1, 0)),
        sig * (CI(0, 2) - CI(2, 0)) + (CI(0, 1) + CI(1, 0)));
   accC(acc, D_FR, CR(1, 1) + sig * h5 * (CR(1, 2) - CR(2, 1)), CI(1, 1) + sig * h5 * (CI(1, 2) - CI(2, 1)));
   {
-    const float ar = sig * CR(2, 2) + h5 * (CR(2, 1) - CR(1, 2));
-    const float ai = sig * CI(2, 2) + h5 * (CI(2, 1) - CI(1, 2));
+    const T ar = sig * CR(2, 2) + h5 * (CR(2, 1) - CR(1, 2));
+    const T ai = sig * CI(2, 2) + h5 * (CI(2, 1) - CI(1, 2));
     accC(acc, D_FP, -ai, ar);
   }
   accC(acc, D_FZ, h5 * (CR(3, 1) + sig * CR(3, 2) + CR(1, 3) - sig * CR(2, 3)),

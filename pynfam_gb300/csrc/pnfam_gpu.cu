@@ -8,6 +8,7 @@
 #include "../../include/pnfam_gpu.h"
 #include "pnfam_kernels.cuh"
 #include "pair_gemm.cuh"
+#include "separable.cuh"
 #include "tbc.cuh"
 #include "hfb.cuh"
 
@@ -49,6 +50,8 @@ namespace {
 
 // asynchronous FP64 anchor batches an engine keeps in flight at most
 constexpr int ANCH_RING = 8;
+// shortest Broyden history of an FP64 run that takes the unit sums (pnfam_ctx::sep64)
+constexpr int SEP_MIN_HISTORY = 16;
 
 template <class T>
 struct DBuf {
@@ -305,6 +308,41 @@ struct pnfam_ctx {
   DBuf<PGTask> d_pg_tproj, d_pg_tdens;
   DBuf<PGBChunk> d_pg_bproj, d_pg_bdens;
   DBuf<float> d_pg_a, d_pg_b, d_pg_d;
+  // basis of z x radial products (separable.cuh): found and checked at creation
+  // (PNFAM_GB300_SEPARABLE=0: not looked for).  sep32: the FP32 evaluations take it too,
+  // unless a setting of the general FP32 kernels (PNFAM_GB300_TC_DENSITY, _PAIR_GEMM,
+  // _PAIR_MIN, _PAIR_KSPAN) asks for those
+  bool sep = false, sep32 = false;
+  SepBasis sepb;
+  SepStruct seps[5];          // F, X^T, Y^T, X, Y
+  struct SepBufs {            // device copy of one structure
+    DBuf<SepUnit> units;
+    DBuf<SepEnt> ents;
+    DBuf<int> rows, offs, ubeg, order;
+    DBuf<SepItem> items;
+    DBuf<SepWarp> warps;
+    void release() {
+      units.release(); ents.release(); rows.release(); offs.release(); ubeg.release(); order.release();
+      items.release(); warps.release();
+    }
+  } d_seps[5];
+  DBuf<double> d_sepf;        // z, r, v, y, e, lam, sgn
+  DBuf<float> d_sepf32;
+  DBuf<double> d_sepg;        // [P][gstride] unit sums
+  DBuf<float> d_sepg32;
+  long long sep_gstride = 0, sep_gpair[2] = {0, 0};
+  // Which evaluations of the current run take it (engine_setup):
+  // sep64: the FP64 ones.  A Broyden history shorter than SEP_MIN_HISTORY wraps early, and
+  // the iteration then amplifies rounding 1.6-fold per step (measured: 40S, N_sh = 8,
+  // M = 7, alpha = 0.4: final states of runs that differ by 2e-16 in the first field are
+  // 1e-8 apart after 42 steps); such FP64 runs keep the sums over the mesh, and with them
+  // the trajectories that they had.
+  // pair32: a mixed-form run that does not certify its strengths (opts.reserved[3] = 0)
+  // returns what its FP32 evaluations lead to, so it keeps the pair-tensor GEMMs from the
+  // tuned point count on: their long tensor-core sums differ from the unit sums by 1e-5 in
+  // 12 steps, while the strengths of certified runs agree to 1e-8 for either.
+  bool sep64 = false, pair32 = false, tuning = false;
+  bool pg_ready = false;      // pg_setup done for the current operator
   int nchunk_bro = 1, nchunk_c = 1;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -357,6 +395,8 @@ struct pnfam_ctx {
     k2a.d_tasks.release(); k2a.d_tile2task.release();
     k2b.d_tasks.release(); k2b.d_tile2task.release();
     t1a.d_tasks.release(); t1b.d_tasks.release(); t2a.d_tasks.release(); t2b.d_tasks.release();
+    for (SepBufs& b : d_seps) b.release();
+    d_sepf.release(); d_sepf32.release(); d_sepg.release(); d_sepg32.release();
     if (ev[0]) cudaEventDestroy(ev[0]);
     if (ev[1]) cudaEventDestroy(ev[1]);
     if (evt[0]) cudaEventDestroy(evt[0]);
@@ -918,7 +958,8 @@ static int ensure_buffers(pnfam_ctx* c, int P, int M) {
   CK(dalloc(c->d_rsp, (size_t)P * 8 * nxy));
   CK(dalloc(c->d_hsp, (size_t)P * 8 * nxy));
   CK(dalloc(c->d_hqp, (size_t)P * nv));
-  CK(dalloc(c->d_dpart, (size_t)P * 2 * c->G * 2 * ND * c->nghl));
+  CK(dalloc(c->d_dpart, (size_t)P * 2 * std::max(4, c->G) * 2 * ND * c->nghl));
+  if (c->sep) CK(dalloc(c->d_sepg, (size_t)P * c->sep_gstride));
   CK(dalloc(c->d_mf, (size_t)P * 2 * NMF * 2 * c->nghl));
   const int Mh = std::max(M, 1);
   CK(dalloc(c->d_df, (size_t)P * Mh * nv));
@@ -982,6 +1023,165 @@ static int launch_gemm(pnfam_ctx* c, TaskList& tl, int P, const int* active) {
   return launch_gemm<double>(c, tl, P, active, c->d_bufs.p, c->stream);
 }
 
+// fields in the SP basis -> dH_qp
+template <class T, class Tic, class Toc>
+static int residual_k2(pnfam_ctx* c, int P, int nact, const int* act, const BufDescT<T>* bufs, cudaStream_t st,
+                       Tic&& tic, Toc&& toc) {
+  int rc;
+  tic();
+  if constexpr (std::is_same<T, float>::value) {
+    if ((rc = launch_gemm_tc(c, c->t2a, nact, st))) return rc;
+    if ((rc = launch_gemm_tc(c, c->t2b, nact, st))) return rc;
+  } else {
+    if ((rc = launch_gemm<T>(c, c->k2a, P, act, bufs, st))) return rc;
+    if ((rc = launch_gemm<T>(c, c->k2b, P, act, bufs, st))) return rc;
+  }
+  toc(4);
+  return PNFAM_OK;
+}
+
+// ---------------------------------------------------------------------------
+// basis of z x radial products (separable.cuh)
+// ---------------------------------------------------------------------------
+static constexpr int SEP_SMEM_MAX = 200 * 1024;   // dynamic shared memory of k_sep_field
+
+// look for the factors (once per context); c->sep stays false when the basis functions
+// are not products or a size is beyond what the kernels take
+static int sep_init(pnfam_ctx* c, const double* phi) {
+  const int nb = c->nb, dqp = c->dqp, nghl = c->nghl;
+  for (int i = 0; i < nb; ++i)
+    for (int a = 0; a < c->db[i]; ++a)
+      if (c->ns[c->st[i] + a] != (a < c->nup[i] ? 1 : -1)) return PNFAM_OK;
+  const int ngh = dqp > 0 ? sep_mesh(dqp, nghl, phi) : 0;
+  if (!ngh || ngh > 128 || sep_field_smem<double>(ngh) > SEP_SMEM_MAX) return PNFAM_OK;
+  SepBasis& B = c->sepb;
+  if (!sep_factors(nb, c->db.data(), c->st.data(), c->nup.data(), dqp, nghl, ngh, phi, B)) return PNFAM_OK;
+  std::vector<double> f;
+  for (const auto* v : {&B.r, &B.z, &B.v, &B.y, &B.e, &B.lam, &B.sgn}) f.insert(f.end(), v->begin(), v->end());
+  CK(upload(c->d_sepf, f.data(), f.size()));
+  std::vector<int> idx(3 * (size_t)dqp);
+  for (int i = 0; i < nb; ++i)
+    for (int a = 0; a < c->db[i]; ++a) {
+      const int k = c->st[i] + a;
+      idx[k] = B.zi[k]; idx[dqp + k] = B.ri[k]; idx[2 * (size_t)dqp + k] = 2 * i + (a >= c->nup[i]);
+    }
+  DBuf<int> d_idx, d_bad;
+  int bad = 1;
+  const double* p = c->d_sepf.p;
+  const double *r = p, *z = r + B.r.size(), *v = z + B.z.size(), *y = v + B.v.size(), *e = y + B.y.size(),
+               *lam = e + B.e.size(), *sgn = lam + B.lam.size();
+  cudaError_t err = upload(d_idx, idx.data(), idx.size());
+  if (err == cudaSuccess) err = dalloc(d_bad, 1);
+  if (err == cudaSuccess) err = cudaMemsetAsync(d_bad.p, 0, sizeof(int), c->stream);
+  if (err == cudaSuccess) {
+    k_sep_check<<<dqp, 128, 0, c->stream>>>(c->d_phi.p, dqp, nghl, ngh, z, r, v, y, e, lam, sgn, d_idx.p, d_idx.p + dqp,
+                                            d_idx.p + 2 * dqp, d_bad.p);
+    err = cudaGetLastError();
+  }
+  if (err == cudaSuccess) err = cudaMemcpyAsync(&bad, d_bad.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
+  if (err == cudaSuccess) err = cudaStreamSynchronize(c->stream);
+  d_idx.release();
+  d_bad.release();
+  CK(err);
+  c->sep = bad == 0;
+  return PNFAM_OK;
+}
+
+// the operator's units (once per operator); a structure that does not fit keeps the
+// general kernels for this context
+static int sep_operator(pnfam_ctx* c) {
+  if (!c->sep) return PNFAM_OK;
+  const std::vector<int>* cols[5] = {&c->fc, &c->xtc, &c->ytc, &c->xc, &c->yc};
+  const std::vector<long long>* offs[5] = {&c->foff, &c->xtoff, &c->ytoff, &c->xoff, &c->yoff};
+  for (int k = 0; k < 5; ++k) {
+    if (!sep_structure(c->sepb, c->nb, c->db.data(), c->st.data(), c->nup.data(), cols[k]->data(), offs[k]->data(),
+                       k == 0 || k >= 3, c->seps[k])) {
+      c->sep = c->sep32 = false;
+      return PNFAM_OK;
+    }
+    const SepStruct& s = c->seps[k];
+    auto& d = c->d_seps[k];
+    CK(upload(d.units, s.units.data(), s.units.size()));
+    CK(upload(d.ents, s.ents.data(), s.ents.size()));
+    CK(upload(d.rows, s.rows.data(), s.rows.size()));
+    CK(upload(d.offs, s.offs.data(), s.offs.size()));
+    CK(upload(d.ubeg, s.ubeg.data(), s.ubeg.size()));
+    CK(upload(d.order, s.order.data(), s.order.size()));
+    CK(upload(d.items, s.items.data(), s.items.size()));
+    CK(upload(d.warps, s.warps.data(), s.warps.size()));
+  }
+  const long long ngl = c->sepb.ngl, nf = (long long)c->seps[0].units.size();
+  c->sep_gpair[0] = 2 * ngl * nf * 2 * SH_N;
+  c->sep_gpair[1] = c->sep_gpair[0] + 2 * ngl * (long long)std::max(c->seps[1].units.size(), c->seps[3].units.size());
+  c->sep_gstride = c->sep_gpair[1] + 2 * ngl * (long long)std::max(c->seps[2].units.size(), c->seps[4].units.size());
+  return PNFAM_OK;
+}
+
+template <class T>
+static SepDev<T> sep_dev(const pnfam_ctx* c, const T* factors, T* g) {
+  const SepBasis& B = c->sepb;
+  SepDev<T> S;
+  S.ngh = B.ngh; S.ngl = B.ngl; S.nzf = B.nzf; S.nghl = c->nghl;
+  S.r = reinterpret_cast<const typename Vec2<T>::t*>(factors);
+  S.z = factors + B.r.size(); S.v = S.z + B.z.size(); S.y = S.v + B.v.size(); S.e = S.y + B.y.size();
+  S.lam = S.e + B.e.size(); S.sgn = S.lam + B.lam.size();
+  SepStructDev* to[5] = {&S.f, &S.k[0], &S.k[1], &S.d[0], &S.d[1]};
+  for (int k = 0; k < 5; ++k) {
+    const auto& d = c->d_seps[k];
+    *to[k] = {d.units.p, d.ents.p, d.rows.p, d.offs.p, d.ubeg.p, d.order.p, d.items.p, d.warps.p,
+              (int)c->seps[k].units.size(), (int)c->seps[k].warps.size()};
+  }
+  S.gstride = c->sep_gstride; S.gpair[0] = c->sep_gpair[0]; S.gpair[1] = c->sep_gpair[1];
+  S.g = g; S.list = nullptr; S.act = nullptr; S.n = 0;
+  return S;
+}
+
+// densities, mean field and projection of the points flagged in act (FP64) or listed in
+// c->d_actlist (FP32, nact of them)
+template <class T, class Tic, class Toc>
+static int sep_field(pnfam_ctx* c, int P, int nact, const int* act, const T* rsp, T* dpart, T* mf, T* hsp,
+                     cudaStream_t st, Tic&& tic, Toc&& toc) {
+  constexpr bool f32 = std::is_same<T, float>::value;
+  SepDev<T> S;
+  if constexpr (f32) {
+    S = sep_dev<float>(c, c->d_sepf32.p, c->d_sepg32.p);
+    S.list = c->d_actlist.p; S.n = std::max(nact, 1);
+  } else {
+    S = sep_dev<double>(c, c->d_sepf.p, c->d_sepg.p);
+    S.act = act; S.n = P;
+  }
+  const int ngh = S.ngh, ngl = S.ngl;
+  tic();
+  const int lv = f32 ? live_begin(c, st) : -1;
+  const unsigned nunit = (unsigned)(S.f.nu + S.k[0].nu + S.k[1].nu);
+  auto threads = [&](int npt) { return std::min(256, (4 * npt * ngl + 31) / 32 * 32); };
+  // two points per CTA in FP32 fill its last warp (160 threads at 20 radial points, not 80
+  // of 96): 0.23 against 0.24 ms for 40 points at N_sh = 16
+  if (f32 && S.n > 1)
+    k_sep_radial<T, 2><<<dim3(nunit, (S.n + 1) / 2), threads(2), 0, st>>>(S, rsp, c->nxy);
+  else
+    k_sep_radial<T, 1><<<dim3(nunit, S.n), threads(1), 0, st>>>(S, rsp, c->nxy);
+  const int ng = std::max(1, std::min(S.nzf, 128 / ngh));
+  k_sep_density<T><<<dim3(ngl, 8, S.n), ngh * ng, sep_dens_smem<T>(ngh, ng), st>>>(S, ng, dpart);
+  if (f32) live_end(c, lv, 0, st);
+  CK(cudaGetLastError());
+  toc(1);
+  tic();
+  k_meanfield<T><<<dim3((c->nghl + 31) / 32, 2 * P), 32, 0, st>>>(c->devbasis<T>(), 4, dpart, mf, act);
+  CK(cudaGetLastError());
+  toc(2);
+  tic();
+  const int lw = f32 ? live_begin(c, st) : -1;
+  k_sep_field<T><<<dim3(ngl, 8, S.n), 128, sep_field_smem<T>(ngh), st>>>(S, mf);
+  const int nw = 2 * S.f.nwarp + S.d[0].nwarp + S.d[1].nwarp;
+  k_sep_project<T><<<dim3((nw + 3) / 4, S.n), 128, 0, st>>>(S, hsp, c->nxy);
+  if (f32) live_end(c, lw, 1, st);
+  c->launches += 5;
+  CK(cudaGetLastError());
+  toc(3);
+  return PNFAM_OK;
+}
+
 // residual interaction of the points flagged in `act`: state (X, Y[, P, Q]) -> hqp
 // (H20, H02[, H11, H11t] stored), computed in precision T (the FP32 form reads the FP32
 // copy of the state and writes the FP32 hqp)
@@ -1016,6 +1216,13 @@ static int residual_t(pnfam_ctx* c, int P, int nact, const int* act, bool timed,
   }
   toc(0);
   const long long nxy = c->nxy;
+  const bool unit_sums = f32 ? c->sep32 && !c->tuning &&
+                                   !(c->pair32 && c->pg_on && c->pg_built && nact >= c->pg_min)
+                             : c->sep64;
+  if (unit_sums) {
+    if ((rc = sep_field<T>(c, P, nact, act, rsp, dpart, mf, hsp, st, tic, toc))) return rc;
+    return residual_k2<T>(c, P, nact, act, bufs, st, tic, toc);
+  }
   DensCallT<T> d0, d1;
   d0.rho = rsp + 0 * nxy; d0.rho_sp = 8 * nxy; d0.rho_spl = 4 * nxy;
   d0.rcols = c->d_fc.p; d0.roffs = c->d_foff.p;
@@ -1101,16 +1308,7 @@ static int residual_t(pnfam_ctx* c, int P, int nact, const int* act, bool timed,
     CK(cudaGetLastError());
   }
   toc(3);
-  tic();
-  if constexpr (f32) {
-    if ((rc = launch_gemm_tc(c, c->t2a, nact, st))) return rc;
-    if ((rc = launch_gemm_tc(c, c->t2b, nact, st))) return rc;
-  } else {
-    if ((rc = launch_gemm<T>(c, c->k2a, P, act, bufs, st))) return rc;
-    if ((rc = launch_gemm<T>(c, c->k2b, P, act, bufs, st))) return rc;
-  }
-  toc(4);
-  return PNFAM_OK;
+  return residual_k2<T>(c, P, nact, act, bufs, st, tic, toc);
 }
 
 
@@ -1180,6 +1378,11 @@ static int pg_autotune(pnfam_ctx* c, int P) {
     for (int i = 0; i < P; ++i) flags[i] = i < n;
     CK(upload(c->d_act32, flags.data(), flags.size()));
     c->pg_min = pair ? 1 : (1 << 30);
+    struct Tuning {   // the general kernels, also on a separable basis
+      pnfam_ctx* c;
+      explicit Tuning(pnfam_ctx* x) : c(x) { c->tuning = true; }
+      ~Tuning() { c->tuning = false; }
+    } tuning(c);
     int rc = residual_t<float>(c, P, n, c->d_act32.p, false, st);   // warm
     if (rc) return rc;
     const int reps = 2;
@@ -1244,8 +1447,9 @@ static int pg_autotune(pnfam_ctx* c, int P) {
   return PNFAM_OK;
 }
 
-// FP32 copies of the ground state and FP32 scratch for P points
-static int ensure_buffers32(pnfam_ctx* c, int P) {
+// FP32 copies of the ground state and FP32 scratch for P points; pair: for evaluations
+// that may take the pair-tensor GEMMs
+static int ensure_buffers32(pnfam_ctx* c, int P, bool pair) {
   const long long nxy = c->nxy;
   const size_t mo = (size_t)(c->uoff.back() + (long long)c->db.back() * c->db.back());
   if (!c->have32) {
@@ -1269,7 +1473,15 @@ static int ensure_buffers32(pnfam_ctx* c, int P) {
   CK(dalloc(c->d_rsp32, (size_t)P * 8 * nxy));
   CK(dalloc(c->d_hsp32, (size_t)P * 8 * nxy));
   CK(dalloc(c->d_hqp32, (size_t)P * nv));
-  CK(dalloc(c->d_dpart32, (size_t)P * 2 * c->G * 2 * ND * c->nghl));
+  CK(dalloc(c->d_dpart32, (size_t)P * 2 * std::max(4, c->G) * 2 * ND * c->nghl));
+  if (c->sep32) {
+    CK(dalloc(c->d_sepg32, (size_t)P * c->sep_gstride));
+    if (c->d_sepf32.n < c->d_sepf.n) {
+      CK(dalloc(c->d_sepf32, c->d_sepf.n));
+      k_to_f32<<<64, 256, 0, c->stream>>>(c->d_sepf.p, c->d_sepf32.p, (long long)c->d_sepf.n, 1, 0, nullptr);
+      CK(cudaGetLastError());
+    }
+  }
   CK(dalloc(c->d_mf32, (size_t)P * 2 * NMF * 2 * c->nghl));
   CK(dalloc(c->d_xsave, (size_t)P * nv));
   CK(dalloc(c->d_radd, (size_t)P * nv));
@@ -1278,7 +1490,14 @@ static int ensure_buffers32(pnfam_ctx* c, int P) {
   CK(dalloc(c->d_lastv, (size_t)P * nv));
   CK(dalloc(c->d_tf, (size_t)P * nv));
   CK(dalloc(c->d_tv, (size_t)P * nv));
-  if (c->tc_density) {
+  // what the general kernels need (a separable basis: only for the pair-tensor GEMMs of
+  // uncertified runs, whose point count is tuned against the per-block kernels)
+  const bool general = !c->sep32 || pair;
+  if (general && !c->pg_ready) {
+    pg_setup(c);
+    c->pg_ready = true;
+  }
+  if (c->tc_density && general) {
     CK(dalloc(c->d_bsplit, (size_t)P * c->bstride));
     if (!c->have_aphi) {
       const int ntr = (c->nghl + 31) / 32, na = (int)c->achunks.size();
@@ -1301,7 +1520,7 @@ static int ensure_buffers32(pnfam_ctx* c, int P) {
   bd[B_HSP] = {c->d_hsp32.p, 8 * nxy, 4 * nxy};
   bd[B_HQP] = {c->d_hqp32.p, nv, nv / 2};
   CK(upload(c->d_bufs32, bd, NBUF));
-  if (!c->have_hphi) {
+  if (!c->have_hphi && general) {
     const int nrc = (c->nghl + HTC_K - 1) / HTC_K;
     CK(dalloc(c->d_hphi, (size_t)std::max(1LL, c->hphi_floats)));
     if (!c->hptiles.empty()) {
@@ -1324,6 +1543,7 @@ static int ensure_buffers32(pnfam_ctx* c, int P) {
     }
     c->have_gsplit = true;
   }
+  if (!general) return PNFAM_OK;
   {
     const int rc = pg_build(c);
     if (rc) return rc;
@@ -1393,6 +1613,12 @@ extern "C" int pnfam_gpu_init(const pnfam_basis_t* basis, const double* Ep, cons
     c->autotune = !(v && v[0] == '0');
     v = std::getenv("PNFAM_GB300_PAIR_KSPAN");
     if (v && std::atoi(v) > 0) c->pg_kspan_env = std::atoi(v);
+    v = std::getenv("PNFAM_GB300_SEPARABLE");
+    c->sep = !(v && v[0] == '0');
+    c->sep32 = c->sep;
+    for (const char* s : {"PNFAM_GB300_TC_DENSITY", "PNFAM_GB300_PAIR_GEMM", "PNFAM_GB300_PAIR_MIN",
+                          "PNFAM_GB300_PAIR_KSPAN"})
+      if (std::getenv(s)) c->sep32 = false;
     v = std::getenv("PNFAM_GB300_PAIR_SMEM_KB");
     if (v && std::atoi(v) >= 64) c->pg_smem = std::min(std::atoi(v), PG_SMEM_MAX / 1024) * 1024;
   }
@@ -1448,9 +1674,18 @@ extern "C" int pnfam_gpu_init(const pnfam_basis_t* basis, const double* Ep, cons
                            (int)density_tc2_smem_bytes()) != cudaSuccess ||
       cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)gemm_tc_smem_bytes()) != cudaSuccess ||
-      cudaFuncSetAttribute(k_pg_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, PG_SMEM_MAX) != cudaSuccess) {
+      cudaFuncSetAttribute(k_pg_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, PG_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_field<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SEP_SMEM_MAX) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_field<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SEP_SMEM_MAX) !=
+          cudaSuccess) {
     delete c;
     return fail(PNFAM_ECUDA, "pnfam_gpu_init: cannot configure shared memory");
+  }
+  if (c->sep) {
+    c->sep = false;
+    if ((rc = sep_init(c, phi))) { delete c; return rc; }
+    c->sep32 = c->sep32 && c->sep;
   }
   *out = c;
   return PNFAM_OK;
@@ -1546,7 +1781,11 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
   c->nchunk_bro = (int)((2 * nq * nf + BRO_CHUNK - 1) / BRO_CHUNK);
   c->nchunk_c = (int)std::min<long long>(32, std::max<long long>(1, (nq * nf) / 4096));
   build_tasks(c);
-  pg_setup(c);
+  {
+    const int rcs = sep_operator(c);
+    if (rcs) return rcs;
+  }
+  c->pg_ready = c->pg_on = c->pg_built = false;
   CK(c->k1a.finalize()); CK(c->k1b.finalize()); CK(c->k2a.finalize()); CK(c->k2b.finalize());
   {
     TaskList* src[4] = {&c->k1a, &c->k1b, &c->k2a, &c->k2b};
@@ -1690,7 +1929,9 @@ static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver
   if (rc) return rc;
   c->cap_P = std::max(P, c->cap_P); c->cap_M = std::max(std::max(e->M, 1), c->cap_M);
   e->mixed = o->precision == 1 && !e->no_res;
-  if (e->mixed && (rc = ensure_buffers32(c, c->cap_P))) return rc;
+  c->sep64 = c->sep && (e->mixed || e->M <= 0 || e->M >= SEP_MIN_HISTORY);
+  c->pair32 = o->reserved[3] <= 0;
+  if (e->mixed && (rc = ensure_buffers32(c, c->cap_P, c->pair32))) return rc;
   // Mixed form (precision 1): one Broyden iteration per evaluation, as in the FP64
   // form, but the residual interaction is evaluated in FP32 on the increment
   // d = X - X_a from an anchor X_a whose image g(X_a) is known in FP64:
@@ -2305,22 +2546,28 @@ extern "C" int pnfam_gpu_calc_hamiltonian(pnfam_ctx_t* c, const double* re_rho_p
     CK(cudaMemcpyAsync(c->d_rsp.p + (k & 1) * 4 * nxy + qin[k] * nxy, in[k], nb, cudaMemcpyHostToDevice, c->stream));
   std::vector<int> one = {1};
   CK(cudaMemcpyAsync(c->d_active.p, one.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  DensCall d0, d1;
-  d0.rho = c->d_rsp.p + 0 * nxy; d0.rho_sp = 8 * nxy; d0.rho_spl = 4 * nxy;
-  d0.rcols = c->d_fc.p; d0.roffs = c->d_foff.p;
-  d0.kap = c->d_rsp.p + 1 * nxy; d0.kap_sp = 8 * nxy; d0.kap_spl = 4 * nxy;
-  d0.kcols = c->d_xtc.p; d0.koffs = c->d_xtoff.p;
-  d1.rho = c->d_rsp.p + 3 * nxy; d1.rho_sp = 8 * nxy; d1.rho_spl = 4 * nxy;
-  d1.rcols = c->d_fc.p; d1.roffs = c->d_foff.p;
-  d1.kap = c->d_rsp.p + 2 * nxy; d1.kap_sp = 8 * nxy; d1.kap_spl = 4 * nxy;
-  d1.kcols = c->d_ytc.p; d1.koffs = c->d_ytoff.p;
-  const DevBasis B = c->devbasis<double>();
   const int* act = c->d_active.p;
-  k_density_fp64<<<dim3((c->nghl + DRT - 1) / DRT, c->G, 2), 256, 0, c->stream>>>(B, d0, d1, c->G, c->d_dpart.p,
-                                                                                 act);
-  k_meanfield<<<dim3((c->nghl + 127) / 128, 2), 128, 0, c->stream>>>(B, c->G, c->d_dpart.p, c->d_mf.p, act);
-  k_hproj_fp64<<<dim3((unsigned)c->htasks.size(), 1), 256, hproj_fp64_smem_bytes(), c->stream>>>(
-      B, c->d_htasks.p, c->d_mf.p, c->d_hsp.p, nxy, act);
+  if (c->sep) {
+    auto none = [](int = 0) {};
+    if ((rc = sep_field<double>(c, 1, 1, act, c->d_rsp.p, c->d_dpart.p, c->d_mf.p, c->d_hsp.p, c->stream, none, none)))
+      return rc;
+  } else {
+    DensCall d0, d1;
+    d0.rho = c->d_rsp.p + 0 * nxy; d0.rho_sp = 8 * nxy; d0.rho_spl = 4 * nxy;
+    d0.rcols = c->d_fc.p; d0.roffs = c->d_foff.p;
+    d0.kap = c->d_rsp.p + 1 * nxy; d0.kap_sp = 8 * nxy; d0.kap_spl = 4 * nxy;
+    d0.kcols = c->d_xtc.p; d0.koffs = c->d_xtoff.p;
+    d1.rho = c->d_rsp.p + 3 * nxy; d1.rho_sp = 8 * nxy; d1.rho_spl = 4 * nxy;
+    d1.rcols = c->d_fc.p; d1.roffs = c->d_foff.p;
+    d1.kap = c->d_rsp.p + 2 * nxy; d1.kap_sp = 8 * nxy; d1.kap_spl = 4 * nxy;
+    d1.kcols = c->d_ytc.p; d1.koffs = c->d_ytoff.p;
+    const DevBasis B = c->devbasis<double>();
+    k_density_fp64<<<dim3((c->nghl + DRT - 1) / DRT, c->G, 2), 256, 0, c->stream>>>(B, d0, d1, c->G, c->d_dpart.p,
+                                                                                   act);
+    k_meanfield<<<dim3((c->nghl + 127) / 128, 2), 128, 0, c->stream>>>(B, c->G, c->d_dpart.p, c->d_mf.p, act);
+    k_hproj_fp64<<<dim3((unsigned)c->htasks.size(), 1), 256, hproj_fp64_smem_bytes(), c->stream>>>(
+        B, c->d_htasks.p, c->d_mf.p, c->d_hsp.p, nxy, act);
+  }
   CK(cudaGetLastError());
   const int qout[8] = {0, 0, 1, 1, 3, 3, 2, 2};
   for (int k = 0; k < 8; ++k)
@@ -2344,7 +2591,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* c, const double* re
   int rc = ensure_buffers(c, std::max(1, c->cap_P), std::max(1, c->cap_M));
   if (rc) return rc;
   c->cap_P = std::max(1, c->cap_P); c->cap_M = std::max(1, c->cap_M);
-  if ((rc = ensure_buffers32(c, c->cap_P))) return rc;
+  if ((rc = ensure_buffers32(c, c->cap_P, false))) return rc;
   const long long nxy = c->nxy;
   const size_t nb = sizeof(double) * nxy;
   const int qin[8] = {0, 0, 1, 1, 3, 3, 2, 2};
@@ -2354,34 +2601,41 @@ extern "C" int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* c, const double* re
   CK(cudaMemcpyAsync(c->d_active.p, one.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
   CK(cudaMemcpyAsync(c->d_actlist.p, zero.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
   k_to_f32<<<1024, 256, 0, c->stream>>>(c->d_rsp.p, c->d_rsp32.p, 8 * nxy, 1, 0, nullptr);
-  DensCallT<float> d0, d1;
-  d0.rho = c->d_rsp32.p + 0 * nxy; d0.rho_sp = 8 * nxy; d0.rho_spl = 4 * nxy;
-  d0.rcols = c->d_fc.p; d0.roffs = c->d_foff.p;
-  d0.kap = c->d_rsp32.p + 1 * nxy; d0.kap_sp = 8 * nxy; d0.kap_spl = 4 * nxy;
-  d0.kcols = c->d_xtc.p; d0.koffs = c->d_xtoff.p;
-  d1.rho = c->d_rsp32.p + 3 * nxy; d1.rho_sp = 8 * nxy; d1.rho_spl = 4 * nxy;
-  d1.rcols = c->d_fc.p; d1.roffs = c->d_foff.p;
-  d1.kap = c->d_rsp32.p + 2 * nxy; d1.kap_sp = 8 * nxy; d1.kap_spl = 4 * nxy;
-  d1.kcols = c->d_ytc.p; d1.koffs = c->d_ytoff.p;
-  const DevBasisT<float> B = c->devbasis<float>();
   const int* act = c->d_active.p;
-  if (c->tc_density) {
-    DensTCArgs t0{d0.rho, d0.rho_sp, d0.rho_spl, d0.rcols, d0.roffs, d0.kap, d0.kap_sp, d0.kap_spl, d0.kcols, d0.koffs};
-    DensTCArgs t1{d1.rho, d1.rho_sp, d1.rho_spl, d1.rcols, d1.roffs, d1.kap, d1.kap_sp, d1.kap_spl, d1.kcols, d1.koffs};
-    if (!c->bchunks.empty())
-      k_dens_bsplit<<<dim3((unsigned)c->bchunks.size(), 1), 256, 0, c->stream>>>(B, t0, t1, c->d_bchunks.p,
-                                                                                c->d_actlist.p, c->d_bsplit.p,
-                                                                                c->bstride);
-    k_density_tc2<<<dim3((c->nghl + 31) / 32, c->G, 2), DTC2_THREADS, density_tc2_smem_bytes(), c->stream>>>(
-        B, c->d_dunits0.p, (int)c->dunits[0].size(), c->d_dunits1.p, (int)c->dunits[1].size(), c->d_aphi.p,
-        (int)c->achunks.size(), c->d_bsplit.p, c->bstride, c->G, c->d_actlist.p, c->d_dpart32.p, c->d_err.p);
+  if (c->sep32) {
+    auto none = [](int = 0) {};
+    if ((rc = sep_field<float>(c, 1, 1, act, c->d_rsp32.p, c->d_dpart32.p, c->d_mf32.p, c->d_hsp32.p, c->stream, none,
+                               none)))
+      return rc;
   } else {
-    k_density<float><<<dim3((c->nghl + DRT - 1) / DRT, c->G, 2), 256, density_smem_bytes<float>(), c->stream>>>(
-        B, d0, d1, c->G, c->d_dpart32.p, act);
+    DensCallT<float> d0, d1;
+    d0.rho = c->d_rsp32.p + 0 * nxy; d0.rho_sp = 8 * nxy; d0.rho_spl = 4 * nxy;
+    d0.rcols = c->d_fc.p; d0.roffs = c->d_foff.p;
+    d0.kap = c->d_rsp32.p + 1 * nxy; d0.kap_sp = 8 * nxy; d0.kap_spl = 4 * nxy;
+    d0.kcols = c->d_xtc.p; d0.koffs = c->d_xtoff.p;
+    d1.rho = c->d_rsp32.p + 3 * nxy; d1.rho_sp = 8 * nxy; d1.rho_spl = 4 * nxy;
+    d1.rcols = c->d_fc.p; d1.roffs = c->d_foff.p;
+    d1.kap = c->d_rsp32.p + 2 * nxy; d1.kap_sp = 8 * nxy; d1.kap_spl = 4 * nxy;
+    d1.kcols = c->d_ytc.p; d1.koffs = c->d_ytoff.p;
+    const DevBasisT<float> B = c->devbasis<float>();
+    if (c->tc_density) {
+      DensTCArgs t0{d0.rho, d0.rho_sp, d0.rho_spl, d0.rcols, d0.roffs, d0.kap, d0.kap_sp, d0.kap_spl, d0.kcols, d0.koffs};
+      DensTCArgs t1{d1.rho, d1.rho_sp, d1.rho_spl, d1.rcols, d1.roffs, d1.kap, d1.kap_sp, d1.kap_spl, d1.kcols, d1.koffs};
+      if (!c->bchunks.empty())
+        k_dens_bsplit<<<dim3((unsigned)c->bchunks.size(), 1), 256, 0, c->stream>>>(B, t0, t1, c->d_bchunks.p,
+                                                                                  c->d_actlist.p, c->d_bsplit.p,
+                                                                                  c->bstride);
+      k_density_tc2<<<dim3((c->nghl + 31) / 32, c->G, 2), DTC2_THREADS, density_tc2_smem_bytes(), c->stream>>>(
+          B, c->d_dunits0.p, (int)c->dunits[0].size(), c->d_dunits1.p, (int)c->dunits[1].size(), c->d_aphi.p,
+          (int)c->achunks.size(), c->d_bsplit.p, c->bstride, c->G, c->d_actlist.p, c->d_dpart32.p, c->d_err.p);
+    } else {
+      k_density<float><<<dim3((c->nghl + DRT - 1) / DRT, c->G, 2), 256, density_smem_bytes<float>(), c->stream>>>(
+          B, d0, d1, c->G, c->d_dpart32.p, act);
+    }
+    k_meanfield<float><<<dim3((c->nghl + 127) / 128, 2), 128, 0, c->stream>>>(B, c->G, c->d_dpart32.p, c->d_mf32.p, act);
+    k_hproj_tc<<<dim3((unsigned)c->htasks_tc.size(), 1), HTC_THREADS, hproj_tc_smem_bytes(c->tc_npmax), c->stream>>>(
+        B, c->d_htasks_tc.p, c->d_actlist.p, 1, c->tc_npmax, c->d_mf32.p, c->d_hphi.p, c->d_hsp32.p, nxy, c->d_err.p);
   }
-  k_meanfield<float><<<dim3((c->nghl + 127) / 128, 2), 128, 0, c->stream>>>(B, c->G, c->d_dpart32.p, c->d_mf32.p, act);
-  k_hproj_tc<<<dim3((unsigned)c->htasks_tc.size(), 1), HTC_THREADS, hproj_tc_smem_bytes(c->tc_npmax), c->stream>>>(
-      B, c->d_htasks_tc.p, c->d_actlist.p, 1, c->tc_npmax, c->d_mf32.p, c->d_hphi.p, c->d_hsp32.p, nxy, c->d_err.p);
   k_to_f64<<<dim3(1024, 1), 256, 0, c->stream>>>(c->d_hsp32.p, c->d_hsp.p, 8 * nxy, 0, nullptr);
   CK(cudaGetLastError());
   const int qout[8] = {0, 0, 1, 1, 3, 3, 2, 2};
