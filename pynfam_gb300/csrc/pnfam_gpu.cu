@@ -101,6 +101,7 @@ struct TaskList {
   DBuf<GemmTask> d_tasks;
   DBuf<int> d_tile2task;
   int ntiles = 0;
+  long long outputs = 0;
 
   void add(int M, int N, int K, const std::vector<GemmTerm>& terms, int cbuf, long long coff, int ldc) {
     if (M <= 0 || N <= 0) return;
@@ -109,28 +110,37 @@ struct TaskList {
     t.M = M; t.N = N; t.K = K; t.nterm = (int)terms.size();
     for (size_t i = 0; i < terms.size(); ++i) t.t[i] = terms[i];
     t.cbuf = cbuf; t.coff = coff; t.ldc = ldc;
-    // tile shape: the fewest 1024-element tiles covering M x N (32 x 32 on ties); every
-    // tile costs the same DFMAs, so this is the fewest padded outputs
-    int best = 32, bt = -1;
-    for (int tm : {32, 64, 16, 128, 8}) {
-      const int tn = 1024 / tm;
-      const int nt = ((M + tm - 1) / tm) * ((N + tn - 1) / tn);
-      if (bt < 0 || nt < bt) { bt = nt; best = tm; }
-    }
-    t.tm = best;
-    const int ntm = (M + best - 1) / best, ntn = (N + 1024 / best - 1) / (1024 / best);
-    t.tile0 = ntiles; t.ntn = ntn;
-    for (int k = 0; k < ntm * ntn; ++k) tile2task.push_back((int)tasks.size());
-    ntiles += ntm * ntn;
     tasks.push_back(t);
+    outputs += 2LL * M * N;
+  }
+  // tiles of at most `cap` outputs (Re and Im), in nearly equal parts of the rows and then
+  // of the columns: 2048 (8 per thread), fewer while the list would leave SMs idle for one
+  // point (at N_sh = 6 blocks up to 16: 256)
+  void tile() {
+    int cap = GT_R * GT_THREADS;
+    while (cap > GT_THREADS && outputs < 2LL * 152 * cap) cap /= 2;
+    auto cdiv = [](int x, int y) { return (x + y - 1) / y; };
+    tile2task.clear();
+    ntiles = 0;
+    for (size_t k = 0; k < tasks.size(); ++k) {
+      GemmTask& t = tasks[k];
+      t.ntm = cdiv(t.M, std::min<int>(GT_SIDE, cap / 2));
+      t.mr = cdiv(t.M, t.ntm);
+      const int ntn = cdiv(t.N, std::max(1, std::min<int>(GT_SIDE, cap / (2 * t.mr))));
+      t.nc = cdiv(t.N, ntn);
+      t.tile0 = ntiles;
+      ntiles += t.ntm * ntn;
+      tile2task.insert(tile2task.end(), (size_t)t.ntm * ntn, (int)k);
+    }
   }
   cudaError_t finalize() {
+    tile();
     cudaError_t e = upload(d_tasks, tasks.data(), tasks.size());
     if (e != cudaSuccess) return e;
     return upload(d_tile2task, tile2task.data(), tile2task.size());
   }
   void clear() {
-    tasks.clear(); tile2task.clear(); ntiles = 0;
+    tasks.clear(); tile2task.clear(); ntiles = 0; outputs = 0;
   }
 };
 
@@ -224,12 +234,19 @@ struct pnfam_ctx {
   DBuf<long long> d_foff, d_xtoff, d_ytoff;
   DBuf<double> d_fops;   // [nops][2*nxy] operator and cross terms in the QP basis
   TaskList k1a, k1b, k2a, k2b;
-  TaskListTC t1a, t1b, t2a, t2b;   // FP32 evaluation on the tensor cores
+  bool shared = false;                // the same transforms with shared products
+  TaskList s1a, s1b, s2a, s2b;
+  // FP32 evaluation on the tensor cores: the tasks of the four lists, in the general (0)
+  // and the shared (1) form, and their ground-state operands, pre-split
+  struct TCSet {
+    TaskListTC l[4];
+    DBuf<float> gsplit;
+    long long floats = 0;
+    bool built = false;
+  } tc32[2];
+  int tcset = 0;              // the form that the current run takes
   std::vector<HTask> htasks;
   DBuf<HTask> d_htasks;
-  DBuf<float> d_gsplit;               // ground-state operands of the tensor-core GEMM tasks, pre-split
-  long long gsplit_floats = 0;
-  bool have_gsplit = false;
   std::vector<HTaskTC> htasks_tc;   // tensor-core field projection (FP32 data)
   int tc_npmax = 16;                  // largest N of those tiles
   DBuf<HTaskTC> d_htasks_tc;
@@ -341,7 +358,8 @@ struct pnfam_ctx {
   // returns what its FP32 evaluations lead to, so it keeps the pair-tensor GEMMs from the
   // tuned point count on: their long tensor-core sums differ from the unit sums by 1e-5 in
   // 12 steps, while the strengths of certified runs agree to 1e-8 for either.
-  bool sep64 = false, pair32 = false, tuning = false;
+  // shared64: the FP64 transforms with shared products, under the rule of sep64.
+  bool sep64 = false, pair32 = false, tuning = false, shared64 = false;
   bool pg_ready = false;      // pg_setup done for the current operator
   int nchunk_bro = 1, nchunk_c = 1;
   cudaStream_t stream = nullptr;
@@ -387,14 +405,21 @@ struct pnfam_ctx {
     for (auto* b : dbs) b->release();
     d_foff.release(); d_xtoff.release(); d_ytoff.release();
     d_htasks.release(); d_bufs.release(); d_htasks_tc.release(); d_actlist.release(); d_err.release();
-    d_gsplit.release(); d_hptiles.release(); d_hphi.release();
+    for (TCSet& t : tc32) {
+      for (TaskListTC& l : t.l) l.d_tasks.release();
+      t.gsplit.release();
+    }
+    d_hptiles.release(); d_hphi.release();
     d_pg_probs.release(); d_pg_elems.release(); d_pg_tproj.release(); d_pg_tdens.release();
     d_pg_bproj.release(); d_pg_bdens.release(); d_pg_a.release(); d_pg_b.release(); d_pg_d.release();
     k1a.d_tasks.release(); k1a.d_tile2task.release();
+    s1a.d_tasks.release(); s1a.d_tile2task.release();
     k1b.d_tasks.release(); k1b.d_tile2task.release();
+    s1b.d_tasks.release(); s1b.d_tile2task.release();
     k2a.d_tasks.release(); k2a.d_tile2task.release();
+    s2a.d_tasks.release(); s2a.d_tile2task.release();
     k2b.d_tasks.release(); k2b.d_tile2task.release();
-    t1a.d_tasks.release(); t1b.d_tasks.release(); t2a.d_tasks.release(); t2b.d_tasks.release();
+    s2b.d_tasks.release(); s2b.d_tile2task.release();
     for (SepBufs& b : d_seps) b.release();
     d_sepf.release(); d_sepf32.release(); d_sepg.release(); d_sepg32.release();
     if (ev[0]) cudaEventDestroy(ev[0]);
@@ -461,6 +486,110 @@ static void emit_triple(TaskList& s1, TaskList& s2, long long& toff, const std::
     st2.push_back(mkterm(t.A, T, t.alpha[0], t.alpha[1]));
   }
   s2.add(orows, ocols, terms[0].A.ocols(), st2, obuf, ooff, orows);
+}
+
+// The same transforms with the first products shared: T1 = UL X - VL Q, T2 = VL Y - UL P
+// and their time-reversed partners serve both SP quadrants that contain them, and the two
+// products with one outer factor are summed before it: 12 block products for X and Y
+// (16 for X, Y, P and Q) in each direction instead of 16 (32).  Needs F's block map to be
+// symmetric under time reversal.  Sums are associated differently, so results differ by
+// rounding.
+static void build_shared_tasks(pnfam_ctx* c) {
+  const int nb = c->nb;
+  const long long nxy = c->nxy;
+  const int UL = c->left_u(), VL = c->left_v(), UR = c->right_u(), VR = c->right_v();
+  const bool stat = c->nq == 4;
+  TaskList &a1 = c->s1a, &b1 = c->s1b, &a2 = c->s2a, &b2 = c->s2b;
+  a1.clear(); b1.clear(); a2.clear(); b2.clear();
+  auto part = [&](int q, int i, const std::vector<long long>& off, const std::vector<int>& cols) {
+    return MatRef{B_STATE, q * nxy + off[i], c->db[i], c->db[cols[i]], 0};
+  };
+  auto X = [&](int i) { return part(0, i, c->xoff, c->xc); };
+  auto Y = [&](int i) { return part(1, i, c->yoff, c->yc); };
+  auto Pq = [&](int i) { return part(2, i, c->poff, c->pc); };
+  auto Qq = [&](int i) { return part(3, i, c->qoff, c->qc); };
+  auto H = [&](int q, int row, const std::vector<long long>& off, const std::vector<int>& cols, int tr_) {
+    return MatRef{B_HSP, q * nxy + off[row], c->db[row], c->db[cols[row]], tr_};
+  };
+  auto flip = [](MatRef m) { m.trans ^= 1; return m; };
+  struct Prod { MatRef A, B; double re, im; };
+  long long toff = 0;
+  auto sum = [&](TaskList& tl, const std::vector<Prod>& ps, int buf, long long off) {
+    std::vector<GemmTerm> g;
+    for (const Prod& q : ps) g.push_back(mkterm(q.A, q.B, q.re, q.im));
+    tl.add(ps[0].A.orows(), ps[0].B.ocols(), ps[0].A.ocols(), g, buf, off, ps[0].A.orows());
+  };
+  auto temp = [&](TaskList& tl, const std::vector<Prod>& ps) {
+    const MatRef T{B_T, toff, ps[0].A.orows(), ps[0].B.ocols(), 0};
+    sum(tl, ps, B_T, toff);
+    toff += (long long)T.rows * T.cols;
+    return T;
+  };
+  // ---- K1 ----
+  std::vector<MatRef> T3(nb), T4(nb);
+  for (int i = 0; i < nb; ++i) {
+    const int t = c->tr[i];
+    if (c->fc[i] >= 0) {
+      const int j = c->fc[i], x = c->xc[i];
+      std::vector<Prod> p1 = {{c->ublk(UL, i, 0), X(i), 1.0, 1.0}}, p2 = {{c->vblk(VL, i, 0), Y(t), 1.0, 1.0}};
+      if (stat) {
+        p1.push_back({c->vblk(VL, i, 0), Qq(t), -1.0, -1.0});
+        p2.push_back({c->ublk(UL, i, 0), Pq(i), -1.0, -1.0});
+      }
+      const MatRef T1 = temp(a1, p1), T2 = temp(a1, p2);
+      sum(b1, {{T1, c->vblk(VR, j, 1), 1.0, 1.0}, {T2, c->ublk(UR, j, 1), -1.0, -1.0}}, B_RSP, c->foff[i]);
+      sum(b1, {{c->ublk(UR, x, 0), flip(T1), -1.0, -1.0}, {c->vblk(VR, x, 0), flip(T2), 1.0, 1.0}}, B_RSP,
+          nxy + c->xtoff[x]);
+    }
+    if (c->yc[i] >= 0) {
+      const int y = c->yc[i];
+      std::vector<Prod> p3 = {{c->vblk(VL, i, 0), X(t), 1.0, 1.0}}, p4 = {{c->ublk(UL, i, 0), Y(i), 1.0, 1.0}};
+      if (stat) {
+        p3.push_back({c->ublk(UL, i, 0), Qq(i), -1.0, -1.0});
+        p4.push_back({c->vblk(VL, i, 0), Pq(t), -1.0, -1.0});
+      }
+      T3[i] = temp(a1, p3);
+      T4[i] = temp(a1, p4);
+      sum(b1, {{c->vblk(VR, y, 0), flip(T3[i]), 1.0, -1.0}, {c->ublk(UR, y, 0), flip(T4[i]), -1.0, 1.0}}, B_RSP,
+          2 * nxy + c->ytoff[y]);
+    }
+  }
+  for (int j = 0; j < nb; ++j) {
+    if (c->fc[j] < 0) continue;
+    const int i = c->fc[j];
+    sum(b1, {{c->ublk(UR, j, 0), flip(T3[i]), -1.0, -1.0}, {c->vblk(VR, j, 0), flip(T4[i]), 1.0, 1.0}}, B_RSP,
+        3 * nxy + c->foff[j]);
+  }
+  // ---- K2 ----
+  toff = 0;
+  std::vector<MatRef> T5(nb), T6(nb), T7(nb), T8(nb);
+  for (int i = 0; i < nb; ++i) {
+    if (c->fc[i] >= 0) {
+      const int j = c->fc[i], x = c->xc[i];
+      const MatRef h11 = H(0, i, c->foff, c->fc, 0), h12 = H(1, i, c->xoff, c->xc, 0);
+      T5[i] = temp(a2, {{h11, c->vblk(VR, j, 0), 1.0, 1.0}, {h12, c->ublk(UR, x, 0), 1.0, 1.0}});
+      T7[i] = temp(a2, {{h11, c->ublk(UR, j, 0), 1.0, 1.0}, {h12, c->vblk(VR, x, 0), 1.0, 1.0}});
+    }
+    if (c->yc[i] >= 0) {
+      const int y = c->yc[i], x = c->tr[y];
+      const MatRef m21 = H(2, i, c->yoff, c->yc, 0), m22 = H(3, x, c->foff, c->fc, 1);
+      T6[i] = temp(a2, {{m21, c->vblk(VR, y, 0), -1.0, 1.0}, {m22, c->ublk(UR, x, 0), -1.0, -1.0}});
+      T8[i] = temp(a2, {{m21, c->ublk(UR, y, 0), 1.0, -1.0}, {m22, c->vblk(VR, x, 0), 1.0, 1.0}});
+    }
+  }
+  for (int i = 0; i < nb; ++i) {
+    const int t = c->tr[i];
+    if (c->fc[i] >= 0)
+      sum(b2, {{c->ublk(UL, i, 1), T5[i], 1.0, 1.0}, {c->vblk(VL, t, 1), T6[t], 1.0, 1.0}}, B_HQP, c->xoff[i]);
+    if (c->yc[i] >= 0)
+      sum(b2, {{c->vblk(VL, t, 1), T7[t], -1.0, -1.0}, {c->ublk(UL, i, 1), T8[i], 1.0, 1.0}}, B_HQP, nxy + c->yoff[i]);
+    if (stat && c->pc[i] >= 0)
+      sum(b2, {{c->ublk(UL, i, 1), T7[i], 1.0, 1.0}, {c->vblk(VL, t, 1), T8[t], -1.0, -1.0}}, B_HQP,
+          2 * nxy + c->poff[i]);
+    if (stat && c->qc[i] >= 0)
+      sum(b2, {{c->vblk(VL, t, 1), T5[t], -1.0, -1.0}, {c->ublk(UL, i, 1), T6[i], -1.0, -1.0}}, B_HQP,
+          3 * nxy + c->qoff[i]);
+  }
 }
 
 static void build_tasks(pnfam_ctx* c) {
@@ -576,6 +705,11 @@ static void build_tasks(pnfam_ctx* c) {
     }
   }
   c->tplane = std::max(c->tplane, toff);
+  // shared products where F's block map is symmetric (every operator of the reference)
+  c->shared = true;
+  for (int i = 0; i < nb; ++i)
+    if (c->fc[i] >= 0 && c->fc[c->tr[c->fc[i]]] != c->tr[i]) c->shared = false;
+  if (c->shared) build_shared_tasks(c);
   // ---- FP64 field projection tasks: spin-uniform tiles of 1024 / tn rows x tn columns ----
   // The shape of each (block pair, spin segment) is the one that issues the fewest DFMAs:
   // per tile, tn columns x the rows up to the warp granularity of the shape (a warp holds
@@ -997,44 +1131,38 @@ static int ensure_buffers(pnfam_ctx* c, int P, int M) {
   return PNFAM_OK;
 }
 
-template <class T>
-static int launch_gemm(pnfam_ctx* c, TaskList& tl, int P, const int* active, const BufDescT<T>* bufs,
-                       cudaStream_t st) {
+static int launch_gemm(pnfam_ctx* c, TaskList& tl, int P, const int* active, cudaStream_t st) {
   if (tl.ntiles == 0) return PNFAM_OK;
-  dim3 grid(tl.ntiles, 2 * P);
-  k_gemm<T><<<grid, 256, 0, st>>>(tl.d_tasks.p, tl.d_tile2task.p, bufs, active);
+  k_gemm<<<dim3(tl.ntiles, P), GT_THREADS, 0, st>>>(tl.d_tasks.p, tl.d_tile2task.p, c->d_bufs.p, active);
   c->launches++;
   CK(cudaGetLastError());
   return PNFAM_OK;
 }
 
 // FP32 stage on the tensor cores for the nact points listed in c->d_actlist
-static int launch_gemm_tc(pnfam_ctx* c, TaskListTC& tl, int nact, cudaStream_t st) {
+static int launch_gemm_tc(pnfam_ctx* c, int list, int nact, cudaStream_t st) {
+  const TaskListTC& tl = c->tc32[c->tcset].l[list];
   if (tl.tasks.empty() || nact <= 0) return PNFAM_OK;
   dim3 grid((unsigned)tl.tasks.size(), (unsigned)((2 * nact * tl.maxrows + 127) / 128));
-  k_gemm_tc<<<grid, GTC_THREADS, gemm_tc_smem_bytes(tl.maxnp), st>>>(tl.d_tasks.p, c->d_bufs32.p, c->d_gsplit.p,
-                                                                      c->d_actlist.p, nact, tl.maxnp, c->d_err.p);
+  k_gemm_tc<<<grid, GTC_THREADS, gemm_tc_smem_bytes(tl.maxnp), st>>>(tl.d_tasks.p, c->d_bufs32.p,
+                                                                      c->tc32[c->tcset].gsplit.p, c->d_actlist.p, nact, tl.maxnp, c->d_err.p);
   c->launches++;
   CK(cudaGetLastError());
   return PNFAM_OK;
 }
 
-static int launch_gemm(pnfam_ctx* c, TaskList& tl, int P, const int* active) {
-  return launch_gemm<double>(c, tl, P, active, c->d_bufs.p, c->stream);
-}
-
 // fields in the SP basis -> dH_qp
 template <class T, class Tic, class Toc>
-static int residual_k2(pnfam_ctx* c, int P, int nact, const int* act, const BufDescT<T>* bufs, cudaStream_t st,
-                       Tic&& tic, Toc&& toc) {
+static int residual_k2(pnfam_ctx* c, int P, int nact, const int* act, cudaStream_t st, Tic&& tic, Toc&& toc) {
   int rc;
   tic();
   if constexpr (std::is_same<T, float>::value) {
-    if ((rc = launch_gemm_tc(c, c->t2a, nact, st))) return rc;
-    if ((rc = launch_gemm_tc(c, c->t2b, nact, st))) return rc;
+    if ((rc = launch_gemm_tc(c, 2, nact, st))) return rc;
+    if ((rc = launch_gemm_tc(c, 3, nact, st))) return rc;
   } else {
-    if ((rc = launch_gemm<T>(c, c->k2a, P, act, bufs, st))) return rc;
-    if ((rc = launch_gemm<T>(c, c->k2b, P, act, bufs, st))) return rc;
+    const bool sh = c->shared64;
+    if ((rc = launch_gemm(c, sh ? c->s2a : c->k2a, P, act, st))) return rc;
+    if ((rc = launch_gemm(c, sh ? c->s2b : c->k2b, P, act, st))) return rc;
   }
   toc(4);
   return PNFAM_OK;
@@ -1198,21 +1326,21 @@ static int residual_t(pnfam_ctx* c, int P, int nact, const int* act, bool timed,
     (std::is_same<T, float>::value ? c->stage32_ms : c->stage_ms)[k] += ms;
   };
   constexpr bool f32 = std::is_same<T, float>::value;
-  const BufDescT<T>* bufs;
   T *rsp, *hsp, *dpart, *mf;
   if constexpr (f32) {
-    bufs = c->d_bufs32.p; rsp = c->d_rsp32.p; hsp = c->d_hsp32.p; dpart = c->d_dpart32.p; mf = c->d_mf32.p;
+    rsp = c->d_rsp32.p; hsp = c->d_hsp32.p; dpart = c->d_dpart32.p; mf = c->d_mf32.p;
   } else {
-    bufs = c->d_bufs.p; rsp = c->d_rsp.p; hsp = c->d_hsp.p; dpart = c->d_dpart.p; mf = c->d_mf.p;
+    rsp = c->d_rsp.p; hsp = c->d_hsp.p; dpart = c->d_dpart.p; mf = c->d_mf.p;
   }
   int rc;
   tic();
   if constexpr (f32) {
-    if ((rc = launch_gemm_tc(c, c->t1a, nact, st))) return rc;
-    if ((rc = launch_gemm_tc(c, c->t1b, nact, st))) return rc;
+    if ((rc = launch_gemm_tc(c, 0, nact, st))) return rc;
+    if ((rc = launch_gemm_tc(c, 1, nact, st))) return rc;
   } else {
-    if ((rc = launch_gemm<T>(c, c->k1a, P, act, bufs, st))) return rc;
-    if ((rc = launch_gemm<T>(c, c->k1b, P, act, bufs, st))) return rc;
+    const bool sh = c->shared64;
+    if ((rc = launch_gemm(c, sh ? c->s1a : c->k1a, P, act, st))) return rc;
+    if ((rc = launch_gemm(c, sh ? c->s1b : c->k1b, P, act, st))) return rc;
   }
   toc(0);
   const long long nxy = c->nxy;
@@ -1221,7 +1349,7 @@ static int residual_t(pnfam_ctx* c, int P, int nact, const int* act, bool timed,
                              : c->sep64;
   if (unit_sums) {
     if ((rc = sep_field<T>(c, P, nact, act, rsp, dpart, mf, hsp, st, tic, toc))) return rc;
-    return residual_k2<T>(c, P, nact, act, bufs, st, tic, toc);
+    return residual_k2<T>(c, P, nact, act, st, tic, toc);
   }
   DensCallT<T> d0, d1;
   d0.rho = rsp + 0 * nxy; d0.rho_sp = 8 * nxy; d0.rho_spl = 4 * nxy;
@@ -1308,7 +1436,7 @@ static int residual_t(pnfam_ctx* c, int P, int nact, const int* act, bool timed,
     CK(cudaGetLastError());
   }
   toc(3);
-  return residual_k2<T>(c, P, nact, act, bufs, st, tic, toc);
+  return residual_k2<T>(c, P, nact, act, st, tic, toc);
 }
 
 
@@ -1448,8 +1576,8 @@ static int pg_autotune(pnfam_ctx* c, int P) {
 }
 
 // FP32 copies of the ground state and FP32 scratch for P points; pair: for evaluations
-// that may take the pair-tensor GEMMs
-static int ensure_buffers32(pnfam_ctx* c, int P, bool pair) {
+// that may take the pair-tensor GEMMs; run: for an engine's run (its block GEMMs too)
+static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
   const long long nxy = c->nxy;
   const size_t mo = (size_t)(c->uoff.back() + (long long)c->db.back() * c->db.back());
   if (!c->have32) {
@@ -1530,18 +1658,22 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair) {
     }
     c->have_hphi = true;
   }
-  if (!c->have_gsplit) {
-    CK(dalloc(c->d_gsplit, (size_t)std::max(1LL, c->gsplit_floats)));
-    TaskListTC* lists[4] = {&c->t1a, &c->t1b, &c->t2a, &c->t2b};
-    for (TaskListTC* tl : lists) {
-      int mc = 0;
-      for (const GemmTaskTC& t : tl->tasks) mc = std::max(mc, t.nterm * ((t.K + GTC_K - 1) / GTC_K));
-      if (tl->tasks.empty() || mc == 0) continue;
-      k_gemm_bsplit<<<dim3((unsigned)tl->tasks.size(), (unsigned)mc), 256, 0, c->stream>>>(tl->d_tasks.p,
-                                                                                      c->d_bufs32.p, c->d_gsplit.p);
-      CK(cudaGetLastError());
+  if (run) {
+    // uncertified runs that take the pair-tensor GEMMs keep the general form (pnfam_ctx::pair32)
+    c->tcset = c->shared && !(pair && c->pg_on) ? 1 : 0;
+    pnfam_ctx::TCSet& set = c->tc32[c->tcset];
+    if (!set.built) {
+      CK(dalloc(set.gsplit, (size_t)std::max(1LL, set.floats)));
+      for (const TaskListTC& tl : set.l) {
+        int mc = 0;
+        for (const GemmTaskTC& t : tl.tasks) mc = std::max(mc, t.nterm * ((t.K + GTC_K - 1) / GTC_K));
+        if (tl.tasks.empty() || mc == 0) continue;
+        k_gemm_bsplit<<<dim3((unsigned)tl.tasks.size(), (unsigned)mc), 256, 0, c->stream>>>(
+            tl.d_tasks.p, c->d_bufs32.p, set.gsplit.p);
+        CK(cudaGetLastError());
+      }
+      set.built = true;
     }
-    c->have_gsplit = true;
   }
   if (!general) return PNFAM_OK;
   {
@@ -1787,21 +1919,24 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
   }
   c->pg_ready = c->pg_on = c->pg_built = false;
   CK(c->k1a.finalize()); CK(c->k1b.finalize()); CK(c->k2a.finalize()); CK(c->k2b.finalize());
+  if (c->shared) { CK(c->s1a.finalize()); CK(c->s1b.finalize()); CK(c->s2a.finalize()); CK(c->s2b.finalize()); }
   {
-    TaskList* src[4] = {&c->k1a, &c->k1b, &c->k2a, &c->k2b};
-    TaskListTC* dst[4] = {&c->t1a, &c->t1b, &c->t2a, &c->t2b};
-    long long goff = 0;
-    for (int k = 0; k < 4; ++k) {
-      dst[k]->build(*src[k]);
-      for (GemmTaskTC& t : dst[k]->tasks) {
-        if (t.ncols > 256) return fail(PNFAM_EINVAL, "pnfam_gpu_set_operator: block larger than 256");
-        t.bsoff = goff;   // the task's pre-split ground-state chunks
-        goff += (long long)t.nterm * ((t.K + GTC_K - 1) / GTC_K) * t.npad * 2 * GTC_K;
+    const TaskList* src[2][4] = {{&c->k1a, &c->k1b, &c->k2a, &c->k2b}, {&c->s1a, &c->s1b, &c->s2a, &c->s2b}};
+    for (int f = 0; f < 1 + c->shared; ++f) {
+      pnfam_ctx::TCSet& set = c->tc32[f];
+      long long goff = 0;
+      for (int k = 0; k < 4; ++k) {
+        set.l[k].build(*src[f][k]);
+        for (GemmTaskTC& t : set.l[k].tasks) {
+          if (t.ncols > 256) return fail(PNFAM_EINVAL, "pnfam_gpu_set_operator: block larger than 256");
+          t.bsoff = goff;   // the task's pre-split ground-state chunks
+          goff += (long long)t.nterm * ((t.K + GTC_K - 1) / GTC_K) * t.npad * 2 * GTC_K;
+        }
+        CK(upload(set.l[k].d_tasks, set.l[k].tasks.data(), set.l[k].tasks.size()));
       }
-      CK(upload(dst[k]->d_tasks, dst[k]->tasks.data(), dst[k]->tasks.size()));
+      set.floats = goff;
+      set.built = false;
     }
-    c->gsplit_floats = goff;
-    c->have_gsplit = false;
   }
   CK(upload(c->d_htasks, c->htasks.data(), c->htasks.size()));
   CK(upload(c->d_htasks_tc, c->htasks_tc.data(), c->htasks_tc.size()));
@@ -1822,8 +1957,8 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
     const double* src = k == 0 ? Fsp : Gsp[k - 1];
     CK(cudaMemsetAsync(c->d_hsp.p, 0, sizeof(double) * 8 * nf, c->stream));
     CK(cudaMemcpyAsync(c->d_hsp.p, src, sizeof(double) * nf, cudaMemcpyHostToDevice, c->stream));
-    if ((rc = launch_gemm(c, c->k2a, 1, c->d_active.p))) return rc;
-    if ((rc = launch_gemm(c, c->k2b, 1, c->d_active.p))) return rc;
+    if ((rc = launch_gemm(c, c->k2a, 1, c->d_active.p, c->stream))) return rc;
+    if ((rc = launch_gemm(c, c->k2b, 1, c->d_active.p, c->stream))) return rc;
     CK(cudaMemcpyAsync(c->d_fops.p + (long long)k * nq * nf, c->d_hqp.p, sizeof(double) * nq * nf,
                        cudaMemcpyDeviceToDevice, c->stream));
   }
@@ -1929,9 +2064,11 @@ static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver
   if (rc) return rc;
   c->cap_P = std::max(P, c->cap_P); c->cap_M = std::max(std::max(e->M, 1), c->cap_M);
   e->mixed = o->precision == 1 && !e->no_res;
-  c->sep64 = c->sep && (e->mixed || e->M <= 0 || e->M >= SEP_MIN_HISTORY);
+  const bool rounding_free = e->mixed || e->M <= 0 || e->M >= SEP_MIN_HISTORY;
+  c->sep64 = c->sep && rounding_free;
+  c->shared64 = c->shared && rounding_free;
   c->pair32 = o->reserved[3] <= 0;
-  if (e->mixed && (rc = ensure_buffers32(c, c->cap_P, c->pair32))) return rc;
+  if (e->mixed && (rc = ensure_buffers32(c, c->cap_P, c->pair32, true))) return rc;
   // Mixed form (precision 1): one Broyden iteration per evaluation, as in the FP64
   // form, but the residual interaction is evaluated in FP32 on the increment
   // d = X - X_a from an anchor X_a whose image g(X_a) is known in FP64:
@@ -2591,7 +2728,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* c, const double* re
   int rc = ensure_buffers(c, std::max(1, c->cap_P), std::max(1, c->cap_M));
   if (rc) return rc;
   c->cap_P = std::max(1, c->cap_P); c->cap_M = std::max(1, c->cap_M);
-  if ((rc = ensure_buffers32(c, c->cap_P, false))) return rc;
+  if ((rc = ensure_buffers32(c, c->cap_P, false, false))) return rc;
   const long long nxy = c->nxy;
   const size_t nb = sizeof(double) * nxy;
   const int qin[8] = {0, 0, 1, 1, 3, 3, 2, 2};
@@ -2682,7 +2819,8 @@ extern "C" int pnfam_gpu_task_tables(int nb, const int* db, const int* num_spin_
   c.nq = statistical ? 4 : 2;
   if ((rc = host_structure(&c, beta_minus, fcols))) return rc;
   build_tasks(&c);
-  const TaskList& tl = stage == 0 ? c.k1a : stage == 1 ? c.k1b : stage == 2 ? c.k2a : c.k2b;
+  const TaskList* lists[2][4] = {{&c.k1a, &c.k1b, &c.k2a, &c.k2b}, {&c.s1a, &c.s1b, &c.s2a, &c.s2b}};
+  const TaskList& tl = *lists[c.shared][stage];
   *ntask = (int)tl.tasks.size();
   if (nxy) *nxy = c.nxy;
   if (scratch) *scratch = c.tplane;

@@ -48,12 +48,11 @@ struct GemmTask {
   GemmTerm t[PNFAM_MAXTERM];
   long long coff;
   int cbuf, ldc;
-  int tile0, ntn;      // first tile in the flattened grid, tiles along N
-  int tm, pad_;        // tile shape: tm rows x 1024 / tm columns (tm = 8 ... 128)
+  int tile0, ntm;      // first tile in the flattened grid, tiles along M
+  int mr, nc;          // rows and columns of a tile
 };
 
-#define GT 32
-#define GK 16
+enum { GT_K = 16, GT_THREADS = 256, GT_R = 8, GT_SIDE = 96 };   // GT_SIDE: most rows or columns of a tile
 
 template <class T>
 __device__ __forceinline__ const T* bufptr(const BufDescT<T>* b, int id, int p, int plane, long long off) {
@@ -61,75 +60,100 @@ __device__ __forceinline__ const T* bufptr(const BufDescT<T>* b, int id, int p, 
   return d.base + (long long)p * d.sp + (long long)plane * d.spl + off;
 }
 
-// C = sum_t alpha_t op(A_t) op(B_t); blockIdx.y = point*2 + plane; T = compute type.
-// Output tiles of TM x TN = 1024 elements (TM = 8 ... 128, chosen per task from its M
-// and N), 2 x 2 per thread; every element sums over k in the same order whatever the
-// shape.
-template <class T, int TM>
-__device__ __forceinline__ void gemm_tile(const GemmTask& Tk, int lt, const BufDescT<T>* __restrict__ bufs, int p,
-                                          int plane, T* smem) {
-  constexpr int TN = 1024 / TM, TX = TN / 2;
-  T* As = smem;                    // [GK][TM + 1]
-  T* Bs = smem + GK * (TM + 1);    // [GK][TN + 1]
-  const int m0 = (lt / Tk.ntn) * TM, n0 = (lt % Tk.ntn) * TN;
-  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  T acc00 = 0, acc01 = 0, acc10 = 0, acc11 = 0;
+// C = sum_t alpha_t op(A_t) op(B_t) in FP64 for both planes (Re, Im) of one point.
+// The DFMA rate bounds it (a warp's DFMA takes the SM's FP64 pipe 16 cycles, its two
+// shared-memory reads 3), so what counts is that no lane works on padding: the mr x nc x 2
+// outputs of a tile are dealt to the threads in one row, element e = thread + 256 i (rows
+// fastest: reads of the row operand are consecutive, those of the column operand mostly
+// one address), K runs over the block's own size, and the ground-state operand is staged
+// once for both planes.  Against tiles of 1024 outputs padded in M, N and K: N_sh = 8, 40
+// points, 28 against 56 ms per solve, N_sh = 6 11 against 22 us per launch; at N_sh = 16
+// (blocks 1 to 81, nine points, shared products) 0.52 ms per point against 1.01, 1.0
+// TFLOP/s of the 1.1 that a DGEMM reaches.  Every output sums over the terms and k in order.  Of the two operands of a
+// term one is the point's (two planes), one the ground state's; alpha (+-1) goes into the
+// point's.  grid (tiles, P)
+__global__ void __launch_bounds__(GT_THREADS) k_gemm(const GemmTask* __restrict__ tasks,
+                                                     const int* __restrict__ tile2task,
+                                                     const BufDescT<double>* __restrict__ bufs,
+                                                     const int* __restrict__ active) {
+  const int p = blockIdx.y;
+  if (!active[p]) return;
+  const GemmTask& Tk = tasks[tile2task[blockIdx.x]];
+  const int lt = blockIdx.x - Tk.tile0;
   const int M = Tk.M, N = Tk.N, K = Tk.K;
+  const int m0 = (lt % Tk.ntm) * Tk.mr, n0 = (lt / Tk.ntm) * Tk.nc;
+  const int mr = min(Tk.mr, M - m0), nc = min(Tk.nc, N - n0);
+  const int ma = mr | 1, nb = nc | 1;          // odd strides: conflict-free transposed stores
+  __shared__ double sm[3 * GT_K * (GT_SIDE + 1)];
+  const bool pa = Tk.t[0].abuf >= B_STATE;     // the point's operand on the left
+  double* As = sm;                             // [2 planes if pa][GT_K][ma]
+  double* Bs = sm + (pa ? 2 : 1) * GT_K * ma;  // [2 planes if !pa][GT_K][nb]
+  const int total = 2 * mr * nc, w0 = threadIdx.x & ~31;
+  double acc[GT_R];
+  int ia[GT_R], ib[GT_R];
+#pragma unroll
+  for (int i = 0; i < GT_R; ++i) {
+    const int e = min((int)threadIdx.x + GT_THREADS * i, total - 1);
+    const int pl = e >= mr * nc, q = e - pl * mr * nc;
+    ia[i] = q % mr + (pa ? pl * GT_K * ma : 0);
+    ib[i] = q / mr + (pa ? 0 : pl * GT_K * nb);
+    acc[i] = 0.0;
+  }
+  const int nr = (total - w0 + GT_THREADS - 1) / GT_THREADS;   // this warp's outputs per thread
   for (int it = 0; it < Tk.nterm; ++it) {
     const GemmTerm& tm = Tk.t[it];
-    const T* A = bufptr(bufs, tm.abuf, p, plane, tm.aoff);
-    const T* B = bufptr(bufs, tm.bbuf, p, plane, tm.boff);
-    const T alpha = (T)tm.alpha[plane];
-    for (int k0 = 0; k0 < K; k0 += GK) {
-      for (int e = threadIdx.x; e < GK * TM; e += 256) {
-        const int kk = e / TM, mm = e % TM;
-        const int gm = m0 + mm, gk = k0 + kk;
-        T v = 0;
-        if (gm < M && gk < K) v = tm.tA ? A[gk + (long long)gm * tm.lda] : A[gm + (long long)gk * tm.lda];
-        As[kk * (TM + 1) + mm] = alpha * v;
+    for (int k0 = 0; k0 < K; k0 += GT_K) {
+      const int kl = min((int)GT_K, K - k0);
+      __syncthreads();
+      for (int pl = 0; pl < (pa ? 2 : 1); ++pl) {
+        const double* A = bufptr(bufs, tm.abuf, p, pl, tm.aoff);
+        const double al = pa ? tm.alpha[pl] : 1.0;
+        double* d = As + pl * GT_K * ma;
+        if (tm.tA) {   // k is consecutive in memory
+          for (int e = threadIdx.x; e < mr * GT_K; e += GT_THREADS) {
+            const int kk = e % GT_K, mm = e / GT_K;
+            if (kk < kl) d[kk * ma + mm] = al * A[k0 + kk + (long long)(m0 + mm) * tm.lda];
+          }
+        } else {
+          for (int e = threadIdx.x; e < mr * kl; e += GT_THREADS) {
+            const int mm = e % mr, kk = e / mr;
+            d[kk * ma + mm] = al * A[m0 + mm + (long long)(k0 + kk) * tm.lda];
+          }
+        }
       }
-      for (int e = threadIdx.x; e < GK * TN; e += 256) {
-        const int kk = e / TN, nn = e % TN;
-        const int gn = n0 + nn, gk = k0 + kk;
-        T w = 0;
-        if (gn < N && gk < K) w = tm.tB ? B[gn + (long long)gk * tm.ldb] : B[gk + (long long)gn * tm.ldb];
-        Bs[kk * (TN + 1) + nn] = w;
+      for (int pl = 0; pl < (pa ? 1 : 2); ++pl) {
+        const double* B = bufptr(bufs, tm.bbuf, p, pl, tm.boff);
+        const double al = pa ? 1.0 : tm.alpha[pl];
+        double* d = Bs + pl * GT_K * nb;
+        if (!tm.tB) {   // k is consecutive in memory
+          for (int e = threadIdx.x; e < nc * GT_K; e += GT_THREADS) {
+            const int kk = e % GT_K, nn = e / GT_K;
+            if (kk < kl) d[kk * nb + nn] = al * B[k0 + kk + (long long)(n0 + nn) * tm.ldb];
+          }
+        } else {
+          for (int e = threadIdx.x; e < nc * kl; e += GT_THREADS) {
+            const int nn = e % nc, kk = e / nc;
+            d[kk * nb + nn] = al * B[n0 + nn + (long long)(k0 + kk) * tm.ldb];
+          }
+        }
       }
       __syncthreads();
+#pragma unroll 4
+      for (int kk = 0; kk < kl; ++kk) {
+        const double *a = As + kk * ma, *b = Bs + kk * nb;
 #pragma unroll
-      for (int kk = 0; kk < GK; ++kk) {
-        const T a0 = As[kk * (TM + 1) + ty * 2], a1 = As[kk * (TM + 1) + ty * 2 + 1];
-        const T b0 = Bs[kk * (TN + 1) + tx * 2], b1 = Bs[kk * (TN + 1) + tx * 2 + 1];
-        acc00 = fma(a0, b0, acc00); acc01 = fma(a0, b1, acc01);
-        acc10 = fma(a1, b0, acc10); acc11 = fma(a1, b1, acc11);
+        for (int i = 0; i < GT_R; ++i)
+          if (i < nr) acc[i] = fma(a[ia[i]], b[ib[i]], acc[i]);
       }
-      __syncthreads();
     }
   }
-  T* C = const_cast<T*>(bufptr(bufs, Tk.cbuf, p, plane, Tk.coff));
-  const int r0 = m0 + ty * 2, c0 = n0 + tx * 2;
-  if (r0 < M && c0 < N) C[r0 + (long long)c0 * Tk.ldc] = acc00;
-  if (r0 < M && c0 + 1 < N) C[r0 + (long long)(c0 + 1) * Tk.ldc] = acc01;
-  if (r0 + 1 < M && c0 < N) C[r0 + 1 + (long long)c0 * Tk.ldc] = acc10;
-  if (r0 + 1 < M && c0 + 1 < N) C[r0 + 1 + (long long)(c0 + 1) * Tk.ldc] = acc11;
-}
-
-template <class T>
-__global__ void __launch_bounds__(256) k_gemm(const GemmTask* __restrict__ tasks, const int* __restrict__ tile2task,
-                                              const BufDescT<T>* __restrict__ bufs, const int* __restrict__ active) {
-  const int z = blockIdx.y;
-  const int p = z >> 1, plane = z & 1;
-  if (active && !active[p]) return;
-  const int tile = blockIdx.x;
-  const GemmTask& Tk = tasks[tile2task[tile]];
-  const int lt = tile - Tk.tile0;
-  __shared__ T smem[GK * (128 + 1) + GK * (8 + 1)];
-  switch (Tk.tm) {
-    case 8: gemm_tile<T, 8>(Tk, lt, bufs, p, plane, smem); break;
-    case 16: gemm_tile<T, 16>(Tk, lt, bufs, p, plane, smem); break;
-    case 64: gemm_tile<T, 64>(Tk, lt, bufs, p, plane, smem); break;
-    case 128: gemm_tile<T, 128>(Tk, lt, bufs, p, plane, smem); break;
-    default: gemm_tile<T, 32>(Tk, lt, bufs, p, plane, smem); break;
+#pragma unroll
+  for (int i = 0; i < GT_R; ++i) {
+    const int e = threadIdx.x + GT_THREADS * i;
+    if (e >= total) break;
+    const int pl = e >= mr * nc, q = e - pl * mr * nc;
+    double* C = const_cast<double*>(bufptr(bufs, Tk.cbuf, p, pl, Tk.coff));
+    C[m0 + q % mr + (long long)(n0 + q / mr) * Tk.ldc] = acc[i];
   }
 }
 
