@@ -113,21 +113,31 @@ struct TaskList {
     tasks.push_back(t);
     outputs += 2LL * M * N;
   }
-  // tiles of at most `cap` outputs (Re and Im), in nearly equal parts of the rows and then
-  // of the columns: 2048 (8 per thread), fewer while the list would leave SMs idle for one
-  // point (at N_sh = 6 blocks up to 16: 256)
+  // tiles of at most `cap` outputs (Re and Im): 2048 (8 per thread), fewer while the list
+  // would leave SMs idle for one point (at N_sh = 6, blocks up to 16: 256).  Of the splits
+  // into nearly equal rows and columns the one with the least work per k: 16 cycles of the
+  // FP64 pipe per warp of outputs, about 6 per warp of staged elements (the point's operand
+  // has two planes)
   void tile() {
     int cap = GT_R * GT_THREADS;
-    while (cap > GT_THREADS && outputs < 2LL * 152 * cap) cap /= 2;
+    while (cap > GT_THREADS && outputs < 152LL * cap) cap /= 2;
     auto cdiv = [](int x, int y) { return (x + y - 1) / y; };
     tile2task.clear();
     ntiles = 0;
     for (size_t k = 0; k < tasks.size(); ++k) {
       GemmTask& t = tasks[k];
-      t.ntm = cdiv(t.M, std::min<int>(GT_SIDE, cap / 2));
-      t.mr = cdiv(t.M, t.ntm);
-      const int ntn = cdiv(t.N, std::max(1, std::min<int>(GT_SIDE, cap / (2 * t.mr))));
-      t.nc = cdiv(t.N, ntn);
+      const bool pa = t.t[0].abuf >= B_STATE;
+      long long best = -1;
+      int ntn = 1;
+      for (int a = cdiv(t.M, GT_SIDE); a <= t.M; ++a) {
+        const int mr = cdiv(t.M, a);
+        if (2 * mr > cap) continue;
+        const int b = cdiv(t.N, std::max(1, std::min<int>(GT_SIDE, cap / (2 * mr)))), nc = cdiv(t.N, b);
+        const long long cost = (long long)a * b * (16 * cdiv(2 * mr * nc, 32) + 6 * cdiv((1 + pa) * mr + (2 - pa) * nc, 32));
+        if (best < 0 || cost < best) { best = cost; t.ntm = a; t.mr = mr; ntn = b; t.nc = nc; }
+      }
+      t.ntm = cdiv(t.M, t.mr);
+      ntn = cdiv(t.N, t.nc);
       t.tile0 = ntiles;
       ntiles += t.ntm * ntn;
       tile2task.insert(tile2task.end(), (size_t)t.ntm * ntn, (int)k);
@@ -229,6 +239,23 @@ struct pnfam_ctx {
   std::vector<int> pc, qc;
   std::vector<long long> poff, qoff;
   DBuf<double> d_fp, d_fn;   // [dqp] quasiparticle occupations
+  // Active quasiparticles: the columns of U and V beyond the last non-zero one of a block
+  // (the reference erases those above the pairing window) leave their elements of the QP
+  // quadrants at zero: F_qp and H_qp vanish there, and so do X, Y, P and Q.  Runs in the
+  // fast form (form = 1) keep and iterate the leading dap[i] x dan[j] part of each block
+  // only, an elements per quadrant instead of nxy (162Gd at N_sh = 16: 0.36).
+  // form 0 is the general one: whole blocks, unshared products.
+  int form = 0;
+  std::vector<int> dap, dan;
+  long long an = 0;
+  std::vector<long long> axoff, ayoff, apoff, aqoff;
+  std::vector<int> agather;  // [nq * an] element of the whole quadrants
+  DBuf<int> d_agather, d_aerow, d_aecol;
+  DBuf<double> d_afops;
+  long long qn() const { return form ? an : nxy; }
+  const int* erow() const { return form ? d_aerow.p : d_erow.p; }
+  const int* ecol() const { return form ? d_aecol.p : d_ecol.p; }
+  const double* fops() const { return form ? d_afops.p : d_fops.p; }
   long long tplane = 0;      // elements per plane of the GEMM scratch (B_T)
   DBuf<int> d_fc, d_xtc, d_ytc, d_erow, d_ecol;
   DBuf<long long> d_foff, d_xtoff, d_ytoff;
@@ -244,7 +271,6 @@ struct pnfam_ctx {
     long long floats = 0;
     bool built = false;
   } tc32[2];
-  int tcset = 0;              // the form that the current run takes
   std::vector<HTask> htasks;
   DBuf<HTask> d_htasks;
   std::vector<HTaskTC> htasks_tc;   // tensor-core field projection (FP32 data)
@@ -358,8 +384,8 @@ struct pnfam_ctx {
   // returns what its FP32 evaluations lead to, so it keeps the pair-tensor GEMMs from the
   // tuned point count on: their long tensor-core sums differ from the unit sums by 1e-5 in
   // 12 steps, while the strengths of certified runs agree to 1e-8 for either.
-  // shared64: the FP64 transforms with shared products, under the rule of sep64.
-  bool sep64 = false, pair32 = false, tuning = false, shared64 = false;
+  // Both kinds of run also keep the general form of the transforms (form 0).
+  bool sep64 = false, pair32 = false, tuning = false;
   bool pg_ready = false;      // pg_setup done for the current operator
   int nchunk_bro = 1, nchunk_c = 1;
   cudaStream_t stream = nullptr;
@@ -404,6 +430,7 @@ struct pnfam_ctx {
                            &d_beta, &d_gamma, &d_cpart, &d_wre, &d_wim, &d_gfn, &d_fp, &d_fn};
     for (auto* b : dbs) b->release();
     d_foff.release(); d_xtoff.release(); d_ytoff.release();
+    d_agather.release(); d_aerow.release(); d_aecol.release(); d_afops.release();
     d_htasks.release(); d_bufs.release(); d_htasks_tc.release(); d_actlist.release(); d_err.release();
     for (TCSet& t : tc32) {
       for (TaskListTC& l : t.l) l.d_tasks.release();
@@ -488,6 +515,31 @@ static void emit_triple(TaskList& s1, TaskList& s2, long long& toff, const std::
   s2.add(orows, ocols, terms[0].A.ocols(), st2, obuf, ooff, orows);
 }
 
+// offsets of the active parts of the QP quadrants, and their elements in the whole ones
+static void active_layout(pnfam_ctx* c) {
+  if (c->dap.empty()) c->dap = c->dan = c->db;
+  const std::vector<int>&dl = c->beta_minus ? c->dap : c->dan, &dr = c->beta_minus ? c->dan : c->dap;
+  const std::vector<int>* cols[4] = {&c->xc, &c->yc, &c->pc, &c->qc};
+  const std::vector<long long>* full[4] = {&c->xoff, &c->yoff, &c->poff, &c->qoff};
+  std::vector<long long>* act[4] = {&c->axoff, &c->ayoff, &c->apoff, &c->aqoff};
+  c->agather.clear();
+  for (int q = 0; q < 4; ++q) {
+    long long n = 0;
+    act[q]->assign(c->nb, -1);
+    for (int i = 0; i < c->nb; ++i) {
+      const int j = (*cols[q])[i];
+      if (j < 0) continue;
+      (*act[q])[i] = n;
+      n += (long long)dl[i] * dr[j];
+      if (q >= c->nq) continue;
+      for (int b = 0; b < dr[j]; ++b)
+        for (int a = 0; a < dl[i]; ++a)
+          c->agather.push_back((int)(q * c->nxy + (*full[q])[i] + a + (long long)b * c->db[i]));
+    }
+    c->an = n;   // one value: dl and dr are the same for TR partners
+  }
+}
+
 // The same transforms with the first products shared: T1 = UL X - VL Q, T2 = VL Y - UL P
 // and their time-reversed partners serve both SP quadrants that contain them, and the two
 // products with one outer factor are summed before it: 12 block products for X and Y
@@ -496,18 +548,24 @@ static void emit_triple(TaskList& s1, TaskList& s2, long long& toff, const std::
 // rounding.
 static void build_shared_tasks(pnfam_ctx* c) {
   const int nb = c->nb;
-  const long long nxy = c->nxy;
-  const int UL = c->left_u(), VL = c->left_v(), UR = c->right_u(), VR = c->right_v();
+  const long long nxy = c->nxy, an = c->an;
+  const std::vector<int>&dl = c->beta_minus ? c->dap : c->dan, &dr = c->beta_minus ? c->dan : c->dap;
   const bool stat = c->nq == 4;
   TaskList &a1 = c->s1a, &b1 = c->s1b, &a2 = c->s2a, &b2 = c->s2b;
   a1.clear(); b1.clear(); a2.clear(); b2.clear();
+  // U and V with their active columns; V of block i couples to the QPs of its TR partner
+  const int ul = c->left_u(), vl = c->left_v(), ur = c->right_u(), vr = c->right_v();
+  auto UL = [&](int i, int t) { return MatRef{ul, c->uoff[i], c->db[i], dl[i], t}; };
+  auto VL = [&](int i, int t) { return MatRef{vl, c->uoff[i], c->db[i], dl[c->tr[i]], t}; };
+  auto UR = [&](int i, int t) { return MatRef{ur, c->uoff[i], c->db[i], dr[i], t}; };
+  auto VR = [&](int i, int t) { return MatRef{vr, c->uoff[i], c->db[i], dr[c->tr[i]], t}; };
   auto part = [&](int q, int i, const std::vector<long long>& off, const std::vector<int>& cols) {
-    return MatRef{B_STATE, q * nxy + off[i], c->db[i], c->db[cols[i]], 0};
+    return MatRef{B_STATE, q * an + off[i], dl[i], dr[cols[i]], 0};
   };
-  auto X = [&](int i) { return part(0, i, c->xoff, c->xc); };
-  auto Y = [&](int i) { return part(1, i, c->yoff, c->yc); };
-  auto Pq = [&](int i) { return part(2, i, c->poff, c->pc); };
-  auto Qq = [&](int i) { return part(3, i, c->qoff, c->qc); };
+  auto X = [&](int i) { return part(0, i, c->axoff, c->xc); };
+  auto Y = [&](int i) { return part(1, i, c->ayoff, c->yc); };
+  auto Pq = [&](int i) { return part(2, i, c->apoff, c->pc); };
+  auto Qq = [&](int i) { return part(3, i, c->aqoff, c->qc); };
   auto H = [&](int q, int row, const std::vector<long long>& off, const std::vector<int>& cols, int tr_) {
     return MatRef{B_HSP, q * nxy + off[row], c->db[row], c->db[cols[row]], tr_};
   };
@@ -531,33 +589,33 @@ static void build_shared_tasks(pnfam_ctx* c) {
     const int t = c->tr[i];
     if (c->fc[i] >= 0) {
       const int j = c->fc[i], x = c->xc[i];
-      std::vector<Prod> p1 = {{c->ublk(UL, i, 0), X(i), 1.0, 1.0}}, p2 = {{c->vblk(VL, i, 0), Y(t), 1.0, 1.0}};
+      std::vector<Prod> p1 = {{UL(i, 0), X(i), 1.0, 1.0}}, p2 = {{VL(i, 0), Y(t), 1.0, 1.0}};
       if (stat) {
-        p1.push_back({c->vblk(VL, i, 0), Qq(t), -1.0, -1.0});
-        p2.push_back({c->ublk(UL, i, 0), Pq(i), -1.0, -1.0});
+        p1.push_back({VL(i, 0), Qq(t), -1.0, -1.0});
+        p2.push_back({UL(i, 0), Pq(i), -1.0, -1.0});
       }
       const MatRef T1 = temp(a1, p1), T2 = temp(a1, p2);
-      sum(b1, {{T1, c->vblk(VR, j, 1), 1.0, 1.0}, {T2, c->ublk(UR, j, 1), -1.0, -1.0}}, B_RSP, c->foff[i]);
-      sum(b1, {{c->ublk(UR, x, 0), flip(T1), -1.0, -1.0}, {c->vblk(VR, x, 0), flip(T2), 1.0, 1.0}}, B_RSP,
+      sum(b1, {{T1, VR(j, 1), 1.0, 1.0}, {T2, UR(j, 1), -1.0, -1.0}}, B_RSP, c->foff[i]);
+      sum(b1, {{UR(x, 0), flip(T1), -1.0, -1.0}, {VR(x, 0), flip(T2), 1.0, 1.0}}, B_RSP,
           nxy + c->xtoff[x]);
     }
     if (c->yc[i] >= 0) {
       const int y = c->yc[i];
-      std::vector<Prod> p3 = {{c->vblk(VL, i, 0), X(t), 1.0, 1.0}}, p4 = {{c->ublk(UL, i, 0), Y(i), 1.0, 1.0}};
+      std::vector<Prod> p3 = {{VL(i, 0), X(t), 1.0, 1.0}}, p4 = {{UL(i, 0), Y(i), 1.0, 1.0}};
       if (stat) {
-        p3.push_back({c->ublk(UL, i, 0), Qq(i), -1.0, -1.0});
-        p4.push_back({c->vblk(VL, i, 0), Pq(t), -1.0, -1.0});
+        p3.push_back({UL(i, 0), Qq(i), -1.0, -1.0});
+        p4.push_back({VL(i, 0), Pq(t), -1.0, -1.0});
       }
       T3[i] = temp(a1, p3);
       T4[i] = temp(a1, p4);
-      sum(b1, {{c->vblk(VR, y, 0), flip(T3[i]), 1.0, -1.0}, {c->ublk(UR, y, 0), flip(T4[i]), -1.0, 1.0}}, B_RSP,
+      sum(b1, {{VR(y, 0), flip(T3[i]), 1.0, -1.0}, {UR(y, 0), flip(T4[i]), -1.0, 1.0}}, B_RSP,
           2 * nxy + c->ytoff[y]);
     }
   }
   for (int j = 0; j < nb; ++j) {
     if (c->fc[j] < 0) continue;
     const int i = c->fc[j];
-    sum(b1, {{c->ublk(UR, j, 0), flip(T3[i]), -1.0, -1.0}, {c->vblk(VR, j, 0), flip(T4[i]), 1.0, 1.0}}, B_RSP,
+    sum(b1, {{UR(j, 0), flip(T3[i]), -1.0, -1.0}, {VR(j, 0), flip(T4[i]), 1.0, 1.0}}, B_RSP,
         3 * nxy + c->foff[j]);
   }
   // ---- K2 ----
@@ -567,32 +625,33 @@ static void build_shared_tasks(pnfam_ctx* c) {
     if (c->fc[i] >= 0) {
       const int j = c->fc[i], x = c->xc[i];
       const MatRef h11 = H(0, i, c->foff, c->fc, 0), h12 = H(1, i, c->xoff, c->xc, 0);
-      T5[i] = temp(a2, {{h11, c->vblk(VR, j, 0), 1.0, 1.0}, {h12, c->ublk(UR, x, 0), 1.0, 1.0}});
-      T7[i] = temp(a2, {{h11, c->ublk(UR, j, 0), 1.0, 1.0}, {h12, c->vblk(VR, x, 0), 1.0, 1.0}});
+      T5[i] = temp(a2, {{h11, VR(j, 0), 1.0, 1.0}, {h12, UR(x, 0), 1.0, 1.0}});
+      T7[i] = temp(a2, {{h11, UR(j, 0), 1.0, 1.0}, {h12, VR(x, 0), 1.0, 1.0}});
     }
     if (c->yc[i] >= 0) {
       const int y = c->yc[i], x = c->tr[y];
       const MatRef m21 = H(2, i, c->yoff, c->yc, 0), m22 = H(3, x, c->foff, c->fc, 1);
-      T6[i] = temp(a2, {{m21, c->vblk(VR, y, 0), -1.0, 1.0}, {m22, c->ublk(UR, x, 0), -1.0, -1.0}});
-      T8[i] = temp(a2, {{m21, c->ublk(UR, y, 0), 1.0, -1.0}, {m22, c->vblk(VR, x, 0), 1.0, 1.0}});
+      T6[i] = temp(a2, {{m21, VR(y, 0), -1.0, 1.0}, {m22, UR(x, 0), -1.0, -1.0}});
+      T8[i] = temp(a2, {{m21, UR(y, 0), 1.0, -1.0}, {m22, VR(x, 0), 1.0, 1.0}});
     }
   }
   for (int i = 0; i < nb; ++i) {
     const int t = c->tr[i];
     if (c->fc[i] >= 0)
-      sum(b2, {{c->ublk(UL, i, 1), T5[i], 1.0, 1.0}, {c->vblk(VL, t, 1), T6[t], 1.0, 1.0}}, B_HQP, c->xoff[i]);
+      sum(b2, {{UL(i, 1), T5[i], 1.0, 1.0}, {VL(t, 1), T6[t], 1.0, 1.0}}, B_HQP, c->axoff[i]);
     if (c->yc[i] >= 0)
-      sum(b2, {{c->vblk(VL, t, 1), T7[t], -1.0, -1.0}, {c->ublk(UL, i, 1), T8[i], 1.0, 1.0}}, B_HQP, nxy + c->yoff[i]);
+      sum(b2, {{VL(t, 1), T7[t], -1.0, -1.0}, {UL(i, 1), T8[i], 1.0, 1.0}}, B_HQP, an + c->ayoff[i]);
     if (stat && c->pc[i] >= 0)
-      sum(b2, {{c->ublk(UL, i, 1), T7[i], 1.0, 1.0}, {c->vblk(VL, t, 1), T8[t], -1.0, -1.0}}, B_HQP,
-          2 * nxy + c->poff[i]);
+      sum(b2, {{UL(i, 1), T7[i], 1.0, 1.0}, {VL(t, 1), T8[t], -1.0, -1.0}}, B_HQP,
+          2 * an + c->apoff[i]);
     if (stat && c->qc[i] >= 0)
-      sum(b2, {{c->vblk(VL, t, 1), T5[t], -1.0, -1.0}, {c->ublk(UL, i, 1), T6[i], -1.0, -1.0}}, B_HQP,
-          3 * nxy + c->qoff[i]);
+      sum(b2, {{VL(t, 1), T5[t], -1.0, -1.0}, {UL(i, 1), T6[i], -1.0, -1.0}}, B_HQP,
+          3 * an + c->aqoff[i]);
   }
 }
 
-static void build_tasks(pnfam_ctx* c) {
+// the QP <-> SP transforms
+static void build_transforms(pnfam_ctx* c) {
   const int nb = c->nb;
   const long long nxy = c->nxy;
   const int UL = c->left_u(), VL = c->left_v(), UR = c->right_u(), VR = c->right_v();
@@ -709,7 +768,15 @@ static void build_tasks(pnfam_ctx* c) {
   c->shared = true;
   for (int i = 0; i < nb; ++i)
     if (c->fc[i] >= 0 && c->fc[c->tr[c->fc[i]]] != c->tr[i]) c->shared = false;
-  if (c->shared) build_shared_tasks(c);
+  if (c->shared) {
+    active_layout(c);
+    build_shared_tasks(c);
+  }
+}
+
+// the general kernels' field projection and density tasks
+static void build_field_tasks(pnfam_ctx* c) {
+  const int nb = c->nb;
   // ---- FP64 field projection tasks: spin-uniform tiles of 1024 / tn rows x tn columns ----
   // The shape of each (block pair, spin segment) is the one that issues the fewest DFMAs:
   // per tile, tn columns x the rows up to the warp granularity of the shape (a warp holds
@@ -1009,6 +1076,11 @@ static void pg_setup(pnfam_ctx* c) {
   }
 }
 
+static void pg_prepare(pnfam_ctx* c) {
+  if (!c->pg_ready) pg_setup(c);
+  c->pg_ready = true;
+}
+
 // device tables and the pair tensor (once per operator)
 static int pg_build(pnfam_ctx* c) {
   if (!c->pg_on || c->pg_built) return PNFAM_OK;
@@ -1084,7 +1156,7 @@ static int pg_projection(pnfam_ctx* c, int nact, const float* mf, float* hsp, cu
 
 static int ensure_buffers(pnfam_ctx* c, int P, int M) {
   const long long nxy = c->nxy;
-  const long long nv = 2 * c->nq * nxy;   // Re and Im of the QP state (X, Y[, P, Q])
+  const long long nv = 2 * c->nq * c->qn();   // Re and Im of the QP state (X, Y[, P, Q])
   const long long tpl = std::max(c->tplane, 8 * nxy);
   CK(dalloc(c->d_state, (size_t)P * nv));
   CK(dalloc(c->d_vout, (size_t)P * nv));
@@ -1141,11 +1213,11 @@ static int launch_gemm(pnfam_ctx* c, TaskList& tl, int P, const int* active, cud
 
 // FP32 stage on the tensor cores for the nact points listed in c->d_actlist
 static int launch_gemm_tc(pnfam_ctx* c, int list, int nact, cudaStream_t st) {
-  const TaskListTC& tl = c->tc32[c->tcset].l[list];
+  const TaskListTC& tl = c->tc32[c->form].l[list];
   if (tl.tasks.empty() || nact <= 0) return PNFAM_OK;
   dim3 grid((unsigned)tl.tasks.size(), (unsigned)((2 * nact * tl.maxrows + 127) / 128));
   k_gemm_tc<<<grid, GTC_THREADS, gemm_tc_smem_bytes(tl.maxnp), st>>>(tl.d_tasks.p, c->d_bufs32.p,
-                                                                      c->tc32[c->tcset].gsplit.p, c->d_actlist.p, nact, tl.maxnp, c->d_err.p);
+                                                                      c->tc32[c->form].gsplit.p, c->d_actlist.p, nact, tl.maxnp, c->d_err.p);
   c->launches++;
   CK(cudaGetLastError());
   return PNFAM_OK;
@@ -1160,7 +1232,7 @@ static int residual_k2(pnfam_ctx* c, int P, int nact, const int* act, cudaStream
     if ((rc = launch_gemm_tc(c, 2, nact, st))) return rc;
     if ((rc = launch_gemm_tc(c, 3, nact, st))) return rc;
   } else {
-    const bool sh = c->shared64;
+    const bool sh = c->form != 0;
     if ((rc = launch_gemm(c, sh ? c->s2a : c->k2a, P, act, st))) return rc;
     if ((rc = launch_gemm(c, sh ? c->s2b : c->k2b, P, act, st))) return rc;
   }
@@ -1338,7 +1410,7 @@ static int residual_t(pnfam_ctx* c, int P, int nact, const int* act, bool timed,
     if ((rc = launch_gemm_tc(c, 0, nact, st))) return rc;
     if ((rc = launch_gemm_tc(c, 1, nact, st))) return rc;
   } else {
-    const bool sh = c->shared64;
+    const bool sh = c->form != 0;
     if ((rc = launch_gemm(c, sh ? c->s1a : c->k1a, P, act, st))) return rc;
     if ((rc = launch_gemm(c, sh ? c->s1b : c->k1b, P, act, st))) return rc;
   }
@@ -1494,7 +1566,7 @@ static int pg_autotune(pnfam_ctx* c, int P) {
     }
   }
   cudaStream_t st = c->stream;
-  const long long nv = 2 * c->nq * c->nxy;
+  const long long nv = 2 * c->nq * c->qn();
   CK(cudaMemsetAsync(c->d_state32.p, 0, sizeof(float) * (size_t)nmax * nv, st));
   std::vector<int> list(nmax), flags(P, 0);
   for (int i = 0; i < nmax; ++i) list[i] = i;
@@ -1594,7 +1666,7 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
   }
   // QP-state arrays: nv = Re and Im of X, Y (and P, Q in the statistical FAM); GEMM
   // scratch as in the FP64 form
-  const long long nv = 2 * c->nq * nxy;
+  const long long nv = 2 * c->nq * c->qn();
   const long long tpl = std::max(c->tplane, 8 * nxy);
   CK(dalloc(c->d_state32, (size_t)P * nv));
   CK(dalloc(c->d_T32, (size_t)P * 2 * tpl));
@@ -1621,10 +1693,7 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
   // what the general kernels need (a separable basis: only for the pair-tensor GEMMs of
   // uncertified runs, whose point count is tuned against the per-block kernels)
   const bool general = !c->sep32 || pair;
-  if (general && !c->pg_ready) {
-    pg_setup(c);
-    c->pg_ready = true;
-  }
+  if (general) pg_prepare(c);
   if (c->tc_density && general) {
     CK(dalloc(c->d_bsplit, (size_t)P * c->bstride));
     if (!c->have_aphi) {
@@ -1659,9 +1728,7 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
     c->have_hphi = true;
   }
   if (run) {
-    // uncertified runs that take the pair-tensor GEMMs keep the general form (pnfam_ctx::pair32)
-    c->tcset = c->shared && !(pair && c->pg_on) ? 1 : 0;
-    pnfam_ctx::TCSet& set = c->tc32[c->tcset];
+    pnfam_ctx::TCSet& set = c->tc32[c->form];
     if (!set.built) {
       CK(dalloc(set.gsplit, (size_t)std::max(1LL, set.floats)));
       for (const TaskListTC& tl : set.l) {
@@ -1762,6 +1829,26 @@ extern "C" int pnfam_gpu_init(const pnfam_basis_t* basis, const double* Ep, cons
     c->ns[k] = (signed char)basis->ns[k];
   }
   for (int i = 0; i < 12; ++i) c->sc[i] = coupl->scalars[i];
+  // active quasiparticles: up to the last column of U and V that is not all zero (at least
+  // one per block), the same number for TR partners
+  auto active = [&](const double* U, const double* V) {
+    std::vector<int> n(c->nb);
+    auto last = [&](const double* m, int i) {
+      const int d = c->db[i];
+      int k = d;
+      for (; k > 1; --k) {
+        const double* col = m + c->uoff[i] + (long long)(k - 1) * d;
+        if (std::any_of(col, col + d, [](double x) { return !(x == 0.0); })) break;
+      }
+      return std::min(k, d);
+    };
+    for (int i = 0; i < c->nb; ++i) n[i] = std::max(last(U, i), last(V, c->tr[i]));
+    std::vector<int> m(c->nb);
+    for (int i = 0; i < c->nb; ++i) m[i] = std::max(n[i], n[c->tr[i]]);
+    return m;
+  };
+  c->dap = active(Up, Vp);
+  c->dan = active(Un, Vn);
   auto up = [&](auto& buf, const auto* h, size_t n) -> int { CK(upload(buf, h, n)); return 0; };
   int rc = 0;
   const size_t nphi = (size_t)5 * s * c->nghl;
@@ -1863,6 +1950,13 @@ static int host_structure(pnfam_ctx* c, int beta_minus, const int* fcols) {
   return PNFAM_OK;
 }
 
+// partial sums of the Broyden and strength kernels for the current form
+static void set_chunks(pnfam_ctx* c) {
+  const long long n = c->nq * c->qn();
+  c->nchunk_bro = (int)((2 * n + BRO_CHUNK - 1) / BRO_CHUNK);
+  c->nchunk_c = (int)std::min<long long>(32, std::max<long long>(1, n / 4096));
+}
+
 extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int* fcols, const double* Fsp,
                                       int n_xterms, const double* const* Gsp) {
   g_err.clear();
@@ -1910,9 +2004,10 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
     for (int i = 0; i < nb; ++i) nrows += c->fc[i] >= 0;
     c->G = std::max(1, std::min(nrows, (2 * std::max(nsm, 1) + ntr - 1) / ntr));
   }
-  c->nchunk_bro = (int)((2 * nq * nf + BRO_CHUNK - 1) / BRO_CHUNK);
-  c->nchunk_c = (int)std::min<long long>(32, std::max<long long>(1, (nq * nf) / 4096));
-  build_tasks(c);
+  c->form = 0;   // F_qp below; a run chooses its own (engine_setup)
+  set_chunks(c);
+  build_transforms(c);
+  build_field_tasks(c);
   {
     const int rcs = sep_operator(c);
     if (rcs) return rcs;
@@ -1961,6 +2056,18 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
     if ((rc = launch_gemm(c, c->k2b, 1, c->d_active.p, c->stream))) return rc;
     CK(cudaMemcpyAsync(c->d_fops.p + (long long)k * nq * nf, c->d_hqp.p, sizeof(double) * nq * nf,
                        cudaMemcpyDeviceToDevice, c->stream));
+  }
+  if (c->shared) {
+    const size_t na = c->agather.size();
+    std::vector<int> ar(na), ac(na);
+    for (size_t e = 0; e < na; ++e) { ar[e] = erow[c->agather[e]]; ac[e] = ecol[c->agather[e]]; }
+    CK(upload(c->d_agather, c->agather.data(), na));
+    CK(upload(c->d_aerow, ar.data(), na));
+    CK(upload(c->d_aecol, ac.data(), na));
+    CK(dalloc(c->d_afops, c->nops * na));
+    k_gather<<<dim3((unsigned)((na + 255) / 256), c->nops), 256, 0, c->stream>>>(
+        c->d_fops.p, (long long)nq * nf, c->d_agather.p, (long long)na, c->d_afops.p);
+    CK(cudaGetLastError());
   }
   CK(cudaStreamSynchronize(c->stream));
   return PNFAM_OK;
@@ -2049,7 +2156,8 @@ void pnfam_ctx::detach_engine() {
   }
 }
 
-static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver_opts_t* o) {
+// active: a start vector, if there is one, vanishes outside the active quasiparticles
+static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver_opts_t* o, bool active = true) {
   if (!c->have_op) return fail(PNFAM_ESTATE, "call pnfam_gpu_set_operator first");
   if (o->max_iter < 0) return fail(PNFAM_EINVAL, "max_iter < 0");
   if (o->precision != 0 && o->precision != 1)
@@ -2059,15 +2167,20 @@ static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver
   e->M = e->no_res ? -1 : o->broyden_history_size;
   if (e->M > 64) return fail(PNFAM_EINVAL, "broyden_history_size > 64 is not supported");
   e->bmode = e->M < 0 ? BRO_NOMIX : e->M == 0 ? BRO_LINEAR : BRO_BROYDEN;
-  e->nxy = c->nxy; e->N = (int)(2 * c->nq * c->nxy); e->nops = c->nops;
+  e->mixed = o->precision == 1 && !e->no_res;
+  c->sep64 = c->sep && (e->mixed || e->M <= 0 || e->M >= SEP_MIN_HISTORY);
+  c->pair32 = e->mixed && o->reserved[3] <= 0;
+  bool general = !c->shared || !active || (!e->mixed && e->M > 0 && e->M < SEP_MIN_HISTORY);
+  if (c->pair32 && c->sep32) {
+    pg_prepare(c);
+    general |= c->pg_on;
+  }
+  c->form = general ? 0 : 1;
+  set_chunks(c);
+  e->nxy = c->qn(); e->N = (int)(2 * c->nq * e->nxy); e->nops = c->nops;
   int rc = ensure_buffers(c, std::max(P, c->cap_P), std::max(std::max(e->M, 1), c->cap_M));
   if (rc) return rc;
   c->cap_P = std::max(P, c->cap_P); c->cap_M = std::max(std::max(e->M, 1), c->cap_M);
-  e->mixed = o->precision == 1 && !e->no_res;
-  const bool rounding_free = e->mixed || e->M <= 0 || e->M >= SEP_MIN_HISTORY;
-  c->sep64 = c->sep && rounding_free;
-  c->shared64 = c->shared && rounding_free;
-  c->pair32 = o->reserved[3] <= 0;
   if (e->mixed && (rc = ensure_buffers32(c, c->cap_P, c->pair32, true))) return rc;
   // Mixed form (precision 1): one Broyden iteration per evaluation, as in the FP64
   // form, but the residual interaction is evaluated in FP32 on the increment
@@ -2169,8 +2282,15 @@ static int engine_set_state(pnfam_engine* e, int p, const double* x) {
   if (p < 0 || p >= e->P || !e->active[p] || e->it[p] != 0)
     return fail(PNFAM_ESTATE, "a start vector needs a slot that was just admitted");
   e->x0[p] = 1;
-  std::vector<double> v(e->N);
-  state_from_ref((int)(e->N / (2 * e->nxy)), e->nxy, x, v.data());
+  const pnfam_ctx* c = e->c;
+  std::vector<double> v((size_t)2 * c->nq * c->nxy);
+  state_from_ref(c->nq, c->nxy, x, v.data());
+  if (c->form) {
+    std::vector<double> w(e->N);
+    const size_t na = c->agather.size(), nf = (size_t)c->nq * c->nxy;
+    for (size_t i = 0; i < na; ++i) { w[i] = v[c->agather[i]]; w[na + i] = v[nf + c->agather[i]]; }
+    v = std::move(w);
+  }
   e->x0q.emplace_back(p, std::move(v));
   return PNFAM_OK;
 }
@@ -2324,7 +2444,7 @@ static int engine_launch(pnfam_engine* e, bool block_if_idle) {
     const int gx = (int)std::min<long long>(4096, (nq * nxy + 255) / 256);
     const double* f1 = nq == 4 ? (c->beta_minus ? c->d_fp.p : c->d_fn.p) : nullptr;
     const double* f2 = nq == 4 ? (c->beta_minus ? c->d_fn.p : c->d_fp.p) : nullptr;
-    k_green_prep<<<dim3(gx, P), 256, 0, c->stream>>>(nxy, nq, c->d_erow.p, c->d_ecol.p, E1, E2, f1, f2, c->d_wre.p,
+    k_green_prep<<<dim3(gx, P), 256, 0, c->stream>>>(nxy, nq, c->erow(), c->ecol(), E1, E2, f1, f2, c->d_wre.p,
                                                      c->d_wim.p, c->d_gfn.p, d_fresh);
     c->launches += 2;
   }
@@ -2391,7 +2511,7 @@ static int engine_launch(pnfam_engine* e, bool block_if_idle) {
   {
     const int gx = (int)std::min<long long>(4096, (nq * nxy + 255) / 256);
     k_green<<<dim3(gx, P), 256, 0, c->stream>>>(nxy, nq, P, e->no_res ? nullptr : c->d_hqp.p,
-                                                e->mixed ? c->d_hqp32.p : nullptr, c->d_fops.p, c->d_gfn.p,
+                                                e->mixed ? c->d_hqp32.p : nullptr, c->fops(), c->d_gfn.p,
                                                 e->o.quench_residual_int, c->d_vout.p, act,
                                                 e->mixed ? d_incr : nullptr, c->d_radd.p, d_zero);
     c->launches++;
@@ -2410,7 +2530,7 @@ static int engine_launch(pnfam_engine* e, bool block_if_idle) {
   tic();
   {
     dim3 grid(c->nchunk_c, P);
-    k_contract<<<grid, 256, 0, c->stream>>>(nxy, nq, e->nops, c->d_fops.p, c->d_state.p, c->nchunk_c, c->d_cpart.p,
+    k_contract<<<grid, 256, 0, c->stream>>>(nxy, nq, e->nops, c->fops(), c->d_state.p, c->nchunk_c, c->d_cpart.p,
                                             act);
     c->launches++;
     CK(cudaGetLastError());
@@ -2518,14 +2638,25 @@ static int solve_impl(pnfam_ctx_t* c, int P, const double* re_w, const double* i
     return fail(PNFAM_EINVAL, "pnfam_gpu_solve: bad argument");
   if (c->engine) return fail(PNFAM_ESTATE, "pnfam_gpu_solve: the context's solve buffers belong to an engine");
   pnfam_engine e;
-  int rc = engine_setup(&e, c, P, o);
+  const long long nst = c->have_op ? 2LL * c->nq * c->nxy : 0;   // length of a state vector
+  bool active = true;
+  if (x0 && c->have_op && c->shared) {
+    std::vector<double> v((size_t)nst);
+    std::vector<char> in((size_t)c->nq * c->nxy, 0);
+    for (int k : c->agather) in[k] = 1;
+    for (int p = 0; p < P && active; ++p) {
+      state_from_ref(c->nq, c->nxy, x0 + (size_t)p * nst, v.data());
+      for (size_t k = 0; k < in.size() && active; ++k) active = in[k] || (v[k] == 0.0 && v[in.size() + k] == 0.0);
+    }
+  }
+  int rc = engine_setup(&e, c, P, o, active);
   if (rc) { g_err = "pnfam_gpu_solve: " + g_err; return rc; }
   e.hist = hist;
   CK(cudaEventRecord(c->evt[0], c->stream));
   engine_admit(&e, P, re_w, im_w, nullptr);
   if (x0) {
     for (int p = 0; p < P; ++p)
-      if (e.active[p] && (rc = engine_set_state(&e, p, x0 + (size_t)p * e.N))) return rc;
+      if (e.active[p] && (rc = engine_set_state(&e, p, x0 + (size_t)p * nst))) return rc;
   }
   while (engine_nactive(&e) > 0) {
     if ((rc = engine_launch(&e, true)) || (rc = engine_finish(&e))) {
@@ -2554,9 +2685,18 @@ static int solve_impl(pnfam_ctx_t* c, int P, const double* re_w, const double* i
   }
   // the final state vectors (point p was admitted into slot p)
   if (x_out) {
-    std::vector<double> v((size_t)P * e.N);
+    std::vector<double> v((size_t)P * e.N), full;
     CK(cudaMemcpy(v.data(), c->d_state.p, sizeof(double) * v.size(), cudaMemcpyDeviceToHost));
-    for (int p = 0; p < P; ++p) state_to_ref(c->nq, c->nxy, v.data() + (size_t)p * e.N, x_out + (size_t)p * e.N);
+    const size_t na = c->agather.size(), nf = (size_t)nst / 2;
+    if (c->form) full.assign((size_t)nst, 0.0);
+    for (int p = 0; p < P; ++p) {
+      const double* d = v.data() + (size_t)p * e.N;
+      if (c->form) {
+        for (size_t i = 0; i < na; ++i) { full[c->agather[i]] = d[i]; full[nf + c->agather[i]] = d[na + i]; }
+        d = full.data();
+      }
+      state_to_ref(c->nq, c->nxy, d, x_out + (size_t)p * nst);
+    }
   }
   return PNFAM_OK;
 }
@@ -2818,7 +2958,7 @@ extern "C" int pnfam_gpu_task_tables(int nb, const int* db, const int* num_spin_
   if (rc) return rc;
   c.nq = statistical ? 4 : 2;
   if ((rc = host_structure(&c, beta_minus, fcols))) return rc;
-  build_tasks(&c);
+  build_transforms(&c);
   const TaskList* lists[2][4] = {{&c.k1a, &c.k1b, &c.k2a, &c.k2b}, {&c.s1a, &c.s1b, &c.s2a, &c.s2b}};
   const TaskList& tl = *lists[c.shared][stage];
   *ntask = (int)tl.tasks.size();
@@ -2991,7 +3131,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian_noalloc(
     return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_noalloc: inconsistent block structure");
   if (nf > NA_MAX_NXY) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_noalloc: nxy <= 32768 is the limit");
   c.nxy = nf;
-  build_tasks(&c);
+  build_field_tasks(&c);
   if ((int)c.htasks.size() > NA_MAX_HTASKS)
     return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_noalloc: more than 4096 field-projection tiles");
   unsigned char* base = nullptr;

@@ -60,6 +60,28 @@ __device__ __forceinline__ const T* bufptr(const BufDescT<T>* b, int id, int p, 
   return d.base + (long long)p * d.sp + (long long)plane * d.spl + off;
 }
 
+// dst[kk * ld + i] = al * element (x0 + i, k0 + kk) for i < n, kk < kl; kfast: k is
+// consecutive in memory (i at stride lds), otherwise i is (k at stride lds)
+__device__ __forceinline__ void gemm_stage(const double* __restrict__ src, int lds, bool kfast, int x0, int n, int k0,
+                                           int kl, double al, double* __restrict__ dst, int ld) {
+  if (kfast) {
+    const int kk = threadIdx.x % GT_K;
+    if (kk >= kl) return;
+    const double* s = src + k0 + kk + (long long)x0 * lds;
+    for (int i = threadIdx.x / GT_K; i < n; i += GT_THREADS / GT_K) dst[kk * ld + i] = al * s[(long long)i * lds];
+  } else {
+    // (i, kk) of element threadIdx.x + 256 j without a division per element
+    const int di = GT_THREADS % n, dk = GT_THREADS / n;
+    int i = threadIdx.x % n, kk = threadIdx.x / n;
+    const double* s = src + x0 + (long long)k0 * lds;
+    while (kk < kl) {
+      dst[kk * ld + i] = al * s[i + (long long)kk * lds];
+      i += di; kk += dk;
+      if (i >= n) { i -= n; ++kk; }
+    }
+  }
+}
+
 // C = sum_t alpha_t op(A_t) op(B_t) in FP64 for both planes (Re, Im) of one point.
 // The DFMA rate bounds it (a warp's DFMA takes the SM's FP64 pipe 16 cycles, its two
 // shared-memory reads 3), so what counts is that no lane works on padding: the mr x nc x 2
@@ -67,9 +89,9 @@ __device__ __forceinline__ const T* bufptr(const BufDescT<T>* b, int id, int p, 
 // fastest: reads of the row operand are consecutive, those of the column operand mostly
 // one address), K runs over the block's own size, and the ground-state operand is staged
 // once for both planes.  Against tiles of 1024 outputs padded in M, N and K: N_sh = 8, 40
-// points, 28 against 56 ms per solve, N_sh = 6 11 against 22 us per launch; at N_sh = 16
-// (blocks 1 to 81, nine points, shared products) 0.52 ms per point against 1.01, 1.0
-// TFLOP/s of the 1.1 that a DGEMM reaches.  Every output sums over the terms and k in order.  Of the two operands of a
+// points, 23 against 56 ms per solve, N_sh = 6 11 against 22 us per launch; at N_sh = 16
+// (blocks 1 to 81, nine points) 1.1 TFLOP/s, what a DGEMM reaches, against 0.69, and with
+// shared products and active quasiparticles only 0.33 ms per point against 1.01.  Every output sums over the terms and k in order.  Of the two operands of a
 // term one is the point's (two planes), one the ground state's; alpha (+-1) goes into the
 // point's.  grid (tiles, P)
 __global__ void __launch_bounds__(GT_THREADS) k_gemm(const GemmTask* __restrict__ tasks,
@@ -105,38 +127,13 @@ __global__ void __launch_bounds__(GT_THREADS) k_gemm(const GemmTask* __restrict_
     for (int k0 = 0; k0 < K; k0 += GT_K) {
       const int kl = min((int)GT_K, K - k0);
       __syncthreads();
-      for (int pl = 0; pl < (pa ? 2 : 1); ++pl) {
-        const double* A = bufptr(bufs, tm.abuf, p, pl, tm.aoff);
-        const double al = pa ? tm.alpha[pl] : 1.0;
-        double* d = As + pl * GT_K * ma;
-        if (tm.tA) {   // k is consecutive in memory
-          for (int e = threadIdx.x; e < mr * GT_K; e += GT_THREADS) {
-            const int kk = e % GT_K, mm = e / GT_K;
-            if (kk < kl) d[kk * ma + mm] = al * A[k0 + kk + (long long)(m0 + mm) * tm.lda];
-          }
-        } else {
-          for (int e = threadIdx.x; e < mr * kl; e += GT_THREADS) {
-            const int mm = e % mr, kk = e / mr;
-            d[kk * ma + mm] = al * A[m0 + mm + (long long)(k0 + kk) * tm.lda];
-          }
-        }
-      }
-      for (int pl = 0; pl < (pa ? 1 : 2); ++pl) {
-        const double* B = bufptr(bufs, tm.bbuf, p, pl, tm.boff);
-        const double al = pa ? 1.0 : tm.alpha[pl];
-        double* d = Bs + pl * GT_K * nb;
-        if (!tm.tB) {   // k is consecutive in memory
-          for (int e = threadIdx.x; e < nc * GT_K; e += GT_THREADS) {
-            const int kk = e % GT_K, nn = e / GT_K;
-            if (kk < kl) d[kk * nb + nn] = al * B[k0 + kk + (long long)(n0 + nn) * tm.ldb];
-          }
-        } else {
-          for (int e = threadIdx.x; e < nc * kl; e += GT_THREADS) {
-            const int nn = e % nc, kk = e / nc;
-            d[kk * nb + nn] = al * B[n0 + nn + (long long)(k0 + kk) * tm.ldb];
-          }
-        }
-      }
+      // op(A) rows, op(B) columns
+      for (int pl = 0; pl < (pa ? 2 : 1); ++pl)
+        gemm_stage(bufptr(bufs, tm.abuf, p, pl, tm.aoff), tm.lda, tm.tA != 0, m0, mr, k0, kl,
+                   pa ? tm.alpha[pl] : 1.0, As + pl * GT_K * ma, ma);
+      for (int pl = 0; pl < (pa ? 1 : 2); ++pl)
+        gemm_stage(bufptr(bufs, tm.bbuf, p, pl, tm.boff), tm.ldb, tm.tB == 0, n0, nc, k0, kl,
+                   pa ? 1.0 : tm.alpha[pl], Bs + pl * GT_K * nb, nb);
       __syncthreads();
 #pragma unroll 4
       for (int kk = 0; kk < kl; ++kk) {
@@ -2507,6 +2504,13 @@ __global__ void k_vecop(int op, double a, double* __restrict__ dst, const double
     else if (op == 2) d[e] = 0.0;
     else d[e] = a * s_[e];
   }
+}
+
+// out[k][e] = in[k][idx[e]]; grid (ceil(n / 256), rows)
+__global__ void __launch_bounds__(256) k_gather(const double* __restrict__ in, long long ld, const int* __restrict__ idx,
+                                                long long n, double* __restrict__ out) {
+  const long long e = blockIdx.x * 256LL + threadIdx.x;
+  if (e < n) out[blockIdx.y * n + e] = in[blockIdx.y * ld + idx[e]];
 }
 
 // S_k = -1/pi * (F_k . Re, F_k . Im) for the operator (k=0) and cross terms
