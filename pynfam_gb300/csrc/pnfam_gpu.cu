@@ -362,11 +362,11 @@ struct pnfam_ctx {
     DBuf<SepUnit> units;
     DBuf<SepEnt> ents;
     DBuf<int> rows, offs, ubeg, order;
-    DBuf<SepItem> items;
-    DBuf<SepWarp> warps;
+    DBuf<int> items;
+    DBuf<SepWarp> warps[2];
     void release() {
       units.release(); ents.release(); rows.release(); offs.release(); ubeg.release(); order.release();
-      items.release(); warps.release();
+      items.release(); warps[0].release(); warps[1].release();
     }
   } d_seps[5];
   DBuf<double> d_sepf;        // z, r, v, y, e, lam, sgn
@@ -1258,6 +1258,10 @@ static int sep_init(pnfam_ctx* c, const double* phi) {
   if (!sep_factors(nb, c->db.data(), c->st.data(), c->nup.data(), dqp, nghl, ngh, phi, B)) return PNFAM_OK;
   std::vector<double> f;
   for (const auto* v : {&B.r, &B.z, &B.v, &B.y, &B.e, &B.lam, &B.sgn}) f.insert(f.end(), v->begin(), v->end());
+  if (f.size() % 2) f.push_back(0.0);   // pairs are read as such
+  for (int l = 0; l < B.ngl; ++l)
+    for (int k = 0; k < B.nrow; ++k)
+      for (int d = 0; d < 2; ++d) f.push_back(B.r[((size_t)k * B.ngl + l) * 2 + d]);
   CK(upload(c->d_sepf, f.data(), f.size()));
   std::vector<int> idx(3 * (size_t)dqp);
   for (int i = 0; i < nb; ++i)
@@ -1283,7 +1287,8 @@ static int sep_init(pnfam_ctx* c, const double* phi) {
   d_idx.release();
   d_bad.release();
   CK(err);
-  c->sep = bad == 0;
+  const int ng = std::max(1, std::min(B.nzf, 128 / ngh));
+  c->sep = bad == 0 && sep_dens_smem<double>(ngh, ng, B.nzf) <= SEP_SMEM_MAX;
   return PNFAM_OK;
 }
 
@@ -1307,8 +1312,9 @@ static int sep_operator(pnfam_ctx* c) {
     CK(upload(d.offs, s.offs.data(), s.offs.size()));
     CK(upload(d.ubeg, s.ubeg.data(), s.ubeg.size()));
     CK(upload(d.order, s.order.data(), s.order.size()));
-    CK(upload(d.items, s.items.data(), s.items.size()));
-    CK(upload(d.warps, s.warps.data(), s.warps.size()));
+    const std::vector<int> items = sep_item_columns(s.items);
+    CK(upload(d.items, items.data(), items.size()));
+    for (int h = 0; h < 2; ++h) CK(upload(d.warps[h], s.warps[h].data(), s.warps[h].size()));
   }
   const long long ngl = c->sepb.ngl, nf = (long long)c->seps[0].units.size();
   c->sep_gpair[0] = 2 * ngl * nf * 2 * SH_N;
@@ -1325,11 +1331,14 @@ static SepDev<T> sep_dev(const pnfam_ctx* c, const T* factors, T* g) {
   S.r = reinterpret_cast<const typename Vec2<T>::t*>(factors);
   S.z = factors + B.r.size(); S.v = S.z + B.z.size(); S.y = S.v + B.v.size(); S.e = S.y + B.y.size();
   S.lam = S.e + B.e.size(); S.sgn = S.lam + B.lam.size();
+  const T* rt = S.sgn + B.sgn.size();
+  S.rt = reinterpret_cast<const typename Vec2<T>::t*>(rt + (rt - factors) % 2); S.nrow = B.nrow;
   SepStructDev* to[5] = {&S.f, &S.k[0], &S.k[1], &S.d[0], &S.d[1]};
   for (int k = 0; k < 5; ++k) {
     const auto& d = c->d_seps[k];
-    *to[k] = {d.units.p, d.ents.p, d.rows.p, d.offs.p, d.ubeg.p, d.order.p, d.items.p, d.warps.p,
-              (int)c->seps[k].units.size(), (int)c->seps[k].warps.size()};
+    const SepStruct& s = c->seps[k];
+    *to[k] = {d.units.p, d.ents.p, d.rows.p, d.offs.p, d.ubeg.p, d.order.p, d.items.p, {d.warps[0].p, d.warps[1].p},
+              (int)s.items.size(), s.umax, (int)s.units.size(), {(int)s.warps[0].size(), (int)s.warps[1].size()}};
   }
   S.gstride = c->sep_gstride; S.gpair[0] = c->sep_gpair[0]; S.gpair[1] = c->sep_gpair[1];
   S.g = g; S.list = nullptr; S.act = nullptr; S.n = 0;
@@ -1339,7 +1348,7 @@ static SepDev<T> sep_dev(const pnfam_ctx* c, const T* factors, T* g) {
 // densities, mean field and projection of the points flagged in act (FP64) or listed in
 // c->d_actlist (FP32, nact of them)
 template <class T, class Tic, class Toc>
-static int sep_field(pnfam_ctx* c, int P, int nact, const int* act, const T* rsp, T* dpart, T* mf, T* hsp,
+static int sep_field(pnfam_ctx* c, int P, int nact, const int* act, const T* rsp, T* dpart, T* hsp,
                      cudaStream_t st, Tic&& tic, Toc&& toc) {
   constexpr bool f32 = std::is_same<T, float>::value;
   SepDev<T> S;
@@ -1354,29 +1363,37 @@ static int sep_field(pnfam_ctx* c, int P, int nact, const int* act, const T* rsp
   tic();
   const int lv = f32 ? live_begin(c, st) : -1;
   const unsigned nunit = (unsigned)(S.f.nu + S.k[0].nu + S.k[1].nu);
-  auto threads = [&](int npt) { return std::min(256, (4 * npt * ngl + 31) / 32 * 32); };
-  // two points per CTA in FP32 fill its last warp (160 threads at 20 radial points, not 80
-  // of 96): 0.23 against 0.24 ms for 40 points at N_sh = 16
-  if (f32 && S.n > 1)
-    k_sep_radial<T, 2><<<dim3(nunit, (S.n + 1) / 2), threads(2), 0, st>>>(S, rsp, c->nxy);
-  else
-    k_sep_radial<T, 1><<<dim3(nunit, S.n), threads(1), 0, st>>>(S, rsp, c->nxy);
+  // points per CTA: see k_sep_radial
+  const int npt = f32 ? (S.n >= 4 ? 4 : 1) : (nact > 1 && 2 * nact > P ? 2 : 1);
+  const int thr = std::min(192, ((f32 ? 2 : 4) * npt * ngl + 31) / 32 * 32);
+  const dim3 rgrid(nunit, (S.n + npt - 1) / npt);
+  if (npt == 4) k_sep_radial<T, f32 ? 4 : 1><<<rgrid, thr, 0, st>>>(S, rsp, c->nxy);
+  else if (npt == 2) k_sep_radial<T, f32 ? 1 : 2><<<rgrid, thr, 0, st>>>(S, rsp, c->nxy);
+  else k_sep_radial<T, 1><<<rgrid, thr, 0, st>>>(S, rsp, c->nxy);
   const int ng = std::max(1, std::min(S.nzf, 128 / ngh));
-  k_sep_density<T><<<dim3(ngl, 8, S.n), ngh * ng, sep_dens_smem<T>(ngh, ng), st>>>(S, ng, dpart);
+  k_sep_density<T><<<dim3(ngl, 8, S.n), ngh * ng, sep_dens_smem<T>(ngh, ng, S.nzf), st>>>(S, ng, dpart);
   if (f32) live_end(c, lv, 0, st);
   CK(cudaGetLastError());
   toc(1);
   tic();
-  k_meanfield<T><<<dim3((c->nghl + 31) / 32, 2 * P), 32, 0, st>>>(c->devbasis<T>(), 4, dpart, mf, act);
-  CK(cudaGetLastError());
-  toc(2);
-  tic();
   const int lw = f32 ? live_begin(c, st) : -1;
-  k_sep_field<T><<<dim3(ngl, 8, S.n), 128, sep_field_smem<T>(ngh), st>>>(S, mf);
-  const int nw = 2 * S.f.nwarp + S.d[0].nwarp + S.d[1].nwarp;
-  k_sep_project<T><<<dim3((nw + 3) / 4, S.n), 128, 0, st>>>(S, hsp, c->nxy);
+  k_sep_field<T><<<dim3(ngl, 8, S.n), 128, sep_field_smem<T>(ngh), st>>>(S, c->devbasis<T>(), dpart);
+  // FP32 on a large basis (a unit of F fills a warp) keeps an item in one lane
+  const bool whole = f32 && (long long)c->seps[0].items.size() >= 32LL * S.f.nu;
+  const int h = whole ? 0 : 1, nw = S.f.nwarp[h] * 2 + S.d[0].nwarp[h] + S.d[1].nwarp[h];
+  // eight warps per CTA, one while that would leave SMs without any
+  const bool stage = (long long)nw * nact >= 8LL * 4 * c->nsm &&
+                     sep_project_smem<T>(ngl, S.nrow, 8, true) <= (size_t)SEP_SMEM_MAX;
+  const int wpc = stage ? 8 : 1;
+  const dim3 pgrid((nw + wpc - 1) / wpc, S.n);
+  const size_t psm = sep_project_smem<T>(ngl, S.nrow, wpc, stage);
+  constexpr int SPL1 = f32 ? 1 : SEP_SPL;
+  if (whole && stage) k_sep_project<T, SPL1, true><<<pgrid, 32 * wpc, psm, st>>>(S, hsp, c->nxy);
+  else if (whole) k_sep_project<T, SPL1, false><<<pgrid, 32 * wpc, psm, st>>>(S, hsp, c->nxy);
+  else if (stage) k_sep_project<T, SEP_SPL, true><<<pgrid, 32 * wpc, psm, st>>>(S, hsp, c->nxy);
+  else k_sep_project<T, SEP_SPL, false><<<pgrid, 32 * wpc, psm, st>>>(S, hsp, c->nxy);
   if (f32) live_end(c, lw, 1, st);
-  c->launches += 5;
+  c->launches += 4;
   CK(cudaGetLastError());
   toc(3);
   return PNFAM_OK;
@@ -1420,7 +1437,7 @@ static int residual_t(pnfam_ctx* c, int P, int nact, const int* act, bool timed,
                                    !(c->pair32 && c->pg_on && c->pg_built && nact >= c->pg_min)
                              : c->sep64;
   if (unit_sums) {
-    if ((rc = sep_field<T>(c, P, nact, act, rsp, dpart, mf, hsp, st, tic, toc))) return rc;
+    if ((rc = sep_field<T>(c, P, nact, act, rsp, dpart, hsp, st, tic, toc))) return rc;
     return residual_k2<T>(c, P, nact, act, st, tic, toc);
   }
   DensCallT<T> d0, d1;
@@ -1897,7 +1914,17 @@ extern "C" int pnfam_gpu_init(const pnfam_basis_t* basis, const double* Ep, cons
       cudaFuncSetAttribute(k_sep_field<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SEP_SMEM_MAX) !=
           cudaSuccess ||
       cudaFuncSetAttribute(k_sep_field<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SEP_SMEM_MAX) !=
-          cudaSuccess) {
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_density<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, SEP_SMEM_MAX) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_density<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SEP_SMEM_MAX) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_project<double, SEP_SPL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SEP_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_project<float, SEP_SPL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SEP_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_project<float, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SEP_SMEM_MAX) != cudaSuccess) {
     delete c;
     return fail(PNFAM_ECUDA, "pnfam_gpu_init: cannot configure shared memory");
   }
@@ -2826,7 +2853,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian(pnfam_ctx_t* c, const double* re_rho_p
   const int* act = c->d_active.p;
   if (c->sep) {
     auto none = [](int = 0) {};
-    if ((rc = sep_field<double>(c, 1, 1, act, c->d_rsp.p, c->d_dpart.p, c->d_mf.p, c->d_hsp.p, c->stream, none, none)))
+    if ((rc = sep_field<double>(c, 1, 1, act, c->d_rsp.p, c->d_dpart.p, c->d_hsp.p, c->stream, none, none)))
       return rc;
   } else {
     DensCall d0, d1;
@@ -2881,7 +2908,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* c, const double* re
   const int* act = c->d_active.p;
   if (c->sep32) {
     auto none = [](int = 0) {};
-    if ((rc = sep_field<float>(c, 1, 1, act, c->d_rsp32.p, c->d_dpart32.p, c->d_mf32.p, c->d_hsp32.p, c->stream, none,
+    if ((rc = sep_field<float>(c, 1, 1, act, c->d_rsp32.p, c->d_dpart32.p, c->d_hsp32.p, c->stream, none,
                                none)))
       return rc;
   } else {

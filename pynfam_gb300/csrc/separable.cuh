@@ -22,7 +22,9 @@
 // against 3.5 GFLOP of the sums over the whole mesh.  Measured there, per point, FP64
 // (nine points): densities 0.14 ms against 2.2 ms, projection 0.18 against 2.7 ms; FP32
 // (40 points): 23 and 18 us against 39 and 41 us of the pair-tensor GEMMs, whose operand
-// (12 GB) is not needed; errors against FP64 2e-7 instead of 8e-6.
+// (12 GB) is not needed; errors against FP64 2e-7 instead of 8e-6.  (First form; with the
+// staging that the kernels below describe 16 and 17 us in FP32, 24 points: radial sums
+// 264, z sums 111, unit fields 121, projection 298 us.)
 //
 // The factors are recovered from the basis functions that the caller passes
 // (sep_factors) and every value of the products is compared with them (k_sep_check);
@@ -239,20 +241,43 @@ struct SepUnit { int cls, nz, nzp, ent0, nent; };   // spin class 2 (s_a < 0) + 
 // ngp of its column states, the elements in the order (column state, row state)
 struct SepEnt { int ng, ngp, row0, rowp0, el0, seg, segp; };
 
-enum { SEP_GC = 5, SEP_STAGE = 512 };   // column states per projection item; elements staged at a time
+// column states per projection item; elements, parts and rows staged at a time
+enum { SEP_GC = 5, SEP_STAGE = 256, SEP_STAGE_E = 64, SEP_STAGE_R = SEP_STAGE + SEP_STAGE_E };
 
 struct SepItem {        // one row state against up to SEP_GC column states of a unit
   int seg, segp, ja, row, n;
   int jb[SEP_GC], rowp[SEP_GC], off[SEP_GC];
 };
-struct SepWarp { int unit, item0, nitem, nmax; };   // 32 items of one unit (nmax: their largest n)
+// the same as columns of integers, so that the lanes of a warp read them side by side:
+// [SI_N][items]
+enum { SI_SEG = 0, SI_SEGP, SI_JA, SI_ROW, SI_CNT, SI_JB, SI_ROWP = SI_JB + SEP_GC, SI_OFF = SI_ROWP + SEP_GC,
+       SI_N = SI_OFF + SEP_GC };
+inline std::vector<int> sep_item_columns(const std::vector<SepItem>& it) {
+  const size_t n = it.size();
+  std::vector<int> v(SI_N * n);
+  for (size_t k = 0; k < n; ++k) {
+    const SepItem& i = it[k];
+    const int head[5] = {i.seg, i.segp, i.ja, i.row, i.n};
+    for (int j = 0; j < 5; ++j) v[j * n + k] = head[j];
+    for (int j = 0; j < SEP_GC; ++j) {   // absent column states repeat the first
+      const int q = j < i.n ? j : 0;
+      v[(SI_JB + j) * n + k] = i.jb[q];
+      v[(SI_ROWP + j) * n + k] = i.rowp[q];
+      v[(SI_OFF + j) * n + k] = i.off[q];
+    }
+  }
+  return v;
+}
+struct SepWarp { int unit, item0, nitem, nmax; };   // up to 32 / SPL items of one unit (nmax: their largest n)
+enum { SEP_SPL = 4 };   // lanes that share an item where the kernel splits its radial points
 
 struct SepStruct {
   std::vector<SepUnit> units;      // by (class, n_z', n_z)
   std::vector<SepEnt> ents;
   std::vector<int> rows, offs, ubeg, order;   // ubeg [4][nzf + 1]: first unit of (class, n_z'); order: largest first
   std::vector<SepItem> items;
-  std::vector<SepWarp> warps;
+  std::vector<SepWarp> warps[2];   // 32 items, 32 / SEP_SPL items
+  int umax = 0;                    // most units of one (class, n_z')
 };
 
 // cols, offs_: the block structure; items: also the projection's items.  false when a
@@ -316,11 +341,15 @@ inline bool sep_structure(const SepBasis& B, int nb, const int* db, const int* s
           // items of one size next to each other, so that a warp's lanes run the same loop
           std::stable_sort(S.items.begin() + item0, S.items.end(),
                            [](const SepItem& x, const SepItem& y) { return x.n > y.n; });
-          for (int k = item0; k < (int)S.items.size(); k += 32)
-            S.warps.push_back({(int)S.units.size(), k, std::min(32, (int)S.items.size() - k), S.items[k].n});
+          for (int h = 0; h < 2; ++h) {
+            const int n = h ? 32 / SEP_SPL : 32;
+            for (int k = item0; k < (int)S.items.size(); k += n)
+              S.warps[h].push_back({(int)S.units.size(), k, std::min(n, (int)S.items.size() - k), S.items[k].n});
+          }
         }
         S.units.push_back(u);
       }
+      S.umax = std::max(S.umax, (int)S.units.size() - S.ubeg.back());
       if (zp == nzf - 1) S.ubeg.push_back((int)S.units.size());
     }
   auto work = [&](const SepUnit& u) {
@@ -331,7 +360,8 @@ inline bool sep_structure(const SepBasis& B, int nb, const int* db, const int* s
   std::vector<long long> w;
   for (const SepUnit& u : S.units) { S.order.push_back((int)w.size()); w.push_back(work(u)); }
   std::stable_sort(S.order.begin(), S.order.end(), [&](int x, int y) { return w[x] > w[y]; });
-  std::stable_sort(S.warps.begin(), S.warps.end(), [](const SepWarp& x, const SepWarp& y) { return x.nmax > y.nmax; });
+  for (auto& w : S.warps)
+    std::stable_sort(w.begin(), w.end(), [](const SepWarp& x, const SepWarp& y) { return x.nmax > y.nmax; });
   return true;
 }
 
@@ -354,15 +384,15 @@ struct SepStructDev {
   const SepUnit* units;
   const SepEnt* ents;
   const int *rows, *offs, *ubeg, *order;
-  const SepItem* items;
-  const SepWarp* warps;
-  int nu, nwarp;
+  const int* items;                // [SI_N][nitem]
+  const SepWarp* warps[2];
+  int nitem, umax, nu, nwarp[2];   // umax: most units of one (class, n_z')
 };
 
 template <class T>
 struct SepDev {
-  int ngh, ngl, nzf, nghl;
-  const typename Vec2<T>::t* r;   // [nrow][ngl] (R, R')
+  int ngh, ngl, nzf, nghl, nrow;
+  const typename Vec2<T>::t *r, *rt;   // (R, R') as [nrow][ngl] and as [ngl][nrow]
   const T *z, *v, *y, *e, *lam, *sgn;
   SepStructDev f, k[2], d[2];     // F; pairing densities (X^T, Y^T); pairing fields (X, Y)
   // unit sums of one point: per call the F units [ngl][nu][SH_N][2 planes], then per
@@ -411,141 +441,204 @@ __global__ void __launch_bounds__(128) k_sep_check(const double* __restrict__ ph
 
 // ---------------------------------------------------------------------------
 // densities 1: the radial sums of every unit.  A CTA takes one unit and NPT points; a
-// thread one radial point and one column (point, call, plane).  The unit's elements are
-// gathered into shared memory and every part is summed over its row states, then over
-// its column states.  FP64: bound by the FP64 pipe (2 DFMA per element, radial point
-// and column); FP32: by shared-memory and L1 loads.
+// thread one radial point and CT columns of (point, call, plane).  The unit's elements
+// are gathered into shared memory (all columns of an element by one thread, so that
+// 4 NPT loads are in flight) and every part is summed over its row states, then over its
+// column states.  FP64 is bound by the FP64 pipe (about 3.7 DFMA per element, radial
+// point and column at N_sh = 16, where a part has 14 elements): one column per thread,
+// two points where they fill the last warp (160 threads at 20 radial points, not 80 of
+// 96).  FP32 is bound by shared-memory and L1 reads: a thread takes Re and Im, so that a
+// radial function is read once for both and the elements as pairs, and four points share
+// a CTA.
 // grid (units of F, X^T and Y^T; point groups)
 // ---------------------------------------------------------------------------
-template <class T, int KT, bool NORMAL>
+template <class T, int KT, int CT, bool NORMAL>
 __device__ __forceinline__ void sep_tile(const typename Vec2<T>::t* __restrict__ r, const int* __restrict__ rows,
-                                         const int* __restrict__ rowsp, int ng, const T* s, int ld, int ir, int ngl,
-                                         T (&o)[4]) {
-  T t0[KT], t1[KT];
+                                         const int* __restrict__ rowsp, int ng, const T* s, int ld, int ir, T (&o)[4][CT]) {
+  T t0[KT][CT], t1[KT][CT];
 #pragma unroll
-  for (int k = 0; k < KT; ++k) t0[k] = t1[k] = T(0);
-#pragma unroll 3
+  for (int k = 0; k < KT; ++k)
+#pragma unroll
+    for (int c = 0; c < CT; ++c) t0[k][c] = t1[k][c] = T(0);
+#pragma unroll 2
   for (int g = 0; g < ng; ++g) {
-    const typename Vec2<T>::t ra = r[rows[g] * ngl + ir];
+    const typename Vec2<T>::t ra = r[rows[g] + ir];
 #pragma unroll
     for (int k = 0; k < KT; ++k) {
-      const T x = s[(k * ng + g) * ld];
-      t0[k] = fma(ra.x, x, t0[k]);
-      if (NORMAL) t1[k] = fma(ra.y, x, t1[k]);
+      T x[CT];
+      if constexpr (CT == 2) {
+        const typename Vec2<T>::t v = *reinterpret_cast<const typename Vec2<T>::t*>(s + (k * ng + g) * ld);
+        x[0] = v.x; x[1] = v.y;
+      } else {
+        x[0] = s[(k * ng + g) * ld];
+      }
+#pragma unroll
+      for (int c = 0; c < CT; ++c) {
+        t0[k][c] = fma(ra.x, x[c], t0[k][c]);
+        if (NORMAL) t1[k][c] = fma(ra.y, x[c], t1[k][c]);
+      }
     }
   }
 #pragma unroll
   for (int k = 0; k < KT; ++k) {
-    const typename Vec2<T>::t rb = r[rowsp[k] * ngl + ir];
-    o[0] = fma(rb.x, t0[k], o[0]);
-    if (NORMAL) {
-      o[1] = fma(rb.x, t1[k], o[1]);
-      o[2] = fma(rb.y, t0[k], o[2]);
-      o[3] = fma(rb.y, t1[k], o[3]);
+    const typename Vec2<T>::t rb = r[rowsp[k] + ir];
+#pragma unroll
+    for (int c = 0; c < CT; ++c) {
+      o[0][c] = fma(rb.x, t0[k][c], o[0][c]);
+      if (NORMAL) {
+        o[1][c] = fma(rb.x, t1[k][c], o[1][c]);
+        o[2][c] = fma(rb.y, t0[k][c], o[2][c]);
+        o[3][c] = fma(rb.y, t1[k][c], o[3][c]);
+      }
     }
   }
 }
 
-template <class T, int NPT, bool NORMAL>
+template <class T, int NPT, int CT, bool NORMAL>
 __device__ __forceinline__ void sep_radial_unit(const SepDev<T>& S, const SepStructDev& X, int ui, int call,
-                                                const T* __restrict__ rsp, long long nxy, T* sx) {
-  constexpr int NC = (NORMAL ? 4 : 2) * NPT;   // columns: (point, call, plane) or (point, plane)
+                                                const T* __restrict__ rsp, long long nxy, T* sx, SepEnt* sent,
+                                                int* srow) {
+  constexpr int NP1 = NORMAL ? 4 : 2, NC = NP1 * NPT;   // columns of a point (call, plane) or (plane), of the CTA
+  constexpr int NN = NORMAL ? SG_N : 1;
   const SepUnit u = X.units[ui];
   const int ngl = S.ngl;
   const SepEnt* en = X.ents + u.ent0;
-  for (int t0 = 0; t0 < ngl * NC; t0 += blockDim.x) {
-    const int t = t0 + threadIdx.x, ir = t % ngl, col = t / ngl;
-    const bool live = t < ngl * NC;
-    T acc[SG_N];
+  const int nthr = ngl * (NC / CT);
+  for (int t0 = 0; t0 < nthr; t0 += blockDim.x) {
+    const int t = t0 + threadIdx.x, ir = t % ngl, col = t / ngl * CT;
+    const bool live = t < nthr;
+    T acc[NN][CT];
 #pragma unroll
-    for (int k = 0; k < SG_N; ++k) acc[k] = T(0);
+    for (int k = 0; k < NN; ++k)
+#pragma unroll
+      for (int c = 0; c < CT; ++c) acc[k][c] = T(0);
     for (int e0 = 0; e0 < u.nent;) {
-      // the parts that fit the staging buffer together
-      int e1 = e0, nel = 0;
-      while (e1 < u.nent && nel + en[e1].ng * en[e1].ngp <= SEP_STAGE) { nel += en[e1].ng * en[e1].ngp; ++e1; }
-      const int el0 = en[e0].el0;
+      // the parts that fit the staging buffers together (a part of n x n' elements has
+      // n + n' <= n n' + 1 rows)
+      int e1 = e0, nel = 0, nrow = 0;
+      while (e1 < u.nent && e1 < e0 + SEP_STAGE_E) {
+        const int n = en[e1].ng * en[e1].ngp;
+        if (nel + n > SEP_STAGE) break;
+        nel += n;
+        nrow += en[e1].ng + en[e1].ngp;
+        ++e1;
+      }
+      const int el0 = en[e0].el0, row0 = en[e0].row0;
       __syncthreads();
-      for (int c = 0; c < NC; ++c) {
-        const int p = sep_point(S, blockIdx.y * NPT + (NORMAL ? c >> 2 : c >> 1));
-        if (p < 0) {
-          for (int k = threadIdx.x; k < nel; k += blockDim.x) sx[k * NC + c] = T(0);
-          continue;
+      for (int k = threadIdx.x; k < nrow; k += blockDim.x) srow[k] = X.rows[row0 + k] * ngl;
+      for (int k = threadIdx.x; k < e1 - e0; k += blockDim.x) sent[k] = en[e0 + k];
+      for (int k = threadIdx.x; k < nel; k += blockDim.x) {
+        const long long off = X.offs[el0 + k];
+        T v[NC];
+#pragma unroll
+        for (int i = 0; i < NPT; ++i) {
+          const int p = sep_point(S, blockIdx.y * NPT + i);
+          const T* src = rsp + (long long)max(p, 0) * 8 * nxy + off;
+#pragma unroll
+          for (int c = 0; c < NP1; ++c) {
+            const int quad = NORMAL ? (c >= 2 ? 3 : 0) : (call ? 2 : 1);
+            v[NP1 * i + c] = p < 0 ? T(0) : src[((c & 1) * 4 + quad) * nxy];
+          }
         }
-        const int quad = NORMAL ? ((c >> 1) & 1 ? 3 : 0) : (call ? 2 : 1);
-        const T* src = rsp + ((long long)p * 2 + (c & 1)) * 4 * nxy + (long long)quad * nxy;
-        for (int k = threadIdx.x; k < nel; k += blockDim.x) sx[k * NC + c] = src[X.offs[el0 + k]];
+#pragma unroll
+        for (int c = 0; c < NC; c += 2) {
+          typename Vec2<T>::t w;
+          w.x = v[c]; w.y = v[c + 1];
+          *reinterpret_cast<typename Vec2<T>::t*>(sx + k * NC + c) = w;
+        }
       }
       __syncthreads();
       if (live) {
         for (int e = e0; e < e1; ++e) {
-          const SepEnt q = en[e];
-          const int *ra = X.rows + q.row0, *rb = X.rows + q.rowp0;
+          const SepEnt q = sent[e - e0];
+          const int *ra = srow + (q.row0 - row0), *rb = srow + (q.rowp0 - row0);
           const T* s = sx + (q.el0 - el0) * NC + col;
-          T o[4] = {T(0), T(0), T(0), T(0)};
+          T o[4][CT];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int c = 0; c < CT; ++c) o[i][c] = T(0);
           int k = 0;
           if (sizeof(T) == 4)
-            for (; k + 4 <= q.ngp; k += 4) sep_tile<T, 4, NORMAL>(S.r, ra, rb + k, q.ng, s + k * q.ng * NC, NC, ir, ngl, o);
-          for (; k + 2 <= q.ngp; k += 2) sep_tile<T, 2, NORMAL>(S.r, ra, rb + k, q.ng, s + k * q.ng * NC, NC, ir, ngl, o);
-          if (k < q.ngp) sep_tile<T, 1, NORMAL>(S.r, ra, rb + k, q.ng, s + k * q.ng * NC, NC, ir, ngl, o);
-          const T sg = S.sgn[q.seg] * S.sgn[q.segp];
-          acc[SG_RR] = fma(sg, o[0], acc[SG_RR]);
-          if (NORMAL) {
-            const T la = S.lam[q.seg] * sg, lb = S.lam[q.segp];
-            acc[SG_DR] = fma(sg, o[1], acc[SG_DR]);
-            acc[SG_RD] = fma(sg, o[2], acc[SG_RD]);
-            acc[SG_DD] = fma(sg, o[3], acc[SG_DD]);
-            acc[SG_ARR] = fma(la, o[0], acc[SG_ARR]);
-            acc[SG_BRR] = fma(lb * sg, o[0], acc[SG_BRR]);
-            acc[SG_ABRR] = fma(la * lb, o[0], acc[SG_ABRR]);
-            acc[SG_BDR] = fma(lb * sg, o[1], acc[SG_BDR]);
-            acc[SG_ARD] = fma(la, o[2], acc[SG_ARD]);
+            for (; k + 4 <= q.ngp; k += 4)
+              sep_tile<T, 4, CT, NORMAL>(S.r, ra, rb + k, q.ng, s + k * q.ng * NC, NC, ir, o);
+          for (; k + 2 <= q.ngp; k += 2)
+            sep_tile<T, 2, CT, NORMAL>(S.r, ra, rb + k, q.ng, s + k * q.ng * NC, NC, ir, o);
+          if (k < q.ngp) sep_tile<T, 1, CT, NORMAL>(S.r, ra, rb + k, q.ng, s + k * q.ng * NC, NC, ir, o);
+          const T sg = S.sgn[q.seg] * S.sgn[q.segp], la = S.lam[q.seg] * sg, lb = S.lam[q.segp];
+#pragma unroll
+          for (int c = 0; c < CT; ++c) {
+            acc[SG_RR][c] = fma(sg, o[0][c], acc[SG_RR][c]);
+            if constexpr (NORMAL) {
+              acc[SG_DR][c] = fma(sg, o[1][c], acc[SG_DR][c]);
+              acc[SG_RD][c] = fma(sg, o[2][c], acc[SG_RD][c]);
+              acc[SG_DD][c] = fma(sg, o[3][c], acc[SG_DD][c]);
+              acc[SG_ARR][c] = fma(la, o[0][c], acc[SG_ARR][c]);
+              acc[SG_BRR][c] = fma(lb * sg, o[0][c], acc[SG_BRR][c]);
+              acc[SG_ABRR][c] = fma(la * lb, o[0][c], acc[SG_ABRR][c]);
+              acc[SG_BDR][c] = fma(lb * sg, o[1][c], acc[SG_BDR][c]);
+              acc[SG_ARD][c] = fma(la, o[2][c], acc[SG_ARD][c]);
+            }
           }
         }
       }
       e0 = e1;
     }
     if (!live) continue;
-    const int p = sep_point(S, blockIdx.y * NPT + (NORMAL ? col >> 2 : col >> 1));
+    const int p = sep_point(S, blockIdx.y * NPT + col / NP1);
     if (p < 0) continue;
     T* g = S.g + p * S.gstride;
-    if (NORMAL) {
+    if constexpr (NORMAL) {
       const T y = S.y[ir];
       g += ((long long)(((col >> 1) & 1) * ngl + ir) * X.nu + ui) * (2 * SH_N) + (col & 1);
-      g[2 * SG_RR] = acc[SG_RR];
-      g[2 * SG_DR] = acc[SG_DR];
-      g[2 * SG_RD] = acc[SG_RD];
-      g[2 * SG_DD] = acc[SG_DD];
-      g[2 * SG_ARR] = y * acc[SG_ARR];
-      g[2 * SG_BRR] = y * acc[SG_BRR];
-      g[2 * SG_ABRR] = y * y * acc[SG_ABRR];
-      g[2 * SG_BDR] = y * acc[SG_BDR];
-      g[2 * SG_ARD] = y * acc[SG_ARD];
+#pragma unroll
+      for (int c = 0; c < CT; ++c) {
+        g[2 * SG_RR + c] = acc[SG_RR][c];
+        g[2 * SG_DR + c] = acc[SG_DR][c];
+        g[2 * SG_RD + c] = acc[SG_RD][c];
+        g[2 * SG_DD + c] = acc[SG_DD][c];
+        g[2 * SG_ARR + c] = y * acc[SG_ARR][c];
+        g[2 * SG_BRR + c] = y * acc[SG_BRR][c];
+        g[2 * SG_ABRR + c] = y * y * acc[SG_ABRR][c];
+        g[2 * SG_BDR + c] = y * acc[SG_BDR][c];
+        g[2 * SG_ARD + c] = y * acc[SG_ARD][c];
+      }
     } else {
-      g[S.gpair[call] + ((long long)ir * X.nu + ui) * 2 + (col & 1)] = acc[SG_RR];
+      g += S.gpair[call] + ((long long)ir * X.nu + ui) * 2 + (col & 1);
+#pragma unroll
+      for (int c = 0; c < CT; ++c) g[c] = acc[0][c];
     }
   }
 }
 
 template <class T, int NPT>
-__global__ void __launch_bounds__(256) k_sep_radial(const __grid_constant__ SepDev<T> S, const T* __restrict__ rsp,
+__global__ void __launch_bounds__(192, sizeof(T) == 4 ? 5 : 1) k_sep_radial(const __grid_constant__ SepDev<T> S, const T* __restrict__ rsp,
                                                     long long nxy) {
+  constexpr int CT = sizeof(T) == 4 ? 2 : 1;
   __shared__ __align__(16) T sx[SEP_STAGE * 4 * NPT];
+  __shared__ SepEnt sent[SEP_STAGE_E];
+  __shared__ int srow[SEP_STAGE_R];
   if (NPT == 1 && sep_point(S, blockIdx.y) < 0) return;
   int b = blockIdx.x;
-  if (b < S.f.nu) { sep_radial_unit<T, NPT, true>(S, S.f, S.f.order[b], 0, rsp, nxy, sx); return; }
+  if (b < S.f.nu) { sep_radial_unit<T, NPT, CT, true>(S, S.f, S.f.order[b], 0, rsp, nxy, sx, sent, srow); return; }
   b -= S.f.nu;
-  if (b < S.k[0].nu) sep_radial_unit<T, NPT, false>(S, S.k[0], S.k[0].order[b], 0, rsp, nxy, sx);
-  else sep_radial_unit<T, NPT, false>(S, S.k[1], S.k[1].order[b - S.k[0].nu], 1, rsp, nxy, sx);
+  if (b < S.k[0].nu) sep_radial_unit<T, NPT, CT, false>(S, S.k[0], S.k[0].order[b], 0, rsp, nxy, sx, sent, srow);
+  else sep_radial_unit<T, NPT, CT, false>(S, S.k[1], S.k[1].order[b - S.k[0].nu], 1, rsp, nxy, sx, sent, srow);
 }
 
 // ---------------------------------------------------------------------------
 // densities 2: the z sums of one radial point, call and class, folded into the class's
 // share of the 28 densities: dpart [P][2 calls][4 classes][2 ND][nghl].  A thread takes
-// one z point and every ng-th n_z' (ng groups of ngh threads).
+// one z point and every ng-th n_z' (ng groups of ngh threads); the unit sums of ng n_z'
+// at a time are staged in shared memory (read from L2 as they are used they stalled 75 %
+// of the issue slots in FP32).
 // grid (ngl, 2 calls x 4 classes, points), ngh * ng threads
 // ---------------------------------------------------------------------------
 template <class T>
-__host__ __device__ inline size_t sep_dens_smem(int ngh, int ng) { return (size_t)ng * 34 * ngh * sizeof(T); }
+__host__ __device__ inline size_t sep_dens_smem(int ngh, int ng, int nzf) {
+  const size_t stage = (size_t)ng * nzf * (SH_N + 1) * 2, red = (size_t)ng * 34 * ngh;
+  return ((stage > red ? stage : red) + (size_t)nzf * 2 * ngh) * sizeof(T) + (size_t)2 * ng * nzf * sizeof(int);
+}
 
 template <class T>
 __global__ void __launch_bounds__(256) k_sep_density(const __grid_constant__ SepDev<T> S, int ng,
@@ -554,19 +647,38 @@ __global__ void __launch_bounds__(256) k_sep_density(const __grid_constant__ Sep
   if (p < 0) return;
   const int ir = blockIdx.x, call = blockIdx.y >> 2, cls = blockIdx.y & 3;
   const int ngh = S.ngh, nzf = S.nzf;
+  using V2 = typename Vec2<T>::t;
   extern __shared__ __align__(16) unsigned char smraw[];
-  T* red = reinterpret_cast<T*>(smraw);   // [ng][34][ngh]
+  T* sz = reinterpret_cast<T*>(smraw);      // [nzf][2][ngh]
+  T* red = sz + (size_t)nzf * 2 * ngh;      // [ng][34][ngh], after the sums
+  V2* sg = reinterpret_cast<V2*>(red);      // [units of ng n_z'][SH_N]
+  V2* sk = sg + (size_t)ng * nzf * SH_N;    // [pairing units of ng n_z']
+  const size_t nred = (size_t)ng * 34 * ngh, nst = (size_t)ng * nzf * (SH_N + 1) * 2;
+  int* snz = reinterpret_cast<int*>(red + (nst > nred ? nst : nred));   // n_z of the staged units
+  int* snk = snz + ng * nzf;
   const int ih = threadIdx.x % ngh, grp = threadIdx.x / ngh;
+  const SepStructDev& X = S.k[call];
+  const T* gp = S.g + p * S.gstride;
+  const V2* gf = reinterpret_cast<const V2*>(gp) + (long long)(call * S.ngl + ir) * S.f.nu * SH_N;
+  const V2* gk = reinterpret_cast<const V2*>(gp + S.gpair[call]) + (long long)ir * X.nu;
   // C(q, q') at q * 4 + q', (re, im); then the pairing sum
   T C[17][2];
 #pragma unroll
   for (int k = 0; k < 17; ++k) C[k][0] = C[k][1] = T(0);
-  using V2 = typename Vec2<T>::t;
-  const T* gp = S.g + p * S.gstride;
-  for (int zp = grp; zp < nzf; zp += ng) {
-    const T Zp = S.z[(2 * zp) * ngh + ih], Zdp = S.z[(2 * zp + 1) * ngh + ih];
+  for (int i = threadIdx.x; i < nzf * 2 * ngh; i += blockDim.x) sz[i] = S.z[i];
+  for (int z0 = 0; z0 < nzf; z0 += ng) {
+    const int z1 = min(nzf, z0 + ng), zp = z0 + grp;
+    const int f0 = S.f.ubeg[cls * (nzf + 1) + z0], f1 = S.f.ubeg[cls * (nzf + 1) + z1];
+    const int k0 = X.ubeg[cls * (nzf + 1) + z0], k1 = X.ubeg[cls * (nzf + 1) + z1];
+    __syncthreads();
+    for (int i = threadIdx.x; i < (f1 - f0) * SH_N; i += blockDim.x)
+      if (i % SH_N < SG_N) sg[i] = gf[(long long)f0 * SH_N + i];
+    for (int i = threadIdx.x; i < k1 - k0; i += blockDim.x) { sk[i] = gk[k0 + i]; snk[i] = X.units[k0 + i].nz; }
+    for (int i = threadIdx.x; i < f1 - f0; i += blockDim.x) snz[i] = S.f.units[f0 + i].nz;
+    __syncthreads();
+    if (zp >= z1) continue;
+    const T Zp = sz[(2 * zp) * ngh + ih], Zdp = sz[(2 * zp + 1) * ngh + ih];
     {
-      const V2* g = reinterpret_cast<const V2*>(gp) + (long long)(call * S.ngl + ir) * S.f.nu * SH_N;
       T A[SG_N][2], D[3][2];
 #pragma unroll
       for (int k = 0; k < SG_N; ++k) A[k][0] = A[k][1] = T(0);
@@ -575,11 +687,9 @@ __global__ void __launch_bounds__(256) k_sep_density(const __grid_constant__ Sep
       const int u0 = S.f.ubeg[cls * (nzf + 1) + zp], u1 = S.f.ubeg[cls * (nzf + 1) + zp + 1];
 #pragma unroll 2
       for (int u = u0; u < u1; ++u) {
-        const int nz = S.f.units[u].nz;
-        const T Z = S.z[(2 * nz) * ngh + ih], Zd = S.z[(2 * nz + 1) * ngh + ih];
-        V2 x[SG_N];
-#pragma unroll
-        for (int k = 0; k < SG_N; ++k) x[k] = g[(long long)u * SH_N + k];
+        const int nz = snz[u - f0];
+        const T Z = sz[(2 * nz) * ngh + ih], Zd = sz[(2 * nz + 1) * ngh + ih];
+        const V2* x = sg + (u - f0) * SH_N;
 #pragma unroll
         for (int k = 0; k < SG_N; ++k) { A[k][0] = fma(Z, x[k].x, A[k][0]); A[k][1] = fma(Z, x[k].y, A[k][1]); }
         D[0][0] = fma(Zd, x[SG_RR].x, D[0][0]); D[0][1] = fma(Zd, x[SG_RR].y, D[0][1]);
@@ -599,19 +709,18 @@ __global__ void __launch_bounds__(256) k_sep_density(const __grid_constant__ Sep
       }
     }
     {
-      const SepStructDev& X = S.k[call];
-      const V2* g = reinterpret_cast<const V2*>(gp + S.gpair[call]) + (long long)ir * X.nu;
       T a0 = T(0), a1 = T(0);
       const int u0 = X.ubeg[cls * (nzf + 1) + zp], u1 = X.ubeg[cls * (nzf + 1) + zp + 1];
 #pragma unroll 4
       for (int u = u0; u < u1; ++u) {
-        const T Z = S.z[(2 * X.units[u].nz) * ngh + ih];
-        const V2 x = g[u];
+        const T Z = sz[(2 * snk[u - k0]) * ngh + ih];
+        const V2 x = sk[u - k0];
         a0 = fma(Z, x.x, a0); a1 = fma(Z, x.y, a1);
       }
       C[16][0] = fma(Zp, a0, C[16][0]); C[16][1] = fma(Zp, a1, C[16][1]);
     }
   }
+  __syncthreads();
 #pragma unroll
   for (int k = 0; k < 17; ++k) {
     red[(grp * 34 + 2 * k) * ngh + ih] = C[k][0];
@@ -647,36 +756,153 @@ __global__ void __launch_bounds__(256) k_sep_density(const __grid_constant__ Sep
 }
 
 // ---------------------------------------------------------------------------
-// projection 1: the unit fields of one radial point, call and class, from the field
-// tensor mf [P][2 calls][NMF][2 planes][nghl].  For SEP_ZC column functions at a time
-// the field is combined with Z' and Z'' into the 13 factors of Z and Z' of the row side
-// (shared memory), then a thread sums one unit and plane over the z points.
+// projection 1: the mean field of one class and the unit fields of one radial point and
+// call.  The class's 18 field components at the CTA's mesh points (k_meanfield computes
+// the same 104 of all classes) are dealt to the threads, so that the FP64 pipe works on
+// them in all CTAs and nothing of the field tensor goes through memory; then, for SEP_ZC
+// column functions at a time, the field is combined with Z' and Z'' into the 13 factors
+// of Z and Z' of the row side (shared memory) and a thread sums two units over the z
+// points, reading each factor once.
 // grid (ngl, 2 calls x 4 classes, points), 128 threads
 // ---------------------------------------------------------------------------
+// component c (q * 4 + q', 16: (0, 4), 17: pairing) of the field of class cls from the
+// densities d (pnfam_hamiltonian_blas.f90:775-1094, 1201-1208, as in k_meanfield; s: the
+// sign that changes between the two classes of same or of opposite spins)
+template <class T>
+__device__ __forceinline__ cplxT<T> sep_meanfield(int c, int cls, const T* d, int ld, const double* sc, T crho, T cs,
+                                                  T cpair, T cspair) {
+  using Z = cplxT<T>;
+  auto D = [&](int k) { return cmk<T>(d[(2 * k) * ld], d[(2 * k + 1) * ld]); };
+  auto add = [](Z a, Z b) { return cadd<T>(a, b); };
+  auto sub = [](Z a, Z b) { return cmk<T>(a.r - b.r, a.i - b.i); };
+  auto mul = [](T a, Z b) { return csc<T>(a, b); };
+  auto im = [](Z a) { return cmk<T>(-a.i, a.r); };   // i a
+  const T cdrho = sc[0], ctau = sc[1], ctj0 = sc[2], ctj1 = sc[3], ctj2 = sc[4], crdj = sc[5];
+  const T cds = sc[6], ct = sc[7], cj = sc[8], cgs = sc[9], cf = sc[10], csdj = sc[11];
+  const bool same = (cls >> 1) == (cls & 1);
+  const T s = (cls & 2) ? T(-1) : T(1), h5 = T(0.5);
+  const T e = (c == 4 || c == 8 || c == 12) ? T(-1) : T(1);   // (q', q) of (0, q): antisymmetric parts change sign
+  const T t3 = T(1) / T(3);
+  if (c == 17) {
+    const Z rb = D(D_RB), sz = D(D_SBZ), sr = D(D_SBR), sp = im(D(D_SBP));
+    switch (cls) {
+      case 0: return mul(cspair, sub(sr, sp));
+      case 1: return sub(mul(cpair, rb), mul(cspair, sz));
+      case 2: return sub(mul(-cpair, rb), mul(cspair, sz));
+      default: return mul(-cspair, add(sr, sp));
+    }
+  }
+  if (same) {
+    switch (c) {
+      case 0:
+        return add(add(mul(T(2) * crho, D(D_RHO)), mul(ctau, D(D_TAU))),
+                   mul(s, add(add(mul(T(2) * cs, D(D_SZ)), mul(ct, D(D_TZ))), mul(cf, D(D_FZ)))));
+      case 1: case 4: {
+        const Z a = add(mul(-crdj, sub(D(D_TJPZ), D(D_TJZP))), mul(-s * csdj, D(D_JP)));
+        const Z t1 = mul(ctj1, sub(D(D_TJZR), D(D_TJRZ))), t2 = mul(ctj2, add(D(D_TJRZ), D(D_TJZR)));
+        return add(a, mul(e, sub(mul(s, im(sub(t1, mul(h5, t2)))), im(mul(cj, D(D_JR))))));
+      }
+      case 2: case 8: {
+        const Z t1 = mul(ctj1, sub(D(D_TJPZ), D(D_TJZP))), t2 = mul(ctj2, add(D(D_TJPZ), D(D_TJZP)));
+        const Z a = add(mul(cj, D(D_JP)), mul(s, add(t1, mul(h5, t2))));
+        return add(a, mul(e, sub(im(mul(s * csdj, D(D_JR))), im(mul(crdj, sub(D(D_TJZR), D(D_TJRZ)))))));
+      }
+      case 3: case 12: {
+        const Z a = add(mul(-crdj, sub(D(D_TJRP), D(D_TJPR))), mul(s * T(2) * cgs, D(D_GS)));
+        const Z rr = D(D_TJRR), pp = D(D_TJPP), zz = D(D_TJZZ), rp = add(rr, pp);
+        const Z t = sub(mul(ctj0, add(rp, zz)), mul(ctj2 * t3, sub(rp, mul(T(2), zz))));
+        return sub(a, mul(e, im(add(mul(s, t), mul(cj, D(D_JZ))))));
+      }
+      case 16: return add(mul(T(2) * cdrho, D(D_RHO)), mul(s * T(2) * cds, D(D_SZ)));
+      case 6: case 9: return add(mul(csdj, D(D_SZ)), mul(s * crdj, D(D_RHO)));
+      case 7: return add(mul(s * h5 * cf, D(D_SR)), im(mul(csdj, D(D_SP))));
+      case 13: return sub(mul(s * h5 * cf, D(D_SR)), im(mul(csdj, D(D_SP))));
+      case 11: return sub(mul(-csdj, D(D_SR)), im(mul(s * h5 * cf, D(D_SP))));
+      case 14: return add(mul(-csdj, D(D_SR)), im(mul(s * h5 * cf, D(D_SP))));
+      default: {   // (1, 1), (2, 2), (3, 3)
+        const Z a = add(mul(T(4) * cdrho + ctau, D(D_RHO)), mul(s * (T(4) * cds + ct), D(D_SZ)));
+        return c == 15 ? add(a, mul(s * cf, D(D_SZ))) : a;
+      }
+    }
+  }
+  switch (c) {
+    case 0:
+      return sub(add(add(mul(T(2) * cs, D(D_SR)), mul(ct, D(D_TR))), mul(cf, D(D_FR))),
+                 im(mul(s, add(add(mul(T(2) * cs, D(D_SP)), mul(ct, D(D_TP))), mul(cf, D(D_FP))))));
+    case 1: case 4: case 2: case 8: {
+      const Z g = sub(mul(T(2) * cgs, D(D_GS)), im(mul(s * csdj, D(D_JZ))));
+      const Z rr = D(D_TJRR), pp = D(D_TJPP), zz = D(D_TJZZ), rp = D(D_TJRP), pr = D(D_TJPR);
+      const Z a1 = mul(-ctj1, sub(rp, pr)), a2 = im(mul(-ctj0, add(add(rr, pp), zz))), a3 = mul(-h5 * ctj2, add(rp, pr));
+      if (c == 1 || c == 4) {
+        const Z a4 = im(mul(ctj2 * t3, add(mul(T(-2), rr), add(pp, zz))));
+        return add(g, mul(e, add(mul(s, add(a1, a3)), add(a2, a4))));
+      }
+      const Z a5 = im(mul(ctj2 * t3, add(add(rr, mul(T(-2), pp)), zz)));
+      return add(mul(s, add(mul(e, g), add(a2, a5))), sub(a1, a3));
+    }
+    case 3: case 12: {
+      const Z f = add(mul(csdj, D(D_JP)), im(mul(s * csdj, D(D_JR))));
+      const Z t1a = mul(ctj1, sub(D(D_TJZR), D(D_TJRZ))), t2a = mul(ctj2, add(D(D_TJRZ), D(D_TJZR)));
+      const Z t1b = mul(ctj1, sub(D(D_TJPZ), D(D_TJZP))), t2b = mul(ctj2, add(D(D_TJPZ), D(D_TJZP)));
+      return add(f, mul(e, sub(mul(s, sub(t1b, mul(h5, t2b))), im(add(t1a, mul(h5, t2a))))));
+    }
+    case 16: return sub(mul(T(2) * cds, D(D_SR)), im(mul(s * T(2) * cds, D(D_SP))));
+    case 6: case 9: {
+      const Z a = add(im(mul(h5 * cf, D(D_SP))), mul(s * h5 * cf, D(D_SR)));
+      return c == 6 ? a : mul(T(-1), a);
+    }
+    case 7: return add(mul(h5 * cf, D(D_SZ)), mul(s * crdj, D(D_RHO)));
+    case 13: return sub(mul(h5 * cf, D(D_SZ)), mul(s * crdj, D(D_RHO)));
+    case 11: return sub(mul(-s * h5 * cf, D(D_SZ)), mul(crdj, D(D_RHO)));
+    case 14: return sub(mul(s * h5 * cf, D(D_SZ)), mul(crdj, D(D_RHO)));
+    default: {   // (1, 1), (2, 2), (3, 3)
+      const T k = ct + T(4) * cds;
+      const Z a = sub(mul(k, D(D_SR)), im(mul(s * k, D(D_SP))));
+      return c == 5 ? add(a, mul(cf, D(D_SR))) : c == 10 ? sub(a, im(mul(s * cf, D(D_SP)))) : a;
+    }
+  }
+}
+
 enum { SEP_ZC = 8, SEP_NX = 13 };
 template <class T>
 __host__ __device__ inline size_t sep_field_smem(int ngh) {
-  return (size_t)(18 * 2 + 1 + SEP_ZC * SEP_NX * 2) * ngh * sizeof(T);
+  const int x = SEP_ZC * SEP_NX * 2;   // the densities (2 ND) share this space
+  return (size_t)(18 * 2 + 1 + (x > 2 * ND ? x : 2 * ND)) * ngh * sizeof(T);
 }
 
+// dpart: the classes' shares of the densities, as k_sep_density leaves them
 template <class T>
-__global__ void __launch_bounds__(128) k_sep_field(const __grid_constant__ SepDev<T> S, const T* __restrict__ mf) {
+__global__ void __launch_bounds__(128) k_sep_field(const __grid_constant__ SepDev<T> S,
+                                                   const __grid_constant__ DevBasisT<T> B,
+                                                   const T* __restrict__ dpart) {
   const int p = sep_point(S, blockIdx.z);
   if (p < 0) return;
   const int ir = blockIdx.x, call = blockIdx.y >> 2, cls = blockIdx.y & 3;
   const int ngh = S.ngh, nzf = S.nzf;
-  const int sa = (cls & 2) ? -1 : 1, sb = (cls & 1) ? -1 : 1;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);     // [16 (q, q') + (0, 4) + pairing][2][ngh]
   T* sv = sm + 18 * 2 * ngh;               // [ngh]
   T* sx = sv + ngh;                        // [SEP_ZC][SEP_NX][2][ngh]
-  const T* mp = mf + ((long long)p * 2 + call) * NMF * 2 * S.nghl + ir * ngh;
-  for (int k = threadIdx.x; k < 36 * ngh; k += blockDim.x) {
-    const int ih = k % ngh, pl = (k / ngh) & 1, c = k / (2 * ngh);
-    const int slot = c < 16 ? mfslot(c >> 2, c & 3, sa, sb) : c == 16 ? mfslot(0, 4, sa, sb) : 100 + cls;
-    sm[k] = mp[((long long)slot * 2 + pl) * S.nghl + ih];
+  {
+    const T* dp = dpart + ((long long)p * 2 + call) * 4 * (2 * ND) * S.nghl + ir * ngh;
+    for (int k = threadIdx.x; k < 2 * ND * ngh; k += blockDim.x) {
+      const T* q = dp + (long long)(k / ngh) * S.nghl + k % ngh;
+      const long long ld = (long long)(2 * ND) * S.nghl;
+      sx[k] = ((q[0] + q[ld]) + (q[2 * ld] + q[3 * ld])) * (T)B.wdcori[ir * ngh + k % ngh];
+    }
+    for (int k = threadIdx.x; k < ngh; k += blockDim.x) sv[k] = S.v[ir * ngh + k];
+    __syncthreads();
+    // a warp takes one component at a time: the components' formulas differ
+    const int nh = (ngh + 31) / 32 * 32;
+    for (int k = threadIdx.x; k < 18 * nh; k += blockDim.x) {
+      const int ih = k % nh, c = k / nh, r = ir * ngh + ih;
+      if (ih >= ngh) continue;
+      const cplxT<T> f = sep_meanfield<T>(c, cls, sx + ih, ngh, B.sc, (T)B.crho[r], (T)B.cs[r], (T)B.cpair[r],
+                                          (T)B.cspair[r]);
+      sm[(2 * c) * ngh + ih] = f.r;
+      sm[(2 * c + 1) * ngh + ih] = f.i;
+    }
   }
-  for (int k = threadIdx.x; k < ngh; k += blockDim.x) sv[k] = S.v[ir * ngh + k];
   T* gp = S.g + p * S.gstride;
   const T y = S.y[ir];
   __syncthreads();
@@ -704,29 +930,36 @@ __global__ void __launch_bounds__(128) k_sep_field(const __grid_constant__ SepDe
 #undef MF_
     }
     __syncthreads();
-    {
-      const int u0 = S.f.ubeg[cls * (nzf + 1) + z0], u1 = S.f.ubeg[cls * (nzf + 1) + z1];
-      for (int k = threadIdx.x; k < 2 * (u1 - u0); k += blockDim.x) {
-        const int pl = k & 1, u = u0 + (k >> 1);
-        const SepUnit U = S.f.units[u];
-        const T* x = sx + ((long long)(U.nzp - z0) * SEP_NX * 2 + pl) * ngh;
-        const T *Z = S.z + (2 * U.nz) * ngh, *Zd = Z + ngh;
-        T h[SH_N];
+    // a thread takes the units (n_z', n_z) and (n_z', next n_z) of one plane
+    const int half = (S.f.umax + 1) / 2;
+    for (int k = threadIdx.x; k < (z1 - z0) * half * 2; k += blockDim.x) {
+      const int pl = k & 1, c = (k >> 1) / half, j = (k >> 1) % half;
+      const int ub = S.f.ubeg[cls * (nzf + 1) + z0 + c], ue = S.f.ubeg[cls * (nzf + 1) + z0 + c + 1];
+      const int u = ub + 2 * j;
+      if (u >= ue) continue;
+      const bool two = u + 1 < ue;
+      const T* x = sx + ((long long)c * SEP_NX * 2 + pl) * ngh;
+      const T *Z0 = S.z + (2 * S.f.units[u].nz) * ngh, *Z1 = S.z + (2 * S.f.units[two ? u + 1 : u].nz) * ngh;
+      T h[2][SH_N];
 #pragma unroll
-        for (int i = 0; i < SH_N; ++i) h[i] = T(0);
-#pragma unroll 2
-        for (int ih = 0; ih < ngh; ++ih) {
-          const T a = Z[ih], b = Zd[ih];
+      for (int i = 0; i < SH_N; ++i) h[0][i] = h[1][i] = T(0);
+      for (int ih = 0; ih < ngh; ++ih) {
+        const T a0 = Z0[ih], b0 = Z0[ngh + ih], a1 = Z1[ih], b1 = Z1[ngh + ih];
 #pragma unroll
-          for (int i = 0; i < SH_N; ++i) h[i] = fma(a, x[i * 2 * ngh + ih], h[i]);
-          h[SG_RR] = fma(b, x[10 * 2 * ngh + ih], h[SG_RR]);
-          h[SG_RD] = fma(b, x[11 * 2 * ngh + ih], h[SG_RD]);
-          h[SG_BRR] = fma(b, x[12 * 2 * ngh + ih], h[SG_BRR]);
+        for (int i = 0; i < SEP_NX; ++i) {
+          const T v = x[i * 2 * ngh + ih];
+          const int o = i < SH_N ? i : i == 10 ? SG_RR : i == 11 ? SG_RD : SG_BRR;
+          h[0][o] = fma(i < SH_N ? a0 : b0, v, h[0][o]);
+          if (two) h[1][o] = fma(i < SH_N ? a1 : b1, v, h[1][o]);
         }
-        h[SG_ARR] *= y; h[SG_BRR] *= y; h[SG_ABRR] *= y * y; h[SG_BDR] *= y; h[SG_ARD] *= y;
-        T* g = gp + ((long long)(call * S.ngl + ir) * S.f.nu + u) * (2 * SH_N) + pl;
+      }
 #pragma unroll
-        for (int i = 0; i < SH_N; ++i) g[2 * i] = h[i];
+      for (int w = 0; w < 2; ++w) {
+        if (w && !two) break;
+        h[w][SG_ARR] *= y; h[w][SG_BRR] *= y; h[w][SG_ABRR] *= y * y; h[w][SG_BDR] *= y; h[w][SG_ARD] *= y;
+        T* g = gp + ((long long)(call * S.ngl + ir) * S.f.nu + u + w) * (2 * SH_N) + pl;
+#pragma unroll
+        for (int i = 0; i < SH_N; ++i) g[2 * i] = h[w][i];
       }
     }
     {
@@ -746,117 +979,178 @@ __global__ void __launch_bounds__(128) k_sep_field(const __grid_constant__ SepDe
 }
 
 // ---------------------------------------------------------------------------
-// projection 2: the radial sums, hsp [P][2 planes][4 quadrants][nxy].  A warp takes 32
-// items of one unit, so that the unit's fields are read once for all lanes; a lane
-// combines them with its row state (5 products per column of Re, Im and the two calls)
-// and sums SEP_GC column states.
-// grid (ceil(warps of F, X and Y / 4), points), 128 threads
+// projection 2: the radial sums, hsp [P][2 planes][4 quadrants][nxy].  A warp takes 32 /
+// SPL items of one unit and call and first brings the unit's fields at all radial points
+// into shared memory (80 or 160 consecutive bytes per point, where reading them as they
+// are used is one load per value); a lane combines them with its row state (10 products
+// per column of Re and Im) and sums SEP_GC column states, over every SPL-th radial point.
+// SPL = 1 on large bases in FP32, where a unit's items fill warps; SPL = 4 in FP64, which
+// is bound by its pipe and so by lanes without an item (units have 9 items at N_sh = 6,
+// 52 at N_sh = 16), and on small bases, bound by the chain of a lane.  CTAs of eight
+// warps also keep the radial functions in shared memory (STAGE; not when few warps make
+// one-warp CTAs).
+// grid (warps of F x 2 calls, X and Y, over the warps of a CTA; points)
 // ---------------------------------------------------------------------------
 template <class T>
+__host__ __device__ inline size_t sep_project_smem(int ngl, int nrow, int nwarp, bool stage) {
+  return ((size_t)nwarp * ngl * SH_N + (stage ? (size_t)ngl * nrow : 0)) * 2 * sizeof(T);
+}
+
+template <class T, int SPL>
 __device__ __forceinline__ void sep_project_normal(const SepDev<T>& S, const SepWarp& W, int p, T* __restrict__ hsp,
-                                                   long long nxy, int call) {
+                                                   long long nxy, int call, const typename Vec2<T>::t* rt,
+                                                   typename Vec2<T>::t* sh) {
   using V2 = typename Vec2<T>::t;
-  const int lane = threadIdx.x & 31, ngl = S.ngl;
-  const SepItem& it = S.f.items[W.item0 + min(lane, W.nitem - 1)];
-  const T la = S.lam[it.seg], lb = S.lam[it.segp], lab = la * lb;
-  const V2* ra = S.r + it.row * ngl;
+  const int lane = threadIdx.x & 31, li = lane / SPL, part = lane % SPL, ngl = S.ngl;
+  {
+    const V2* g = reinterpret_cast<const V2*>(S.g + p * S.gstride) +
+                  ((long long)call * ngl * S.f.nu + W.unit) * SH_N;
+    const long long gs = (long long)S.f.nu * SH_N;
+    if constexpr (sizeof(T) == 4) {   // 16 bytes at a time: SH_N pairs are five of them
+      for (int k = lane; k < ngl * (SH_N / 2); k += 32)
+        reinterpret_cast<float4*>(sh)[k] =
+            reinterpret_cast<const float4*>(g + (long long)(k / (SH_N / 2)) * gs)[k % (SH_N / 2)];
+    } else {
+      for (int k = lane; k < ngl * SH_N; k += 32) sh[k] = g[(long long)(k / SH_N) * gs + k % SH_N];
+    }
+  }
+  const int* it = S.f.items + W.item0 + min(li, W.nitem - 1);
+  const long long ni = S.f.nitem;
+  const int seg = it[SI_SEG * ni], segp = it[SI_SEGP * ni], row = it[SI_ROW * ni];
+  const T la = S.lam[seg], lb = S.lam[segp], lab = la * lb;
   int rp[SEP_GC];
 #pragma unroll
-  for (int k = 0; k < SEP_GC; ++k) rp[k] = it.rowp[k < it.n ? k : 0] * ngl;
+  for (int k = 0; k < SEP_GC; ++k) rp[k] = it[(SI_ROWP + k) * ni];
   T acc[SEP_GC][2], lap[SEP_GC][2];
 #pragma unroll
-  for (int k = 0; k < SEP_GC; ++k) { acc[k][0] = acc[k][1] = lap[k][0] = lap[k][1] = T(0); }
-  const V2* g = reinterpret_cast<const V2*>(S.g + p * S.gstride) + ((long long)call * ngl * S.f.nu + W.unit) * SH_N;
-  const long long gs = (long long)S.f.nu * SH_N;
-  for (int ir = 0; ir < ngl; ++ir, g += gs) {
-    V2 h[SH_N];
-#pragma unroll
-    for (int i = 0; i < SH_N; ++i) h[i] = g[i];
-    const V2 a = ra[ir];
+  for (int k = 0; k < SEP_GC; ++k) acc[k][0] = acc[k][1] = lap[k][0] = lap[k][1] = T(0);
+  const int nmax = W.nmax;
+  __syncwarp();
+#pragma unroll 2
+  for (int ir = part; ir < ngl; ir += SPL) {
+    const V2 *r = rt + ir * S.nrow, *h = sh + ir * SH_N;
+    const V2 a = r[row];
     T vr[2], vd[2], vl[2];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-#define H_(k) (i ? h[k].y : h[k].x)
+    for (int c = 0; c < 2; ++c) {
+#define H_(k) (c ? h[k].y : h[k].x)
       const T rr = fma(lab, H_(SG_ABRR), fma(lb, H_(SG_BRR), fma(la, H_(SG_ARR), H_(SG_RR))));
       const T dr = fma(lb, H_(SG_BDR), H_(SG_DR));
       const T rd = fma(la, H_(SG_ARD), H_(SG_RD));
-      vr[i] = fma(a.x, rr, a.y * dr);
-      vd[i] = fma(a.x, rd, a.y * H_(SG_DD));
-      vl[i] = a.x * H_(SH_L);
+      vr[c] = fma(a.x, rr, a.y * dr);
+      vd[c] = fma(a.x, rd, a.y * H_(SG_DD));
+      vl[c] = a.x * H_(SH_L);
 #undef H_
     }
 #pragma unroll
     for (int k = 0; k < SEP_GC; ++k) {
-      if (k >= W.nmax) break;
-      const V2 b = S.r[rp[k] + ir];
+      if (k >= nmax) break;
+      const V2 b = r[rp[k]];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        acc[k][i] = fma(b.x, vr[i], fma(b.y, vd[i], acc[k][i]));
-        lap[k][i] = fma(b.x, vl[i], lap[k][i]);
+      for (int c = 0; c < 2; ++c) {
+        acc[k][c] = fma(b.x, vr[c], fma(b.y, vd[c], acc[k][c]));
+        lap[k][c] = fma(b.x, vl[c], lap[k][c]);
       }
     }
   }
-  if (lane >= W.nitem) return;
-  const T s = T(2) * S.sgn[it.seg] * S.sgn[it.segp], ea = S.e[it.ja];
+  const T s = T(2) * S.sgn[seg] * S.sgn[segp], ea = S.e[it[SI_JA * ni]];
+  const int cnt = it[SI_CNT * ni];
   T* out = hsp + (long long)p * 8 * nxy + (call ? 3 * nxy : 0);
 #pragma unroll
   for (int k = 0; k < SEP_GC; ++k) {
-    if (k >= it.n) break;
-    const T ee = ea + S.e[it.jb[k]];
+    if (k >= nmax) break;
+    const bool mine = part == 0 && li < W.nitem && k < cnt;
+    const T ee = ea + S.e[it[(SI_JB + k) * ni]];
+    const int off = it[(SI_OFF + k) * ni];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) out[(long long)i * 4 * nxy + it.off[k]] = s * fma(-ee, lap[k][i], acc[k][i]);
+    for (int c = 0; c < 2; ++c) {
+      T x = acc[k][c], y = lap[k][c];
+#pragma unroll
+      for (int o = 1; o < SPL; o *= 2) {
+        x += __shfl_xor_sync(0xffffffffu, x, o);
+        y += __shfl_xor_sync(0xffffffffu, y, o);
+      }
+      if (mine) out[c * 4 * nxy + off] = s * fma(-ee, y, x);
+    }
   }
 }
 
-template <class T>
+template <class T, int SPL>
 __device__ __forceinline__ void sep_project_pair(const SepDev<T>& S, const SepWarp& W, int call, int p,
-                                                 T* __restrict__ hsp, long long nxy) {
+                                                 T* __restrict__ hsp, long long nxy,
+                                                 const typename Vec2<T>::t* rt, typename Vec2<T>::t* sh) {
   using V2 = typename Vec2<T>::t;
   const SepStructDev& X = S.d[call];
-  const int lane = threadIdx.x & 31, ngl = S.ngl;
-  const SepItem& it = X.items[W.item0 + min(lane, W.nitem - 1)];
-  const V2* ra = S.r + it.row * ngl;
+  const int lane = threadIdx.x & 31, li = lane / SPL, part = lane % SPL, ngl = S.ngl;
+  {
+    const V2* g = reinterpret_cast<const V2*>(S.g + p * S.gstride + S.gpair[call]) + W.unit;
+    for (int k = lane; k < ngl; k += 32) sh[k] = g[(long long)k * X.nu];
+  }
+  const int* it = X.items + W.item0 + min(li, W.nitem - 1);
+  const long long ni = X.nitem;
+  const int seg = it[SI_SEG * ni], segp = it[SI_SEGP * ni], row = it[SI_ROW * ni];
   int rp[SEP_GC];
 #pragma unroll
-  for (int k = 0; k < SEP_GC; ++k) rp[k] = it.rowp[k < it.n ? k : 0] * ngl;
+  for (int k = 0; k < SEP_GC; ++k) rp[k] = it[(SI_ROWP + k) * ni];
   T acc[SEP_GC][2];
 #pragma unroll
   for (int k = 0; k < SEP_GC; ++k) acc[k][0] = acc[k][1] = T(0);
-  const V2* g = reinterpret_cast<const V2*>(S.g + p * S.gstride + S.gpair[call]) + W.unit;
+  const int nmax = W.nmax;
+  __syncwarp();
 #pragma unroll 2
-  for (int ir = 0; ir < ngl; ++ir) {
-    const V2 h = g[(long long)ir * X.nu];
-    const T a = ra[ir].x, v0 = a * h.x, v1 = a * h.y;
+  for (int ir = part; ir < ngl; ir += SPL) {
+    const V2* r = rt + ir * S.nrow;
+    const V2 h = sh[ir];
+    const T a = r[row].x, v0 = a * h.x, v1 = a * h.y;
 #pragma unroll
     for (int k = 0; k < SEP_GC; ++k) {
-      if (k >= W.nmax) break;
-      const T b = S.r[rp[k] + ir].x;
+      if (k >= nmax) break;
+      const T b = r[rp[k]].x;
       acc[k][0] = fma(b, v0, acc[k][0]);
       acc[k][1] = fma(b, v1, acc[k][1]);
     }
   }
-  if (lane >= W.nitem) return;
-  const T s = T(2) * S.sgn[it.seg] * S.sgn[it.segp];
+  const T s = T(2) * S.sgn[seg] * S.sgn[segp];
+  const int cnt = it[SI_CNT * ni];
   T* out = hsp + (long long)p * 8 * nxy + (call ? 2 : 1) * nxy;
 #pragma unroll
   for (int k = 0; k < SEP_GC; ++k) {
-    if (k >= it.n) break;
-    out[it.off[k]] = s * acc[k][0];
-    out[4 * nxy + it.off[k]] = s * acc[k][1];
+    if (k >= nmax) break;
+    const bool mine = part == 0 && li < W.nitem && k < cnt;
+    const int off = it[(SI_OFF + k) * ni];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      T v = acc[k][c];
+#pragma unroll
+      for (int o = 1; o < SPL; o *= 2) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (mine) out[c * 4 * nxy + off] = s * v;
+    }
   }
 }
 
-template <class T>
-__global__ void __launch_bounds__(128) k_sep_project(const __grid_constant__ SepDev<T> S, T* __restrict__ hsp,
+template <class T, int SPL, bool STAGE>
+__global__ void __launch_bounds__(256) k_sep_project(const __grid_constant__ SepDev<T> S, T* __restrict__ hsp,
                                                      long long nxy) {
+  using V2 = typename Vec2<T>::t;
+  constexpr int H = SPL > 1;
   const int p = sep_point(S, blockIdx.y);
   if (p < 0) return;
-  int w = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (w < 2 * S.f.nwarp) { sep_project_normal<T>(S, S.f.warps[w >> 1], p, hsp, nxy, w & 1); return; }
-  w -= 2 * S.f.nwarp;
-  if (w < S.d[0].nwarp) { sep_project_pair<T>(S, S.d[0].warps[w], 0, p, hsp, nxy); return; }
-  w -= S.d[0].nwarp;
-  if (w < S.d[1].nwarp) sep_project_pair<T>(S, S.d[1].warps[w], 1, p, hsp, nxy);
+  extern __shared__ __align__(16) unsigned char smraw[];
+  V2* sh = reinterpret_cast<V2*>(smraw) + (size_t)(threadIdx.x >> 5) * S.ngl * SH_N;
+  const V2* rt = S.rt;
+  if (STAGE) {
+    V2* sr = reinterpret_cast<V2*>(smraw) + (size_t)(blockDim.x >> 5) * S.ngl * SH_N;
+    for (int k = threadIdx.x; k < S.ngl * S.nrow; k += blockDim.x) sr[k] = rt[k];
+    rt = sr;
+    __syncthreads();
+  }
+  int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int nf = S.f.nwarp[H] * 2;
+  if (w < nf) { sep_project_normal<T, SPL>(S, S.f.warps[H][w >> 1], p, hsp, nxy, w & 1, rt, sh); return; }
+  w -= nf;
+  if (w < S.d[0].nwarp[H]) { sep_project_pair<T, SPL>(S, S.d[0].warps[H][w], 0, p, hsp, nxy, rt, sh); return; }
+  w -= S.d[0].nwarp[H];
+  if (w < S.d[1].nwarp[H]) sep_project_pair<T, SPL>(S, S.d[1].warps[H][w], 1, p, hsp, nxy, rt, sh);
 }
 
 }  // namespace pnfam

@@ -66,7 +66,13 @@ extern "C" int sep_host_check(int nb, const int* db, const int* nup, int nghl, c
               Z(u.nz, c / 4 == 3, ih) * Z(u.nzp, c % 4 == 3, ih) * g[zz[c]];
     }
   }
-  for (const SepWarp& w : S.warps) {
+  // both groupings hold the same items
+  std::vector<int> seen(S.items.size(), 0);
+  for (const SepWarp& w : S.warps[1])
+    for (int k = w.item0; k < w.item0 + w.nitem; ++k) seen[k] += w.nitem <= 32 / SEP_SPL && S.items[k].n <= w.nmax;
+  for (int k : seen)
+    if (k != 1) return 0;
+  for (const SepWarp& w : S.warps[0]) {
     const SepUnit& u = S.units[w.unit];
     for (int k = w.item0; k < w.item0 + w.nitem; ++k) {
       const SepItem& it = S.items[k];
