@@ -300,7 +300,7 @@ struct pnfam_ctx {
   DBuf<BufDescT<float>> d_bufs32;
   DBuf<double> d_xsave, d_radd;   // [P][4nxy] mixed form: anchor X_a and its FP64 image g(X_a)
   DBuf<unsigned long long> d_dmax;  // [P] max|X - X_a| of the last increment evaluation
-  DBuf<double> d_lastf, d_lastv, d_tf, d_tv;  // [P][4nxy] mixed-form Broyden: raw vectors of the last step, raw differences
+  DBuf<double> d_lastf, d_lastv, d_bcs;  // mixed-form Broyden: BroState2::v1 (v0 is d_vout), lastv, cs
   // tensor-core densities: unit tables per call, B chunks to lay out, pre-split A
   std::vector<DUnitTC> dunits[2];
   std::vector<DBChunkTC> bchunks;
@@ -419,7 +419,7 @@ struct pnfam_ctx {
     for (auto* b : fb) b->release();
     d_bufs32.release();
     d_xsave.release(); d_radd.release(); d_dmax.release();
-    d_lastf.release(); d_lastv.release(); d_tf.release(); d_tv.release();
+    d_lastf.release(); d_lastv.release(); d_bcs.release();
     d_dunits0.release(); d_dunits1.release(); d_bchunks.release(); d_achunks.release(); d_aphi.release();
     d_bsplit.release();
     for (auto* b : ib) b->release();
@@ -1175,6 +1175,7 @@ static int ensure_buffers(pnfam_ctx* c, int P, int M) {
   CK(dalloc(c->d_norm, (size_t)P));
   CK(dalloc(c->d_beta, (size_t)P * Mh * Mh));
   CK(dalloc(c->d_gamma, (size_t)P * 64));
+  CK(dalloc(c->d_bcs, (size_t)P * Mh));
   CK(dalloc(c->d_cpart, (size_t)P * c->nchunk_c * 2 * c->nops));
   CK(dalloc(c->d_wre, (size_t)P));
   CK(dalloc(c->d_wim, (size_t)P));
@@ -1705,8 +1706,6 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
   CK(dalloc(c->d_dmax, (size_t)P));
   CK(dalloc(c->d_lastf, (size_t)P * nv));
   CK(dalloc(c->d_lastv, (size_t)P * nv));
-  CK(dalloc(c->d_tf, (size_t)P * nv));
-  CK(dalloc(c->d_tv, (size_t)P * nv));
   // what the general kernels need (a separable basis: only for the pair-tensor GEMMs of
   // uncertified runs, whose point count is tuned against the per-block kernels)
   const bool general = !c->sep32 || pair;
@@ -2324,7 +2323,8 @@ static int engine_set_state(pnfam_engine* e, int p, const double* x) {
 
 // one Broyden step of every active slot: FP64 history (FP64 form), pair-arithmetic
 // history (mixed form)
-static int broyden_step(pnfam_ctx* c, pnfam_engine* e, int any_bro, const int* d_itp, const int* d_mode) {
+static int broyden_step(pnfam_ctx* c, pnfam_engine* e, int any_bro, const int* d_itp, const int* d_mode,
+                        const int* d_incr, const int* d_anch, const int* d_zero) {
   const int P = e->P, N = e->N;
   const int* act = c->d_active.p;
   BroState S;
@@ -2332,27 +2332,34 @@ static int broyden_step(pnfam_ctx* c, pnfam_engine* e, int any_bro, const int* d
   S.vin = c->d_state.p; S.vout = c->d_vout.p; S.df = c->d_df.p; S.dv = c->d_dv.p;
   S.part = c->d_bpart.p; S.nchunk = c->nchunk_bro;
   S.itp = d_itp; S.modep = d_mode;
-  BroState2 S2;
-  S2.N = N; S2.M = S.M; S2.alpha = S.alpha; S2.vin = S.vin; S2.vout = S.vout;
-  S2.df = reinterpret_cast<float2*>(c->d_df.p); S2.u = reinterpret_cast<float2*>(c->d_dv.p);
-  S2.lastf = c->d_lastf.p; S2.lastv = c->d_lastv.p; S2.tf = c->d_tf.p; S2.tv = c->d_tv.p;
-  S2.part = S.part; S2.nchunk = S.nchunk; S2.itp = d_itp; S2.modep = d_mode;
-  const bool pair = e->mixed;
   const double w0 = 0.01;
-  dim3 grid(c->nchunk_bro, P);
-  if (pair) k_bro_diff2<<<grid, 256, 0, c->stream>>>(S2, act);
-  else k_bro_diff<<<grid, 256, 0, c->stream>>>(S, act);
+  const dim3 grid(c->nchunk_bro, P);
+  if (e->mixed) {
+    BroState2 S2;
+    S2.N = N; S2.M = S.M; S2.alpha = S.alpha; S2.vin = S.vin;
+    S2.v0 = c->d_vout.p; S2.v1 = c->d_lastf.p; S2.lastv = c->d_lastv.p; S2.cs = c->d_bcs.p;
+    S2.df = reinterpret_cast<float2*>(c->d_df.p); S2.u = reinterpret_cast<float2*>(c->d_dv.p);
+    S2.part = S.part; S2.nchunk = S.nchunk; S2.itp = d_itp; S2.modep = d_mode;
+    k_bro_step2<<<grid, 256, 0, c->stream>>>(S2, e->no_res ? nullptr : c->d_hqp.p, c->d_hqp32.p, c->fops(), c->d_gfn.p,
+                                             e->o.quench_residual_int, act, d_incr, d_anch, d_zero, c->d_si.p,
+                                             c->d_xsave.p, c->d_radd.p);
+    k_bro_solve<<<P, 256, 0, c->stream>>>(S, any_bro ? 2 : 0, w0, c->d_si.p, c->d_norm.p, c->d_beta.p, c->d_gamma.p, act,
+                                          c->d_bcs.p);
+    k_bro_update2<<<dim3((unsigned)((N / 2 + 255) / 256), P), 256, 0, c->stream>>>(S2, c->d_gamma.p, c->d_si.p, act);
+    c->launches += 3;
+    CK(cudaGetLastError());
+    return PNFAM_OK;
+  }
+  k_bro_diff<<<grid, 256, 0, c->stream>>>(S, act);
   k_bro_solve<<<P, 256, 0, c->stream>>>(S, 0, w0, c->d_si.p, c->d_norm.p, c->d_beta.p, c->d_gamma.p, act);
   c->launches += 2;
   if (any_bro) {
-    if (pair) k_bro_dots2<<<grid, 256, 0, c->stream>>>(S2, c->d_norm.p, act);
-    else k_bro_dots<<<grid, 256, 0, c->stream>>>(S, c->d_norm.p, act);
+    k_bro_dots<<<grid, 256, 0, c->stream>>>(S, c->d_norm.p, act);
     k_bro_solve<<<P, 256, 0, c->stream>>>(S, 1, w0, c->d_si.p, c->d_norm.p, c->d_beta.p, c->d_gamma.p, act);
     c->launches += 2;
   }
   dim3 ug((unsigned)std::min<long long>(4096, (N + 255) / 256), P);
-  if (pair) k_bro_update2<<<ug, 256, 0, c->stream>>>(S2, c->d_gamma.p, act);
-  else k_bro_update<<<ug, 256, 0, c->stream>>>(S, c->d_gamma.p, act);
+  k_bro_update<<<ug, 256, 0, c->stream>>>(S, c->d_gamma.p, act);
   c->launches++;
   CK(cudaGetLastError());
   return PNFAM_OK;
@@ -2394,7 +2401,7 @@ static int engine_launch(pnfam_engine* e, bool block_if_idle) {
     CK(cudaEventSynchronize(e->aev[e->abatch.front().ring]));
     resume_front();
   }
-  int nact = 0, n32 = 0, n64 = 0, nanch = 0, nfresh = 0, any_bro = 0;
+  int nact = 0, n32 = 0, n64 = 0, nfresh = 0, any_bro = 0;
   for (int p = 0; p < P; ++p) {
     const bool a = e->active[p] != 0 && e->afly[p] != 1;   // steps in this launch
     const bool resumed = a && e->afly[p] == 2;            // its anchor was evaluated earlier
@@ -2424,7 +2431,7 @@ static int engine_launch(pnfam_engine* e, bool block_if_idle) {
     e->pint[3 * P + p] = a && e->mixed && e->anchor[p];
     e->pint[4 * P + p] = first && !e->x0[p];
     e->pint[5 * P + p] = a && e->fresh[p];
-    nanch += e->pint[3 * P + p]; nfresh += e->pint[5 * P + p];
+    nfresh += e->pint[5 * P + p];
     any_bro |= a && e->pint[P + p] == BRO_BROYDEN;
     if (a) e->fresh[p] = 0;
   }
@@ -2524,7 +2531,7 @@ static int engine_launch(pnfam_engine* e, bool block_if_idle) {
         CK(cudaMemcpyAsync(c->d_actlist.p, pi_ + 9 * P, sizeof(int) * n32, cudaMemcpyHostToDevice, c->stream));
         CK(cudaMemsetAsync(c->d_dmax.p, 0, sizeof(unsigned long long) * P, c->stream));
         // a few elements per thread and one atomic per block for max|X - X_a|
-        const dim3 cgrid((unsigned)std::min<long long>(256, (N + 255) / 256), P);
+        const dim3 cgrid((unsigned)std::min<long long>(256, (N + 1023) / 1024), P);
         k_to_f32<<<cgrid, 256, 0, c->stream>>>(c->d_state.p, c->d_state32.p, N, P, N, c->d_act32.p, c->d_xsave.p,
                                                c->d_dmax.p);
         if ((rc = residual_t<float>(c, P, n32, c->d_act32.p, timed, c->stream))) return rc;
@@ -2535,24 +2542,17 @@ static int engine_launch(pnfam_engine* e, bool block_if_idle) {
   }
   if (split) CK(cudaStreamWaitEvent(c->stream, c->evf[1], 0));
   tic();
-  {
+  if (!e->mixed) {   // the mixed form: k_bro_step2
     const int gx = (int)std::min<long long>(4096, (nq * nxy + 255) / 256);
-    k_green<<<dim3(gx, P), 256, 0, c->stream>>>(nxy, nq, P, e->no_res ? nullptr : c->d_hqp.p,
-                                                e->mixed ? c->d_hqp32.p : nullptr, c->fops(), c->d_gfn.p,
-                                                e->o.quench_residual_int, c->d_vout.p, act,
-                                                e->mixed ? d_incr : nullptr, c->d_radd.p, d_zero);
+    k_green<<<dim3(gx, P), 256, 0, c->stream>>>(nxy, nq, e->no_res ? nullptr : c->d_hqp.p, c->fops(), c->d_gfn.p,
+                                                e->o.quench_residual_int, c->d_vout.p, act, d_zero);
     c->launches++;
-    if (nanch) {  // new anchors: X_a = X, g(X_a) = vout
-      k_vecop<<<vgrid, 256, 0, c->stream>>>(0, 0.0, c->d_xsave.p, c->d_state.p, N, d_anch);
-      k_vecop<<<vgrid, 256, 0, c->stream>>>(0, 0.0, c->d_radd.p, c->d_vout.p, N, d_anch);
-      c->launches += 2;
-    }
     CK(cudaGetLastError());
   }
   toc(5);
   // ---- Broyden (pnfam_broyden.f90:117-216), each slot at its own iteration ----
   tic();
-  if ((rc = broyden_step(c, e, any_bro, d_itp, d_mode))) return rc;
+  if ((rc = broyden_step(c, e, any_bro, d_itp, d_mode, d_incr, d_anch, d_zero))) return rc;
   toc(6);
   tic();
   {

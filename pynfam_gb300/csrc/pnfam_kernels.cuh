@@ -18,6 +18,7 @@
 #include <stdint.h>
 
 #include "tc.cuh"
+#include "pair_arith.cuh"
 
 namespace pnfam {
 
@@ -2012,32 +2013,22 @@ __global__ void k_green_prep(long long nxy, int nq, const int* __restrict__ erow
   }
 }
 
-// vout = G o (q*H + F), G from k_green_prep.  corr[p] != 0 (increment evaluation of the
-// mixed form): H is the FP32 field of X - X_anchor (hqp32) and vout = G o (q*H) + radd[p],
-// radd = g(X_anchor) evaluated in FP64
-__global__ void k_green(long long nxy, int nq, int P, const double* __restrict__ hqp, const float* __restrict__ hqp32,
-                        const double* __restrict__ fqp, const double* __restrict__ gfn, double quench,
-                        double* __restrict__ vout, const int* __restrict__ active,
-                        const int* __restrict__ corr, const double* __restrict__ radd,
-                        const int* __restrict__ zeroh) {
+// vout = G o (q*H + F), G from k_green_prep (FP64 form; the mixed form: k_bro_step2)
+__global__ void k_green(long long nxy, int nq, const double* __restrict__ hqp, const double* __restrict__ fqp,
+                        const double* __restrict__ gfn, double quench, double* __restrict__ vout,
+                        const int* __restrict__ active, const int* __restrict__ zeroh) {
   const int p = blockIdx.y;
   if (!active[p]) return;
   const long long n2 = nq * nxy;
-  const bool cstep = corr && corr[p];
-  const bool useh = hqp && !(zeroh && zeroh[p]);  // zeroh: H = 0 (the field of X = 0)
+  const bool useh = hqp && !zeroh[p];  // zeroh: H = 0 (the field of X = 0)
   const long long o = (long long)p * 2 * n2;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n2; e += (long long)gridDim.x * blockDim.x) {
     double hr = 0.0, hi = 0.0;
-    if (useh) {
-      if (cstep) { hr = quench * (double)hqp32[o + e]; hi = quench * (double)hqp32[o + n2 + e]; }
-      else { hr = quench * hqp[o + e]; hi = quench * hqp[o + n2 + e]; }
-    }
-    if (!cstep) hr += fqp[e];
+    if (useh) { hr = quench * hqp[o + e]; hi = quench * hqp[o + n2 + e]; }
+    hr += fqp[e];
     const double gr = gfn[o + e], gi = gfn[o + n2 + e];
-    double vr = gr * hr - gi * hi, vi = gr * hi + gi * hr;
-    if (cstep) { vr += radd[o + e]; vi += radd[o + n2 + e]; }
-    vout[o + e] = vr;
-    vout[o + n2 + e] = vi;
+    vout[o + e] = gr * hr - gi * hi;
+    vout[o + n2 + e] = gr * hi + gi * hr;
   }
 }
 
@@ -2214,15 +2205,22 @@ __global__ void __launch_bounds__(256) k_bro_dots(BroState S, const double* __re
 // definite (the reference factorises it with DSYTRF/DSYTRI, pnfam_broyden.f90:190-206):
 // here L D L^T without pivoting, one barrier per column, then two triangular solves
 // by one warp
+// cs (mixed form, BroState2): the dots are those of unnormalised columns and are made
+// here; stage 2 is both stages in one launch
 __global__ void __launch_bounds__(256) k_bro_solve(BroState S, int stage, double w0, double* __restrict__ si,
                                                    double* __restrict__ norm, double* __restrict__ beta,
-                                                   double* __restrict__ gamma, const int* __restrict__ active) {
+                                                   double* __restrict__ gamma, const int* __restrict__ active,
+                                                   double* __restrict__ cs = nullptr) {
   const int p = blockIdx.x;
   if (!active[p]) return;
   const double* pt = S.part + bro_part(S.nchunk, p, 0);
   const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
   __shared__ double red[8][2];
-  if (stage == 0) {
+  __shared__ double scale[2];   // of the columns and the residual (k_bro_step2), of the update
+  const int it = S.itp[p], mode = S.modep[p];
+  int n, ipos, inext;
+  bro_slots(it, S.M, n, ipos, inext);
+  if (stage != 1) {
     double m = 0.0, s = 0.0;
     for (int c = tid; c < S.nchunk; c += blockDim.x) { m = fmax(m, pt[c]); s += pt[S.nchunk + c]; }
     for (int o = 16; o > 0; o >>= 1) {
@@ -2234,15 +2232,18 @@ __global__ void __launch_bounds__(256) k_bro_solve(BroState S, int stage, double
     if (tid == 0) {
       double mm = 0.0, ss = 0.0;
       for (int i = 0; i < 8; ++i) { mm = fmax(mm, red[i][0]); ss += red[i][1]; }
-      si[p] = mm;
       norm[p] = ss > 0.0 ? 1.0 / sqrt(ss) : 0.0;
+      if (cs && mode == BRO_BROYDEN && it >= 2) {
+        scale[0] = scalbn(1.0, -pair_scale(si[p]));
+        scale[1] = scalbn(1.0, pair_scale(mm));
+        cs[(long long)p * S.M + ipos] = norm[p] * scale[0];
+      }
+      si[p] = mm;
     }
-    return;
+    if (stage == 0) return;
+    __syncthreads();
   }
-  const int it = S.itp[p], mode = S.modep[p];
   if (mode != BRO_BROYDEN || it < 1) return;
-  int n, ipos, inext;
-  bro_slots(it, S.M, n, ipos, inext);
   __shared__ double A[64][65];
   __shared__ double x[64];
   __shared__ double dinv[2];   // 1/D of the current and the next column
@@ -2259,6 +2260,11 @@ __global__ void __launch_bounds__(256) k_bro_solve(BroState S, int stage, double
       wk += __shfl_xor_sync(0xffffffffu, wk, o);
     }
     if (l == 0) {
+      if (cs) {
+        const double ck = cs[(long long)p * M + k];
+        dd *= ck * cs[(long long)p * M + ipos];
+        wk *= ck * scale[0];
+      }
       if (k != ipos) { bp[k * M + ipos] = dd; bp[ipos * M + k] = dd; }
       x[k] = wk;
     }
@@ -2295,7 +2301,7 @@ __global__ void __launch_bounds__(256) k_bro_solve(BroState S, int stage, double
       for (int r = tid; r < c; r += 32) x[r] -= A[r][c] * gc;
       __syncwarp();
     }
-    for (int k = tid; k < n; k += 32) gamma[(long long)p * 64 + k] = x[k];
+    for (int k = tid; k < n; k += 32) gamma[(long long)p * 64 + k] = cs ? x[k] * cs[(long long)p * M + k] * scale[1] : x[k];
   }
 }
 
@@ -2339,139 +2345,184 @@ __global__ void __launch_bounds__(256) k_bro_update(BroState S, const double* __
 // k_bro_update.
 // ---------------------------------------------------------------------------
 struct BroState2 {
-  int N;              // vector length (4*nxy)
+  int N;              // vector length (2*nq*nxy, a multiple of 4)
   int M;              // history size
   double alpha;
   double* vin;        // [P][N]
-  double* vout;       // [P][N]
-  float2* df;         // [P][M][N] finished columns df_k
-  float2* u;          // [P][M][N] finished columns u_k = dv_k + alpha*df_k
-  double* lastf;      // [P][N] raw vout of the previous step
-  double* lastv;      // [P][N] raw vin of the previous step
-  double* tf;         // [P][N] vout - lastf of this step (unnormalised)
-  double* tv;         // [P][N] vin - lastv of this step
+  double* v0;         // [P][N] this step's residual vout - vin and the previous step's by
+  double* v1;         // [P][N] turns: of iteration it in v0 (even) or v1 (odd)
+  double* lastv;      // [P][N] vin of the previous step
+  float2* df;         // [P][M][N] columns 2^s (res - previous res), s of k_bro_step2
+  float2* u;          // [P][M][N] columns 2^s (vin - lastv + alpha (res - previous res))
+  double* cs;         // [P][M] 2^-s / |res - previous res| of a column: what normalises it
   double* part;       // [P][BRO_NPART][nchunk]
   int nchunk;
   const int* itp;
   const int* modep;
+  __device__ double* res(int it) const { return it & 1 ? v1 : v0; }
+  __device__ const double* prev(int it) const { return it & 1 ? v0 : v1; }
 };
 
-__device__ __forceinline__ float2 pair_split(double x) {
-  const float h = __double2float_rn(x);
-  return make_float2(h, __double2float_rn(x - (double)h));
-}
-__device__ __forceinline__ double pair_value(float2 a) { return (double)a.x + (double)a.y; }
-
-// s += a*b in pair arithmetic: the exact error of the leading product (FMA) and the
-// cross terms go to the low part, the leading sum is a two-sum (rounded operations
-// that the compiler may not contract)
-__device__ __forceinline__ void pair_fma(float2& s, float2 a, float2 b) {
-  const float p = __fmul_rn(a.x, b.x);
-  float e = fmaf(a.x, b.x, -p);
-  e = fmaf(a.x, b.y, e);
-  e = fmaf(a.y, b.x, e);
-  const float t = __fadd_rn(s.x, p);
-  const float z = __fsub_rn(t, s.x);
-  const float err = __fadd_rn(__fsub_rn(s.x, __fsub_rn(t, z)), __fsub_rn(p, z));
-  s.x = t;
-  s.y = __fadd_rn(s.y, __fadd_rn(err, e));
-}
-
-// vout -= vin; max|vout|; tf = vout - lastf, tv = vin - lastv, |tf|^2
-__global__ void __launch_bounds__(256) k_bro_diff2(BroState2 S, const int* __restrict__ active) {
+// The Green's function update (as k_green) and the start of the Broyden step of a mixed-
+// form slot: vout = G o (q*H + F) or, on an increment evaluation, G o (q*H32) + g(X_a);
+// the residual vout - vin and its maximum; its difference f to the previous step's, |f|^2,
+// the new columns df and u, and the dots df_k . df_ipos and df_k . res with every column.
+// An anchor evaluation (anch) leaves X_a = vin and g(X_a) = vout.
+// grid (nchunk, P): a CTA takes BRO_CHUNK / 2 complex elements, two per thread, keeps f
+// and the residual as pairs in shared memory and then gives each warp a column in turn.
+// The columns are stored before their norm is known, scaled by the power of two that
+// brings the previous residual's maximum (si) to 1; cs carries the norm.
+// Bound by FP64 (8 operations per element) in the first iterations and by the reads of the
+// columns later.  As k_green, two copies, k_bro_diff2 and k_bro_dots2 with FP64
+// conversions, sums and normalisation these took 1.2, 2.0 and 3.6 ms for 64 points at
+// N_sh = 20 with 3 columns; in this form 3.2 ms.  k_bro_update2 there 1.5 -> 1.16 ms,
+// k_to_f32 0.78 -> 0.53 ms.
+__global__ void __launch_bounds__(256, 4) k_bro_step2(BroState2 S, const double* __restrict__ hqp,
+                                                      const float* __restrict__ hqp32, const double* __restrict__ fqp,
+                                                      const double* __restrict__ gfn, double quench,
+                                                      const int* __restrict__ active, const int* __restrict__ corr,
+                                                      const int* __restrict__ anch, const int* __restrict__ zeroh,
+                                                      const double* __restrict__ si, double* __restrict__ xsave,
+                                                      double* __restrict__ radd) {
   const int p = blockIdx.y;
   if (!active[p]) return;
-  __shared__ double sh[32];
-  const int it = S.itp[p], mode = S.modep[p];
-  const bool upd = mode == BRO_BROYDEN && it >= 2;
-  const long long o = (long long)p * S.N;
-  double mx = 0.0, nn = 0.0;
-  const int e0 = blockIdx.x * BRO_CHUNK, e1 = min(S.N, e0 + BRO_CHUNK);
-  for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    const double vi = S.vin[o + e];
-    const double v = S.vout[o + e] - vi;
-    S.vout[o + e] = v;
-    mx = fmax(mx, fabs(v));
-    if (upd) {
-      const double f = v - S.lastf[o + e];
-      S.tf[o + e] = f;
-      S.tv[o + e] = vi - S.lastv[o + e];
-      nn = fma(f, f, nn);
-    }
-  }
-  const double m = block_max(mx, sh);
-  const double s = block_sum(nn, sh);
-  if (threadIdx.x == 0) {
-    S.part[bro_part(S.nchunk, p, 0) + blockIdx.x] = m;
-    S.part[bro_part(S.nchunk, p, 1) + blockIdx.x] = s;
-  }
-}
-
-// finish column ipos (df = tf/|tf|, u = tv/|tf| + alpha*df, stored as pairs) and form
-// the dots dd[k] = df_k . df_ipos and wk[k] = df_k . vout, one warp per column
-__global__ void __launch_bounds__(256) k_bro_dots2(BroState2 S, const double* __restrict__ norm,
-                                                   const int* __restrict__ active) {
-  const int p = blockIdx.y;
-  if (!active[p]) return;
-  const int it = S.itp[p], mode = S.modep[p];
-  if (mode != BRO_BROYDEN || it < 1) return;
+  constexpr int HC = BRO_CHUNK / 2;
+  __shared__ float4 sf[2][HC / 2], sv[2][HC / 2];   // [Re, Im][pairs of elements]
+  __shared__ double sn[256];
+  __shared__ unsigned long long sm[8];
+  const int it = S.itp[p], mode = S.modep[p], n2 = S.N / 2;
   int iu, ipos, inext;
   bro_slots(it, S.M, iu, ipos, inext);
-  const bool upd = it >= 2;
-  __shared__ float2 sf[BRO_CHUNK], sv[BRO_CHUNK];
+  const bool upd = mode == BRO_BROYDEN && it >= 2;
+  const bool cstep = corr[p] != 0, useh = hqp && !zeroh[p], an = anch[p] != 0;
   const long long o = (long long)p * S.N;
+  const int t = threadIdx.x, w = t >> 5, l = t & 31;
+  const int e0 = blockIdx.x * HC, e = e0 + 2 * t;   // n2 is even: both elements or none
+  const int s = upd ? pair_scale(si[p]) : 0;
   float2* dfp = S.df + (long long)p * S.M * S.N;
-  float2* up = S.u + (long long)p * S.M * S.N;
-  const long long base = (long long)blockIdx.x * BRO_CHUNK;
-  const int len = (int)min((long long)BRO_CHUNK, (long long)S.N - base);
-  const double sc = upd ? norm[p] : 0.0;
-  for (int i = threadIdx.x; i < BRO_CHUNK; i += blockDim.x) {
-    float2 f2 = make_float2(0.f, 0.f), v2 = f2;
-    if (i < len) {
-      const long long e = base + i;
-      if (upd) {
-        const double fn = S.tf[o + e] * sc;
-        f2 = pair_split(fn);
-        dfp[(long long)ipos * S.N + e] = f2;
-        up[(long long)ipos * S.N + e] = pair_split(fma(S.alpha, fn, S.tv[o + e] * sc));
+  unsigned long long mx = 0;
+  double nn = 0.0;
+  float4 f4[2], v4[2];
+#pragma unroll
+  for (int c = 0; c < 2; ++c) f4[c] = v4[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (e < n2) {
+    auto ld2 = [](const double* q) { return *reinterpret_cast<const double2*>(q); };
+    auto st2 = [](double* q, double a, double b) { *reinterpret_cast<double2*>(q) = make_double2(a, b); };
+    double h[2][2] = {{0.0, 0.0}, {0.0, 0.0}};   // [Re, Im][element]
+    if (useh) {
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (cstep) {
+          const float2 q = *reinterpret_cast<const float2*>(hqp32 + o + (c ? n2 : 0) + e);
+          h[c][0] = f64_of(q.x);
+          h[c][1] = f64_of(q.y);
+        } else {
+          const double2 q = ld2(hqp + o + (c ? n2 : 0) + e);
+          h[c][0] = q.x;
+          h[c][1] = q.y;
+        }
+        if (quench != 1.0) { h[c][0] *= quench; h[c][1] *= quench; }
       }
-      v2 = pair_split(S.vout[o + e]);
     }
-    sf[i] = f2;
-    sv[i] = v2;
+    if (!cstep) {
+      const double2 q = ld2(fqp + e);
+      h[0][0] += q.x;
+      h[0][1] += q.y;
+    }
+    const double2 gr = ld2(gfn + o + e), gi = ld2(gfn + o + n2 + e);
+    double v[2][2];
+    v[0][0] = gr.x * h[0][0] - gi.x * h[1][0];
+    v[1][0] = gr.x * h[1][0] + gi.x * h[0][0];
+    v[0][1] = gr.y * h[0][1] - gi.y * h[1][1];
+    v[1][1] = gr.y * h[1][1] + gi.y * h[0][1];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const long long q = o + (c ? n2 : 0) + e;
+      if (cstep) {
+        const double2 ra = ld2(radd + q);
+        v[c][0] += ra.x;
+        v[c][1] += ra.y;
+      }
+      const double2 x = ld2(S.vin + q);
+      if (an) {
+        st2(xsave + q, x.x, x.y);
+        st2(radd + q, v[c][0], v[c][1]);
+      }
+      const double r0 = v[c][0] - x.x, r1 = v[c][1] - x.y;
+      st2(S.res(it) + q, r0, r1);
+      mx = abs_max(abs_max(mx, r0), r1);
+      if (upd) {
+        const double2 pr = ld2(S.prev(it) + q), lv = ld2(S.lastv + q);
+        const double d0 = r0 - pr.x, d1 = r1 - pr.y;
+        nn = fma(d0, d0, nn);
+        nn = fma(d1, d1, nn);
+        const float2 a = pair_split(d0, s), b = pair_split(d1, s);
+        f4[c] = make_float4(a.x, a.y, b.x, b.y);
+        const long long cq = (long long)ipos * S.N + (c ? n2 : 0) + e;
+        *reinterpret_cast<float4*>(dfp + cq) = f4[c];
+        const float2 ua = pair_split(fma(S.alpha, d0, x.x - lv.x), s), ub = pair_split(fma(S.alpha, d1, x.y - lv.y), s);
+        *reinterpret_cast<float4*>(S.u + (long long)p * S.M * S.N + cq) = make_float4(ua.x, ua.y, ub.x, ub.y);
+        const float2 va = pair_split(r0, s), vb = pair_split(r1, s);
+        v4[c] = make_float4(va.x, va.y, vb.x, vb.y);
+      }
+    }
   }
+#pragma unroll
+  for (int c = 0; c < 2; ++c) { sf[c][t] = f4[c]; sv[c][t] = v4[c]; }
+  sn[t] = nn;
+  mx = warp_abs_max(mx);
+  if (l == 0) sm[w] = mx;
   __syncthreads();
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   double* pt = S.part + bro_part(S.nchunk, p, 0) + blockIdx.x;
+  if (w == 7) {   // few FP64 sums: one warp adds the threads' values
+    double q = 0.0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q += sn[32 * i + l];
+    for (int i = 16; i > 0; i >>= 1) q += __shfl_xor_sync(0xffffffffu, q, i);
+    const unsigned long long m = warp_abs_max(l < 8 ? sm[l] : 0ULL);
+    if (l == 0) { pt[0] = __longlong_as_double((long long)m); pt[S.nchunk] = q; }
+  }
+  if (!upd) return;
+  const int half = max(0, min(HC, n2 - e0)) / 2;   // pairs of elements of this CTA, each of Re and Im
   for (int k = w; k < iu; k += 8) {
     float2 a = make_float2(0.f, 0.f), b = a;
-    if (k == ipos && upd) {   // the new column itself: its values are in shared memory
-      for (int j = l; j < len; j += 32) {
-        pair_fma(a, sf[j], sf[j]);
-        pair_fma(b, sf[j], sv[j]);
+    auto add = [&](float4 x, float4 f, float4 v) {
+      pair_fma(a, make_float2(x.x, x.y), make_float2(f.x, f.y));
+      pair_fma(b, make_float2(x.x, x.y), make_float2(v.x, v.y));
+      pair_fma(a, make_float2(x.z, x.w), make_float2(f.z, f.w));
+      pair_fma(b, make_float2(x.z, x.w), make_float2(v.z, v.w));
+    };
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (k == ipos) {   // the new column itself
+        for (int j = l; j < half; j += 32) add(sf[c][j], sf[c][j], sv[c][j]);
+        continue;
       }
-    } else {
-      const float2* fk = dfp + (long long)k * S.N + base;
-#pragma unroll 8
-      for (int j = l; j < len; j += 32) {
-        const float2 x = __ldcs(fk + j);
-        pair_fma(a, x, sf[j]);
-        pair_fma(b, x, sv[j]);
+      const float4* fk = reinterpret_cast<const float4*>(dfp + (long long)k * S.N + (c ? n2 : 0) + e0);
+      if (half == HC / 2) {
+        float4 x[HC / 64];
+#pragma unroll
+        for (int i = 0; i < HC / 64; ++i) x[i] = __ldcs(fk + l + 32 * i);
+#pragma unroll
+        for (int i = 0; i < HC / 64; ++i) add(x[i], sf[c][l + 32 * i], sv[c][l + 32 * i]);
+      } else {
+        for (int j = l; j < half; j += 32) add(__ldcs(fk + j), sf[c][j], sv[c][j]);
       }
     }
-    double ad = pair_value(a), bd = pair_value(b);
-    for (int of = 16; of > 0; of >>= 1) {
-      ad += __shfl_xor_sync(0xffffffffu, ad, of);
-      bd += __shfl_xor_sync(0xffffffffu, bd, of);
+    a = pair_warp_sum(a);
+    b = pair_warp_sum(b);
+    if (l == 0) {
+      pt[(long long)(2 + k) * S.nchunk] = pair_value(a);
+      pt[(long long)(2 + 64 + k) * S.nchunk] = pair_value(b);
     }
-    if (l == 0) { pt[(long long)(2 + k) * S.nchunk] = ad; pt[(long long)(2 + 64 + k) * S.nchunk] = bd; }
   }
 }
 
-// BRO_BROYDEN: vin += alpha*vout - sum_k gamma_k u_k; lastf = vout, lastv = vin (raw)
-// BRO_LINEAR:  vin += alpha*vout;  BRO_NOMIX: vin += vout
+// BRO_BROYDEN: vin += alpha*res - sum_k gamma_k u_k; lastv = vin.  gamma holds the
+// columns' factors and the scale of the residual (k_bro_solve)
+// BRO_LINEAR:  vin += alpha*res;  BRO_NOMIX: vin += res
 __global__ void __launch_bounds__(256) k_bro_update2(BroState2 S, const double* __restrict__ gamma,
-                                                     const int* __restrict__ active) {
+                                                     const double* __restrict__ si, const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (!active[p]) return;
   const int it = S.itp[p], mode = S.modep[p];
@@ -2482,19 +2533,24 @@ __global__ void __launch_bounds__(256) k_bro_update2(BroState2 S, const double* 
   __shared__ float2 g[64];
   if (mode == BRO_BROYDEN && (int)threadIdx.x < iu) g[threadIdx.x] = pair_split(gamma[(long long)p * 64 + threadIdx.x]);
   __syncthreads();
-  const float2* up = S.u + (long long)p * S.M * S.N;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < S.N; e += (long long)gridDim.x * blockDim.x) {
-    const double v = S.vout[o + e];
-    if (mode == BRO_NOMIX) { S.vin[o + e] += v; continue; }
-    if (mode == BRO_LINEAR) { S.vin[o + e] += S.alpha * v; continue; }
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 4
-    for (int k = 0; k < iu; ++k) pair_fma(acc, up[(long long)k * S.N + e], g[k]);
-    const double old = S.vin[o + e];
-    S.lastf[o + e] = v;
-    S.lastv[o + e] = old;
-    S.vin[o + e] = old + (S.alpha * v - pair_value(acc));
+  const int s = pair_scale(si[p]);
+  const int e = 2 * (blockIdx.x * 256 + threadIdx.x);   // N is even
+  if (e >= S.N) return;
+  const float2* up = S.u + (long long)p * S.M * S.N + e;
+  const double2 v = *reinterpret_cast<const double2*>(S.res(it) + o + e);
+  double2* vin = reinterpret_cast<double2*>(S.vin + o + e);
+  const double2 old = *vin;
+  if (mode == BRO_NOMIX) { *vin = make_double2(old.x + v.x, old.y + v.y); return; }
+  if (mode == BRO_LINEAR) { *vin = make_double2(old.x + S.alpha * v.x, old.y + S.alpha * v.y); return; }
+  float2 a = make_float2(0.f, 0.f), b = a;
+#pragma unroll 8
+  for (int k = 0; k < iu; ++k) {
+    const float4 x = __ldcs(reinterpret_cast<const float4*>(up + (long long)k * S.N));
+    pair_fma(a, make_float2(x.x, x.y), g[k]);
+    pair_fma(b, make_float2(x.z, x.w), g[k]);
   }
+  *reinterpret_cast<double2*>(S.lastv + o + e) = old;
+  *vin = make_double2(old.x + (S.alpha * v.x - pair_value(a, -s)), old.y + (S.alpha * v.y - pair_value(b, -s)));
 }
 
 // per-point vector operations, [P][n] layout:
@@ -2561,23 +2617,21 @@ __global__ void __launch_bounds__(256) k_to_f32(const double* __restrict__ in, f
                                                 unsigned long long* __restrict__ dmax = nullptr) {
   const int p = blockIdx.y;
   if (act && !act[p]) return;
-  double m = 0.0;
+  unsigned long long m = 0;
+#pragma unroll 4
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
     const double v = sub ? in[p * ld + e] - sub[p * ld + e] : in[p * ld + e];
-    m = fmax(m, fabs(v));
-    out[p * ld + e] = (float)v;
+    m = abs_max(m, v);
+    out[p * ld + e] = f32_of(v);
   }
-  if (dmax) {
-    // one atomic per block: warp maxima, then the block's (a non-negative double orders
-    // like its bit pattern)
-    __shared__ double wm[32];
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (dmax) {   // one atomic per block
+    __shared__ unsigned long long wm[8];
+    m = warp_abs_max(m);
     if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double b = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) b = fmax(b, wm[w]);
-      atomicMax(dmax + p, (unsigned long long)__double_as_longlong(b));
+    if (threadIdx.x < 32) {
+      m = warp_abs_max(threadIdx.x < 8 ? wm[threadIdx.x] : 0ULL);
+      if (threadIdx.x == 0) atomicMax(dmax + p, m);
     }
   }
 }
