@@ -252,7 +252,7 @@ int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* ctx,
  * allowed): the same computation as pnfam_gpu_calc_hamiltonian, with every
  * input and output given as a DEVICE pointer by the caller and all
  * intermediates kept in one fixed device array inside the library (about
- * 12.5 MB, held on every GPU that loads the library until the process exits).
+ * 13.8 MB, held on every GPU that loads the library until the process exits).
  * This entry point calls no cudaMalloc/cudaFree and no allocating library
  * routine.
  *

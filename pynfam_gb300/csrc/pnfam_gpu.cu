@@ -271,8 +271,10 @@ struct pnfam_ctx {
     long long floats = 0;
     bool built = false;
   } tc32[2];
-  std::vector<HTask> htasks;
-  DBuf<HTask> d_htasks;
+  std::vector<HGroup> hgroups;
+  DBuf<HGroup> d_hgroups;
+  int htiles = 0;           // tiles that the groups' chunk lengths were chosen for
+  size_t hproj_smem = 0;
   std::vector<HTaskTC> htasks_tc;   // tensor-core field projection (FP32 data)
   int tc_npmax = 16;                  // largest N of those tiles
   DBuf<HTaskTC> d_htasks_tc;
@@ -431,7 +433,7 @@ struct pnfam_ctx {
     for (auto* b : dbs) b->release();
     d_foff.release(); d_xtoff.release(); d_ytoff.release();
     d_agather.release(); d_aerow.release(); d_aecol.release(); d_afops.release();
-    d_htasks.release(); d_bufs.release(); d_htasks_tc.release(); d_actlist.release(); d_err.release();
+    d_hgroups.release(); d_bufs.release(); d_htasks_tc.release(); d_actlist.release(); d_err.release();
     for (TCSet& t : tc32) {
       for (TaskListTC& l : t.l) l.d_tasks.release();
       t.gsplit.release();
@@ -777,13 +779,18 @@ static void build_transforms(pnfam_ctx* c) {
 // the general kernels' field projection and density tasks
 static void build_field_tasks(pnfam_ctx* c) {
   const int nb = c->nb;
-  // ---- FP64 field projection tasks: spin-uniform tiles of 1024 / tn rows x tn columns ----
-  // The shape of each (block pair, spin segment) is the one that issues the fewest DFMAs:
-  // per tile, tn columns x the rows up to the warp granularity of the shape (a warp holds
-  // 64 / (tn / 2) rows and skips when they are all beyond the tile), twice (Re, Im), plus
-  // the hpsi generation (10 DFMAs per column and mesh point of each component)
-  c->htasks.clear();
+  // ---- FP64 field projection ----
+  // The mesh points of a (block pair, spin segment) are summed in chunks of 16, or of 8 where
+  // tiles of 128 rows x 8 columns would issue fewer DFMAs than 64 x 16 or 32 x 32 (per
+  // tile the columns x the rows up to the warp granularity of the shape, twice, plus the
+  // hpsi generation): a rule of an earlier tiling, kept because the chunk length is part of
+  // the result's rounding.  The tiles are cut into pieces of at most HP_ITEMS outputs and
+  // HP_ROWS rows, and pieces with the same field tensor are packed into groups.
+  c->hgroups.clear();
+  c->htiles = 0;
   auto cdiv = [](int a, int b) { return (a + b - 1) / b; };
+  struct Cut { int call, sa, mode, hr; HPiece p; };
+  std::vector<Cut> cuts;
   auto add_h = [&](int ix, int iy, int mode, int call, int outq, long long ooff) {
     const int d = c->db[ix], dc = c->db[iy], nu = c->nup[ix];
     const int seg[3] = {0, nu, d};
@@ -804,11 +811,19 @@ static void build_field_tasks(pnfam_ctx* c) {
       const int tm = 1024 / best;
       for (int a0 = seg[s]; a0 < seg[s + 1]; a0 += tm)
         for (int b0 = 0; b0 < dc; b0 += best) {
-          HTask h{};
-          h.ix = ix; h.iy = iy; h.a0 = a0; h.na = std::min(tm, seg[s + 1] - a0);
-          h.b0 = b0; h.nbc = std::min(best, dc - b0); h.sa = s == 0 ? 1 : -1;
-          h.mode = mode; h.call = call; h.outq = outq; h.tn = best; h.ooff = ooff;
-          c->htasks.push_back(h);
+          c->htiles++;
+          const int ne = std::min(a0 + tm, seg[s + 1]), be = std::min(b0 + best, dc);
+          for (int a = a0; a < ne; a += HP_ROWS) {
+            const int na = std::min<int>(HP_ROWS, ne - a), wb = HP_ITEMS / na;
+            for (int b = b0; b < be; b += wb) {
+              Cut q{call, s == 0 ? 1 : -1, mode, best == 8 ? 8 : (int)HRC, {}};
+              q.p.ja = c->st[ix] + a; q.p.na = na;
+              q.p.jb = c->st[iy] + b; q.p.nb = std::min(wb, be - b);
+              q.p.off = (long long)outq * c->nxy + ooff + a + (long long)b * d;
+              q.p.ld = d;
+              cuts.push_back(q);
+            }
+          }
         }
     }
   };
@@ -845,6 +860,35 @@ static void build_field_tasks(pnfam_ctx* c) {
     if (c->fc[i] >= 0) { add_tc(i, c->fc[i], 0, 0, 0, c->foff[i]); add_tc(i, c->fc[i], 0, 1, 3, c->foff[i]); }
     if (c->xc[i] >= 0) add_tc(i, c->xc[i], 1, 0, 1, c->xoff[i]);
     if (c->yc[i] >= 0) add_tc(i, c->yc[i], 1, 1, 2, c->yoff[i]);
+  }
+  // largest pieces first, each into the first open group of its kind that has room
+  std::stable_sort(cuts.begin(), cuts.end(), [](const Cut& x, const Cut& y) {
+    return x.mode != y.mode ? x.mode < y.mode : x.p.na * x.p.nb > y.p.na * y.p.nb;
+  });
+  std::map<std::tuple<int, int, int, int>, std::vector<size_t>> open;
+  c->hproj_smem = 0;
+  for (Cut& q : cuts) {
+    const int n = q.p.na * q.p.nb;
+    std::vector<size_t>& list = open[std::make_tuple(q.call, q.sa, q.mode, q.hr)];
+    size_t at = c->hgroups.size();
+    for (size_t i = 0; i < list.size() && at == c->hgroups.size(); ++i) {
+      const HGroup& g = c->hgroups[list[i]];
+      if (g.np < HP_PIECES && g.nitem + n <= HP_ITEMS && g.nrow + q.p.na <= HP_TAB && g.ncol + q.p.nb <= HP_TAB &&
+          hproj_fp64_smem(q.hr, q.mode, g.nrow + q.p.na, g.ncol + q.p.nb) <= HP_SMEM_FILL)
+        at = list[i];
+    }
+    if (at == c->hgroups.size()) {
+      HGroup g{};
+      g.call = q.call; g.sa = q.sa; g.mode = q.mode; g.hr = q.hr;
+      c->hgroups.push_back(g);
+      list.push_back(at);
+    }
+    HGroup& g = c->hgroups[at];
+    q.p.item0 = g.nitem;
+    g.piece[g.np++] = q.p;
+    g.nitem += n; g.nrow += q.p.na; g.ncol += q.p.nb;
+    c->hproj_smem = std::max(c->hproj_smem, hproj_fp64_smem(g.hr, g.mode, g.nrow, g.ncol));
+    if (g.np == HP_PIECES || g.nitem == HP_ITEMS) list.erase(std::find(list.begin(), list.end(), at));
   }
   // pre-split row basis functions of the projection tiles, one copy per distinct
   // (block, first row, rows)
@@ -1520,8 +1564,8 @@ static int residual_t(pnfam_ctx* c, int P, int nact, const int* act, bool timed,
       CK(cudaGetLastError());
     }
   } else {
-    dim3 grid((unsigned)c->htasks.size(), P);
-    k_hproj_fp64<<<grid, 256, hproj_fp64_smem_bytes(), st>>>(B, c->d_htasks.p, mf, hsp, nxy, act);
+    dim3 grid((unsigned)c->hgroups.size(), P);
+    k_hproj_fp64<<<grid, 256, c->hproj_smem, st>>>(B, c->d_hgroups.p, mf, hsp, nxy, act);
     c->launches++;
     CK(cudaGetLastError());
   }
@@ -1902,7 +1946,7 @@ extern "C" int pnfam_gpu_init(const pnfam_basis_t* basis, const double* Ep, cons
     return fail(PNFAM_ECUDA, "pnfam_gpu_init: stream/event creation failed");
   }
   if (cudaFuncSetAttribute(k_hproj_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)hproj_fp64_smem_bytes()) != cudaSuccess ||
+                           (int)HP_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(k_hproj_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)hproj_tc_smem_bytes(HTC_MAXN)) != cudaSuccess ||
       cudaFuncSetAttribute(k_density_tc2, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2059,7 +2103,7 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
       set.built = false;
     }
   }
-  CK(upload(c->d_htasks, c->htasks.data(), c->htasks.size()));
+  CK(upload(c->d_hgroups, c->hgroups.data(), c->hgroups.size()));
   CK(upload(c->d_htasks_tc, c->htasks_tc.data(), c->htasks_tc.size()));
   CK(upload(c->d_hptiles, c->hptiles.data(), c->hptiles.size()));
   CK(upload(c->d_dunits0, c->dunits[0].data(), c->dunits[0].size()));
@@ -2869,8 +2913,8 @@ extern "C" int pnfam_gpu_calc_hamiltonian(pnfam_ctx_t* c, const double* re_rho_p
     k_density_fp64<<<dim3((c->nghl + DRT - 1) / DRT, c->G, 2), 256, 0, c->stream>>>(B, d0, d1, c->G, c->d_dpart.p,
                                                                                    act);
     k_meanfield<<<dim3((c->nghl + 127) / 128, 2), 128, 0, c->stream>>>(B, c->G, c->d_dpart.p, c->d_mf.p, act);
-    k_hproj_fp64<<<dim3((unsigned)c->htasks.size(), 1), 256, hproj_fp64_smem_bytes(), c->stream>>>(
-        B, c->d_htasks.p, c->d_mf.p, c->d_hsp.p, nxy, act);
+    k_hproj_fp64<<<dim3((unsigned)c->hgroups.size(), 1), 256, c->hproj_smem, c->stream>>>(
+        B, c->d_hgroups.p, c->d_mf.p, c->d_hsp.p, nxy, act);
   }
   CK(cudaGetLastError());
   const int qout[8] = {0, 0, 1, 1, 3, 3, 2, 2};
@@ -3037,7 +3081,7 @@ extern "C" const char* pnfam_gpu_last_error(void) { return g_err.c_str(); }
 // allocation is not allowed): the caller passes device pointers for every
 // input and output, and all intermediates live in one file-scope device array
 // of fixed size.  Every GPU that loads this library holds that array (about
-// 12.5 MB) until the process exits.
+// 13.8 MB) until the process exits.
 // ---------------------------------------------------------------------------
 namespace {
 constexpr long long NA_MAX_NXY = 32768;   // FAM matrix elements (N_sh <= 12)
@@ -3045,6 +3089,9 @@ constexpr int NA_MAX_NGHL = 1600;         // mesh points (40 x 40)
 constexpr int NA_MAX_DQP = 1024;          // basis states incl. time-reversed partners
 constexpr int NA_MAX_NB = 64;             // blocks incl. time-reversed partners
 constexpr int NA_MAX_HTASKS = 4096;       // field-projection tiles
+// their groups: a piece that does not end a row range of its tile (two at most) has more
+// than HP_ITEMS - HP_ROWS of the 4 nxy outputs
+constexpr int NA_MAX_HGROUPS = 2 * NA_MAX_HTASKS + 4 * (int)NA_MAX_NXY / (HP_ITEMS - HP_ROWS);
 constexpr int NA_G = 2;                   // block-row groups of the density kernel
 
 constexpr size_t na_align(size_t n) { return (n + 255) / 256 * 256; }
@@ -3055,7 +3102,7 @@ constexpr size_t NA_MF = na_align(sizeof(double) * 2 * NMF * 2 * NA_MAX_NGHL);
 constexpr size_t NA_INTS = na_align(sizeof(int) * (6 * NA_MAX_NB + 1));
 constexpr size_t NA_LONGS = na_align(sizeof(long long) * 3 * NA_MAX_NB);
 constexpr size_t NA_NS = na_align(NA_MAX_DQP);
-constexpr size_t NA_TASKS = na_align(sizeof(HTask) * NA_MAX_HTASKS);
+constexpr size_t NA_TASKS = na_align(sizeof(HGroup) * NA_MAX_HGROUPS);
 constexpr size_t NA_BYTES = NA_RSP + NA_HSP + NA_DPART + NA_MF + NA_INTS + NA_LONGS + NA_NS + NA_TASKS;
 }  // namespace
 
@@ -3085,7 +3132,7 @@ int noalloc_setup(unsigned char** out) {
       return fail(PNFAM_ECUDA, std::string("pnfam_gpu_calc_hamiltonian_noalloc: cudaGetSymbolAddress: ") +
                                    cudaGetErrorString(e));
     e = cudaFuncSetAttribute(k_hproj_fp64, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)hproj_fp64_smem_bytes());
+                             (int)HP_SMEM_MAX);
     if (e != cudaSuccess)
       return fail(PNFAM_ECUDA, std::string("pnfam_gpu_calc_hamiltonian_noalloc: cudaFuncSetAttribute: ") +
                                    cudaGetErrorString(e));
@@ -3159,7 +3206,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian_noalloc(
   if (nf > NA_MAX_NXY) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_noalloc: nxy <= 32768 is the limit");
   c.nxy = nf;
   build_field_tasks(&c);
-  if ((int)c.htasks.size() > NA_MAX_HTASKS)
+  if (c.htiles > NA_MAX_HTASKS)
     return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_noalloc: more than 4096 field-projection tiles");
   unsigned char* base = nullptr;
   int rc = noalloc_setup(&base);
@@ -3172,7 +3219,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian_noalloc(
   int* ints = reinterpret_cast<int*>(base + NA_RSP + NA_HSP + NA_DPART + NA_MF);
   long long* longs = reinterpret_cast<long long*>(base + NA_RSP + NA_HSP + NA_DPART + NA_MF + NA_INTS);
   signed char* dns = reinterpret_cast<signed char*>(base + NA_RSP + NA_HSP + NA_DPART + NA_MF + NA_INTS + NA_LONGS);
-  HTask* dtasks = reinterpret_cast<HTask*>(base + NA_RSP + NA_HSP + NA_DPART + NA_MF + NA_INTS + NA_LONGS + NA_NS);
+  HGroup* dgroups = reinterpret_cast<HGroup*>(base + NA_RSP + NA_HSP + NA_DPART + NA_MF + NA_INTS + NA_LONGS + NA_NS);
   std::vector<int> hints(6 * NA_MAX_NB + 1, 0);
   std::vector<long long> hlongs(3 * NA_MAX_NB, 0);
   for (int i = 0; i < nb; ++i) {
@@ -3192,7 +3239,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian_noalloc(
   CK(cudaMemcpyAsync(ints, hints.data(), sizeof(int) * hints.size(), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(longs, hlongs.data(), sizeof(long long) * hlongs.size(), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(dns, ns.data(), (size_t)s, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(dtasks, c.htasks.data(), sizeof(HTask) * c.htasks.size(), cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(dgroups, c.hgroups.data(), sizeof(HGroup) * c.hgroups.size(), cudaMemcpyHostToDevice, st));
   // inputs in the solver's quadrant layout: plane pl at pl*4nxy, quadrant q at q*nxy
   // (0 rho_pn, 1 kappa+, 2 kappa-, 3 rho_np)
   const int qin[8] = {0, 0, 1, 1, 3, 3, 2, 2};
@@ -3216,8 +3263,7 @@ extern "C" int pnfam_gpu_calc_hamiltonian_noalloc(
   d1.kcols = ints + 5 * NA_MAX_NB; d1.koffs = longs + 2 * NA_MAX_NB;
   k_density_fp64<<<dim3((nghl + DRT - 1) / DRT, NA_G, 2), 256, 0, st>>>(B, d0, d1, NA_G, dpart, act);
   k_meanfield<<<dim3((nghl + 127) / 128, 2), 128, 0, st>>>(B, NA_G, dpart, mf, act);
-  k_hproj_fp64<<<dim3((unsigned)c.htasks.size(), 1), 256, hproj_fp64_smem_bytes(), st>>>(B, dtasks, mf, hsp, nf,
-                                                                                       act);
+  k_hproj_fp64<<<dim3((unsigned)c.hgroups.size(), 1), 256, c.hproj_smem, st>>>(B, dgroups, mf, hsp, nf, act);
   CK(cudaGetLastError());
   const int qout[8] = {0, 0, 1, 1, 3, 3, 2, 2};
   for (int k = 0; k < 8; ++k)

@@ -1595,150 +1595,155 @@ __global__ void __launch_bounds__(128) k_meanfield(DevBasisT<T> B, int G, const 
 // ---------------------------------------------------------------------------
 // field projection: out_ab = 2 sum_r sum_iy phi_iy(a,r) hpsi(iy)(r,b)
 // ---------------------------------------------------------------------------
-struct HTask {
-  int ix, iy;      // block row / column
-  int a0, na;      // row tile inside block ix (spin-uniform), na <= 1024 / tn
-  int b0, nbc;     // column tile inside block iy, nbc <= tn
+// part of an output block of the FP64 projection: na rows (of one spin) from state ja on,
+// nb columns from state jb on; output element (a, b) at off + a + b*ld of the quadrants
+struct HPiece {
+  int ja, na, jb, nb;
+  long long off;
+  int ld, item0;   // first output of the piece in its group
+};
+// pieces with the same field tensor that one CTA computes: at most HP_ITEMS outputs, one
+// per thread
+enum { HP_PIECES = 4, HP_ITEMS = 256, HP_ROWS = 64, HP_TAB = 128, HRC = 16 };
+struct HGroup {
+  int call;        // 0: pn, 1: np
   int sa;          // spin of the rows (+1/-1)
   int mode;        // 0: mean field (5 components), 1: pairing (1 component)
-  int call;        // 0: pn, 1: np
-  int outq;        // HSP quadrant 0..3 (m11, m12, m21, m22)
-  int tn, pad_;    // tile shape: (1024 / tn) rows x tn columns, tn = 32, 16 or 8
-  long long ooff;  // block offset inside the quadrant
+  int hr;          // mesh points per chunk: 16 or 8
+  int np, nrow, ncol, nitem;
+  HPiece piece[HP_PIECES];
 };
-
-#define HRC 16   // mesh points per K chunk
-
-// FP64 field projection: output tiles of TM = 1024 / TN rows x TN columns (TN = 32, 16
-// or 8, chosen per block pair from the block sizes so that little of the FP64 pipe goes
-// to padding), 2 x 2 outputs per thread; warps whose rows lie beyond the tile's na skip
-// the FMAs (the DFMA rate is the bound).  grid (ntasks, P); 256 threads; dynamic smem
-// hproj_fp64_smem_bytes()
-// mesh points per K chunk of a shape: 16, or 8 for the 128-row tiles, so that every
-// shape stays within the 94.7 KB of the 32 x 32 tiles and a CTA of the FP32 kernels
-// (pair-tensor GEMM: 128 KB) still fits beside one on an SM
-__host__ __device__ constexpr int hproj_fp64_hr(int tn) { return tn == 8 ? 8 : HRC; }
-__host__ __device__ constexpr size_t hproj_fp64_smem_tn(int tn) {
-  return (size_t)(5 * (1024 / tn) + 5 * tn + 25 * 4 + 5 * tn * 2) * hproj_fp64_hr(tn) * sizeof(double);
+// dynamic shared memory of a group: row functions, field tensor (18 component pairs: the
+// others vanish, see k_meanfield), hpsi; the padding keeps 16-byte reads of different
+// rows or columns on different banks
+__host__ __device__ constexpr size_t hproj_fp64_smem(int hr, int mode, int nrow, int ncol) {
+  return sizeof(double) * (mode == 0 ? 5 * nrow * (hr + 2) + 18 * 4 * hr + 5 * ncol * (2 * hr + 2)
+                                     : nrow * (hr + 2) + 4 * hr + ncol * (2 * hr + 2));
 }
-__host__ __device__ constexpr size_t hproj_fp64_smem_bytes() {
-  return hproj_fp64_smem_tn(8) > hproj_fp64_smem_tn(32) ? hproj_fp64_smem_tn(8) : hproj_fp64_smem_tn(32);
-}
+// groups are filled up to the first figure (5 CTAs on an SM); a single piece stays below
+// the second: 64 rows and 4 columns, or 8 and 32
+constexpr size_t HP_SMEM_FILL = 44 * 1024, HP_SMEM_MAX = 64 * 1024;
 
-template <int TN, int HR>
-__device__ __forceinline__ void hproj_fp64_tile(const DevBasis& B, const HTask& Th, const double* __restrict__ mfp,
-                                                double* __restrict__ hsp, long long nxy, int p,
-                                                unsigned char* smraw, signed char* sns) {
-  using T = double;
-  constexpr int TM = 1024 / TN, TX = TN / 2;
-  const int nghl = B.nghl;
+// FP64 field projection.  Per chunk of mesh points a CTA stages the row functions and the
+// field tensor, forms hpsi of its columns and adds each thread's output:
+//   out_ab = 2 sum_r sum_iy phi_iy(a, r) hpsi(iy)(r, b)
+// over the chunks, in each over the components, in each over the points (this order and the
+// chunk length of a block pair are part of the result: an iteration that amplifies
+// rounding repeats to the last digit).
+// Bound by the FP64 pipe (one warp instruction per 16 cycles of an SM), so the outputs are
+// dealt to the threads in one row over several block pairs: with tiles of 32 x 32, 64 x 16 or
+// 128 x 8 outputs, 2 x 2 per thread, the small blocks of N_sh = 8 left most warps without
+// rows (46 % of the pipe, 23 of 33 cycles per instruction at barriers) and formed hpsi with
+// the 7 vanishing pairs of the field tensor: 40 points there 20.2 ms, now 5.5 ms.
+// grid (ngroups, P); 256 threads; dynamic smem: the largest hproj_fp64_smem of the groups
+template <int HR>
+__device__ __forceinline__ void hproj_fp64_group(const DevBasis& B, const HGroup& g, const double* __restrict__ mfp,
+                                                 double* __restrict__ out, long long nxy, double* sm, const int* srow,
+                                                 const int* scol, int row, int col, long long off) {
+  constexpr int SA = HR + 2, SH = 2 * HR + 2;
+  const int nghl = B.nghl, nc = g.mode == 0 ? 5 : 1, nrow = g.nrow, ncol = g.ncol, tid = threadIdx.x;
   const long long ps = (long long)B.dqp * nghl;
-  const int nc = Th.mode == 0 ? 5 : 1;
-  T* sA = reinterpret_cast<T*>(smraw);     // [5][TM][HR]
-  T* sPb = sA + 5 * TM * HR;               // [5][TN][HR]
-  T* sMF = sPb + 5 * TN * HR;              // [25][2 sb][2 re/im][HR]
-  T* sH = sMF + 25 * 2 * 2 * HR;           // [5][TN][2][HR]
-  const int ja0 = B.st[Th.ix] + Th.a0, jb0 = B.st[Th.iy] + Th.b0;
-  if (threadIdx.x < TN) sns[threadIdx.x] = threadIdx.x < Th.nbc ? B.ns[jb0 + threadIdx.x] : (signed char)1;
-  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
-  // rows 2 ty, 2 ty + 1; the rows of warp w start at 64 w / TX
-  const bool rows_live = (64 * (int)(threadIdx.x >> 5)) / TX < Th.na;
-  T ar[2][2] = {{0, 0}, {0, 0}}, ai[2][2] = {{0, 0}, {0, 0}};
+  double* sA = sm;                      // [nc][nrow][SA]
+  double* sM = sA + nc * nrow * SA;     // [18 or 1][2 sb][2 re/im][HR]
+  double* sH = sM + (g.mode == 0 ? 18 : 1) * 4 * HR;   // [nc][ncol][2 re/im][HR], a column SH apart
+  double ar = 0.0, ai = 0.0;
   for (int r0 = 0; r0 < nghl; r0 += HR) {
     const int nr = min(HR, nghl - r0);
     __syncthreads();
-    for (int e = threadIdx.x; e < nc * TM * HR; e += 256) {
-      const int q = e / (TM * HR), rem = e % (TM * HR), aa = rem / HR, rr = rem % HR;
-      T va = 0;
-      if (rr < nr && aa < Th.na) va = B.phi[q * ps + (long long)(ja0 + aa) * nghl + r0 + rr];
-      sA[(q * TM + aa) * HR + rr] = va;
-    }
-    for (int e = threadIdx.x; e < nc * TN * HR; e += 256) {
-      const int q = e / (TN * HR), rem = e % (TN * HR), bb = rem / HR, rr = rem % HR;
-      T vb = 0;
-      if (rr < nr && bb < Th.nbc) vb = B.phi[q * ps + (long long)(jb0 + bb) * nghl + r0 + rr];
-      sPb[(q * TN + bb) * HR + rr] = vb;
-    }
-    if (Th.mode == 0) {
-      for (int e = threadIdx.x; e < 25 * 2 * 2 * HR; e += 256) {
-        const int pair = e / (4 * HR), rem = e % (4 * HR), sb = rem / (2 * HR), rem2 = rem % (2 * HR);
-        const int ri = rem2 / HR, rr = rem2 % HR;
-        const int iy = pair / 5, iz = pair % 5;
-        T v = 0;
-        if (rr < nr) v = mfp[((long long)mfslot(iy, iz, Th.sa, sb == 0 ? 1 : -1) * 2 + ri) * nghl + r0 + rr];
-        sMF[e] = v;
+    for (int q = 0; q < nc; ++q)
+      for (int e = tid; e < nrow * HR; e += 256) {
+        const int rr = e % HR, a = e / HR;
+        sA[(q * nrow + a) * SA + rr] = rr < nr ? B.phi[q * ps + (long long)srow[a] * nghl + r0 + rr] : 0.0;
       }
-    } else {
-      for (int e = threadIdx.x; e < 2 * 2 * HR; e += 256) {
-        const int sb = e / (2 * HR), rem = e % (2 * HR), ri = rem / HR, rr = rem % HR;
-        const int slot = 100 + (Th.sa < 0 ? 2 : 0) + sb;
-        sMF[e] = rr < nr ? mfp[((long long)slot * 2 + ri) * nghl + r0 + rr] : (T)0;
+    for (int e = tid; e < (g.mode == 0 ? 18 : 1) * 4 * HR; e += 256) {
+      const int rr = e % HR, m = e / HR, pair = m >> 2, sb = (m >> 1) & 1, ri = m & 1;
+      int slot;
+      if (g.mode == 0) {
+        const int iy = pair < 16 ? pair >> 2 : pair == 16 ? 0 : 4, iz = pair < 16 ? pair & 3 : pair == 16 ? 4 : 0;
+        slot = mfslot(iy, iz, g.sa, sb == 0 ? 1 : -1);
+      } else {
+        slot = 100 + (g.sa < 0 ? 2 : 0) + sb;
       }
+      sM[e] = rr < nr ? mfp[((long long)slot * 2 + ri) * nghl + r0 + rr] : 0.0;
     }
     __syncthreads();
-    // hpsi(iy, b, r) = sum_iz mf(iy, iz, sa, s_b)(r) phi_iz(b, r), for the tile's live columns
-    for (int e = threadIdx.x; e < nc * TN * HR; e += 256) {
-      const int iy = e / (TN * HR), rem = e % (TN * HR), bb = rem / HR, rr = rem % HR;
-      T hr = 0, hi = 0;
-      if (bb < Th.nbc) {
-        const int sb = sns[bb] > 0 ? 0 : 1;
-        if (Th.mode == 0) {
+    // hpsi(iy, b, r) = sum_iz mf(iy, iz, sa, s_b)(r) phi_iz(b, r)
+    for (int e = tid; e < ncol * HR; e += 256) {
+      const int rr = e % HR, b = e / HR, jb = scol[b];
+      const double* f = B.phi + (long long)jb * nghl + r0 + rr;
+      const double* m = sM + (B.ns[jb] > 0 ? 0 : 2 * HR) + rr;
+      double* h = sH + b * SH + rr;
+      if (g.mode == 0) {
+        double p[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) p[q] = rr < nr ? f[q * ps] : 0.0;
+#pragma unroll
+        for (int iy = 0; iy < 5; ++iy) {
+          double hr = 0.0, hi = 0.0;
 #pragma unroll
           for (int iz = 0; iz < 5; ++iz) {
-            const T f = sPb[(iz * TN + bb) * HR + rr];
-            const T* m = &sMF[((iy * 5 + iz) * 4 + sb * 2) * HR];
-            hr = fma(m[rr], f, hr); hi = fma(m[HR + rr], f, hi);
+            if (iz == 4 ? iy != 0 : iy == 4 && iz != 0) continue;   // vanishes
+            const int pair = iz == 4 ? 16 : iy == 4 ? 17 : iy * 4 + iz;
+            hr = fma(m[pair * 4 * HR], p[iz], hr);
+            hi = fma(m[pair * 4 * HR + HR], p[iz], hi);
           }
-        } else {
-          const T f = sPb[bb * HR + rr];
-          hr = sMF[(sb * 2) * HR + rr] * f; hi = sMF[(sb * 2 + 1) * HR + rr] * f;
+          h[iy * ncol * SH] = hr;
+          h[iy * ncol * SH + HR] = hi;
         }
+      } else {
+        const double p = rr < nr ? f[0] : 0.0;
+        h[0] = m[0] * p;
+        h[HR] = m[HR] * p;
       }
-      sH[((iy * TN + bb) * 2) * HR + rr] = hr;
-      sH[((iy * TN + bb) * 2 + 1) * HR + rr] = hi;
     }
     __syncthreads();
-    if (rows_live)
-    for (int q = 0; q < nc; ++q) {
-      for (int rr = 0; rr < HR; ++rr) {
-        const T a0 = sA[(q * TM + ty * 2) * HR + rr], a1 = sA[(q * TM + ty * 2 + 1) * HR + rr];
-        const T h0r = sH[((q * TN + tx * 2) * 2) * HR + rr], h0i = sH[((q * TN + tx * 2) * 2 + 1) * HR + rr];
-        const T h1r = sH[((q * TN + tx * 2 + 1) * 2) * HR + rr], h1i = sH[((q * TN + tx * 2 + 1) * 2 + 1) * HR + rr];
-        ar[0][0] = fma(a0, h0r, ar[0][0]); ai[0][0] = fma(a0, h0i, ai[0][0]);
-        ar[0][1] = fma(a0, h1r, ar[0][1]); ai[0][1] = fma(a0, h1i, ai[0][1]);
-        ar[1][0] = fma(a1, h0r, ar[1][0]); ai[1][0] = fma(a1, h0i, ai[1][0]);
-        ar[1][1] = fma(a1, h1r, ar[1][1]); ai[1][1] = fma(a1, h1i, ai[1][1]);
+    if (row >= 0)
+      for (int q = 0; q < nc; ++q) {
+        const double2* a = reinterpret_cast<const double2*>(sA + (q * nrow + row) * SA);
+        const double2* h = reinterpret_cast<const double2*>(sH + (q * ncol + col) * SH);
+#pragma unroll
+        for (int i = 0; i < HR / 2; ++i) {
+          const double2 x = a[i], u = h[i], v = h[HR / 2 + i];
+          ar = fma(x.x, u.x, ar); ai = fma(x.x, v.x, ai);
+          ar = fma(x.y, u.y, ar); ai = fma(x.y, v.y, ai);
+        }
       }
-    }
   }
-  const int ld = B.db[Th.ix];
-  T* ore = hsp + ((long long)p * 2 + 0) * 4 * nxy + (long long)Th.outq * nxy + Th.ooff;
-  T* oim = hsp + ((long long)p * 2 + 1) * 4 * nxy + (long long)Th.outq * nxy + Th.ooff;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int a = ty * 2 + i, b = tx * 2 + j;
-      if (a < Th.na && b < Th.nbc) {
-        const long long e = (Th.a0 + a) + (long long)(Th.b0 + b) * ld;
-        ore[e] = (T)2 * ar[i][j];
-        oim[e] = (T)2 * ai[i][j];
-      }
-    }
+  if (row >= 0) {
+    out[off] = 2.0 * ar;
+    out[4 * nxy + off] = 2.0 * ai;
+  }
 }
 
-__global__ void __launch_bounds__(256) k_hproj_fp64(DevBasis B, const HTask* __restrict__ tasks,
+__global__ void __launch_bounds__(256) k_hproj_fp64(DevBasis B, const HGroup* __restrict__ groups,
                                                     const double* __restrict__ mf, double* __restrict__ hsp,
                                                     long long nxy, const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (!active[p]) return;
-  const HTask Th = tasks[blockIdx.x];
+  const HGroup& g = groups[blockIdx.x];
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ signed char sns[32];
-  const double* mfp = mf + ((long long)p * 2 + Th.call) * NMF * 2 * B.nghl;
-  if (Th.tn == 8) hproj_fp64_tile<8, hproj_fp64_hr(8)>(B, Th, mfp, hsp, nxy, p, smraw, sns);
-  else if (Th.tn == 16) hproj_fp64_tile<16, hproj_fp64_hr(16)>(B, Th, mfp, hsp, nxy, p, smraw, sns);
-  else hproj_fp64_tile<32, hproj_fp64_hr(32)>(B, Th, mfp, hsp, nxy, p, smraw, sns);
+  __shared__ int srow[HP_TAB], scol[HP_TAB];   // states of the rows and columns
+  int row = -1, col = 0, r0 = 0, c0 = 0;
+  long long off = 0;
+  for (int k = 0; k < g.np; ++k) {
+    const HPiece& q = g.piece[k];
+    for (int a = threadIdx.x; a < q.na; a += 256) srow[r0 + a] = q.ja + a;
+    for (int b = threadIdx.x; b < q.nb; b += 256) scol[c0 + b] = q.jb + b;
+    const int i = (int)threadIdx.x - q.item0;
+    if (i >= 0 && i < q.na * q.nb) {
+      const int a = i % q.na, b = i / q.na;
+      row = r0 + a;
+      col = c0 + b;
+      off = q.off + a + (long long)b * q.ld;
+    }
+    r0 += q.na;
+    c0 += q.nb;
+  }
+  const double* mfp = mf + ((long long)p * 2 + g.call) * NMF * 2 * B.nghl;
+  double* out = hsp + (long long)p * 8 * nxy;
+  double* sm = reinterpret_cast<double*>(smraw);
+  if (g.hr == 8) hproj_fp64_group<8>(B, g, mfp, out, nxy, sm, srow, scol, row, col, off);
+  else hproj_fp64_group<HRC>(B, g, mfp, out, nxy, sm, srow, scol, row, col, off);
 }
 
 // ---------------------------------------------------------------------------
