@@ -679,38 +679,31 @@ __global__ void __launch_bounds__(256, sizeof(T) >= 8 ? 1 : 2) k_density(DevBasi
 }
 
 // ---------------------------------------------------------------------------
-// FP64 densities (the drop-in form and the anchors of the mixed form): a CTA of
-// 32 mesh points x 8 column lanes; each lane accumulates W for one column b over
-// chunks of DAK rows and folds it into its own 28 complex densities (registers),
-// which are summed over the 8 lanes once, at the end.  FP64 is bound by the DFMA
-// rate, so the tiles follow the blocks closely (8 columns per chunk, rows exact).
+// FP64 densities over the whole mesh: a CTA takes 32 mesh points, a warp the columns
+// b = warp, warp + 8, ... of the blocks; a lane accumulates W of its point for a column
+// over the rows, folds it into its own 28 complex densities (registers), and these are
+// summed over the 8 warps at the end (as a tree: the order is part of the result,
+// an iteration that amplifies rounding repeats to the last digit).
+// Bound by the FP64 pipe.  With 8 lanes of a warp on 8 columns and the rows staged in
+// shared memory the pipe was 83 % busy, 40 % of it with columns that a block of 1 ... 25
+// does not have and with factors 1/2 that the sums can take along; a warp of one column
+// skips what is missing and needs neither staging nor barriers.  40 points at N_sh = 8:
+// 11.5 ms before, @NEW@ ms.
 // ---------------------------------------------------------------------------
-#define DBC 8    // b columns per chunk
-#define DAK 16   // a rows per chunk
 
-__device__ __forceinline__ double red8(double v) {
-  v += __shfl_xor_sync(0xffffffffu, v, 4);
-  v += __shfl_xor_sync(0xffffffffu, v, 2);
-  v += __shfl_xor_sync(0xffffffffu, v, 1);
-  return v;
-}
-
-// grid (ceil(nghl/DRT), G, P*2 calls); block 256 = DRT r x DBC b
+// grid (ceil(nghl/DRT), G, P*2 calls); block 256 = 8 warps x DRT mesh points
 // dpart: [P][2][G][2*ND][nghl]
-__global__ void __maxnreg__(192) k_density_fp64(DevBasis B, DensCall c0, DensCall c1, int G,
-                                                      double* __restrict__ dpart, const int* __restrict__ active) {
+__global__ void __launch_bounds__(256, 1) k_density_fp64(DevBasis B, DensCall c0, DensCall c1, int G,
+                                                         double* __restrict__ dpart, const int* __restrict__ active) {
   using T = double;
   const int p = blockIdx.z >> 1, call = blockIdx.z & 1;
   if (!active[p]) return;
   const DensCall& C = call ? c1 : c0;
   const int g = blockIdx.y;
-  const int r0 = blockIdx.x * DRT;
-  const int rl = threadIdx.x >> 3, bl = threadIdx.x & 7;
+  const int w8 = threadIdx.x >> 5, l = threadIdx.x & 31;
   const int nghl = B.nghl;
-  const int r = r0 + rl;
-  const bool rok = r < nghl;
-  __shared__ T sphi[4][DAK][DRT];  // static smem: ~20 KB
-  __shared__ T srho[2][DAK][DBC];
+  const bool rok = (int)blockIdx.x * DRT + l < nghl;
+  const int r = rok ? blockIdx.x * DRT + l : nghl - 1;   // lanes past the mesh repeat its last point
   T al[2 * ND];   // this lane's densities at mesh point r
 #pragma unroll
   for (int k = 0; k < 2 * ND; ++k) al[k] = 0;
@@ -718,67 +711,42 @@ __global__ void __maxnreg__(192) k_density_fp64(DevBasis B, DensCall c0, DensCal
   const T h5 = (T)0.5, two = (T)2;
 
 #define ACC(k, re, im) { al[2 * (k)] += (re); al[2 * (k) + 1] += (im); }
+// with a factor that is exact: 1/2 or 2, and the sign s
+#define ACCF(k, f, re, im) { al[2 * (k)] = fma((f), (re), al[2 * (k)]); al[2 * (k) + 1] = fma((f), (im), al[2 * (k) + 1]); }
 
   // ---------------- normal densities ----------------
   for (int ix = g; ix < B.nb; ix += G) {
     const int iy = C.rcols[ix];
     if (iy < 0) continue;
     const int d = B.db[ix], dc = B.db[iy], nu = B.nup[ix];
-    const int sa = B.st[ix], sb = B.st[iy];
+    const T* phi = B.phi + (long long)B.st[ix] * nghl + r;
     const T* rho = C.rho + (long long)p * C.rho_sp + C.roffs[ix];
-    for (int b0 = 0; b0 < dc; b0 += DBC) {
-      const int b = b0 + bl;
+    for (int b = w8; b < dc; b += 8) {
+      const T *cr = rho + (long long)b * d, *ci = cr + C.rho_spl;
       T w[2][4][2];
 #pragma unroll
       for (int s = 0; s < 2; ++s)
 #pragma unroll
         for (int q = 0; q < 4; ++q) { w[s][q][0] = 0; w[s][q][1] = 0; }
-      for (int a0 = 0; a0 < d; a0 += DAK) {
-        const int na = min(DAK, d - a0);
-        for (int e = threadIdx.x; e < 4 * DAK * DRT; e += 256) {
-          const int q = e / (DAK * DRT), rem = e % (DAK * DRT), aa = rem / DRT, rr = rem % DRT;
-          T v = 0;
-          if (aa < na && r0 + rr < nghl) v = B.phi[q * ps + (long long)(sa + a0 + aa) * nghl + r0 + rr];
-          sphi[q][aa][rr] = v;
-        }
-        for (int e = threadIdx.x; e < 2 * DAK * DBC; e += 256) {
-          const int pl = e / (DAK * DBC), rem = e % (DAK * DBC), aa = rem / DBC, bb = rem % DBC;
-          T v = 0;
-          if (aa < na && b0 + bb < dc) v = rho[(long long)pl * C.rho_spl + (a0 + aa) + (long long)(b0 + bb) * d];
-          srho[pl][aa][bb] = v;
-        }
-        __syncthreads();
-        // spin-up rows first: split the chunk at the spin boundary
-        const int nup_here = max(0, min(na, nu - a0));
-        for (int aa = 0; aa < nup_here; ++aa) {
-          const T re = srho[0][aa][bl], im = srho[1][aa][bl];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {   // spin-up rows first
+#pragma unroll 4
+        for (int a = s ? nu : 0; a < (s ? d : nu); ++a) {
+          const T re = cr[a], im = ci[a];
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            const T f = sphi[q][aa][rl];
-            w[0][q][0] = fma(f, re, w[0][q][0]); w[0][q][1] = fma(f, im, w[0][q][1]);
+            const T f = phi[q * ps + (long long)a * nghl];
+            w[s][q][0] = fma(f, re, w[s][q][0]); w[s][q][1] = fma(f, im, w[s][q][1]);
           }
         }
-        for (int aa = nup_here; aa < na; ++aa) {
-          const T re = srho[0][aa][bl], im = srho[1][aa][bl];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const T f = sphi[q][aa][rl];
-            w[1][q][0] = fma(f, re, w[1][q][0]); w[1][q][1] = fma(f, im, w[1][q][1]);
-          }
-        }
-        __syncthreads();
       }
-      // epilogue: contributions of column b at mesh point r
-      T P0 = 0, P1 = 0, P2 = 0, P3 = 0, sg = 0;
-      const bool ok = rok && b < dc;
-      if (ok) {
-        const int jb = sb + b;
-        P0 = B.phi[0 * ps + (long long)jb * nghl + r];
-        P1 = B.phi[1 * ps + (long long)jb * nghl + r];
-        P2 = B.phi[2 * ps + (long long)jb * nghl + r];
-        P3 = B.phi[3 * ps + (long long)jb * nghl + r];
-        sg = (T)B.ns[jb];
-      }
+      // contributions of column b at mesh point r
+      const int jb = B.st[iy] + b;
+      const T P0 = B.phi[0 * ps + (long long)jb * nghl + r];
+      const T P1 = B.phi[1 * ps + (long long)jb * nghl + r];
+      const T P2 = B.phi[2 * ps + (long long)jb * nghl + r];
+      const T P3 = B.phi[3 * ps + (long long)jb * nghl + r];
+      const T sg = (T)B.ns[jb];
       const int si = (sg > 0) ? 0 : 1;  // same-spin set of wfa
       // select S (same spin as b) and O (opposite)
       T Sr[4], Si[4], Or[4], Oi[4];
@@ -786,26 +754,26 @@ __global__ void __maxnreg__(192) k_density_fp64(DevBasis B, DensCall c0, DensCal
       for (int q = 0; q < 4; ++q) {
         Sr[q] = si == 0 ? w[0][q][0] : w[1][q][0]; Si[q] = si == 0 ? w[0][q][1] : w[1][q][1];
         Or[q] = si == 0 ? w[1][q][0] : w[0][q][0]; Oi[q] = si == 0 ? w[1][q][1] : w[0][q][1];
-        if (!ok) { Sr[q] = Si[q] = Or[q] = Oi[q] = 0; }
       }
       const T sig = (sg < 0) ? (T)1 : (T)-1;  // +1 if b is spin down
+      const T hs = h5 * sg, hg = h5 * sig;
       T xr, xi;
       // diagonal in spin
       xr = Sr[0] * P0; xi = Si[0] * P0;
       ACC(D_RHO, xr, xi);
       ACC(D_SZ, sg * xr, sg * xi);
-      xr = h5 * (Sr[0] * P2 + Sr[2] * P0); xi = h5 * (Si[0] * P2 + Si[2] * P0);
-      ACC(D_JP, xr, xi);
-      ACC(D_TJPZ, sg * xr, sg * xi);
+      xr = Sr[0] * P2 + Sr[2] * P0; xi = Si[0] * P2 + Si[2] * P0;
+      ACCF(D_JP, h5, xr, xi);
+      ACCF(D_TJPZ, hs, xr, xi);
       xr = Sr[1] * P1 + Sr[2] * P2 + Sr[3] * P3; xi = Si[1] * P1 + Si[2] * P2 + Si[3] * P3;
       ACC(D_TAU, xr, xi);
       ACC(D_TZ, sg * xr, sg * xi);
-      xr = h5 * (Sr[0] * P1 - Sr[1] * P0); xi = h5 * (Si[0] * P1 - Si[1] * P0);
-      ACC(D_JR, -xi, xr);
-      ACC(D_TJRZ, -sg * xi, sg * xr);
-      xr = h5 * (Sr[0] * P3 - Sr[3] * P0); xi = h5 * (Si[0] * P3 - Si[3] * P0);
-      ACC(D_JZ, -xi, xr);
-      ACC(D_TJZZ, -sg * xi, sg * xr);
+      xr = Sr[0] * P1 - Sr[1] * P0; xi = Si[0] * P1 - Si[1] * P0;
+      ACCF(D_JR, h5, -xi, xr);
+      ACCF(D_TJRZ, hs, -xi, xr);
+      xr = Sr[0] * P3 - Sr[3] * P0; xi = Si[0] * P3 - Si[3] * P0;
+      ACCF(D_JZ, h5, -xi, xr);
+      ACCF(D_TJZZ, hs, -xi, xr);
       // gs: diagonal part + off-diagonal parts
       {
         T gr = sg * (Sr[0] * P3 + Sr[3] * P0), gi = sg * (Si[0] * P3 + Si[3] * P0);
@@ -814,19 +782,19 @@ __global__ void __maxnreg__(192) k_density_fp64(DevBasis B, DensCall c0, DensCal
         ACC(D_GS, gr, gi);
       }
       {
-                T fr = h5 * sg * (Sr[1] * P3 + Sr[3] * P1), fi = h5 * sg * (Si[1] * P3 + Si[3] * P1);
+        T fr = h5 * sg * (Sr[1] * P3 + Sr[3] * P1), fi = h5 * sg * (Si[1] * P3 + Si[3] * P1);
         fr += Or[1] * P1 + sig * h5 * (Or[1] * P2 - Or[2] * P1);
         fi += Oi[1] * P1 + sig * h5 * (Oi[1] * P2 - Oi[2] * P1);
         ACC(D_FR, fr, fi);
       }
       {
         // fp += i*sg*(S2P3 - S3P2)/2 + i*(sig*O2P2 + (O2P1 - O1P2)/2)
-                const T ar = h5 * sg * (Sr[2] * P3 - Sr[3] * P2) + sig * Or[2] * P2 + h5 * (Or[2] * P1 - Or[1] * P2);
+        const T ar = h5 * sg * (Sr[2] * P3 - Sr[3] * P2) + sig * Or[2] * P2 + h5 * (Or[2] * P1 - Or[1] * P2);
         const T ai = h5 * sg * (Si[2] * P3 - Si[3] * P2) + sig * Oi[2] * P2 + h5 * (Oi[2] * P1 - Oi[1] * P2);
         ACC(D_FP, -ai, ar);
       }
       {
-                T zr = sg * Sr[3] * P3, zi = sg * Si[3] * P3;
+        T zr = sg * Sr[3] * P3, zi = sg * Si[3] * P3;
         zr += h5 * (Or[3] * P1 + sig * Or[3] * P2 + Or[1] * P3 - sig * Or[2] * P3);
         zi += h5 * (Oi[3] * P1 + sig * Oi[3] * P2 + Oi[1] * P3 - sig * Oi[2] * P3);
         ACC(D_FZ, zr, zi);
@@ -835,18 +803,18 @@ __global__ void __maxnreg__(192) k_density_fp64(DevBasis B, DensCall c0, DensCal
       xr = Or[0] * P0; xi = Oi[0] * P0;
       ACC(D_SR, xr, xi);
       ACC(D_SP, -sig * xi, sig * xr);
-      xr = h5 * (Or[2] * P0 + Or[0] * P2); xi = h5 * (Oi[2] * P0 + Oi[0] * P2);
-      ACC(D_TJPR, xr, xi);
-      ACC(D_TJPP, -sig * xi, sig * xr);
+      xr = Or[2] * P0 + Or[0] * P2; xi = Oi[2] * P0 + Oi[0] * P2;
+      ACCF(D_TJPR, h5, xr, xi);
+      ACCF(D_TJPP, hg, -xi, xr);
       xr = Or[1] * P1 + Or[2] * P2 + Or[3] * P3; xi = Oi[1] * P1 + Oi[2] * P2 + Oi[3] * P3;
       ACC(D_TR, xr, xi);
       ACC(D_TP, -sig * xi, sig * xr);
-      xr = h5 * (Or[0] * P1 - Or[1] * P0); xi = h5 * (Oi[0] * P1 - Oi[1] * P0);
-      ACC(D_TJRR, -xi, xr);
-      ACC(D_TJRP, -sig * xr, -sig * xi);
-      xr = h5 * (Or[0] * P3 - Or[3] * P0); xi = h5 * (Oi[0] * P3 - Oi[3] * P0);
-      ACC(D_TJZR, -xi, xr);
-      ACC(D_TJZP, -sig * xr, -sig * xi);
+      xr = Or[0] * P1 - Or[1] * P0; xi = Oi[0] * P1 - Oi[1] * P0;
+      ACCF(D_TJRR, h5, -xi, xr);
+      ACCF(D_TJRP, hg, -xr, -xi);
+      xr = Or[0] * P3 - Or[3] * P0; xi = Oi[0] * P3 - Oi[3] * P0;
+      ACCF(D_TJZR, h5, -xi, xr);
+      ACCF(D_TJZP, hg, -xr, -xi);
     }
   }
   // ---------------- pairing densities ----------------
@@ -854,48 +822,25 @@ __global__ void __maxnreg__(192) k_density_fp64(DevBasis B, DensCall c0, DensCal
     const int iy = C.kcols[ix];
     if (iy < 0) continue;
     const int d = B.db[ix], dc = B.db[iy], nu = B.nup[ix];
-    const int sa = B.st[ix], sb = B.st[iy];
+    const T* phi = B.phi + (long long)B.st[ix] * nghl + r;
     const T* kap = C.kap + (long long)p * C.kap_sp + C.koffs[ix];
-    for (int b0 = 0; b0 < dc; b0 += DBC) {
-      const int b = b0 + bl;
+    for (int b = w8; b < dc; b += 8) {
+      const T *cr = kap + (long long)b * d, *ci = cr + C.kap_spl;
       T w[2][2] = {{0, 0}, {0, 0}};
-      for (int a0 = 0; a0 < d; a0 += DAK) {
-        const int na = min(DAK, d - a0);
-        for (int e = threadIdx.x; e < DAK * DRT; e += 256) {
-          const int aa = e / DRT, rr = e % DRT;
-          T v = 0;
-          if (aa < na && r0 + rr < nghl) v = B.phi[(long long)(sa + a0 + aa) * nghl + r0 + rr];
-          sphi[0][aa][rr] = v;
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+#pragma unroll 4
+        for (int a = s ? nu : 0; a < (s ? d : nu); ++a) {
+          const T f = phi[(long long)a * nghl];
+          w[s][0] = fma(f, cr[a], w[s][0]); w[s][1] = fma(f, ci[a], w[s][1]);
         }
-        for (int e = threadIdx.x; e < 2 * DAK * DBC; e += 256) {
-          const int pl = e / (DAK * DBC), rem = e % (DAK * DBC), aa = rem / DBC, bb = rem % DBC;
-          T v = 0;
-          if (aa < na && b0 + bb < dc) v = kap[(long long)pl * C.kap_spl + (a0 + aa) + (long long)(b0 + bb) * d];
-          srho[pl][aa][bb] = v;
-        }
-        __syncthreads();
-        const int nup_here = max(0, min(na, nu - a0));
-        for (int aa = 0; aa < nup_here; ++aa) {
-          const T f = sphi[0][aa][rl];
-          w[0][0] = fma(f, srho[0][aa][bl], w[0][0]); w[0][1] = fma(f, srho[1][aa][bl], w[0][1]);
-        }
-        for (int aa = nup_here; aa < na; ++aa) {
-          const T f = sphi[0][aa][rl];
-          w[1][0] = fma(f, srho[0][aa][bl], w[1][0]); w[1][1] = fma(f, srho[1][aa][bl], w[1][1]);
-        }
-        __syncthreads();
       }
-      T P0 = 0, sg = 0;
-      const bool ok = rok && b < dc;
-      if (ok) {
-        const int jb = sb + b;
-        P0 = B.phi[(long long)jb * nghl + r];
-        sg = (T)B.ns[jb];
-      }
+      const int jb = B.st[iy] + b;
+      const T P0 = B.phi[(long long)jb * nghl + r];
+      const T sg = (T)B.ns[jb];
       const int si = (sg > 0) ? 0 : 1;
-      T Sr = si == 0 ? w[0][0] : w[1][0], Si = si == 0 ? w[0][1] : w[1][1];
-      T Or = si == 0 ? w[1][0] : w[0][0], Oi = si == 0 ? w[1][1] : w[0][1];
-      if (!ok) { Sr = Si = Or = Oi = 0; }
+      const T Sr = si == 0 ? w[0][0] : w[1][0], Si = si == 0 ? w[0][1] : w[1][1];
+      const T Or = si == 0 ? w[1][0] : w[0][0], Oi = si == 0 ? w[1][1] : w[0][1];
       const T sig = (sg < 0) ? (T)1 : (T)-1;
       T xr = two * Or * P0, xi = two * Oi * P0;
       ACC(D_RB, -sg * xr, -sg * xi);
@@ -906,11 +851,21 @@ __global__ void __maxnreg__(192) k_density_fp64(DevBasis B, DensCall c0, DensCal
     }
   }
 #undef ACC
+#undef ACCF
+  // over the warps, DSUM densities at a time
+  constexpr int DSUM = 8;
+  __shared__ T red[DSUM][8][DRT];
   T* out = dpart + (((long long)p * 2 + call) * G + g) * (2 * ND) * nghl;
 #pragma unroll
-  for (int k = 0; k < 2 * ND; ++k) {
-    const T v = red8(al[k]);
-    if (bl == 0 && rok) out[(long long)k * nghl + r] = v;
+  for (int k0 = 0; k0 < 2 * ND; k0 += DSUM) {
+    if (k0) __syncthreads();
+#pragma unroll
+    for (int k = 0; k < DSUM; ++k) red[k][w8][l] = al[k0 + k];
+    __syncthreads();
+    T v[8];   // warp w8 sums density k0 + w8
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = red[w8][i][l];
+    if (rok) out[(long long)(k0 + w8) * nghl + r] = ((v[0] + v[4]) + (v[2] + v[6])) + ((v[1] + v[5]) + (v[3] + v[7]));
   }
 }
 
