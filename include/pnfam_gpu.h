@@ -243,6 +243,13 @@ int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* ctx,
                                      double* re_dm, double* im_dm);
 
 /*
+ * Either evaluation on arrays of complex numbers (Re and Im in turn, nxy of them): in
+ * rho_pn, kappa(+), rho_np, kappa(-), out h_pn, Delta(+), h_np, Delta(-).  The results are
+ * those of the entry points above (mixed != 0: of the second) without their separate planes.
+ */
+int pnfam_gpu_calc_hamiltonian_z(pnfam_ctx_t* ctx, int mixed, const double* const* in, double* const* out);
+
+/*
  * Allocation-free field evaluation.  No counterpart in the reference: the
  * reference evaluates the field only inside its own process.
  *

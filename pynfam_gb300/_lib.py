@@ -17,7 +17,7 @@ EXPORTS = ("pnfam_gpu_init", "pnfam_gpu_set_operator", "pnfam_gpu_solve", "pnfam
            "pnfam_gpu_nxy", "pnfam_gpu_last_profile", "pnfam_gpu_free", "pnfam_gpu_last_error",
            "pnfam_gpu_engine_create", "pnfam_gpu_engine_admit", "pnfam_gpu_engine_launch",
            "pnfam_gpu_engine_finish", "pnfam_gpu_engine_active", "pnfam_gpu_engine_ready", "pnfam_gpu_engine_free",
-           "pnfam_gpu_calc_hamiltonian_mixed", "pnfam_gpu_set_occupations", "pnfam_gpu_task_tables",
+           "pnfam_gpu_calc_hamiltonian_mixed", "pnfam_gpu_calc_hamiltonian_z", "pnfam_gpu_set_occupations", "pnfam_gpu_task_tables",
            "pnfam_gpu_solve_state", "pnfam_gpu_state_size", "pnfam_gpu_2bc_field", "pnfam_gpu_hfb_basis",
            "pnfam_gpu_hfb_matrices", "pnfam_gpu_sym_eigen", "pnfam_gpu_hfb_densities")
 
@@ -89,6 +89,8 @@ def load(path: str = LIBPATH):
     lib.pnfam_gpu_calc_hamiltonian.restype = C.c_int
     lib.pnfam_gpu_calc_hamiltonian_mixed.argtypes = [C.c_void_p] + [dp] * 16
     lib.pnfam_gpu_calc_hamiltonian_mixed.restype = C.c_int
+    lib.pnfam_gpu_calc_hamiltonian_z.argtypes = [C.c_void_p, C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p)]
+    lib.pnfam_gpu_calc_hamiltonian_z.restype = C.c_int
     lib.pnfam_gpu_nxy.argtypes = [C.c_void_p]
     lib.pnfam_gpu_nxy.restype = C.c_longlong
     lib.pnfam_gpu_last_profile.argtypes = [C.c_void_p, dp, C.c_int, C.POINTER(C.c_longlong)]

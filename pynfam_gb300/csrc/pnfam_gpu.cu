@@ -288,6 +288,7 @@ struct pnfam_ctx {
   // per-solve buffers
   int cap_P = 0, cap_M = 0;
   DBuf<double> d_state, d_vout, d_T, d_rsp, d_hsp, d_hqp, d_dpart, d_mf;
+  DBuf<double> d_zio;   // [4][nxy] complex: arrays of calc_hamiltonian_z
   DBuf<double> d_df, d_dv, d_bpart, d_si, d_norm, d_beta, d_gamma, d_cpart, d_wre, d_wim;
   DBuf<double> d_gfn;   // [P][Re | Im][nq*nxy] Green's function of each slot's omega
   DBuf<int> d_active, d_act32, d_act64;
@@ -429,7 +430,7 @@ struct pnfam_ctx {
     DBuf<double>* dbs[] = {&d_up, &d_vp, &d_un, &d_vn, &d_ep, &d_en, &d_phi, &d_wd, &d_crho, &d_cs,
                            &d_cpair, &d_cspair, &d_fops, &d_state, &d_vout, &d_T, &d_rsp, &d_hsp,
                            &d_hqp, &d_dpart, &d_mf, &d_df, &d_dv, &d_bpart, &d_si, &d_norm,
-                           &d_beta, &d_gamma, &d_cpart, &d_wre, &d_wim, &d_gfn, &d_fp, &d_fn};
+                           &d_beta, &d_gamma, &d_cpart, &d_wre, &d_wim, &d_gfn, &d_fp, &d_fn, &d_zio};
     for (auto* b : dbs) b->release();
     d_foff.release(); d_xtoff.release(); d_ytoff.release();
     d_agather.release(); d_aerow.release(); d_aecol.release(); d_afops.release();
@@ -2872,33 +2873,14 @@ extern "C" void pnfam_gpu_engine_free(pnfam_engine_t* e) {
   delete e;
 }
 
-extern "C" int pnfam_gpu_calc_hamiltonian(pnfam_ctx_t* c, const double* re_rho_pn, const double* im_rho_pn,
-                                          const double* re_kp, const double* im_kp, const double* re_rho_np,
-                                          const double* im_rho_np, const double* re_km, const double* im_km,
-                                          double* re_h_pn, double* im_h_pn, double* re_dp, double* im_dp,
-                                          double* re_h_np, double* im_h_np, double* re_dm, double* im_dm) {
-  g_err.clear();
-  if (!c) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian: NULL context");
-  if (!c->have_op) return fail(PNFAM_ESTATE, "pnfam_gpu_calc_hamiltonian: call pnfam_gpu_set_operator first");
-  const void* in[8] = {re_rho_pn, im_rho_pn, re_kp, im_kp, re_rho_np, im_rho_np, re_km, im_km};
-  void* outp[8] = {re_h_pn, im_h_pn, re_dp, im_dp, re_h_np, im_h_np, re_dm, im_dm};
-  for (int k = 0; k < 8; ++k)
-    if (!in[k] || !outp[k]) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian: NULL array");
-  int rc = ensure_buffers(c, std::max(1, c->cap_P), std::max(1, c->cap_M));
-  if (rc) return rc;
+// the field of the densities in d_rsp (point 0) into d_hsp; d_active[0] = 1
+static int field_fp64(pnfam_ctx* c) {
   const long long nxy = c->nxy;
-  const size_t nb = sizeof(double) * nxy;
-  // RSP quadrant q, plane pl at pl*4nxy + q*nxy (point 0): 0 rho_pn, 1 kappa+, 2 kappa-, 3 rho_np
-  const int qin[8] = {0, 0, 1, 1, 3, 3, 2, 2};
-  for (int k = 0; k < 8; ++k)
-    CK(cudaMemcpyAsync(c->d_rsp.p + (k & 1) * 4 * nxy + qin[k] * nxy, in[k], nb, cudaMemcpyHostToDevice, c->stream));
-  std::vector<int> one = {1};
-  CK(cudaMemcpyAsync(c->d_active.p, one.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
   const int* act = c->d_active.p;
   if (c->sep) {
     auto none = [](int = 0) {};
-    if ((rc = sep_field<double>(c, 1, 1, act, c->d_rsp.p, c->d_dpart.p, c->d_hsp.p, c->stream, none, none)))
-      return rc;
+    const int rc = sep_field<double>(c, 1, 1, act, c->d_rsp.p, c->d_dpart.p, c->d_hsp.p, c->stream, none, none);
+    if (rc) return rc;
   } else {
     DensCall d0, d1;
     d0.rho = c->d_rsp.p + 0 * nxy; d0.rho_sp = 8 * nxy; d0.rho_spl = 4 * nxy;
@@ -2917,44 +2899,17 @@ extern "C" int pnfam_gpu_calc_hamiltonian(pnfam_ctx_t* c, const double* re_rho_p
         B, c->d_hgroups.p, c->d_mf.p, c->d_hsp.p, nxy, act);
   }
   CK(cudaGetLastError());
-  const int qout[8] = {0, 0, 1, 1, 3, 3, 2, 2};
-  for (int k = 0; k < 8; ++k)
-    CK(cudaMemcpyAsync(outp[k], c->d_hsp.p + (k & 1) * 4 * nxy + qout[k] * nxy, nb, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
   return PNFAM_OK;
 }
 
-extern "C" int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* c, const double* re_rho_pn, const double* im_rho_pn,
-                                                const double* re_kp, const double* im_kp, const double* re_rho_np,
-                                                const double* im_rho_np, const double* re_km, const double* im_km,
-                                                double* re_h_pn, double* im_h_pn, double* re_dp, double* im_dp,
-                                                double* re_h_np, double* im_h_np, double* re_dm, double* im_dm) {
-  g_err.clear();
-  if (!c) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_mixed: NULL context");
-  if (!c->have_op) return fail(PNFAM_ESTATE, "pnfam_gpu_calc_hamiltonian_mixed: call pnfam_gpu_set_operator first");
-  const void* in[8] = {re_rho_pn, im_rho_pn, re_kp, im_kp, re_rho_np, im_rho_np, re_km, im_km};
-  void* outp[8] = {re_h_pn, im_h_pn, re_dp, im_dp, re_h_np, im_h_np, re_dm, im_dm};
-  for (int k = 0; k < 8; ++k)
-    if (!in[k] || !outp[k]) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_mixed: NULL array");
-  int rc = ensure_buffers(c, std::max(1, c->cap_P), std::max(1, c->cap_M));
-  if (rc) return rc;
-  c->cap_P = std::max(1, c->cap_P); c->cap_M = std::max(1, c->cap_M);
-  if ((rc = ensure_buffers32(c, c->cap_P, false, false))) return rc;
+// the same in FP32, d_rsp32 into d_hsp32; also d_actlist[0] = 0
+static int field_fp32(pnfam_ctx* c) {
   const long long nxy = c->nxy;
-  const size_t nb = sizeof(double) * nxy;
-  const int qin[8] = {0, 0, 1, 1, 3, 3, 2, 2};
-  for (int k = 0; k < 8; ++k)
-    CK(cudaMemcpyAsync(c->d_rsp.p + (k & 1) * 4 * nxy + qin[k] * nxy, in[k], nb, cudaMemcpyHostToDevice, c->stream));
-  std::vector<int> one = {1}, zero = {0};
-  CK(cudaMemcpyAsync(c->d_active.p, one.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(c->d_actlist.p, zero.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
-  k_to_f32<<<1024, 256, 0, c->stream>>>(c->d_rsp.p, c->d_rsp32.p, 8 * nxy, 1, 0, nullptr);
   const int* act = c->d_active.p;
   if (c->sep32) {
     auto none = [](int = 0) {};
-    if ((rc = sep_field<float>(c, 1, 1, act, c->d_rsp32.p, c->d_dpart32.p, c->d_hsp32.p, c->stream, none,
-                               none)))
-      return rc;
+    const int rc = sep_field<float>(c, 1, 1, act, c->d_rsp32.p, c->d_dpart32.p, c->d_hsp32.p, c->stream, none, none);
+    if (rc) return rc;
   } else {
     DensCallT<float> d0, d1;
     d0.rho = c->d_rsp32.p + 0 * nxy; d0.rho_sp = 8 * nxy; d0.rho_spl = 4 * nxy;
@@ -2984,19 +2939,134 @@ extern "C" int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* c, const double* re
     k_hproj_tc<<<dim3((unsigned)c->htasks_tc.size(), 1), HTC_THREADS, hproj_tc_smem_bytes(c->tc_npmax), c->stream>>>(
         B, c->d_htasks_tc.p, c->d_actlist.p, 1, c->tc_npmax, c->d_mf32.p, c->d_hphi.p, c->d_hsp32.p, nxy, c->d_err.p);
   }
+  CK(cudaGetLastError());
+  return PNFAM_OK;
+}
+
+// the waits of the tensor-core kernels of field_fp32 (the product-basis kernels have none);
+// after the stream's work was waited for
+static int field_fp32_status(pnfam_ctx* c, const char* who) {
+  if (c->sep32) return PNFAM_OK;
+  int herr = 0;
+  CK(cudaMemcpyAsync(&herr, c->d_err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  if (!herr) return PNFAM_OK;
+  cudaMemsetAsync(c->d_err.p, 0, sizeof(int), c->stream);
+  return fail(PNFAM_ECUDA, std::string(who) + ": a wait on the tensor cores gave up");
+}
+
+static int field_buffers(pnfam_ctx* c, bool mixed) {
+  int rc = ensure_buffers(c, std::max(1, c->cap_P), std::max(1, c->cap_M));
+  if (rc) return rc;
+  if (!mixed) return PNFAM_OK;
+  c->cap_P = std::max(1, c->cap_P); c->cap_M = std::max(1, c->cap_M);
+  return ensure_buffers32(c, c->cap_P, false, false);
+}
+
+extern "C" int pnfam_gpu_calc_hamiltonian(pnfam_ctx_t* c, const double* re_rho_pn, const double* im_rho_pn,
+                                          const double* re_kp, const double* im_kp, const double* re_rho_np,
+                                          const double* im_rho_np, const double* re_km, const double* im_km,
+                                          double* re_h_pn, double* im_h_pn, double* re_dp, double* im_dp,
+                                          double* re_h_np, double* im_h_np, double* re_dm, double* im_dm) {
+  g_err.clear();
+  if (!c) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian: NULL context");
+  if (!c->have_op) return fail(PNFAM_ESTATE, "pnfam_gpu_calc_hamiltonian: call pnfam_gpu_set_operator first");
+  const void* in[8] = {re_rho_pn, im_rho_pn, re_kp, im_kp, re_rho_np, im_rho_np, re_km, im_km};
+  void* outp[8] = {re_h_pn, im_h_pn, re_dp, im_dp, re_h_np, im_h_np, re_dm, im_dm};
+  for (int k = 0; k < 8; ++k)
+    if (!in[k] || !outp[k]) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian: NULL array");
+  int rc = field_buffers(c, false);
+  if (rc) return rc;
+  const long long nxy = c->nxy;
+  const size_t nb = sizeof(double) * nxy;
+  // RSP quadrant q, plane pl at pl*4nxy + q*nxy (point 0): 0 rho_pn, 1 kappa+, 2 kappa-, 3 rho_np
+  const int qin[8] = {0, 0, 1, 1, 3, 3, 2, 2};
+  for (int k = 0; k < 8; ++k)
+    CK(cudaMemcpyAsync(c->d_rsp.p + (k & 1) * 4 * nxy + qin[k] * nxy, in[k], nb, cudaMemcpyHostToDevice, c->stream));
+  std::vector<int> one = {1};
+  CK(cudaMemcpyAsync(c->d_active.p, one.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  if ((rc = field_fp64(c))) return rc;
+  const int qout[8] = {0, 0, 1, 1, 3, 3, 2, 2};
+  for (int k = 0; k < 8; ++k)
+    CK(cudaMemcpyAsync(outp[k], c->d_hsp.p + (k & 1) * 4 * nxy + qout[k] * nxy, nb, cudaMemcpyDeviceToHost, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
+  return PNFAM_OK;
+}
+
+extern "C" int pnfam_gpu_calc_hamiltonian_mixed(pnfam_ctx_t* c, const double* re_rho_pn, const double* im_rho_pn,
+                                                const double* re_kp, const double* im_kp, const double* re_rho_np,
+                                                const double* im_rho_np, const double* re_km, const double* im_km,
+                                                double* re_h_pn, double* im_h_pn, double* re_dp, double* im_dp,
+                                                double* re_h_np, double* im_h_np, double* re_dm, double* im_dm) {
+  g_err.clear();
+  if (!c) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_mixed: NULL context");
+  if (!c->have_op) return fail(PNFAM_ESTATE, "pnfam_gpu_calc_hamiltonian_mixed: call pnfam_gpu_set_operator first");
+  const void* in[8] = {re_rho_pn, im_rho_pn, re_kp, im_kp, re_rho_np, im_rho_np, re_km, im_km};
+  void* outp[8] = {re_h_pn, im_h_pn, re_dp, im_dp, re_h_np, im_h_np, re_dm, im_dm};
+  for (int k = 0; k < 8; ++k)
+    if (!in[k] || !outp[k]) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_mixed: NULL array");
+  int rc = field_buffers(c, true);
+  if (rc) return rc;
+  const long long nxy = c->nxy;
+  const size_t nb = sizeof(double) * nxy;
+  const int qin[8] = {0, 0, 1, 1, 3, 3, 2, 2};
+  for (int k = 0; k < 8; ++k)
+    CK(cudaMemcpyAsync(c->d_rsp.p + (k & 1) * 4 * nxy + qin[k] * nxy, in[k], nb, cudaMemcpyHostToDevice, c->stream));
+  std::vector<int> one = {1}, zero = {0};
+  CK(cudaMemcpyAsync(c->d_active.p, one.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->d_actlist.p, zero.data(), sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  k_to_f32<<<1024, 256, 0, c->stream>>>(c->d_rsp.p, c->d_rsp32.p, 8 * nxy, 1, 0, nullptr);
+  if ((rc = field_fp32(c))) return rc;
   k_to_f64<<<dim3(1024, 1), 256, 0, c->stream>>>(c->d_hsp32.p, c->d_hsp.p, 8 * nxy, 0, nullptr);
   CK(cudaGetLastError());
   const int qout[8] = {0, 0, 1, 1, 3, 3, 2, 2};
   for (int k = 0; k < 8; ++k)
     CK(cudaMemcpyAsync(outp[k], c->d_hsp.p + (k & 1) * 4 * nxy + qout[k] * nxy, nb, cudaMemcpyDeviceToHost, c->stream));
-  int herr = 0;
-  CK(cudaMemcpyAsync(&herr, c->d_err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
-  if (herr) {
-    cudaMemsetAsync(c->d_err.p, 0, sizeof(int), c->stream);
-    return fail(PNFAM_ECUDA, "pnfam_gpu_calc_hamiltonian_mixed: a wait on the tensor cores gave up");
+  return field_fp32_status(c, "pnfam_gpu_calc_hamiltonian_mixed");
+}
+
+// Complex arrays as a caller holds them: one copy per array, split and merged on the device.
+// The pages of new result arrays are touched while the device computes.
+extern "C" int pnfam_gpu_calc_hamiltonian_z(pnfam_ctx_t* c, int mixed, const double* const* in, double* const* out) {
+  g_err.clear();
+  if (!c) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_z: NULL context");
+  if (!c->have_op) return fail(PNFAM_ESTATE, "pnfam_gpu_calc_hamiltonian_z: call pnfam_gpu_set_operator first");
+  if (!in || !out) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_z: NULL array");
+  for (int k = 0; k < 4; ++k)
+    if (!in[k] || !out[k]) return fail(PNFAM_EINVAL, "pnfam_gpu_calc_hamiltonian_z: NULL array");
+  int rc = field_buffers(c, mixed != 0);
+  if (rc) return rc;
+  const long long nxy = c->nxy;
+  const size_t nz = sizeof(double) * 2 * nxy;
+  CK(dalloc(c->d_zio, (size_t)8 * nxy));
+  double* z = c->d_zio.p;
+  for (int k = 0; k < 4; ++k) CK(cudaMemcpyAsync(z + 2 * k * nxy, in[k], nz, cudaMemcpyHostToDevice, c->stream));
+  const dim3 grid((unsigned)((nxy + 255) / 256), 4);
+  const double2* zc = reinterpret_cast<const double2*>(z);
+  if (mixed) {
+    k_split_z<float><<<grid, 256, 0, c->stream>>>(nxy, zc, c->d_rsp32.p, c->d_active.p, c->d_actlist.p);
+    if ((rc = field_fp32(c))) return rc;
+    k_merge_z<float><<<grid, 256, 0, c->stream>>>(nxy, c->d_hsp32.p, reinterpret_cast<double2*>(z));
+  } else {
+    k_split_z<double><<<grid, 256, 0, c->stream>>>(nxy, zc, c->d_rsp.p, c->d_active.p, nullptr);
+    if ((rc = field_fp64(c))) return rc;
+    k_merge_z<double><<<grid, 256, 0, c->stream>>>(nxy, c->d_hsp.p, reinterpret_cast<double2*>(z));
   }
-  return PNFAM_OK;
+  CK(cudaGetLastError());
+  for (int k = 0; k < 4; ++k) {
+    volatile char* o = reinterpret_cast<volatile char*>(out[k]);
+    for (size_t i = 0; i < nz; i += 4096) o[i] = o[i];
+  }
+  bool one = true;   // the four arrays in one piece: one copy
+  for (int k = 1; k < 4; ++k) one = one && out[k] == out[0] + 2 * k * nxy;
+  if (one) {
+    CK(cudaMemcpyAsync(out[0], z, 4 * nz, cudaMemcpyDeviceToHost, c->stream));
+  } else {
+    for (int k = 0; k < 4; ++k) CK(cudaMemcpyAsync(out[k], z + 2 * k * nxy, nz, cudaMemcpyDeviceToHost, c->stream));
+  }
+  CK(cudaStreamSynchronize(c->stream));
+  return mixed ? field_fp32_status(c, "pnfam_gpu_calc_hamiltonian_z") : PNFAM_OK;
 }
 
 extern "C" int pnfam_gpu_set_occupations(pnfam_ctx_t* c, const double* fp, const double* fn) {

@@ -2602,4 +2602,28 @@ __global__ void k_to_f64(const float* __restrict__ in, double* __restrict__ out,
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
     out[p * ld + e] = (double)in[p * ld + e];
 }
+
+// the four densities of calc_hamiltonian_z ([4][nxy] complex: rho_pn, kappa+, rho_np, kappa-)
+// into the planes and quadrants of point 0 ([2 re/im][4]: rho_pn, kappa+, kappa-, rho_np), and
+// its slot flags; k_merge_z: the fields back.  grid (ceil(nxy/256), 4)
+template <class T>
+__global__ void __launch_bounds__(256) k_split_z(long long nxy, const double2* __restrict__ z, T* __restrict__ rsp,
+                                                 int* __restrict__ active, int* __restrict__ actlist) {
+  const int k = blockIdx.y, q = k < 2 ? k : 5 - k;
+  const long long i = blockIdx.x * 256LL + threadIdx.x;
+  if (k == 0 && i == 0) {
+    active[0] = 1;
+    if (actlist) actlist[0] = 0;
+  }
+  if (i >= nxy) return;
+  const double2 v = z[k * nxy + i];
+  rsp[q * nxy + i] = (T)v.x;
+  rsp[(4 + q) * nxy + i] = (T)v.y;
+}
+template <class T>
+__global__ void __launch_bounds__(256) k_merge_z(long long nxy, const T* __restrict__ hsp, double2* __restrict__ z) {
+  const int k = blockIdx.y, q = k < 2 ? k : 5 - k;
+  const long long i = blockIdx.x * 256LL + threadIdx.x;
+  if (i < nxy) z[k * nxy + i] = make_double2((double)hsp[q * nxy + i], (double)hsp[(4 + q) * nxy + i]);
+}
 }  // namespace pnfam

@@ -187,14 +187,13 @@ class GPUSolver:
         mixed=True evaluates in FP32 with the tensor-core projection (the
         kernels of the mixed form's increment evaluations)."""
         n = self.nxy
-        ins = []
-        for a in (rho_pn, kp, rho_np, km):
-            a = np.asarray(a, dtype=complex)
-            ins += [np.ascontiguousarray(a.real), np.ascontiguousarray(a.imag)]
-        outs = [np.zeros(n) for _ in range(8)]
-        fn = self.lib.pnfam_gpu_calc_hamiltonian_mixed if mixed else self.lib.pnfam_gpu_calc_hamiltonian
-        _lib.check(fn(self.ctx, *[_lib.dptr(x) for x in ins], *[_lib.dptr(x) for x in outs]))
-        return tuple(outs[2 * k] + 1j * outs[2 * k + 1] for k in range(4))
+        ins = [np.ascontiguousarray(a, dtype=complex) for a in (rho_pn, kp, rho_np, km)]
+        if min(a.size for a in ins) < n:
+            raise ValueError(f"calc_hamiltonian: arrays of {n} elements are needed")
+        out = np.empty((4, n), dtype=complex)   # one piece: one copy from the device
+        ptrs = [(C.c_void_p * 4)(*[a.ctypes.data for a in group]) for group in (ins, out)]
+        _lib.check(self.lib.pnfam_gpu_calc_hamiltonian_z(self.ctx, int(bool(mixed)), *ptrs))
+        return tuple(out)
 
     def close(self):
         if getattr(self, "ctx", None) is not None and self.ctx.value:
