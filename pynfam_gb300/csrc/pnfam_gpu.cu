@@ -18,6 +18,8 @@
 #include <chrono>
 #include <deque>
 #include <map>
+#include <new>
+#include <thread>
 #include <tuple>
 #include <type_traits>
 #include <mutex>
@@ -1344,9 +1346,35 @@ static int sep_operator(pnfam_ctx* c) {
   if (!c->sep) return PNFAM_OK;
   const std::vector<int>* cols[5] = {&c->fc, &c->xtc, &c->ytc, &c->xc, &c->yc};
   const std::vector<long long>* offs[5] = {&c->foff, &c->xtoff, &c->ytoff, &c->xoff, &c->yoff};
+  // the five structures do not depend on each other: a thread for each where building one
+  // takes longer than starting a thread (2 ms against 0.05 at N_sh = 16, 0.1 ms at 6)
+  std::vector<int> items[5];
+  int state[5] = {0, 0, 0, 0, 0};   // 1: built, -1: not of this form, 0: out of memory
+  auto make = [&](int k) {
+    try {
+      const bool ok = sep_structure(c->sepb, c->nb, c->db.data(), c->st.data(), c->nup.data(), cols[k]->data(),
+                                    offs[k]->data(), k == 0 || k >= 3, c->seps[k]);
+      if (ok) items[k] = sep_item_columns(c->seps[k].items);
+      state[k] = ok ? 1 : -1;
+    } catch (const std::bad_alloc&) {
+    }
+  };
+  {
+    std::vector<std::thread> team;
+    int next = 0;
+    if (c->nxy >= 16384) {
+      try {
+        team.reserve(4);
+        for (; next < 4; ++next) team.emplace_back(make, next);
+      } catch (const std::exception&) {   // no further thread: the rest here
+      }
+    }
+    for (int k = next; k < 5; ++k) make(k);
+    for (std::thread& t : team) t.join();
+  }
   for (int k = 0; k < 5; ++k) {
-    if (!sep_structure(c->sepb, c->nb, c->db.data(), c->st.data(), c->nup.data(), cols[k]->data(), offs[k]->data(),
-                       k == 0 || k >= 3, c->seps[k])) {
+    if (!state[k]) return fail(PNFAM_ENOMEM, "pnfam_gpu_set_operator: out of memory");
+    if (state[k] < 0) {
       c->sep = c->sep32 = false;
       return PNFAM_OK;
     }
@@ -1358,8 +1386,7 @@ static int sep_operator(pnfam_ctx* c) {
     CK(upload(d.offs, s.offs.data(), s.offs.size()));
     CK(upload(d.ubeg, s.ubeg.data(), s.ubeg.size()));
     CK(upload(d.order, s.order.data(), s.order.size()));
-    const std::vector<int> items = sep_item_columns(s.items);
-    CK(upload(d.items, items.data(), items.size()));
+    CK(upload(d.items, items[k].data(), items[k].size()));
     for (int h = 0; h < 2; ++h) CK(upload(d.warps[h], s.warps[h].data(), s.warps[h].size()));
   }
   const long long ngl = c->sepb.ngl, nf = (long long)c->seps[0].units.size();
