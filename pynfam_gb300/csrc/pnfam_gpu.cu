@@ -3418,8 +3418,12 @@ extern "C" int pnfam_gpu_2bc_field(const pnfam_2bc_input_t* in, double* pieces, 
   const int NZ = P.nzx + 1;
   const long long nzt = (long long)NZ * NZ * v.nt;
   CK(dalloc(d.zbuf, (size_t)nzt * tbc::NQ * tbc::NCG));
-  CK(dalloc(d.acc, (size_t)in->nxy * 6));
-  CK(cudaMemset(d.acc.p, 0, (size_t)in->nxy * 6 * sizeof(double)));
+  // a share per term chunk until there are enough groups for a dozen rounds of CTAs (two
+  // fit on an SM), so that the last round does not count
+  const int nchunk = (v.nt + tbc::TBC_TCH - 1) / tbc::TBC_TCH;
+  const int shares = v.ngroups < 12 * 304 ? std::max(1, nchunk) : 1;
+  CK(dalloc(d.acc, (size_t)in->nxy * 6 * shares));
+  CK(cudaMemset(d.acc.p, 0, (size_t)in->nxy * 6 * shares * sizeof(double)));
   v.zbuf = d.zbuf.p; v.acc = d.acc.p;
   for (auto& e : d.ev) CK(cudaEventCreate(&e));
 
@@ -3430,7 +3434,9 @@ extern "C" int pnfam_gpu_2bc_field(const pnfam_2bc_input_t* in, double* pieces, 
   CK(cudaGetLastError());
   CK(cudaEventRecord(d.ev[1], 0));
   CK(cudaFuncSetAttribute(tbc::k_tbc_field, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tbc::TBC_SMEM));
-  if (v.ngroups > 0) tbc::k_tbc_field<<<v.ngroups, tbc::TBC_THREADS, tbc::TBC_SMEM>>>(v);
+  if (v.ngroups > 0) tbc::k_tbc_field<<<dim3(v.ngroups, shares), tbc::TBC_THREADS, tbc::TBC_SMEM>>>(v);
+  if (shares > 1)
+    tbc::k_tbc_sum<<<(unsigned)((in->nxy * 6 + 255) / 256), 256>>>(d.acc.p, in->nxy * 6, shares);
   CK(cudaGetLastError());
   CK(cudaEventRecord(d.ev[2], 0));
   std::vector<double> acc((size_t)in->nxy * 6);

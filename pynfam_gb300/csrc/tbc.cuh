@@ -809,46 +809,72 @@ constexpr int TBC_TCH = 32;         // terms per chunk
 constexpr int TBC_THREADS = 256;    // 8 warps
 constexpr size_t TBC_SMEM = sizeof(double) * TBC_TCH * 4 * NCG;
 
-__device__ __forceinline__ void warp_sum6(double* s) {
+// sums of six values over the warp, left in different lanes: the lane returns the one with
+// the index g = warp_sum6_at(lane).  8 additions instead of the 30 of six full sums (a
+// quarter of the FP64 work of the short Cartesian sums)
+__device__ __forceinline__ double warp_sum6(const double* s, int lane) {
+  const bool a = lane & 16, b = lane & 8, c = lane & 4;
+  double k[3], m[2];
 #pragma unroll
-  for (int g = 0; g < NG; ++g)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s[g] += __shfl_xor_sync(0xffffffffu, s[g], o);
+  for (int i = 0; i < 3; ++i) k[i] = (a ? s[3 + i] : s[i]) + __shfl_xor_sync(0xffffffffu, a ? s[i] : s[3 + i], 16);
+  m[0] = (b ? k[2] : k[0]) + __shfl_xor_sync(0xffffffffu, b ? k[0] : k[2], 8);
+  m[1] = k[1] + __shfl_xor_sync(0xffffffffu, k[1], 8);
+  double r = (!b && c ? m[1] : m[0]) + __shfl_xor_sync(0xffffffffu, b || c ? m[0] : m[1], 4);
+  r += __shfl_xor_sync(0xffffffffu, r, 2);
+  return r + __shfl_xor_sync(0xffffffffu, r, 1);
+}
+// -1: the sum is another lane's to use
+__device__ __forceinline__ int warp_sum6_at(int lane) {
+  return lane & 3 ? -1 : (lane & 8) && (lane & 4) ? -1 : (lane & 16 ? 3 : 0) + (lane & 8 ? 2 : lane & 4 ? 1 : 0);
 }
 
-// radx6 with the 32 lanes of a warp splitting the (ny_i, ny_j, ny_k) combinations;
-// every lane returns the full sums.  Called by all lanes with the same arguments.
-__device__ void radx6_warp(const View& v, int lane, int tab, int ni, int li, int nj, int lj, int nk, int lk, int nl,
-                           int ll, double* s) {
+// radx6 with the 32 lanes of a warp splitting the (ny_i, ny_j, ny_k) combinations, for NT
+// tables tab that share the coefficients and the ny elements; sum[k]: that of this lane's
+// index (warp_sum6).  Called by all lanes with the same arguments.
+template <int NT>
+__device__ void radx6_warp(const View& v, int lane, const int* tab, int ni, int li, int nj, int lj, int nk, int lk,
+                           int nl, int ll, double* sum) {
   const int n1 = v.nrl + 1;
-  const double* X = v.xr + (size_t)tab * n1 * n1 * n1 * n1 * NG;
-  const double* Y = v.xr + (size_t)X00 * n1 * n1 * n1 * n1 * NG;
+  const size_t nx = (size_t)n1 * n1 * n1 * n1 * NG;
+  const double* Y = v.xr + X00 * nx;
   const int Ai = 2 * ni + abs(li), Aj = 2 * nj + abs(lj), Ak = 2 * nk + abs(lk), Al = 2 * nl + abs(ll);
   const int n3 = (Ai + 1) * (Aj + 1) * (Ak + 1);
-  for (int g = 0; g < NG; ++g) s[g] = 0.0;
+  double s[NT][NG];
+  const double* X[NT];
+#pragma unroll
+  for (int k = 0; k < NT; ++k) {
+    X[k] = v.xr + tab[k] * nx;
+#pragma unroll
+    for (int g = 0; g < NG; ++g) s[k][g] = 0.0;
+  }
   for (int c = lane; c < n3; c += 32) {
     const int yk = c % (Ak + 1), r = c / (Ak + 1), yj = r % (Aj + 1), yi = r / (Aj + 1);
     const double cijk = cp2c_at(v, ni, li, yi) * cp2c_at(v, nj, lj, yj) * cp2c_at(v, nk, lk, yk);
     for (int yl = (yi + yj + yk) & 1; yl <= Al; yl += 2) {
       const int sgn = (yi + yj + ((yi + yj + yk + yl) >> 1)) & 1;
       const double w = (sgn ? -cijk : cijk) * cp2c_at(v, nl, ll, yl);
-      const double* x = X + idx4(n1, Ai - yi, Aj - yj, Ak - yk, Al - yl) * NG;
+      const size_t x = idx4(n1, Ai - yi, Aj - yj, Ak - yk, Al - yl) * NG;
       const double* y = Y + idx4(n1, yi, yj, yk, yl) * NG;
 #pragma unroll
-      for (int g = 0; g < NG; ++g) s[g] += w * x[g] * y[g];
+      for (int k = 0; k < NT; ++k)
+#pragma unroll
+        for (int g = 0; g < NG; ++g) s[k][g] += w * X[k][x + g] * y[g];
     }
   }
-  warp_sum6(s);
+#pragma unroll
+  for (int k = 0; k < NT; ++k) sum[k] = warp_sum6(s[k], lane);
 }
 
 // radc6_imag with the lanes of a warp splitting the (ny_i, ny_j, ny_k) combinations
-__device__ void radc6_imag_warp(const View& v, int lane, int dip, int ni, int li, int nj, int lj, int nk, int lk,
-                                int nl, int ll, double* s) {
+__device__ double radc6_imag_warp(const View& v, int lane, int dip, int ni, int li, int nj, int lj, int nk, int lk,
+                                  int nl, int ll) {
   const int n1 = v.nrl + 1;
   const double* X = v.xr + (size_t)X10 * n1 * n1 * n1 * n1 * NG;
   const double* Y = v.xr + (size_t)(dip == 1 ? X01 : X02) * n1 * n1 * n1 * n1 * NG;
   const int Ai = 2 * ni + abs(li), Aj = 2 * nj + abs(lj), Ak = 2 * nk + abs(lk), Al = 2 * nl + abs(ll);
   const int n3 = (Ai + 1) * (Aj + 1) * (Ak + 1);
+  double s[NG];
+#pragma unroll
   for (int g = 0; g < NG; ++g) s[g] = 0.0;
   for (int c = lane; c < n3; c += 32) {
     const int yk = c % (Ak + 1), r = c / (Ak + 1), yj = r % (Aj + 1), yi = r / (Aj + 1);
@@ -859,37 +885,44 @@ __device__ void radc6_imag_warp(const View& v, int lane, int dip, int ni, int li
       const double w = (e == 1 ? cijk : -cijk) * cp2c_at(v, nl, ll, yl);
       const double* x = X + idx4(n1, Ai - yi, Aj - yj, Ak - yk, Al - yl) * NG;
       const double* y = Y + idx4(n1, yi, yj, yk, yl) * NG;
+#pragma unroll
       for (int g = 0; g < NG; ++g) s[g] += w * x[g] * y[g];
     }
   }
-  warp_sum6(s);
+  return warp_sum6(s, lane);
 }
 
-// ddgr6 by a warp: lane 0 writes out[g]
+// ddgr6 by a warp: the lane of g writes out[g]
 __device__ void ddgr6_warp(const View& v, int lane, int ni, int li, int nj, int lj, int nk, int lk, int nl, int ll,
                            int di, int dj, int dip, double* out) {
   if (-li - lj + lk + ll + di + dj != 0) return;          // out stays 0
   const double r2 = 1.4142135623730951;
-  const int p = dip ? 1 : 0, sm = di + dj;
+  const int p = dip ? 1 : 0, sm = di + dj, g = warp_sum6_at(lane);
   auto tab = [&](int d, int pp) {
     if (pp == 0) return d == 0 ? (int)X00 : d == 1 ? (int)X10 : (int)X20;
     if (d == 1) return pp == 1 ? (int)X11 : (int)X12;
     return pp == 1 ? (int)X01 : (int)X02;
   };
-  double s[NG], sc;
+  double s, sc;
   int tb;
   if (di == 0 && dj == 0) { tb = X00; sc = 1.0; }
   else if (sm == 2 || sm == -2) { tb = tab(2 - p, dip); sc = 2.0; }
   else if (sm == 1 || sm == -1) { tb = dj == 0 ? tab(1 - p, dip) : (int)X10; sc = -sm * r2; }
   else { tb = tab(2 - p, dip); sc = -1.0; }
-  radx6_warp(v, lane, tb, ni, li, nj, lj, nk, lk, nl, ll, s);
-  if (lane == 0)
-    for (int g = 0; g < NG; ++g) out[g] = sc * s[g];
-  if (sm == 0 && !(di == 0 && dj == 0) && dip) {
-    radc6_imag_warp(v, lane, dip, ni, li, nj, lj, nk, lk, nl, ll, s);
-    if (lane == 0)
-      for (int g = 0; g < NG; ++g) out[g] += s[g];
-  }
+  radx6_warp<1>(v, lane, &tb, ni, li, nj, lj, nk, lk, nl, ll, &s);
+  s *= sc;
+  if (sm == 0 && !(di == 0 && dj == 0) && dip)
+    s += radc6_imag_warp(v, lane, dip, ni, li, nj, lj, nk, lk, nl, ll);
+  if (g >= 0) out[g] = s;
+}
+// its pieces (0, 0) and (+1, -1) without a dipole index, which share their sums' terms
+__device__ void ddgr6_pair_warp(const View& v, int lane, int ni, int li, int nj, int lj, int nk, int lk, int nl, int ll,
+                                double* out00, double* outpm) {
+  if (-li - lj + lk + ll != 0) return;
+  const int tab[2] = {X00, X20}, g = warp_sum6_at(lane);
+  double s[2];
+  radx6_warp<2>(v, lane, tab, ni, li, nj, lj, nk, lk, nl, ll, s);
+  if (g >= 0) { out00[g] = s[0]; outpm[g] = -s[1]; }
 }
 
 // jr_vec by a warp into J [NCG] (shared memory)
@@ -904,13 +937,15 @@ __device__ void jr_vec_warp(const View& v, int lane, int na, int la, int nb, int
     TBC_RW(RP0, K, -1, 2); TBC_RW(RZ0, K, 0, 2); TBC_RW(RM0, K, +1, 2);
   }
   if (K == 1) {
-    TBC_RW(RKP, +1, -1, 0); TBC_RW(RKZ, +1, 0, 0); TBC_RW(RKM, +1, +1, 0); TBC_RW(RPZ, 0, 0, 0);
+    TBC_RW(RKZ, +1, 0, 0); TBC_RW(RKM, +1, +1, 0);
   } else if (K == 0) {
-    TBC_RW(RKP, 0, -1, 0); TBC_RW(RKZ, 0, 0, 0); TBC_RW(RKM, +1, 0, 0); TBC_RW(RPM, +1, -1, 0);
+    TBC_RW(RKP, 0, -1, 0); TBC_RW(RKM, +1, 0, 0);
   } else {
-    TBC_RW(RKP, -1, -1, 0); TBC_RW(RKZ, 0, -1, 0); TBC_RW(RKM, +1, -1, 0); TBC_RW(RZM, 0, 0, 0);
+    TBC_RW(RKP, -1, -1, 0); TBC_RW(RKZ, 0, -1, 0);
   }
 #undef TBC_RW
+  ddgr6_pair_warp(v, lane, na, la, nb, lb, nc, lc, nd, ld, J + (K == 1 ? RPZ : K == 0 ? RKZ : RZM) * NG,
+                  J + (K == 1 ? RKP : K == 0 ? RPM : RKM) * NG);
   __syncwarp();
   if (lane < NG) {
     const int g = lane;
@@ -925,18 +960,26 @@ __device__ void jr_vec_warp(const View& v, int lane, int na, int la, int nb, int
   __syncwarp();
 }
 
-// stage 2: one CTA per radial group.  Phase A: the chunk's currents, one (term,
-// branch, direct/exchange) per warp, the lanes splitting each Cartesian sum, into
-// shared memory; phase B: one element per warp, the lanes splitting the chunk's
-// (term, branch) pairs, reduced across the warp into the element's sums.
+// stage 2: one CTA per radial group and share of the term chunks.  Phase A: the chunk's
+// currents, one (term, branch, direct/exchange) per warp, the lanes splitting each
+// Cartesian sum, into shared memory; phase B: one element per warp, the lanes splitting the
+// chunk's (term, branch) pairs, reduced across the warp into the element's sums.
+// Bound by the FP64 pipe.  The cost of a group grows with (2 r_a + |l_a|)(2 r_c + |l_c|), so
+// one CTA per group left the SMs idle for 55 % of the time (208 groups at N_sh = 6); a CTA
+// per chunk evens that out, the costly groups (the last ones) first.  All sums keep their
+// order: a piece that vanishes by symmetry is left with the same rounding.
+// N_sh = 6: 4.5 ms before, now 2.0; N_sh = 8: 24 ms, now 15.
+// grid (ngroups, shares), shares = 1 or the number of chunks; share s sums into
+// acc + s * nelem * 6
 __global__ void __launch_bounds__(TBC_THREADS) k_tbc_field(View v) {
   extern __shared__ double sj[];                 // [TBC_TCH][2][2][NCG]
   __shared__ int ok[TBC_TCH][2];
-  const int grp = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int grp = gridDim.x - 1 - blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int e0 = v.goff[grp], e1 = v.goff[grp + 1];
   const int* q = v.gq + 4 * grp;
   const int ra = q[0], la = q[1], rc = q[2], lc = q[3];
-  for (int t0 = 0; t0 < v.nt; t0 += TBC_TCH) {
+  double* acc = v.acc + (size_t)blockIdx.y * v.goff[gridDim.x] * 6;
+  for (int t0 = blockIdx.y * TBC_TCH; t0 < v.nt; t0 += gridDim.y * TBC_TCH) {
     for (int it = warp; it < TBC_TCH * 4; it += nw) {
       const int tt = it >> 2, br = (it >> 1) & 1, de = it & 1, t = t0 + tt;
       int lb = 0, ld = 0, sd, sb;
@@ -959,14 +1002,21 @@ __global__ void __launch_bounds__(TBC_THREADS) k_tbc_field(View v) {
           stage2_elem(v, grp, e, t0 + tt, br, jd, jd + NCG, gam);
         }
       }
-      warp_sum6(gam);
-      if (lane == 0) {
-        double* a = v.acc + (size_t)e * 6;
-        for (int k = 0; k < 6; ++k) a[k] += gam[k];
-      }
+      const double sum = warp_sum6(gam, lane);
+      const int k = warp_sum6_at(lane);
+      if (k >= 0) acc[(size_t)e * 6 + k] += sum;
     }
     __syncthreads();
   }
+}
+
+// the shares' sums into the first one's, in their order
+__global__ void k_tbc_sum(double* acc, long long n, int shares) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double s = acc[i];
+  for (int k = 1; k < shares; ++k) s += acc[k * n + i];
+  acc[i] = s;
 }
 #endif
 
