@@ -2052,7 +2052,7 @@ static int host_structure(pnfam_ctx* c, int beta_minus, const int* fcols) {
 static void set_chunks(pnfam_ctx* c) {
   const long long n = c->nq * c->qn();
   c->nchunk_bro = (int)((2 * n + BRO_CHUNK - 1) / BRO_CHUNK);
-  c->nchunk_c = (int)std::min<long long>(32, std::max<long long>(1, n / 4096));
+  c->nchunk_c = (int)std::min<long long>(64, std::max<long long>(1, (n + 511) / 512));
 }
 
 extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int* fcols, const double* Fsp,

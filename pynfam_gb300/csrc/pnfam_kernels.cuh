@@ -688,7 +688,7 @@ __global__ void __launch_bounds__(256, sizeof(T) >= 8 ? 1 : 2) k_density(DevBasi
 // shared memory the pipe was 83 % busy, 40 % of it with columns that a block of 1 ... 25
 // does not have and with factors 1/2 that the sums can take along; a warp of one column
 // skips what is missing and needs neither staging nor barriers.  40 points at N_sh = 8:
-// 11.5 ms before, @NEW@ ms.
+// 11.5 ms before, now 7.7 ms.
 // ---------------------------------------------------------------------------
 
 // grid (ceil(nghl/DRT), G, P*2 calls); block 256 = 8 warps x DRT mesh points
@@ -2537,29 +2537,47 @@ __global__ void __launch_bounds__(256) k_gather(const double* __restrict__ in, l
 }
 
 // S_k = -1/pi * (F_k . Re, F_k . Im) for the operator (k=0) and cross terms
-// fops: [nops][nq*nxy]; part: [P][nchunk][2*nops]
+// fops: [nops][nq*nxy]; part: [P][nchunk][2*nops].  grid (nchunk, P)
+// Bound by the chain of loads and sums of a CTA: a chunk is two elements per thread (up to
+// 64 chunks; with one chunk per 4096 elements 16 us for one point at N_sh = 6 and 73 us for
+// five with cross terms in the statistical FAM, now 5.6 and 10.5), and the operators meet at
+// one barrier.
 __global__ void __launch_bounds__(256) k_contract(long long nxy, int nq, int nops, const double* __restrict__ fops,
                                                   const double* __restrict__ vin, int nchunk,
                                                   double* __restrict__ part, const int* __restrict__ active) {
   const int p = blockIdx.y;
   if (!active[p]) return;
-  __shared__ double sh[32];
+  constexpr int KB = 8;
+  __shared__ double sh[8][2 * KB];
+  const int t = threadIdx.x, w = t >> 5;
   const long long n2 = nq * nxy;
   const double* v = vin + (long long)p * 2 * n2;
   const long long chunk = (n2 + nchunk - 1) / nchunk;
   const long long e0 = blockIdx.x * chunk, e1 = min(n2, e0 + chunk);
-  for (int k = 0; k < nops; ++k) {
-    double a = 0.0, b = 0.0;
-    for (long long e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-      const double f = fops[(long long)k * n2 + e];
-      a = fma(f, v[e], a);
-      b = fma(f, v[n2 + e], b);
+  for (int k0 = 0; k0 < nops; k0 += KB) {
+    const int nk = min(KB, nops - k0);
+    if (k0) __syncthreads();
+    for (int k = 0; k < nk; ++k) {
+      double a = 0.0, b = 0.0;
+#pragma unroll 2
+      for (long long e = e0 + t; e < e1; e += 256) {
+        const double f = fops[(k0 + k) * n2 + e];
+        a = fma(f, v[e], a);
+        b = fma(f, v[n2 + e], b);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+      }
+      if ((t & 31) == 0) { sh[w][2 * k] = a; sh[w][2 * k + 1] = b; }
     }
-    const double sa = block_sum(a, sh);
-    const double sb = block_sum(b, sh);
-    if (threadIdx.x == 0) {
-      part[((long long)p * nchunk + blockIdx.x) * 2 * nops + 2 * k] = sa;
-      part[((long long)p * nchunk + blockIdx.x) * 2 * nops + 2 * k + 1] = sb;
+    __syncthreads();
+    if (t < 2 * nk) {
+      double s = 0.0;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) s += sh[i][t];
+      part[((long long)p * nchunk + blockIdx.x) * 2 * nops + 2 * k0 + t] = s;
     }
   }
 }
