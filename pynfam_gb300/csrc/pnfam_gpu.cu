@@ -1301,7 +1301,7 @@ static int sep_init(pnfam_ctx* c, const double* phi) {
     for (int a = 0; a < c->db[i]; ++a)
       if (c->ns[c->st[i] + a] != (a < c->nup[i] ? 1 : -1)) return PNFAM_OK;
   const int ngh = dqp > 0 ? sep_mesh(dqp, nghl, phi) : 0;
-  if (!ngh || ngh > 128 || sep_field_smem<double>(ngh) > SEP_SMEM_MAX) return PNFAM_OK;
+  if (!ngh || ngh > 128 || sep_field_smem<double>(ngh, SEP_ZC) > SEP_SMEM_MAX) return PNFAM_OK;
   SepBasis& B = c->sepb;
   if (!sep_factors(nb, c->db.data(), c->st.data(), c->nup.data(), dqp, nghl, ngh, phi, B)) return PNFAM_OK;
   std::vector<double> f;
@@ -1450,7 +1450,8 @@ static int sep_field(pnfam_ctx* c, int P, int nact, const int* act, const T* rsp
   toc(1);
   tic();
   const int lw = f32 ? live_begin(c, st) : -1;
-  k_sep_field<T><<<dim3(ngl, 8, S.n), 128, sep_field_smem<T>(ngh), st>>>(S, c->devbasis<T>(), dpart);
+  const int zc = sep_field_zc<T>(ngh, S.nzf, S.f.umax);
+  k_sep_field<T><<<dim3(ngl, 8, S.n), SEP_FTHR, sep_field_smem<T>(ngh, zc), st>>>(S, c->devbasis<T>(), zc, dpart);
   // FP32 on a large basis (a unit of F fills a warp) keeps an item in one lane
   const bool whole = f32 && (long long)c->seps[0].items.size() >= 32LL * S.f.nu;
   const int h = whole ? 0 : 1, nw = S.f.nwarp[h] * 2 + S.d[0].nwarp[h] + S.d[1].nwarp[h];

@@ -759,11 +759,11 @@ __global__ void __launch_bounds__(256) k_sep_density(const __grid_constant__ Sep
 // projection 1: the mean field of one class and the unit fields of one radial point and
 // call.  The class's 18 field components at the CTA's mesh points (k_meanfield computes
 // the same 104 of all classes) are dealt to the threads, so that the FP64 pipe works on
-// them in all CTAs and nothing of the field tensor goes through memory; then, for SEP_ZC
+// them in all CTAs and nothing of the field tensor goes through memory; then, for zc
 // column functions at a time, the field is combined with Z' and Z'' into the 13 factors
 // of Z and Z' of the row side (shared memory) and a thread sums two units over the z
 // points, reading each factor once.
-// grid (ngl, 2 calls x 4 classes, points), 128 threads
+// grid (ngl, 2 calls x 4 classes, points), SEP_FTHR threads
 // ---------------------------------------------------------------------------
 // component c (q * 4 + q', 16: (0, 4), 17: pairing) of the field of class cls from the
 // densities d (pnfam_hamiltonian_blas.f90:775-1094, 1201-1208, as in k_meanfield; s: the
@@ -863,18 +863,38 @@ __device__ __forceinline__ cplxT<T> sep_meanfield(int c, int cls, const T* d, in
   }
 }
 
-enum { SEP_ZC = 8, SEP_NX = 13 };
+enum { SEP_ZC = 8, SEP_NX = 13, SEP_FTHR = 128 };
 template <class T>
-__host__ __device__ inline size_t sep_field_smem(int ngh) {
-  const int x = SEP_ZC * SEP_NX * 2;   // the densities (2 ND) share this space
+__host__ __device__ inline size_t sep_field_smem(int ngh, int zc) {
+  const int x = zc * SEP_NX * 2;   // the densities (2 ND) share this space
   return (size_t)(18 * 2 + 1 + (x > 2 * ND ? x : 2 * ND)) * ngh * sizeof(T);
+}
+// column functions per round: the number with the fewest passes of the CTA over its unit
+// sums, a round's factors and barriers counted as a third of a pass.  Up to SEP_ZC, where
+// the space was judged to fit, and beyond while seven CTAs (FP32; four in FP64) fit on an SM.
+// N_sh = 8 has 9 z functions (two rounds at 8, 40 sums of the threads in the second idle),
+// N_sh = 16 17 (8, 8, 1: five passes; 7, 7, 3: three).  FP32, 16 points at N_sh = 8: 60 ->
+// 52 us, 24 at N_sh = 16 121 -> 107 us; FP64, 9 points at N_sh = 16 443 -> 404 us
+template <class T>
+inline int sep_field_zc(int ngh, int nzf, int umax) {
+  const int half = (umax + 1) / 2;
+  int best = 1;
+  long long bcost = -1;
+  for (int zc = 1; zc <= 16 && zc <= nzf; ++zc) {
+    if (zc > SEP_ZC && sep_field_smem<T>(ngh, zc) > (sizeof(T) == 4 ? 31 : 55) * (size_t)1024) break;
+    long long cost = 0;
+    for (int z0 = 0; z0 < nzf; z0 += zc)
+      cost += 3LL * ((std::min(zc, nzf - z0) * half * 2 + SEP_FTHR - 1) / SEP_FTHR) + 1;
+    if (bcost < 0 || cost < bcost) { bcost = cost; best = zc; }
+  }
+  return best;
 }
 
 // dpart: the classes' shares of the densities, as k_sep_density leaves them
 template <class T>
-__global__ void __launch_bounds__(128) k_sep_field(const __grid_constant__ SepDev<T> S,
-                                                   const __grid_constant__ DevBasisT<T> B,
-                                                   const T* __restrict__ dpart) {
+__global__ void __launch_bounds__(SEP_FTHR) k_sep_field(const __grid_constant__ SepDev<T> S,
+                                                        const __grid_constant__ DevBasisT<T> B, int zc,
+                                                        const T* __restrict__ dpart) {
   const int p = sep_point(S, blockIdx.z);
   if (p < 0) return;
   const int ir = blockIdx.x, call = blockIdx.y >> 2, cls = blockIdx.y & 3;
@@ -882,7 +902,7 @@ __global__ void __launch_bounds__(128) k_sep_field(const __grid_constant__ SepDe
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);     // [16 (q, q') + (0, 4) + pairing][2][ngh]
   T* sv = sm + 18 * 2 * ngh;               // [ngh]
-  T* sx = sv + ngh;                        // [SEP_ZC][SEP_NX][2][ngh]
+  T* sx = sv + ngh;                        // [zc][SEP_NX][2][ngh]
   {
     const T* dp = dpart + ((long long)p * 2 + call) * 4 * (2 * ND) * S.nghl + ir * ngh;
     for (int k = threadIdx.x; k < 2 * ND * ngh; k += blockDim.x) {
@@ -906,8 +926,8 @@ __global__ void __launch_bounds__(128) k_sep_field(const __grid_constant__ SepDe
   T* gp = S.g + p * S.gstride;
   const T y = S.y[ir];
   __syncthreads();
-  for (int z0 = 0; z0 < nzf; z0 += SEP_ZC) {
-    const int z1 = min(nzf, z0 + SEP_ZC);
+  for (int z0 = 0; z0 < nzf; z0 += zc) {
+    const int z1 = min(nzf, z0 + zc);
     for (int k = threadIdx.x; k < (z1 - z0) * 2 * ngh; k += blockDim.x) {
       const int ih = k % ngh, pl = (k / ngh) & 1, c = k / (2 * ngh);
       const T Zp = S.z[(2 * (z0 + c)) * ngh + ih], Zdp = S.z[(2 * (z0 + c) + 1) * ngh + ih];
