@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(256) k_sep_density(const __grid_constant__ Sep
 // densities d (pnfam_hamiltonian_blas.f90:775-1094, 1201-1208, as in k_meanfield; s: the
 // sign that changes between the two classes of same or of opposite spins)
 template <class T>
-__device__ __forceinline__ cplxT<T> sep_meanfield(int c, int cls, const T* d, int ld, const double* sc, T crho, T cs,
+__device__ __forceinline__ cplxT<T> sep_meanfield(int c, int cls, const T* d, int ld, const T* sc, T crho, T cs,
                                                   T cpair, T cspair) {
   using Z = cplxT<T>;
   auto D = [&](int k) { return cmk<T>(d[(2 * k) * ld], d[(2 * k + 1) * ld]); };
@@ -867,7 +867,7 @@ enum { SEP_ZC = 8, SEP_NX = 13, SEP_FTHR = 128 };
 template <class T>
 __host__ __device__ inline size_t sep_field_smem(int ngh, int zc) {
   const int x = zc * SEP_NX * 2;   // the densities (2 ND) share this space
-  return (size_t)(18 * 2 + 1 + (x > 2 * ND ? x : 2 * ND)) * ngh * sizeof(T);
+  return (size_t)(18 * 2 + 5 + (x > 2 * ND ? x : 2 * ND)) * ngh * sizeof(T);
 }
 // column functions per round: the number with the fewest passes of the CTA over its unit
 // sums, a round's factors and barriers counted as a third of a pass.  Up to SEP_ZC, where
@@ -890,6 +890,12 @@ inline int sep_field_zc(int ngh, int nzf, int umax) {
   return best;
 }
 
+template <class T>
+__device__ __forceinline__ T sep_to(double x) {
+  if constexpr (sizeof(T) == 4) return f32_of(x);
+  else return x;
+}
+
 // dpart: the classes' shares of the densities, as k_sep_density leaves them
 template <class T>
 __global__ void __launch_bounds__(SEP_FTHR) k_sep_field(const __grid_constant__ SepDev<T> S,
@@ -902,23 +908,36 @@ __global__ void __launch_bounds__(SEP_FTHR) k_sep_field(const __grid_constant__ 
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sm = reinterpret_cast<T*>(smraw);     // [16 (q, q') + (0, 4) + pairing][2][ngh]
   T* sv = sm + 18 * 2 * ngh;               // [ngh]
-  T* sx = sv + ngh;                        // [zc][SEP_NX][2][ngh]
+  T* sc4 = sv + ngh;                       // [crho, cs, cpair, cspair][ngh]
+  T* sx = sc4 + 4 * ngh;                   // [zc][SEP_NX][2][ngh]
+  __shared__ T ssc[12];
   {
     const T* dp = dpart + ((long long)p * 2 + call) * 4 * (2 * ND) * S.nghl + ir * ngh;
     for (int k = threadIdx.x; k < 2 * ND * ngh; k += blockDim.x) {
       const T* q = dp + (long long)(k / ngh) * S.nghl + k % ngh;
       const long long ld = (long long)(2 * ND) * S.nghl;
-      sx[k] = ((q[0] + q[ld]) + (q[2 * ld] + q[3 * ld])) * (T)B.wdcori[ir * ngh + k % ngh];
+      sx[k] = ((q[0] + q[ld]) + (q[2 * ld] + q[3 * ld])) * sep_to<T>(B.wdcori[ir * ngh + k % ngh]);
     }
-    for (int k = threadIdx.x; k < ngh; k += blockDim.x) sv[k] = S.v[ir * ngh + k];
+    // the couplings are FP64: converted once per CTA (and not by the FP64 pipe, which spent
+    // 32 us of 108 on it when every component converted what it used): 24 points at N_sh = 16
+    // 107 -> 103.5 us, 16 at N_sh = 8 52 -> 48 us, FP64 9 points at N_sh = 16 404 -> 375 us
+    for (int k = threadIdx.x; k < ngh; k += blockDim.x) {
+      const int r = ir * ngh + k;
+      sv[k] = S.v[r];
+      sc4[k] = sep_to<T>(B.crho[r]);
+      sc4[ngh + k] = sep_to<T>(B.cs[r]);
+      sc4[2 * ngh + k] = sep_to<T>(B.cpair[r]);
+      sc4[3 * ngh + k] = sep_to<T>(B.cspair[r]);
+    }
+    if (threadIdx.x < 12) ssc[threadIdx.x] = sep_to<T>(B.sc[threadIdx.x]);
     __syncthreads();
     // a warp takes one component at a time: the components' formulas differ
     const int nh = (ngh + 31) / 32 * 32;
     for (int k = threadIdx.x; k < 18 * nh; k += blockDim.x) {
-      const int ih = k % nh, c = k / nh, r = ir * ngh + ih;
+      const int ih = k % nh, c = k / nh;
       if (ih >= ngh) continue;
-      const cplxT<T> f = sep_meanfield<T>(c, cls, sx + ih, ngh, B.sc, (T)B.crho[r], (T)B.cs[r], (T)B.cpair[r],
-                                          (T)B.cspair[r]);
+      const cplxT<T> f = sep_meanfield<T>(c, cls, sx + ih, ngh, ssc, sc4[ih], sc4[ngh + ih], sc4[2 * ngh + ih],
+                                          sc4[3 * ngh + ih]);
       sm[(2 * c) * ngh + ih] = f.r;
       sm[(2 * c + 1) * ngh + ih] = f.i;
     }
