@@ -27,9 +27,7 @@ within 1e-6 (relative) of the FP64 fixed point of the same equations (the FP64
 form converged to 1e-12, computed once and kept in
 tests/golden/bench_fixed_point_nsh16.json).  The plain FP64 form (the drop-in:
 the reference's arithmetic and trajectory, epsilon 1e-7) is measured on the
-same stream and reported beside it.  The pair-tensor GEMMs are tuned once per
-operator when the contexts are set up (outside the timed steps; the choices are
-in the line's "autotune" object).
+same stream and reported beside it.
 
 The same line also carries, unless --no-config4 / --no-stream:
   config4         the large-basis stress configuration: a synthetic Bogoliubov
@@ -94,9 +92,10 @@ TIGHT = 1e-12
 # evaluation there is ~1e-6 of 1e-5, far below epsilon)
 NEAR_EXP = 4
 # DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) over the algorithmic bytes of
-# one pair-tensor GEMM launch, from one ncu capture (N_sh = 12, 16 points)
-TRAFFIC_RATIO = {"density_fp32": 1.662e9 / 1.578e9, "field_projection_fp32": 1.773e9 / 1.739e9}
-TRAFFIC_SOURCE = "profiles/k_pg_gemm_nsh12.md"
+# the two launches of a stage of the unit sums, from one ncu capture (N_sh = 16, 24 points)
+TRAFFIC_RATIO = {"density_fp32": 165.3e6 / 89.8e6, "field_projection_fp32": 95.6e6 / 89.8e6}
+TRAFFIC_SOURCE = "profiles/k_sep_nsh16.md"
+STAGE_KERNELS = {"density_fp32": "k_sep_radial + k_sep_density", "field_projection_fp32": "k_sep_field + k_sep_project"}
 REL = 1e-6
 # mixed form: FP64 anchors beside FP32 increments run asynchronously (--async-anchors)
 ASYNC_ANCHORS = False
@@ -329,15 +328,13 @@ def score(out, fp, nreq):
     return tot, {opname(op): d for op, d in per.items()}
 
 
-def pair_bytes(case, stage, npts):
-    """Algorithmic bytes of one pair-tensor GEMM launch of npts points: the pair tensor
-    (TF32 hi + lo: 16 density pairs or 18 projection pairs per element and mesh point,
-    plus the pairing parts), the points' operands and results."""
+def unit_bytes(case, stage, npts):
+    """Algorithmic bytes of one stage of the FP32 unit sums of npts points: the density
+    matrices in (8 planes of S2) and the classes' shares of the 28 complex densities of both
+    calls out, or these in and the fields out.  The unit sums between a stage's two launches
+    stay in L2."""
     S2 = flops_per_iteration(case)["S2"]
-    n = case.hfb.nghl
-    if stage == "density_fp32":
-        return (16 + 2) * n * S2 * 8 + npts * 8 * S2 * 8 + npts * 4 * 18 * n * 4
-    return (18 + 2) * n * S2 * 8 + npts * (4 * 18 + 4) * n * 8 + npts * 8 * S2 * 4
+    return npts * (8 * S2 + 2 * 4 * 56 * case.hfb.nghl) * 4
 
 
 def cpu_iteration_sample(cases, omegas, n_per_op=1):
@@ -502,23 +499,19 @@ def run_gpu(args):
     h2d = len(OPERATORS) * h2d_ctx + sum(8 * c.F.mat.nelem * (1 + len(c.G)) for c in cases) + 16 * npts
     d2h = sum(npts // len(OPERATORS) * (16 * (1 + len(c.G)) + 4 + 8 + 8) for c in cases)
     e2e_value = world * e2e_ok / e2e_wall
-    # ---- roofline of the dominant FP32 kernel (the pair-tensor GEMMs: HBM-bound) ----
+    # ---- roofline of the dominant FP32 field stage (the unit sums; their bytes are few) ----
     fl = flops_per_iteration(cases[0])
     stages = {}
     for prof, _ in profs_t.values():
         for k, v in prof.items():
             if k != "total" and not k.startswith("live_") and not k.startswith("tuned_") and k != "autotune_ms":
                 stages[k] = stages.get(k, 0.0) + v
-    autotune = {opname(op): {"pair_tensor_from_points": int(p["tuned_pair_min_points"]),
-                             "density_k_chunks_per_task": int(p["tuned_density_kspan"]),
-                             "ms": p["autotune_ms"]}
-                for op, (p, _) in profs_t.items()}
     stage_fl = {"field_projection_fp32": fl["field_projection"], "density_fp32": fl["density"]}
     dom = max(live, key=lambda k: live[k][1])
     nl, ms = live[dom]
     pts_per_launch = pit32 / max(nl, 1)
     launch_ms = ms / max(nl, 1)
-    alg = pair_bytes(cases[0], dom, pts_per_launch)
+    alg = unit_bytes(cases[0], dom, pts_per_launch)
     achieved = alg / (launch_ms / 1e3) / 1e9
     # the same launches alone on the GPU: the serialised stage run
     pit32_t = max(stages.get("point_iterations_fp32", 0.0), 1.0)
@@ -567,13 +560,12 @@ def run_gpu(args):
             "gpu_launches": launches,
             "stages_ms": {k: round(v, 3) for k, v in stages.items()},
             "stages_note": "one extra serialised run with events between stages (not the timed steps)",
-            "autotune": autotune,
-            "roofline": {"bound": "hbm", "kernel": f"k_pg_gemm ({dom})", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "issue", "kernel": f"{STAGE_KERNELS[dom]} ({dom})", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak,
                          "traffic": alg * TRAFFIC_RATIO[dom],
                          "traffic_unit": f"DRAM bytes read + written per launch ({pts_per_launch:.1f} points): "
                                          f"algorithmic bytes x the DRAM/algorithmic ratio of one ncu capture "
-                                         f"({TRAFFIC_SOURCE}); the pair tensor grows with S2, so the ratio carries",
+                                         f"({TRAFFIC_SOURCE})",
                          "algorithmic_bytes": alg, "launches": nl, "mean_launch_ms": launch_ms,
                          "points_per_launch": pts_per_launch,
                          "achieved_alone": achieved_alone, "frac_alone": achieved_alone / peak,
@@ -582,11 +574,13 @@ def run_gpu(args):
                          "reference_tflops_alone": stage_fl[dom] * pts_per_launch / max(alone_ms / 1e3, 1e-12) / 1e12,
                          "tf32_peak_tflops": bf16 / 2,
                          "peak_source": src,
-                         "note": "achieved = algorithmic bytes per launch (pair tensor + the points' operands "
-                                 "and results) / mean launch time, CUDA events around every launch of the kernel "
-                                 "on its own stream in the timed steps, where the five engines' kernels share "
-                                 "the GPU; *_alone: the same launches from the serialised stage run; "
-                                 "reference_tflops: the reference's operation count of the stage at that rate"},
+                         "note": "achieved = algorithmic bytes of the stage's two launches (density matrices and "
+                                 "densities or fields) / their mean time, CUDA events around the two on their "
+                                 "own stream in the timed steps, where the five engines' kernels share the GPU; "
+                                 "*_alone: the same launches from the serialised stage run; the stage is bound "
+                                 "by instruction issue and shared memory, not by these bytes; "
+                                 "reference_tflops: the reference's operation count of the stage (sums over the "
+                                 "whole mesh, which the unit sums do not execute) at that rate"},
             "clocks": ck}
     if rank == 0 and world == 1:
         t_iter = cpu_iteration_sample(cases, omegas)
@@ -839,15 +833,12 @@ def run_config4(args, emit=True):
     state's iteration does not converge, so the measure is FAM point-iterations per
     second), through one continuous-batching engine per operator, in the mixed form and
     in the FP64 form.  A separate timed run gives the per-stage device time, from which
-    the stage rates (reference FLOP counts per TF32 or FP64 peak; HBM bytes of the
-    pair-tensor stream per measured HBM peak) follow."""
+    the stage rates (the reference's FLOP counts over the stage's time) follow."""
     import torch
     from pynfam_gb300.contour import circle
     from pynfam_gb300.serve import Request, Server
     from pynfam_gb300.solver import GPUSolver
     torch.cuda.set_device(0)
-    # the pair tensors of N_sh = 20 (about 62 GB per operator) stay off: the per-block
-    # tensor-core kernels evaluate these points
     t0 = time.perf_counter()
     hfb, cases = config4_cases()
     omegas = circle(-15.0, 35.0, 2 * args.c4_points)
@@ -877,7 +868,7 @@ def run_config4(args, emit=True):
     # the FP64 form (about 40 point-iterations/s here) on the first c4_fp64_points points
     for precision, name, npts in ((1, "mixed", None), (0, "fp64", args.c4_fp64_points)):
         if precision == 1:
-            serve(precision)                   # warm-up (FP32 scratch, autotuning)
+            serve(precision)                   # warm-up (FP32 scratch)
         wall, out = serve(precision, npts=npts)
         npi = sum(iters if o.iters < 0 else o.iters for o in out)
         res[name] = {"point_iterations_per_s": npi / wall, "wall_s": wall, "point_iterations": npi,
@@ -901,11 +892,8 @@ def run_config4(args, emit=True):
         ms = sum(stages.get(k, 0.0) for k in key)
         flops = sum(flops_per_iteration(c)[stage] for c in cases) / len(cases) * pit32
         d = {"ms": ms, "tflops": flops / (ms * 1e-3) / 1e12 if ms > 0 else None}
-        d["tensor_frac_of_tf32_peak"] = d["tflops"] / tf32 if d["tflops"] else None
-        if stage != "block_gemm":
-            key2 = "density_fp32" if stage == "density" else "field_projection_fp32"
-            byts = sum(pair_bytes(c, key2, 0) for c in cases) / len(cases)
-            d["pair_tensor_gb"] = byts / 1e9
+        if stage == "block_gemm":   # the fields' sums do not run on the tensor cores
+            d["tensor_frac_of_tf32_peak"] = d["tflops"] / tf32 if d["tflops"] else None
         per_stage[stage] = d
     per_stage["broyden"] = {"ms": stages.get("broyden", 0.0)}
     line = {"config": "large-basis stress (N_sh=20 synthetic Bogoliubov seed 3, Omega-only blocks up to 231, "
@@ -916,9 +904,9 @@ def run_config4(args, emit=True):
             "unit": "FAM point-iterations/s", "mixed": res["mixed"], "fp64_form": res["fp64"],
             "mixed_over_fp64": res["mixed"]["point_iterations_per_s"] / res["fp64"]["point_iterations_per_s"],
             "stages_mixed": per_stage, "stage_point_iterations": {"fp32": pit32, "fp64": pit64},
-            "note": "stage rates from one serialised run with events between stages; tensor fraction = reference "
-                    "FLOPs per second over the TF32 dense peak (half the measured bf16 peak), 3xTF32 issues three "
-                    "MMAs per product"}
+            "note": "stage rates (the reference's FLOP counts, more than the stages execute) from one serialised run "
+                    "with events between stages; tensor fraction = reference FLOPs per second over the TF32 dense "
+                    "peak (half the measured bf16 peak), 3xTF32 issues three MMAs per product"}
     for g in gpus:
         g.close()
     if emit:

@@ -82,7 +82,8 @@ typedef struct {
                                  (Re and Im of the strength and each cross term) to have
                                  settled, |S - S_previous| <= 10^-n |S| + 1e-13 max|S|, for
                                  at most 20 iterations beyond si < epsilon (0: the
-                                 reference's test si < epsilon alone);
+                                 reference's test si < epsilon alone, and in the mixed form
+                                 the pair-tensor GEMMs where they fit);
                                  [4] = n > 0: the mixed form's "near its anchor" bound is
                                  10^n epsilon instead of 1000 epsilon;
                                  [5] != 0: mixed form, asynchronous anchors: an FP64 anchor
@@ -313,18 +314,21 @@ long long pnfam_gpu_nxy(const pnfam_ctx_t* ctx);
 
 /* Timing of the last solve: per stage accumulated device ms (order:
  * k1_blockgemm, density, meanfield, field_projection, k2_blockgemm, green,
- * broyden, strength; filled only when opts.reserved[0] != 0), then, if
+ * broyden, strength; filled only when opts.reserved[0] != 0; where the fields are
+ * summed direction by direction the mean field is part of field_projection, in the
+ * mixed form the Green's function is part of broyden), then, if
  * nstage > 8, the whole solve's device time (CUDA events on the solver's
  * stream), if nstage > 10 the FP64 and FP32 point-iterations of the solve,
  * then (entries 11-15) the first five stages of the FP32 evaluations of the
  * mixed form (entries 0-4 then hold the FP64 evaluations only), then (entries
  * 16-19, with opts.reserved[2] != 0) the number and total device ms of the FP32
- * density launches and of the FP32 field-projection launches, then (entries
- * 20-22) the autotuner's choices for the context's operator: the point count from
+ * density launches and of the FP32 field-projection launches (one or two kernels each),
+ * then (entries
+ * 20-22) the autotuner's choices for the context's operator, where it ran: the point count from
  * which FP32 evaluations take the pair-tensor GEMMs (2^30: never), the K chunks per
  * density task of those GEMMs, and the autotuner's host time in ms (0: not run; it
- * runs once per operator when the first mixed-form engine or solve sets up its FP32
- * buffers, unless PNFAM_GB300_AUTOTUNE=0), and the number of kernel launches.  An
+ * runs once per operator when the first mixed-form engine or solve that can take those
+ * GEMMs sets up its FP32 buffers, unless PNFAM_GB300_AUTOTUNE=0), and the number of kernel launches.  An
  * engine's figures accumulate from its creation. */
 int pnfam_gpu_last_profile(const pnfam_ctx_t* ctx, double* stage_ms, int nstage,
                            long long* launches);

@@ -184,8 +184,8 @@ class GPUSolver:
     def calc_hamiltonian(self, rho_pn, kp, rho_np, km, mixed=False):
         """Plugin seam: complex flat arrays (nxy) in the structures documented in
         include/pnfam_gpu.h; returns (h_pn, Delta+, h_np, Delta-) complex.
-        mixed=True evaluates in FP32 with the tensor-core projection (the
-        kernels of the mixed form's increment evaluations)."""
+        mixed=True evaluates in FP32 (the kernels of the mixed form's increment
+        evaluations)."""
         n = self.nxy
         ins = [np.ascontiguousarray(a, dtype=complex) for a in (rho_pn, kp, rho_np, km)]
         if min(a.size for a in ins) < n:
