@@ -2547,7 +2547,7 @@ static int engine_launch(pnfam_engine* e, bool block_if_idle) {
   const double* E2 = c->beta_minus ? c->d_en.p : c->d_ep.p;
   const int nq = c->nq;
   if (nfresh) {  // newly admitted slots start from X = 0, with their Green's function
-    k_vecop<<<vgrid, 256, 0, c->stream>>>(2, 0.0, c->d_state.p, nullptr, N, d_fresh);
+    k_zero<<<vgrid, 256, 0, c->stream>>>(c->d_state.p, N, d_fresh);
     const int gx = (int)std::min<long long>(4096, (nq * nxy + 255) / 256);
     const double* f1 = nq == 4 ? (c->beta_minus ? c->d_fp.p : c->d_fn.p) : nullptr;
     const double* f2 = nq == 4 ? (c->beta_minus ? c->d_fn.p : c->d_fp.p) : nullptr;

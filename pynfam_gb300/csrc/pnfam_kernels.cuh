@@ -2299,9 +2299,9 @@ __global__ void __launch_bounds__(256) k_bro_update(BroState S, const double* __
 // Broyden of the mixed form.  The history columns df_k and u_k are kept as pairs
 // of floats (hi + lo, about 48 significant bits) and every product with them is
 // formed in pair arithmetic on the FP32 cores, which GB300 runs at dozens of times
-// its FP64 rate; the raw vout and vin of the previous step and this step's raw
-// differences stay FP64, so the secant pairs are formed before any rounding, and
-// the small solve is FP64 (k_bro_solve).  Same steps as k_bro_diff / k_bro_dots /
+// its FP64 rate; the residuals of this and the previous step and the vectors themselves
+// stay FP64, so the secant pairs are formed before any rounding, and the small solve
+// is FP64 (k_bro_solve).  Same steps as k_bro_diff / k_bro_dots /
 // k_bro_update.
 // ---------------------------------------------------------------------------
 struct BroState2 {
@@ -2333,10 +2333,10 @@ struct BroState2 {
 // The columns are stored before their norm is known, scaled by the power of two that
 // brings the previous residual's maximum (si) to 1; cs carries the norm.
 // Bound by FP64 (8 operations per element) in the first iterations and by the reads of the
-// columns later.  As k_green, two copies, k_bro_diff2 and k_bro_dots2 with FP64
-// conversions, sums and normalisation these took 1.2, 2.0 and 3.6 ms for 64 points at
-// N_sh = 20 with 3 columns; in this form 3.2 ms.  k_bro_update2 there 1.5 -> 1.16 ms,
-// k_to_f32 0.78 -> 0.53 ms.
+// columns later.  As separate passes with FP64 conversions, sums and normalisation (Green's
+// function, copies, differences, dots) these took 1.2, 2.0 and 3.6 ms for 64 points at N_sh =
+// 20 with 3 columns; in this form 3.2 ms.  With 35 to 55 columns (24 points, N_sh = 16) it reads
+// at 4.5-5.4 TB/s.  k_bro_update2 there 1.5 -> 1.16 ms and 6.2 TB/s, k_to_f32 0.78 -> 0.53 ms.
 __global__ void __launch_bounds__(256, 4) k_bro_step2(BroState2 S, const double* __restrict__ hqp,
                                                       const float* __restrict__ hqp32, const double* __restrict__ fqp,
                                                       const double* __restrict__ gfn, double quench,
@@ -2513,20 +2513,13 @@ __global__ void __launch_bounds__(256) k_bro_update2(BroState2 S, const double* 
   *vin = make_double2(old.x + (S.alpha * v.x - pair_value(a, -s)), old.y + (S.alpha * v.y - pair_value(b, -s)));
 }
 
-// per-point vector operations, [P][n] layout:
-// op 0: dst = src; op 1: dst += src; op 2: dst = 0; op 3: dst = a*src
-__global__ void k_vecop(int op, double a, double* __restrict__ dst, const double* __restrict__ src, long long n,
-                        const int* __restrict__ mask) {
+// dst = 0 for the points with mask[p], [P][n] layout
+__global__ void k_zero(double* __restrict__ dst, long long n, const int* __restrict__ mask) {
   const int p = blockIdx.y;
   if (!mask[p]) return;
   double* d = dst + (long long)p * n;
-  const double* s_ = src ? src + (long long)p * n : nullptr;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    if (op == 0) d[e] = s_[e];
-    else if (op == 1) d[e] += s_[e];
-    else if (op == 2) d[e] = 0.0;
-    else d[e] = a * s_[e];
-  }
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+    d[e] = 0.0;
 }
 
 // out[k][e] = in[k][idx[e]]; grid (ceil(n / 256), rows)

@@ -24,7 +24,7 @@
 // (40 points): 23 and 18 us against 39 and 41 us of the pair-tensor GEMMs, whose operand
 // (12 GB) is not needed; errors against FP64 2e-7 instead of 8e-6.  (First form; with the
 // staging that the kernels below describe 16 and 17 us in FP32, 24 points: radial sums
-// 264, z sums 111, unit fields 121, projection 298 us.)
+// 264, z sums 111, unit fields 104, projection 298 us.)
 //
 // The factors are recovered from the basis functions that the caller passes
 // (sep_factors) and every value of the products is compared with them (k_sep_check);
