@@ -1263,6 +1263,7 @@ static int launch_gemm(pnfam_ctx* c, TaskList& tl, int P, const int* active, cud
 static int launch_gemm_tc(pnfam_ctx* c, int list, int nact, cudaStream_t st) {
   const TaskListTC& tl = c->tc32[c->form].l[list];
   if (tl.tasks.empty() || nact <= 0) return PNFAM_OK;
+  if (!c->tc32[c->form].built) return fail(PNFAM_ESTATE, "block GEMMs without their pre-split operands");
   dim3 grid((unsigned)tl.tasks.size(), (unsigned)((2 * nact * tl.maxrows + 127) / 128));
   k_gemm_tc<<<grid, GTC_THREADS, gemm_tc_smem_bytes(tl.maxnp), st>>>(tl.d_tasks.p, c->d_bufs32.p,
                                                                       c->tc32[c->form].gsplit.p, c->d_actlist.p, nact, tl.maxnp, c->d_err.p);
@@ -1739,7 +1740,9 @@ static int pg_autotune(pnfam_ctx* c, int P) {
 }
 
 // FP32 copies of the ground state and FP32 scratch for P points; pair: for evaluations
-// that may take the pair-tensor GEMMs; run: for an engine's run (its block GEMMs too)
+// that may take the pair-tensor GEMMs; run: for an engine's run, which also takes the block
+// GEMMs and, where general, the pair tensor (a field evaluation takes neither, and the
+// tuner's trials need the block GEMMs' operands)
 static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
   const long long nxy = c->nxy;
   const size_t mo = (size_t)(c->uoff.back() + (long long)c->db.back() * c->db.back());
@@ -1782,7 +1785,7 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
   // what the general kernels need (a separable basis: only for the pair-tensor GEMMs of
   // uncertified runs, whose point count is tuned against the per-block kernels)
   const bool general = !c->sep32 || pair;
-  if (general) pg_prepare(c);
+  if (general && run) pg_prepare(c);
   if (c->tc_density && general) {
     CK(dalloc(c->d_bsplit, (size_t)P * c->bstride));
     if (!c->have_aphi) {
@@ -1831,7 +1834,7 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
       set.built = true;
     }
   }
-  if (!general) return PNFAM_OK;
+  if (!general || !run) return PNFAM_OK;
   {
     const int rc = pg_build(c);
     if (rc) return rc;
