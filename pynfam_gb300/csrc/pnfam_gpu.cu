@@ -1390,10 +1390,9 @@ static int sep_operator(pnfam_ctx* c) {
     CK(upload(d.items, items[k].data(), items[k].size()));
     for (int h = 0; h < 2; ++h) CK(upload(d.warps[h], s.warps[h].data(), s.warps[h].size()));
   }
-  const long long ngl = c->sepb.ngl, nf = (long long)c->seps[0].units.size();
-  c->sep_gpair[0] = 2 * ngl * nf * 2 * SH_N;
-  c->sep_gpair[1] = c->sep_gpair[0] + 2 * ngl * (long long)std::max(c->seps[1].units.size(), c->seps[3].units.size());
-  c->sep_gstride = c->sep_gpair[1] + 2 * ngl * (long long)std::max(c->seps[2].units.size(), c->seps[4].units.size());
+  long long nu[5];
+  for (int k = 0; k < 5; ++k) nu[k] = (long long)c->seps[k].units.size();
+  c->sep_gstride = sep_sums(c->sepb.ngl, nu, c->sep_gpair);
   return PNFAM_OK;
 }
 

@@ -371,6 +371,18 @@ enum { SG_RR = 0, SG_DR, SG_RD, SG_DD, SG_ARR, SG_BRR, SG_ABRR, SG_BDR, SG_ARD, 
 // the projection's unit fields: the same nine, then the (0, 4) and (4, 0) field
 enum { SH_L = SG_N, SH_N };
 
+// values of one point's unit sums, for nu units of the structures F, X^T, Y^T, X and Y:
+// per call the F units [ngl][nu][SH_N][2 planes], then per call, from gpair[call] on, the
+// pairing units [ngl][nu][2 planes] (densities and fields in the same place).  A multiple of
+// 4, so that every point's sums start on 16 bytes in FP32 too: k_sep_project reads the F
+// units 16 bytes at a time
+inline long long sep_sums(long long ngl, const long long nu[5], long long gpair[2]) {
+  gpair[0] = 2 * ngl * nu[0] * 2 * SH_N;
+  gpair[1] = gpair[0] + 2 * ngl * std::max(nu[1], nu[3]);
+  const long long n = gpair[1] + 2 * ngl * std::max(nu[2], nu[4]);
+  return (n + 3) / 4 * 4;
+}
+
 }  // namespace pnfam
 
 #ifdef __CUDACC__
@@ -395,9 +407,7 @@ struct SepDev {
   const typename Vec2<T>::t *r, *rt;   // (R, R') as [nrow][ngl] and as [ngl][nrow]
   const T *z, *v, *y, *e, *lam, *sgn;
   SepStructDev f, k[2], d[2];     // F; pairing densities (X^T, Y^T); pairing fields (X, Y)
-  // unit sums of one point: per call the F units [ngl][nu][SH_N][2 planes], then per
-  // call the pairing units [ngl][nu][2 planes]
-  long long gstride, gpair[2];
+  long long gstride, gpair[2];    // of one point's unit sums (sep_sums)
   T* g;                           // [P][gstride]
   // the points of a launch: a list, or (list null) all P with their flags
   const int *list, *act;
