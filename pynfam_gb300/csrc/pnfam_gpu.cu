@@ -1292,7 +1292,7 @@ static int residual_k2(pnfam_ctx* c, int P, int nact, const int* act, cudaStream
 // ---------------------------------------------------------------------------
 // basis of z x radial products (separable.cuh)
 // ---------------------------------------------------------------------------
-static constexpr int SEP_SMEM_MAX = 200 * 1024;   // dynamic shared memory of k_sep_field
+static constexpr int SEP_SMEM_MAX = 200 * 1024;   // dynamic shared memory of the k_sep_* kernels
 
 // look for the factors (once per context); c->sep stays false when the basis functions
 // are not products or a size is beyond what the kernels take
@@ -1337,7 +1337,8 @@ static int sep_init(pnfam_ctx* c, const double* phi) {
   d_bad.release();
   CK(err);
   const int ng = std::max(1, std::min(B.nzf, 128 / ngh));
-  c->sep = bad == 0 && sep_dens_smem<double>(ngh, ng, B.nzf) <= SEP_SMEM_MAX;
+  c->sep = bad == 0 && sep_dens_smem<double>(ngh, ng, B.nzf) <= SEP_SMEM_MAX &&
+           sep_project_smem<double>(B.ngl, B.nrow, 1, false) <= SEP_SMEM_MAX;   // up to 1280 radial points
   return PNFAM_OK;
 }
 
@@ -1998,6 +1999,12 @@ extern "C" int pnfam_gpu_init(const pnfam_basis_t* basis, const double* Ep, cons
       cudaFuncSetAttribute(k_sep_project<float, SEP_SPL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            SEP_SMEM_MAX) != cudaSuccess ||
       cudaFuncSetAttribute(k_sep_project<float, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SEP_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_project<double, SEP_SPL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SEP_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_project<float, SEP_SPL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SEP_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(k_sep_project<float, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            SEP_SMEM_MAX) != cudaSuccess) {
     delete c;
     return fail(PNFAM_ECUDA, "pnfam_gpu_init: cannot configure shared memory");
