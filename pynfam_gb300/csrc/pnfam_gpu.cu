@@ -288,7 +288,7 @@ struct pnfam_ctx {
   DBuf<int> d_actlist;   // [P] points of the current FP32 evaluation (tensor-core tiles)
   DBuf<int> d_err;       // set by a tensor-core kernel whose wait gave up
   // per-solve buffers
-  int cap_P = 0, cap_M = 0;
+  int cap_P = 0, cap_M = 0;   // most points and longest history of the runs so far
   DBuf<double> d_state, d_vout, d_T, d_rsp, d_hsp, d_hqp, d_dpart, d_mf;
   DBuf<double> d_zio;   // [4][nxy] complex: arrays of calc_hamiltonian_z
   DBuf<double> d_df, d_dv, d_bpart, d_si, d_norm, d_beta, d_gamma, d_cpart, d_wre, d_wim;
@@ -2149,9 +2149,10 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
   CK(upload(c->d_bchunks, c->bchunks.data(), c->bchunks.size()));
   if (!c->have_aphi) CK(upload(c->d_achunks, c->achunks.data(), c->achunks.size()));
   c->have_op = true;
-  int rc = ensure_buffers(c, std::max(1, c->cap_P), std::max(1, c->cap_M));
+  // one point for F_qp, in whole blocks: a run sizes the buffers of its form (engine_setup),
+  // so that those of an earlier run in the active form are not made whole here
+  int rc = ensure_buffers(c, 1, 1);
   if (rc) return rc;
-  c->cap_P = std::max(1, c->cap_P); c->cap_M = std::max(1, c->cap_M);
   // F_qp and cross terms: K2 applied to dH_sp = (F, 0, 0, 0) (pnfam_solver.f90:368-381)
   CK(dalloc(c->d_fops, (size_t)c->nops * nq * nf));
   std::vector<int> one = {1};
@@ -2993,11 +2994,8 @@ static int field_fp32_status(pnfam_ctx* c, const char* who) {
 }
 
 static int field_buffers(pnfam_ctx* c, bool mixed) {
-  int rc = ensure_buffers(c, std::max(1, c->cap_P), std::max(1, c->cap_M));
-  if (rc) return rc;
-  if (!mixed) return PNFAM_OK;
-  c->cap_P = std::max(1, c->cap_P); c->cap_M = std::max(1, c->cap_M);
-  return ensure_buffers32(c, c->cap_P, false, false);
+  const int rc = ensure_buffers(c, 1, 1);
+  return rc || !mixed ? rc : ensure_buffers32(c, 1, false, false);
 }
 
 extern "C" int pnfam_gpu_calc_hamiltonian(pnfam_ctx_t* c, const double* re_rho_pn, const double* im_rho_pn,
