@@ -727,7 +727,7 @@ def run_serve_stream(args, emit=True):
     from pynfam_gb300.contour import circle
     from pynfam_gb300.namelist import defaults, parse_namelist_text
     from pynfam_gb300.pnfam_setup import setup_case
-    from pynfam_gb300.serve import Request, Server, poisson_arrivals, slot_bytes
+    from pynfam_gb300.serve import Request, Server, field_bytes, poisson_arrivals, slot_bytes
     from pynfam_gb300.solver import GPUSolver
     from pynfam_gb300.synthetic import ground_state
     rng = np.random.default_rng(args.stream_seed)
@@ -755,7 +755,7 @@ def run_serve_stream(args, emit=True):
         c = cases[key]
         h = c.hfb
         ground = 12 * (5 * h.dqp * h.nghl + 4 * int(sum(int(b.size) for b in h.Up)))
-        return n * slot_bytes(c.F.mat.nelem, M, True) + ground
+        return n * slot_bytes(c.F.mat.nelem, M, True, field=field_bytes(h, c.F.mat.cols, True)) + ground
 
     def factory(key, n):
         c = cases[key]

@@ -66,15 +66,51 @@ class ServeStats:
         return float(np.percentile(self.latencies, q)) if self.latencies else float("nan")
 
 
-def slot_bytes(nxy: int, broyden_m: int, mixed: bool, statistical: bool = False) -> int:
-    """Device memory of one solve slot (the per-point buffers of pnfam_gpu.cu); the
-    statistical FAM doubles the QP-state arrays (quadrants P and Q) and the scratch."""
+def field_bytes(hfb, cols, mixed: bool) -> int:
+    """Device memory that the field evaluations of one solve slot take on the mesh and in the
+    unit sums (pnfam_gpu.cu: d_dpart, d_mf, d_sepg, with their FP32 copies), for an operator
+    with the block columns ``cols``. It does not grow with nxy like the rest of a slot
+    (``slot_bytes``) and is most of it on small bases."""
+    nb, n = int(hfb.nb), int(hfb.nghl)
+    cols = np.asarray(cols)
+    # groups of block rows of the densities over the mesh: two CTAs per SM, 32 points each
+    groups = max(4, min(int(np.sum(cols >= 0)), -(-2 * 152 // -(-n // 32))))
+    doubles = 2 * groups * 2 * 28 * n + 2 * 104 * 2 * n
+    # units: (spin of the row, of the column, n_z, n_z') that occur in a block pair
+    nz = np.asarray(hfb.nz)
+    has = np.zeros((nb, 2, int(nz.max()) + 1), dtype=bool)
+    for i in range(nb):
+        at, up = int(hfb.isstart[i]), int(hfb.num_spin_up[i])
+        has[i, 0, nz[at:at + up]] = True
+        has[i, 1, nz[at + up:at + int(hfb.db[i])]] = True
+
+    def units(c):
+        rows = np.flatnonzero(c >= 0)
+        return int(np.count_nonzero(np.einsum("isz,itw->stzw", has[rows].astype(int), has[c[rows]].astype(int))))
+
+    tr = np.array([hfb.partner(i) for i in range(nb)])
+    x, y = np.where(cols >= 0, tr[cols], -1), cols[tr]
+
+    def transposed(c):
+        t = np.full(nb, -1)
+        t[c[c >= 0]] = np.flatnonzero(c >= 0)
+        return t
+
+    ngl = n // int(hfb.hel.ngh)
+    doubles += 2 * ngl * (20 * units(cols) + max(units(x), units(transposed(x))) + max(units(y), units(transposed(y)))) + 3
+    return doubles * (12 if mixed else 8)
+
+
+def slot_bytes(nxy: int, broyden_m: int, mixed: bool, statistical: bool = False, field: int = 0) -> int:
+    """Device memory of one solve slot (the per-point buffers of pnfam_gpu.cu), quasiparticle
+    states in whole blocks; the statistical FAM doubles the QP-state arrays (quadrants P and
+    Q) and the scratch. field: what its field evaluations take (``field_bytes``)."""
     q = 2 if statistical else 1
     f64 = q * (4 + 4 + 16 + 4 + 4 + 2 * 4 * max(broyden_m, 1)) + 8 + 8   # state, vout, T, hqp, G, df+dv; rsp, hsp
     if mixed:
-        f64 += 4 + 4 + 4 * 4                                     # anchor, its image; Broyden raw vectors
-    f32 = (4 + 16 + 8 + 8 + 4) if mixed else 0
-    return int(nxy) * (8 * f64 + 4 * f32)
+        f64 += q * (4 + 4 + 4 + 4)                               # anchor, its image; the last step's residual and state
+    f32 = (q * (4 + 16 + 4) + 8 + 8) if mixed else 0             # state, T, hqp; rsp, hsp
+    return int(nxy) * (8 * f64 + 4 * f32) + int(field)
 
 
 class Server:
