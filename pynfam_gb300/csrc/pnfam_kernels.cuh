@@ -2469,12 +2469,8 @@ __global__ void __launch_bounds__(256, 4) k_bro_step2(BroState2 S, const double*
         for (int j = l; j < half; j += 32) add(__ldcs(fk + j), sf[c][j], sv[c][j]);
       }
     }
-    a = pair_warp_sum(a);
-    b = pair_warp_sum(b);
-    if (l == 0) {
-      pt[(long long)(2 + k) * S.nchunk] = pair_value(a);
-      pt[(long long)(2 + 64 + k) * S.nchunk] = pair_value(b);
-    }
+    const double sum = pair_warp_sums(a, b, l);
+    if ((l & 15) == 0) pt[(long long)(2 + (l ? 64 : 0) + k) * S.nchunk] = sum;
   }
 }
 
