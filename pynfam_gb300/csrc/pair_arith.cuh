@@ -47,9 +47,9 @@ PAIR_HD float pair_float(unsigned b) {
 }
 
 // x * 2^s as a pair: the leading 24 bits, and the other 29 rounded to 24.  Exact to 2^-49
-// of x for 2^-74 <= |x 2^s| < 2^127 (callers choose s so that the largest value of a
-// vector is about 1); below, the low part is 0, below 2^-126 both are; overflow gives an
-// infinity, as a conversion does
+// of x for 2^-100 <= |x 2^s| < 2^127 (callers choose s so that the largest value of a
+// vector is about 1), below to the least denormal float, 2^-149; overflow gives an infinity,
+// as a conversion does
 PAIR_HD float2 pair_split(double x, int s = 0) {
   const unsigned long long b = pair_bits(x);
   const unsigned h = (unsigned)(b >> 32), l = (unsigned)b;
@@ -63,8 +63,13 @@ PAIR_HD float2 pair_split(double x, int s = 0) {
   if (er == 0 || e < 949 || e > 1150) {
     o.y = 0.f;
     if (er == 2047) o.x = pair_float(sg | 0x7f800000u | (m | r ? 0x400000u : 0u));
-    else if (er == 0 || e < 897) o.x = pair_float(sg);
+    else if (er == 0) o.x = pair_float(sg);
     else if (e > 1150) o.x = pair_float(sg | 0x7f800000u);
+    else if (e >= 872) {   // the scale of the low part, or of both, in two steps
+      const float q = 7.888609052210118e-31f;   // 2^-100
+      if (e < 897) o.x = pair_float(sg | ((127u << 23) + m + up)) * pair_float((unsigned)(e - 796) << 23) * q;
+      else o.y = (float)((int)r - (int)(up << 29)) * pair_float(sg | ((unsigned)(e - 848) << 23)) * q;
+    } else o.x = pair_float(sg);
   }
   return o;
 }
