@@ -77,7 +77,11 @@ SEP_HD double sep_value(int q, const double* z, const double* r, double v, doubl
 }
 
 // the factors of phi [5][dqp][nghl] for a mesh of ngh points along z; false when the
-// functions are plainly not of the product form (sep_value still has to be compared)
+// functions are plainly not of the product form (sep_value still has to be compared).
+// Blocks nb / 2 ... are the time-reversed partners of the first half: their states are tried
+// with the factors of the partner's (same functions, spins exchanged) before a search, and
+// the others' searches look at one value before they compare whole functions. Host time,
+// Grace: 0.11 ms at N_sh = 6 and 1.6 at 16 (0.33 and 4.3 with a full search for every state)
 inline bool sep_factors(int nb, const int* db, const int* st, const int* nup, int dqp, int nghl, int ngh,
                         const double* phi, SepBasis& B) {
   const int ngl = nghl / ngh;
@@ -91,84 +95,117 @@ inline bool sep_factors(int nb, const int* db, const int* st, const int* nup, in
   std::vector<double> ztop;             // and Z there
   std::vector<std::vector<double>> lseg(2 * nb);
   std::vector<double> row(ngl * 2), wbest(ngl);
+  std::vector<int> peer(dqp, -1);       // the state whose factors a state was found to share
   for (int i = 0; i < nb; ++i)
     for (int s = 0; s < 2; ++s) {
       const int lo = st[i] + (s ? nup[i] : 0), hi = s ? st[i] + db[i] : st[i] + nup[i];
+      const int ip = i - nb / 2;        // partner block, if it came before
+      int po = -1;                      // its states of the other spin
+      if (ip >= 0 && nb % 2 == 0 && db[ip] == db[i] && nup[ip] == db[i] - nup[i]) po = st[ip] + (s ? 0 : nup[ip]);
       std::vector<double> c(ngl, 0.0);
       std::fill(wbest.begin(), wbest.end(), 0.0);
       bool first = true;
+      // the state's radial function with the z function c0 divided out, its largest values
+      double rtop = 0.0, dtop = 0.0;
+      int rmax = 0;
+      auto radial = [&](const double* f, int c0) {
+        const double *fd = f + ps, inv = 1.0 / ztop[c0];
+        rtop = dtop = 0.0;
+        for (int l = 0; l < ngl; ++l) {
+          row[2 * l] = f[(size_t)l * ngh + zstar[c0]] * inv;
+          row[2 * l + 1] = fd[(size_t)l * ngh + zstar[c0]] * inv;
+          if (fabs(row[2 * l]) > rtop) { rtop = fabs(row[2 * l]); rmax = l; }
+          if (fabs(row[2 * l + 1]) > dtop) dtop = fabs(row[2 * l + 1]);
+        }
+      };
+      auto same_z = [&](const double* p, int k, double top) {
+        const double q = p[zstar[k]] / ztop[k], *z = &B.z[(size_t)(2 * k) * ngh];
+        for (int h = 0; h < ngh; ++h)
+          if (fabs(p[h] - q * z[h]) > SEP_TOL * top) return false;
+        return true;
+      };
+      auto same_row = [&](int k, double sg) {
+        const double* r = &B.r[(size_t)k * ngl * 2];
+        if (fabs(row[2 * rmax] - sg * r[2 * rmax]) > SEP_TOL * rtop) return false;
+        for (int l = 0; l < ngl; ++l)
+          if (fabs(row[2 * l] - sg * r[2 * l]) > SEP_TOL * rtop || fabs(row[2 * l + 1] - sg * r[2 * l + 1]) > SEP_TOL * dtop)
+            return false;
+        return true;
+      };
+      auto find = [&](double sg) {
+        for (int k = 0; k < B.nrow; ++k)
+          if (same_row(k, sg)) return k;
+        return -1;
+      };
       for (int a = lo; a < hi; ++a) {
         const double* f = phi + (size_t)a * nghl;
-        int m = 0;
-        for (int k = 1; k < nghl; ++k)
-          if (fabs(f[k]) > fabs(f[m])) m = k;
-        const double top = fabs(f[m]);
-        if (!(top > 0.0) || !std::isfinite(top)) return false;
-        const int ls = m / ngh, hs = m % ngh;
-        const double* p = f + (size_t)ls * ngh;   // the state along z at its largest point
-        int c0 = -1;
-        for (int k = 0; k < B.nzf && c0 < 0; ++k) {
-          const double q = p[zstar[k]] / ztop[k];
-          double d = 0.0;
-          for (int h = 0; h < ngh; ++h) d = fmax(d, fabs(p[h] - q * B.z[(size_t)(2 * k) * ngh + h]));
-          if (d <= SEP_TOL * top) c0 = k;
-        }
-        if (c0 < 0) {
-          if (B.nzf >= 256) return false;   // not a product basis of any size in use
-          // scaled so that the state's radial function is a row that is there already,
-          // if there is one: every (n_r, |Lambda|) then has one row for all n_z
-          double scale = 1.0;
-          for (int k = 0; k < B.nrow; ++k) {
-            const double *rk = &B.r[(size_t)k * ngl * 2], sg = B.sgn[2 * i + s];
-            if (rk[2 * ls] == 0.0) continue;
-            const double al = f[(size_t)ls * ngh + hs] / (sg * rk[2 * ls]);
-            double d0 = 0.0, d1 = 0.0, dtop = 0.0;
-            for (int l = 0; l < ngl; ++l) {
-              const double fd = phi[ps + (size_t)a * nghl + (size_t)l * ngh + hs];
-              d0 = fmax(d0, fabs(f[(size_t)l * ngh + hs] - al * sg * rk[2 * l]));
-              d1 = fmax(d1, fabs(fd - al * sg * rk[2 * l + 1]));
-              dtop = fmax(dtop, fabs(fd));
-            }
-            if (d0 <= SEP_TOL * top && d1 <= SEP_TOL * dtop) { scale = al; break; }
+        int c0 = -1, k = -1;
+        if (po >= 0) {
+          const int b = po + a - lo, zb = B.zi[b];
+          radial(f, zb);
+          const double* p = f + (size_t)rmax * ngh;
+          if (rtop > 0.0 && std::isfinite(rtop) && same_z(p, zb, fabs(p[zstar[zb]]))) {
+            if (same_row(B.ri[b], B.sgn[2 * i + s])) k = B.ri[b];
+            else if (first && same_row(B.ri[b], -1.0)) { k = B.ri[b]; B.sgn[2 * i + s] = -1.0; }
           }
-          c0 = B.nzf++;
-          zstar.push_back(hs);
-          ztop.push_back(scale);
-          for (int h = 0; h < ngh; ++h) B.z.push_back(scale * (p[h] / p[hs]));
-          const double* g = phi + 3 * ps + (size_t)a * nghl + (size_t)ls * ngh;
-          for (int h = 0; h < ngh; ++h) B.z.push_back(scale * (g[h] / p[hs]));
+          if (k >= 0) { c0 = zb; peer[a] = b; }
+        }
+        if (k < 0) {
+          double m4[4] = {0.0, 0.0, 0.0, 0.0};   // four chains
+          int q = 0;
+          for (; q + 4 <= nghl; q += 4)
+            for (int u = 0; u < 4; ++u) { const double x = fabs(f[q + u]); m4[u] = x > m4[u] ? x : m4[u]; }
+          for (; q < nghl; ++q) { const double x = fabs(f[q]); m4[0] = x > m4[0] ? x : m4[0]; }
+          const double top = std::max(std::max(m4[0], m4[1]), std::max(m4[2], m4[3]));
+          if (!(top > 0.0) || !std::isfinite(top)) return false;
+          int m = 0;
+          while (fabs(f[m]) != top) ++m;
+          const int ls = m / ngh, hs = m % ngh;
+          const double* p = f + (size_t)ls * ngh;   // the state along z at its largest point
+          for (int z = 0; z < B.nzf && c0 < 0; ++z)
+            if (same_z(p, z, top)) c0 = z;
+          if (c0 < 0) {
+            if (B.nzf >= 256) return false;   // not a product basis of any size in use
+            // scaled so that the state's radial function is a row that is there already,
+            // if there is one: every (n_r, |Lambda|) then has one row for all n_z
+            double scale = 1.0;
+            for (int z = 0; z < B.nrow; ++z) {
+              const double *rk = &B.r[(size_t)z * ngl * 2], sg = B.sgn[2 * i + s];
+              if (rk[2 * ls] == 0.0) continue;
+              const double al = f[(size_t)ls * ngh + hs] / (sg * rk[2 * ls]);
+              double d0 = 0.0, d1 = 0.0, dt = 0.0;
+              for (int l = 0; l < ngl; ++l) {
+                const double fd = phi[ps + (size_t)a * nghl + (size_t)l * ngh + hs];
+                d0 = fmax(d0, fabs(f[(size_t)l * ngh + hs] - al * sg * rk[2 * l]));
+                d1 = fmax(d1, fabs(fd - al * sg * rk[2 * l + 1]));
+                dt = fmax(dt, fabs(fd));
+              }
+              if (d0 <= SEP_TOL * top && d1 <= SEP_TOL * dt) { scale = al; break; }
+            }
+            c0 = B.nzf++;
+            zstar.push_back(hs);
+            ztop.push_back(scale);
+            for (int h = 0; h < ngh; ++h) B.z.push_back(scale * (p[h] / p[hs]));
+            const double* g = phi + 3 * ps + (size_t)a * nghl + (size_t)ls * ngh;
+            for (int h = 0; h < ngh; ++h) B.z.push_back(scale * (g[h] / p[hs]));
+          }
+          radial(f, c0);
+          k = first || B.sgn[2 * i + s] > 0 ? find(1.0) : find(-1.0);
+          if (first && k < 0 && (k = find(-1.0)) >= 0) B.sgn[2 * i + s] = -1.0;
+          if (k < 0) {
+            if (B.nrow >= 4096) return false;
+            k = B.nrow++;
+            for (double x : row) B.r.push_back(B.sgn[2 * i + s] * x);
+          }
         }
         B.zi[a] = c0;
-        double rtop = 0.0, dtop = 0.0;
-        for (int l = 0; l < ngl; ++l) {
-          row[2 * l] = f[(size_t)l * ngh + zstar[c0]] / ztop[c0];
-          row[2 * l + 1] = phi[ps + (size_t)a * nghl + (size_t)l * ngh + zstar[c0]] / ztop[c0];
-          rtop = fmax(rtop, fabs(row[2 * l]));
-          dtop = fmax(dtop, fabs(row[2 * l + 1]));
-          const double g2 = phi[2 * ps + (size_t)a * nghl + (size_t)l * ngh + zstar[c0]];
-          if (fabs(row[2 * l]) > wbest[l]) { wbest[l] = fabs(row[2 * l]); c[l] = g2 / ztop[c0] / row[2 * l]; }
-        }
-        auto find = [&](double sg) {
-          for (int k = 0; k < B.nrow; ++k) {
-            double d0 = 0.0, d1 = 0.0;
-            for (int l = 0; l < ngl; ++l) {
-              d0 = fmax(d0, fabs(row[2 * l] - sg * B.r[((size_t)k * ngl + l) * 2]));
-              d1 = fmax(d1, fabs(row[2 * l + 1] - sg * B.r[((size_t)k * ngl + l) * 2 + 1]));
-              if (d0 > SEP_TOL * rtop) break;
-            }
-            if (d0 <= SEP_TOL * rtop && d1 <= SEP_TOL * dtop) return k;
-          }
-          return -1;
-        };
-        int k = first || B.sgn[2 * i + s] > 0 ? find(1.0) : find(-1.0);
-        if (first && k < 0 && (k = find(-1.0)) >= 0) B.sgn[2 * i + s] = -1.0;
-        if (k < 0) {
-          if (B.nrow >= 4096) return false;
-          k = B.nrow++;
-          for (double x : row) B.r.push_back(B.sgn[2 * i + s] * x);
-        }
         B.ri[a] = k;
         first = false;
+        for (int l = 0; l < ngl; ++l)
+          if (fabs(row[2 * l]) > wbest[l]) {
+            wbest[l] = fabs(row[2 * l]);
+            c[l] = phi[2 * ps + (size_t)a * nghl + (size_t)l * ngh + zstar[c0]] / ztop[c0] / row[2 * l];
+          }
       }
       lseg[2 * i + s] = c;
     }
@@ -188,22 +225,27 @@ inline bool sep_factors(int nb, const int* db, const int* st, const int* nup, in
       B.lam[k] = d / big;
     }
   }
-  // V and e: phi_4 / phi_0 = V - e_a, each taken where the state is large
+  // V and e: phi_4 = (V - e_a) phi_0; e by least squares over the points where V is known, V
+  // from the state that is largest there
   std::vector<double> w(nghl, 0.0);
   for (int pass = 0; pass < 2; ++pass)
     for (int a = 0; a < dqp; ++a) {
+      if (peer[a] >= 0) { B.e[a] = B.e[peer[a]]; continue; }
       const double *f = phi + (size_t)a * nghl, *g = phi + 4 * ps + (size_t)a * nghl;
-      double top = 0.0, s0 = 0.0, s1 = 0.0;
-      for (int k = 0; k < nghl; ++k) top = fmax(top, fabs(f[k]));
-      for (int k = 0; k < nghl; ++k) {
-        const double x = fabs(f[k]);
-        if (x < 1e-2 * top || w[k] == 0.0) continue;
-        s0 += x * w[k];
-        s1 += x * w[k] * (B.v[k] - g[k] / f[k]);
-      }
-      if (s0 > 0.0) B.e[a] = s1 / s0;
+      double s0[4] = {0.0, 0.0, 0.0, 0.0}, s1[4] = {0.0, 0.0, 0.0, 0.0};   // four chains
+      auto add = [&](int k, int u) {
+        const double x = w[k] > 0.0 ? f[k] : 0.0;
+        s0[u] += x * x;
+        s1[u] += x * (B.v[k] * x - g[k]);
+      };
+      int k = 0;
+      for (; k + 4 <= nghl; k += 4)
+        for (int u = 0; u < 4; ++u) add(k + u, u);
+      for (; k < nghl; ++k) add(k, 0);
+      const double d = (s0[0] + s0[1]) + (s0[2] + s0[3]);
+      if (d > 0.0) B.e[a] = ((s1[0] + s1[1]) + (s1[2] + s1[3])) / d;
       if (pass == 0)
-        for (int k = 0; k < nghl; ++k)
+        for (k = 0; k < nghl; ++k)
           if (fabs(f[k]) > w[k]) { w[k] = fabs(f[k]); B.v[k] = g[k] / f[k] + B.e[a]; }
     }
   return true;
@@ -280,67 +322,83 @@ struct SepStruct {
   int umax = 0;                    // most units of one (class, n_z')
 };
 
-// cols, offs_: the block structure; items: also the projection's items.  false when a
-// part of a unit does not fit the staging buffer
+// cols, boff: the block structure; project: also the projection's items.  false when a
+// part of a unit does not fit the staging buffer.  The five structures of an operator with
+// their item columns: 0.19 ms at N_sh = 6, 4.3 at 16 on one Grace core
 inline bool sep_structure(const SepBasis& B, int nb, const int* db, const int* st, const int* nup, const int* cols,
                           const long long* boff, bool project, SepStruct& S) {
   S = SepStruct();
   const int nzf = B.nzf;
-  struct Part { int i, s, j, t; };
-  std::vector<Part> parts[4];
+  // states of each (block, spin) by z function: byz[first[seg * nzf + z] ...]
+  std::vector<int> first(2 * nb * nzf + 1, 0), byz, at;
+  for (int i = 0; i < nb; ++i)
+    for (int a = 0; a < db[i]; ++a) ++first[(2 * i + (a >= nup[i])) * nzf + B.zi[st[i] + a] + 1];
+  for (size_t k = 1; k < first.size(); ++k) first[k] += first[k - 1];
+  byz.resize(first.back());
+  at.assign(first.begin(), first.end() - 1);
+  for (int i = 0; i < nb; ++i)
+    for (int a = 0; a < db[i]; ++a) byz[at[(2 * i + (a >= nup[i])) * nzf + B.zi[st[i] + a]]++] = st[i] + a;
+  auto count = [&](int seg, int z) { return first[seg * nzf + z + 1] - first[seg * nzf + z]; };
+  long long nel = 0;
+  for (int i = 0; i < nb; ++i)
+    if (cols[i] >= 0) nel += (long long)db[i] * db[cols[i]];
+  S.offs.reserve(nel);
+  if (project) S.items.reserve(nel / 2);
+  struct Part { int i, seg, j, segp; };
+  std::vector<Part> parts[4], live;   // of a class; those with column states of a z function
   for (int i = 0; i < nb; ++i) {
     const int j = cols[i];
     if (j < 0) continue;
     for (int s = 0; s < 2; ++s)
-      for (int t = 0; t < 2; ++t) parts[2 * s + t].push_back({i, s, j, t});
+      for (int t = 0; t < 2; ++t) parts[2 * s + t].push_back({i, 2 * i + s, j, 2 * j + t});
   }
-  // states of each (block, spin) by z function
-  std::vector<std::vector<std::vector<int>>> byz(2 * nb, std::vector<std::vector<int>>(nzf));
-  for (int i = 0; i < nb; ++i)
-    for (int a = st[i]; a < st[i] + db[i]; ++a) byz[2 * i + (a - st[i] >= nup[i])][B.zi[a]].push_back(a);
   for (int c = 0; c < 4; ++c)
     for (int zp = 0; zp < nzf; ++zp) {
       S.ubeg.push_back((int)S.units.size());
+      live.clear();
+      for (const Part& p : parts[c])
+        if (count(p.segp, zp)) live.push_back(p);
       for (int z = 0; z < nzf; ++z) {
         SepUnit u{c, z, zp, (int)S.ents.size(), 0};
         const int item0 = (int)S.items.size();
-        for (const Part& p : parts[c]) {
-          const std::vector<int>&A = byz[2 * p.i + p.s][z], &C = byz[2 * p.j + p.t][zp];
-          if (A.empty() || C.empty()) continue;
-          SepEnt en{(int)A.size(), (int)C.size(), (int)S.rows.size(), 0, (int)S.offs.size(), 2 * p.i + p.s,
-                    2 * p.j + p.t};
-          if ((long long)en.ng * en.ngp > SEP_STAGE) return false;
-          for (int a : A) S.rows.push_back(B.ri[a]);
-          en.rowp0 = (int)S.rows.size();
-          for (int b : C) S.rows.push_back(B.ri[b]);
-          auto off = [&](int a, int b) {
-            return (int)(boff[p.i] + (a - st[p.i]) + (long long)(b - st[p.j]) * db[p.i]);
-          };
-          for (int b : C)
-            for (int a : A) S.offs.push_back(off(a, b));
-          if (project) {
-            // columns in nearly equal groups of at most SEP_GC
-            const int nc = ((int)C.size() + SEP_GC - 1) / SEP_GC;
-            for (int k = 0; k < nc; ++k) {
-              const int b0 = (int)C.size() * k / nc, b1 = (int)C.size() * (k + 1) / nc;
-              for (int a : A) {
-                SepItem it{};
-                it.seg = en.seg; it.segp = en.segp; it.ja = a; it.row = B.ri[a]; it.n = b1 - b0;
-                for (int b = b0; b < b1; ++b) {
-                  it.jb[b - b0] = C[b]; it.rowp[b - b0] = B.ri[C[b]]; it.off[b - b0] = off(a, C[b]);
-                }
-                S.items.push_back(it);
-              }
-            }
-          }
+        for (const Part& p : live) {
+          const int na = count(p.seg, z), nc = count(p.segp, zp);
+          if (!na) continue;
+          const int *A = &byz[first[p.seg * nzf + z]], *C = &byz[first[p.segp * nzf + zp]];
+          if ((long long)na * nc > SEP_STAGE) return false;
+          SepEnt en{na, nc, (int)S.rows.size(), (int)S.rows.size() + na, (int)S.offs.size(), p.seg, p.segp};
+          for (int a = 0; a < na; ++a) S.rows.push_back(B.ri[A[a]]);
+          for (int b = 0; b < nc; ++b) S.rows.push_back(B.ri[C[b]]);
+          for (int b = 0; b < nc; ++b)
+            for (int a = 0; a < na; ++a)
+              S.offs.push_back((int)(boff[p.i] + (A[a] - st[p.i]) + (long long)(C[b] - st[p.j]) * db[p.i]));
           S.ents.push_back(en);
         }
         u.nent = (int)S.ents.size() - u.ent0;
         if (!u.nent) continue;
         if (project) {
-          // items of one size next to each other, so that a warp's lanes run the same loop
-          std::stable_sort(S.items.begin() + item0, S.items.end(),
-                           [](const SepItem& x, const SepItem& y) { return x.n > y.n; });
+          // a part's columns in nearly equal groups of at most SEP_GC; items of one size next
+          // to each other, so that a warp's lanes run the same loop
+          for (int n = SEP_GC; n > 0; --n)
+            for (int e = u.ent0; e < u.ent0 + u.nent; ++e) {
+              const SepEnt& en = S.ents[e];
+              const int ng = (en.ngp + SEP_GC - 1) / SEP_GC;
+              if (en.ngp / ng != n && (en.ngp + ng - 1) / ng != n) continue;
+              const int *A = &byz[first[en.seg * nzf + z]], *C = &byz[first[en.segp * nzf + zp]];
+              for (int k = 0; k < ng; ++k) {
+                const int b0 = en.ngp * k / ng;
+                if (en.ngp * (k + 1) / ng - b0 != n) continue;
+                for (int a = 0; a < en.ng; ++a) {
+                  S.items.emplace_back();
+                  SepItem& it = S.items.back();
+                  it.seg = en.seg; it.segp = en.segp; it.ja = A[a]; it.row = S.rows[en.row0 + a]; it.n = n;
+                  for (int b = 0; b < n; ++b) {
+                    it.jb[b] = C[b0 + b]; it.rowp[b] = S.rows[en.rowp0 + b0 + b];
+                    it.off[b] = S.offs[en.el0 + (b0 + b) * en.ng + a];
+                  }
+                }
+              }
+            }
           for (int h = 0; h < 2; ++h) {
             const int n = h ? 32 / SEP_SPL : 32;
             for (int k = item0; k < (int)S.items.size(); k += n)
