@@ -363,17 +363,8 @@ struct pnfam_ctx {
   bool sep = false, sep32 = false;
   SepBasis sepb;
   SepStruct seps[5];          // F, X^T, Y^T, X, Y
-  struct SepBufs {            // device copy of one structure
-    DBuf<SepUnit> units;
-    DBuf<SepEnt> ents;
-    DBuf<int> rows, offs, ubeg, order;
-    DBuf<int> items;
-    DBuf<SepWarp> warps[2];
-    void release() {
-      units.release(); ents.release(); rows.release(); offs.release(); ubeg.release(); order.release();
-      items.release(); warps[0].release(); warps[1].release();
-    }
-  } d_seps[5];
+  DBuf<unsigned char> d_septab;   // their device copies, in one piece
+  SepStructDev sepd[5];           // and where each lies
   DBuf<double> d_sepf;        // z, r, v, y, e, lam, sgn
   DBuf<float> d_sepf32;
   DBuf<double> d_sepg;        // [P][gstride] unit sums
@@ -452,8 +443,7 @@ struct pnfam_ctx {
     s2a.d_tasks.release(); s2a.d_tile2task.release();
     k2b.d_tasks.release(); k2b.d_tile2task.release();
     s2b.d_tasks.release(); s2b.d_tile2task.release();
-    for (SepBufs& b : d_seps) b.release();
-    d_sepf.release(); d_sepf32.release(); d_sepg.release(); d_sepg32.release();
+    d_septab.release(); d_sepf.release(); d_sepf32.release(); d_sepg.release(); d_sepg32.release();
     if (ev[0]) cudaEventDestroy(ev[0]);
     if (ev[1]) cudaEventDestroy(ev[1]);
     if (evt[0]) cudaEventDestroy(evt[0]);
@@ -1380,16 +1370,41 @@ static int sep_operator(pnfam_ctx* c) {
       c->sep = c->sep32 = false;
       return PNFAM_OK;
     }
+  }
+  // one allocation, and one copy while that is quicker than a copy per table (45 of them)
+  struct Piece { const void* src; size_t bytes, at; };
+  std::vector<Piece> pieces;
+  size_t total = 0;
+  auto put = [&](const auto& v) {
+    const size_t at = total, n = v.size() * sizeof(v[0]);
+    pieces.push_back({v.data(), n, at});
+    total += (n + 255) / 256 * 256;
+    return at;
+  };
+  size_t at[5][9];
+  for (int k = 0; k < 5; ++k) {
     const SepStruct& s = c->seps[k];
-    auto& d = c->d_seps[k];
-    CK(upload(d.units, s.units.data(), s.units.size()));
-    CK(upload(d.ents, s.ents.data(), s.ents.size()));
-    CK(upload(d.rows, s.rows.data(), s.rows.size()));
-    CK(upload(d.offs, s.offs.data(), s.offs.size()));
-    CK(upload(d.ubeg, s.ubeg.data(), s.ubeg.size()));
-    CK(upload(d.order, s.order.data(), s.order.size()));
-    CK(upload(d.items, items[k].data(), items[k].size()));
-    for (int h = 0; h < 2; ++h) CK(upload(d.warps[h], s.warps[h].data(), s.warps[h].size()));
+    const size_t a[9] = {put(s.units), put(s.ents), put(s.rows), put(s.offs), put(s.ubeg), put(s.order), put(items[k]),
+                         put(s.warps[0]), put(s.warps[1])};
+    std::copy(a, a + 9, at[k]);
+  }
+  CK(dalloc(c->d_septab, total));
+  if (total <= (size_t)1 << 20) {
+    std::vector<unsigned char> h(total);
+    for (const Piece& q : pieces)
+      if (q.bytes) memcpy(h.data() + q.at, q.src, q.bytes);
+    CK(upload(c->d_septab, h.data(), total));
+  } else {
+    for (const Piece& q : pieces) CK(cudaMemcpy(c->d_septab.p + q.at, q.src, q.bytes, cudaMemcpyHostToDevice));
+  }
+  for (int k = 0; k < 5; ++k) {
+    const SepStruct& s = c->seps[k];
+    const unsigned char* p = c->d_septab.p;
+    auto ints = [&](int i) { return reinterpret_cast<const int*>(p + at[k][i]); };
+    auto warps = [&](int i) { return reinterpret_cast<const SepWarp*>(p + at[k][i]); };
+    c->sepd[k] = {reinterpret_cast<const SepUnit*>(p + at[k][0]), reinterpret_cast<const SepEnt*>(p + at[k][1]),
+                  ints(2), ints(3), ints(4), ints(5), ints(6), {warps(7), warps(8)},
+                  (int)s.items.size(), s.umax, (int)s.units.size(), {(int)s.warps[0].size(), (int)s.warps[1].size()}};
   }
   long long nu[5];
   for (int k = 0; k < 5; ++k) nu[k] = (long long)c->seps[k].units.size();
@@ -1408,12 +1423,7 @@ static SepDev<T> sep_dev(const pnfam_ctx* c, const T* factors, T* g) {
   const T* rt = S.sgn + B.sgn.size();
   S.rt = reinterpret_cast<const typename Vec2<T>::t*>(rt + (rt - factors) % 2); S.nrow = B.nrow;
   SepStructDev* to[5] = {&S.f, &S.k[0], &S.k[1], &S.d[0], &S.d[1]};
-  for (int k = 0; k < 5; ++k) {
-    const auto& d = c->d_seps[k];
-    const SepStruct& s = c->seps[k];
-    *to[k] = {d.units.p, d.ents.p, d.rows.p, d.offs.p, d.ubeg.p, d.order.p, d.items.p, {d.warps[0].p, d.warps[1].p},
-              (int)s.items.size(), s.umax, (int)s.units.size(), {(int)s.warps[0].size(), (int)s.warps[1].size()}};
-  }
+  for (int k = 0; k < 5; ++k) *to[k] = c->sepd[k];
   S.gstride = c->sep_gstride; S.gpair[0] = c->sep_gpair[0]; S.gpair[1] = c->sep_gpair[1];
   S.g = g; S.list = nullptr; S.act = nullptr; S.n = 0;
   return S;
