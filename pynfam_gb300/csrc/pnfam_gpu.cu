@@ -270,7 +270,6 @@ struct pnfam_ctx {
   struct TCSet {
     TaskListTC l[4];
     DBuf<float> gsplit;
-    long long floats = 0;
     bool built = false;
   } tc32[2];
   std::vector<HGroup> hgroups;
@@ -383,6 +382,7 @@ struct pnfam_ctx {
   // Both kinds of run also keep the general form of the transforms (form 0).
   bool sep64 = false, pair32 = false, tuning = false;
   bool pg_ready = false;      // pg_setup done for the current operator
+  bool have_general = false, have_k1 = false;   // general_tables done; k1a and k1b on the device
   int nchunk_bro = 1, nchunk_c = 1;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -1191,6 +1191,50 @@ static int pg_projection(pnfam_ctx* c, int nact, const float* mf, float* hsp, cu
   return PNFAM_OK;
 }
 
+// tables of the kernels over the mesh, made by the first that takes them: a run that keeps
+// its sums (engine_setup), or set_operator where there are no unit sums to take
+static int general_tables(pnfam_ctx* c) {
+  if (c->have_general) return PNFAM_OK;
+  build_field_tasks(c);
+  CK(upload(c->d_hgroups, c->hgroups.data(), c->hgroups.size()));
+  CK(upload(c->d_htasks_tc, c->htasks_tc.data(), c->htasks_tc.size()));
+  CK(upload(c->d_hptiles, c->hptiles.data(), c->hptiles.size()));
+  CK(upload(c->d_dunits0, c->dunits[0].data(), c->dunits[0].size()));
+  CK(upload(c->d_dunits1, c->dunits[1].data(), c->dunits[1].size()));
+  CK(upload(c->d_bchunks, c->bchunks.data(), c->bchunks.size()));
+  if (!c->have_aphi) CK(upload(c->d_achunks, c->achunks.data(), c->achunks.size()));
+  c->have_general = true;
+  return PNFAM_OK;
+}
+
+// the block GEMMs' tasks for the tensor-core kernel and their pre-split operands, by the
+// first run that takes them
+static int tc_tables(pnfam_ctx* c, int form) {
+  pnfam_ctx::TCSet& set = c->tc32[form];
+  if (set.built) return PNFAM_OK;
+  const TaskList* src[2][4] = {{&c->k1a, &c->k1b, &c->k2a, &c->k2b}, {&c->s1a, &c->s1b, &c->s2a, &c->s2b}};
+  long long floats = 0;
+  for (int k = 0; k < 4; ++k) {
+    set.l[k].build(*src[form][k]);
+    for (GemmTaskTC& t : set.l[k].tasks) {
+      t.bsoff = floats;   // the task's pre-split ground-state chunks
+      floats += (long long)t.nterm * ((t.K + GTC_K - 1) / GTC_K) * t.npad * 2 * GTC_K;
+    }
+    CK(upload(set.l[k].d_tasks, set.l[k].tasks.data(), set.l[k].tasks.size()));
+  }
+  CK(dalloc(set.gsplit, (size_t)std::max(1LL, floats)));
+  for (const TaskListTC& tl : set.l) {
+    int mc = 0;
+    for (const GemmTaskTC& t : tl.tasks) mc = std::max(mc, t.nterm * ((t.K + GTC_K - 1) / GTC_K));
+    if (tl.tasks.empty() || mc == 0) continue;
+    k_gemm_bsplit<<<dim3((unsigned)tl.tasks.size(), (unsigned)mc), 256, 0, c->stream>>>(
+        tl.d_tasks.p, c->d_bufs32.p, set.gsplit.p);
+    CK(cudaGetLastError());
+  }
+  set.built = true;
+  return PNFAM_OK;
+}
+
 static int ensure_buffers(pnfam_ctx* c, int P, int M) {
   const long long nxy = c->nxy;
   const long long nv = 2 * c->nq * c->qn();   // Re and Im of the QP state (X, Y[, P, Q])
@@ -1795,6 +1839,10 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
   // what the general kernels need (a separable basis: only for the pair-tensor GEMMs of
   // uncertified runs, whose point count is tuned against the per-block kernels)
   const bool general = !c->sep32 || pair;
+  if (general) {
+    const int rc = general_tables(c);
+    if (rc) return rc;
+  }
   if (general && run) pg_prepare(c);
   if (c->tc_density && general) {
     CK(dalloc(c->d_bsplit, (size_t)P * c->bstride));
@@ -1830,19 +1878,8 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
     c->have_hphi = true;
   }
   if (run) {
-    pnfam_ctx::TCSet& set = c->tc32[c->form];
-    if (!set.built) {
-      CK(dalloc(set.gsplit, (size_t)std::max(1LL, set.floats)));
-      for (const TaskListTC& tl : set.l) {
-        int mc = 0;
-        for (const GemmTaskTC& t : tl.tasks) mc = std::max(mc, t.nterm * ((t.K + GTC_K - 1) / GTC_K));
-        if (tl.tasks.empty() || mc == 0) continue;
-        k_gemm_bsplit<<<dim3((unsigned)tl.tasks.size(), (unsigned)mc), 256, 0, c->stream>>>(
-            tl.d_tasks.p, c->d_bufs32.p, set.gsplit.p);
-        CK(cudaGetLastError());
-      }
-      set.built = true;
-    }
+    const int rc = tc_tables(c, c->form);
+    if (rc) return rc;
   }
   if (!general || !run) return PNFAM_OK;
   {
@@ -2125,39 +2162,22 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
   c->form = 0;   // F_qp below; a run chooses its own (engine_setup)
   set_chunks(c);
   build_transforms(c);
-  build_field_tasks(c);
+  for (const TaskList* l : {&c->k1a, &c->k1b, &c->k2a, &c->k2b})
+    for (const GemmTask& t : l->tasks)   // the ground state's side (TaskListTC::build)
+      if ((t.t[0].abuf >= B_STATE ? t.N : t.M) > 256)
+        return fail(PNFAM_EINVAL, "pnfam_gpu_set_operator: block larger than 256");
   {
     const int rcs = sep_operator(c);
     if (rcs) return rcs;
   }
-  c->pg_ready = c->pg_on = c->pg_built = false;
-  CK(c->k1a.finalize()); CK(c->k1b.finalize()); CK(c->k2a.finalize()); CK(c->k2b.finalize());
+  c->pg_ready = c->pg_on = c->pg_built = c->have_general = c->have_k1 = false;
+  c->tc32[0].built = c->tc32[1].built = false;
+  CK(c->k2a.finalize()); CK(c->k2b.finalize());
   if (c->shared) { CK(c->s1a.finalize()); CK(c->s1b.finalize()); CK(c->s2a.finalize()); CK(c->s2b.finalize()); }
-  {
-    const TaskList* src[2][4] = {{&c->k1a, &c->k1b, &c->k2a, &c->k2b}, {&c->s1a, &c->s1b, &c->s2a, &c->s2b}};
-    for (int f = 0; f < 1 + c->shared; ++f) {
-      pnfam_ctx::TCSet& set = c->tc32[f];
-      long long goff = 0;
-      for (int k = 0; k < 4; ++k) {
-        set.l[k].build(*src[f][k]);
-        for (GemmTaskTC& t : set.l[k].tasks) {
-          if (t.ncols > 256) return fail(PNFAM_EINVAL, "pnfam_gpu_set_operator: block larger than 256");
-          t.bsoff = goff;   // the task's pre-split ground-state chunks
-          goff += (long long)t.nterm * ((t.K + GTC_K - 1) / GTC_K) * t.npad * 2 * GTC_K;
-        }
-        CK(upload(set.l[k].d_tasks, set.l[k].tasks.data(), set.l[k].tasks.size()));
-      }
-      set.floats = goff;
-      set.built = false;
-    }
+  if (!c->sep || !c->sep32) {
+    const int rcg = general_tables(c);
+    if (rcg) return rcg;
   }
-  CK(upload(c->d_hgroups, c->hgroups.data(), c->hgroups.size()));
-  CK(upload(c->d_htasks_tc, c->htasks_tc.data(), c->htasks_tc.size()));
-  CK(upload(c->d_hptiles, c->hptiles.data(), c->hptiles.size()));
-  CK(upload(c->d_dunits0, c->dunits[0].data(), c->dunits[0].size()));
-  CK(upload(c->d_dunits1, c->dunits[1].data(), c->dunits[1].size()));
-  CK(upload(c->d_bchunks, c->bchunks.data(), c->bchunks.size()));
-  if (!c->have_aphi) CK(upload(c->d_achunks, c->achunks.data(), c->achunks.size()));
   c->have_op = true;
   // one point for F_qp, in whole blocks: a run sizes the buffers of its form (engine_setup),
   // so that those of an earlier run in the active form are not made whole here
@@ -2296,9 +2316,14 @@ static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver
   }
   c->form = general ? 0 : 1;
   set_chunks(c);
-  e->nxy = c->qn(); e->N = (int)(2 * c->nq * e->nxy); e->nops = c->nops;
-  int rc = ensure_buffers(c, std::max(P, c->cap_P), std::max(std::max(e->M, 1), c->cap_M));
+  int rc = c->sep64 ? PNFAM_OK : general_tables(c);
   if (rc) return rc;
+  if (!c->form && !c->have_k1) {
+    CK(c->k1a.finalize()); CK(c->k1b.finalize());
+    c->have_k1 = true;
+  }
+  e->nxy = c->qn(); e->N = (int)(2 * c->nq * e->nxy); e->nops = c->nops;
+  if ((rc = ensure_buffers(c, std::max(P, c->cap_P), std::max(std::max(e->M, 1), c->cap_M)))) return rc;
   c->cap_P = std::max(P, c->cap_P); c->cap_M = std::max(std::max(e->M, 1), c->cap_M);
   if (e->mixed && (rc = ensure_buffers32(c, c->cap_P, c->pair32, true))) return rc;
   // Mixed form (precision 1): one Broyden iteration per evaluation, as in the FP64
