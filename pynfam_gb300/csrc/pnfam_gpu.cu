@@ -52,7 +52,17 @@ namespace {
 
 // asynchronous FP64 anchor batches an engine keeps in flight at most
 constexpr int ANCH_RING = 8;
-// shortest Broyden history of an FP64 run that takes the unit sums (pnfam_ctx::sep64)
+// Shortest Broyden history of an FP64 run that takes the unit sums (pnfam_ctx::sep64).  With
+// a shorter one, points near the real axis do not converge in 200 iterations, and what they
+// then return is decided by rounding: unit sums and sums over the mesh, neither of them nearer
+// to the fixed point, differ by (worst of six points, relative, 40S and 162Gd at N_sh = 8 and
+// 40S RS1 at 6, eps = 1e-7, alpha = 0.4 and 0.7)
+//   M = 4: 1e-2 and more   M = 7: 1e-4 to more than 1   M = 10: 1e-5 to 3e-3
+//   M = 13: 9e-8 to 1e-4   M = 16: 9e-10 to 7e-7        M = 20: 9e-11 to 2e-7
+// From 16 on that is below the solve's own error against the fixed point (1e-8 to 1e-6).
+// Below, a run keeps the order of its sums, and with it the values that it returned before:
+// 40 points of 40S at N_sh = 8 with M = 7 take 290 ms so, nine tenths of it in the sums over
+// the mesh
 constexpr int SEP_MIN_HISTORY = 16;
 
 template <class T>
@@ -370,16 +380,14 @@ struct pnfam_ctx {
   DBuf<float> d_sepg32;
   long long sep_gstride = 0, sep_gpair[2] = {0, 0};
   // Which evaluations of the current run take it (engine_setup):
-  // sep64: the FP64 ones.  A Broyden history shorter than SEP_MIN_HISTORY wraps early, and
-  // the iteration then amplifies rounding 1.6-fold per step (measured: 40S, N_sh = 8,
-  // M = 7, alpha = 0.4: final states of runs that differ by 2e-16 in the first field are
-  // 1e-8 apart after 42 steps); such FP64 runs keep the sums over the mesh, and with them
-  // the trajectories that they had.
-  // pair32: a mixed-form run that does not certify its strengths (opts.reserved[3] = 0)
-  // returns what its FP32 evaluations lead to, so it keeps the pair-tensor GEMMs from the
-  // tuned point count on: their long tensor-core sums differ from the unit sums by 1e-5 in
-  // 12 steps, while the strengths of certified runs agree to 1e-8 for either.
-  // Both kinds of run also keep the general form of the transforms (form 0).
+  // sep64: the FP64 ones (SEP_MIN_HISTORY).
+  // pair32: a mixed-form run that does not wait for its strengths (opts.reserved[3] = 0) and
+  // whose pair tensor fits keeps the pair-tensor GEMMs from the tuned point count on, so that
+  // it returns what it did: the two sums' results are 1e-5 apart after 12 steps (strengths of
+  // runs that wait agree to 1e-8). The unit sums are the more accurate ones (2e-7 a field
+  // against 8e-6) and the quicker ones (33 us a point of a 24-point launch at N_sh = 16 against
+  // 80 of a 40-point one); a run whose pair tensor does not fit (N_sh = 20) takes them.
+  // Both kinds of run that keep their sums also keep the general form of the transforms (form 0).
   bool sep64 = false, pair32 = false, tuning = false;
   bool pg_ready = false;      // pg_setup done for the current operator
   bool have_general = false, have_k1 = false;   // general_tables done; k1a and k1b on the device

@@ -91,10 +91,10 @@ __device__ __forceinline__ void gemm_stage(const double* __restrict__ src, int l
 // one address), K runs over the block's own size, and the ground-state operand is staged
 // once for both planes.  Against tiles of 1024 outputs padded in M, N and K: N_sh = 8, 40
 // points, 23 against 56 ms per solve, N_sh = 6 11 against 22 us per launch; at N_sh = 16
-// (blocks 1 to 81, nine points) 1.1 TFLOP/s, what a DGEMM reaches, against 0.69, and with
-// shared products and active quasiparticles only 0.33 ms per point against 1.01.  Every output sums over the terms and k in order.  Of the two operands of a
-// term one is the point's (two planes), one the ground state's; alpha (+-1) goes into the
-// point's.  grid (tiles, P)
+// (blocks 1 to 81, nine points) 1.04 TFLOP/s (a DGEMM reaches 1.1) against 0.69, and with
+// shared products and active quasiparticles only 0.33 ms per point against 1.01.  Every
+// output sums over the terms and k in order.  Of the two operands of a term one is the
+// point's (two planes), one the ground state's; alpha (+-1) goes into the point's.  grid (tiles, P)
 __global__ void __launch_bounds__(GT_THREADS) k_gemm(const GemmTask* __restrict__ tasks,
                                                      const int* __restrict__ tile2task,
                                                      const BufDescT<double>* __restrict__ bufs,

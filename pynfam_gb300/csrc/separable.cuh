@@ -20,11 +20,10 @@
 // direction instead of the whole mesh, and the sums over the blocks come before the
 // other direction is expanded: about 0.15 GFLOP per point at N_sh = 16 (20 x 20 mesh)
 // against 3.5 GFLOP of the sums over the whole mesh.  Measured there, per point, FP64
-// (nine points): densities 0.14 ms against 2.2 ms, projection 0.18 against 2.7 ms; FP32
-// (40 points): 23 and 18 us against 39 and 41 us of the pair-tensor GEMMs, whose operand
-// (12 GB) is not needed; errors against FP64 2e-7 instead of 8e-6.  (First form; with the
-// staging that the kernels below describe 16 and 17 us in FP32, 24 points: radial sums
-// 264, z sums 111, unit fields 104, projection 298 us.)
+// (nine points): densities 0.13 ms against 1.8 ms, projection 0.19 against 1.8 ms; FP32
+// (24 points): 16 and 17 us (radial sums 264, z sums 111, unit fields 104, projection 298 us
+// a launch) against 39 and 41 us of the pair-tensor GEMMs (40 points), whose operand (12 GB)
+// is not needed; errors against FP64 2e-7 instead of 8e-6.
 //
 // The factors are recovered from the basis functions that the caller passes
 // (sep_factors) and every value of the products is compared with them (k_sep_check);

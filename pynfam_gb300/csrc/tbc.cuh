@@ -18,8 +18,9 @@
 //    (r_a, l_a, r_c, l_c);
 //  * k_tbc_z (stage 1): Z[z_a z_c][t][dn, dp, en, ep][14][g] = sum over the pairs of t of
 //    Jz * rho (direct and exchange, neutron and proton densities);
-//  * k_tbc_field (stage 2): one CTA per radial group.  Its threads compute the (r, phi)
-//    current vectors Jr of a chunk of terms once (each a quadruple sum over the
+//  * k_tbc_field (stage 2): one CTA per radial group, or per group and chunk of terms while
+//    the groups are few (the chunks' sums are added by k_tbc_sum).  Its warps compute the
+//    (r, phi) current vectors Jr of a chunk of terms once (each a quadruple sum over the
 //    Cartesian decompositions of the four polar states, all six Gaussians at once) and
 //    then contract them with the Z rows of every element of the group: all z_a, z_c
 //    and spins that share the radial quantum numbers reuse one Jr, which the
