@@ -95,6 +95,11 @@ NEAR_EXP = 4
 # the two launches of a stage of the unit sums, from one ncu capture (N_sh = 16, 24 points)
 TRAFFIC_RATIO = {"density_fp32": 165.3e6 / 89.8e6, "field_projection_fp32": 95.6e6 / 89.8e6}
 TRAFFIC_SOURCE = "profiles/k_sep_nsh16.md"
+# warp schedulers' issue slots in use, of the stage's two kernels by their time, same capture
+ISSUE_ACTIVE = {"density_fp32": (266 * 0.44 + 112 * 0.32) / 378, "field_projection_fp32": (108 * 0.53 + 300 * 0.48) / 408}
+# FP32 multiply-adds per point that the stage executes there (nxy = 94,482), same capture
+EXECUTED_FMA = {"density_fp32": 39e6 + 15e6, "field_projection_fp32": 18e6 + 81e6}
+FP32_TFLOPS = 152 * 128 * 2 * 2.07e9 / 1e12
 STAGE_KERNELS = {"density_fp32": "k_sep_radial + k_sep_density", "field_projection_fp32": "k_sep_field + k_sep_project"}
 REL = 1e-6
 # mixed form: FP64 anchors beside FP32 increments run asynchronously (--async-anchors)
@@ -516,6 +521,7 @@ def run_gpu(args):
     # the same launches alone on the GPU: the serialised stage run
     pit32_t = max(stages.get("point_iterations_fp32", 0.0), 1.0)
     alone_ms = stages.get(dom, 0.0) / pit32_t * pts_per_launch
+    executed = 2 * EXECUTED_FMA[dom] * pts_per_launch * fl["S2"] / 94482
     achieved_alone = alg / max(alone_ms / 1e3, 1e-12) / 1e9
     peaks = measured_peaks()
     peak = peaks.get("hbm_gbs")
@@ -572,13 +578,20 @@ def run_gpu(args):
                          "mean_launch_ms_alone": alone_ms,
                          "reference_tflops": stage_fl[dom] * pts_per_launch / (launch_ms / 1e3) / 1e12,
                          "reference_tflops_alone": stage_fl[dom] * pts_per_launch / max(alone_ms / 1e3, 1e-12) / 1e12,
+                         "issue_active": ISSUE_ACTIVE[dom],
+                         "issue_unit": f"share of the issue slots in use, from one ncu capture ({TRAFFIC_SOURCE}): "
+                                       "the bound of the stage",
+                         "executed_tflops_alone": executed / max(alone_ms / 1e3, 1e-12) / 1e12,
+                         "executed_frac_alone": executed / max(alone_ms / 1e3, 1e-12) / 1e12 / FP32_TFLOPS,
+                         "fp32_peak_tflops": FP32_TFLOPS,
                          "tf32_peak_tflops": bf16 / 2,
                          "peak_source": src,
                          "note": "achieved = algorithmic bytes of the stage's two launches (density matrices and "
                                  "densities or fields) / their mean time, CUDA events around the two on their "
                                  "own stream in the timed steps, where the five engines' kernels share the GPU; "
                                  "*_alone: the same launches from the serialised stage run; the stage is bound "
-                                 "by instruction issue and shared memory, not by these bytes; "
+                                 "by instruction issue and shared memory, not by these bytes: issue_active, and "
+                                 "executed_* for the FP32 operations that it executes; "
                                  "reference_tflops: the reference's operation count of the stage (sums over the "
                                  "whole mesh, which the unit sums do not execute) at that rate"},
             "clocks": ck}
