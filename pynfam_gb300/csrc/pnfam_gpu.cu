@@ -280,7 +280,8 @@ struct pnfam_ctx {
   struct TCSet {
     TaskListTC l[4];
     DBuf<float> gsplit;
-    bool built = false;
+    long long floats = 0;
+    bool listed = false, built = false;
   } tc32[2];
   std::vector<HGroup> hgroups;
   DBuf<HGroup> d_hgroups;
@@ -1215,22 +1216,32 @@ static int general_tables(pnfam_ctx* c) {
   return PNFAM_OK;
 }
 
-// the block GEMMs' tasks for the tensor-core kernel and their pre-split operands, by the
-// first run that takes them
+// the block GEMMs' tasks for the tensor-core kernel: the form that a mixed run usually takes
+// in set_operator, the other by the first run that takes it
 static int tc_tables(pnfam_ctx* c, int form) {
   pnfam_ctx::TCSet& set = c->tc32[form];
-  if (set.built) return PNFAM_OK;
+  if (set.listed) return PNFAM_OK;
   const TaskList* src[2][4] = {{&c->k1a, &c->k1b, &c->k2a, &c->k2b}, {&c->s1a, &c->s1b, &c->s2a, &c->s2b}};
-  long long floats = 0;
+  set.floats = 0;
   for (int k = 0; k < 4; ++k) {
     set.l[k].build(*src[form][k]);
     for (GemmTaskTC& t : set.l[k].tasks) {
-      t.bsoff = floats;   // the task's pre-split ground-state chunks
-      floats += (long long)t.nterm * ((t.K + GTC_K - 1) / GTC_K) * t.npad * 2 * GTC_K;
+      t.bsoff = set.floats;   // the task's pre-split ground-state chunks
+      set.floats += (long long)t.nterm * ((t.K + GTC_K - 1) / GTC_K) * t.npad * 2 * GTC_K;
     }
     CK(upload(set.l[k].d_tasks, set.l[k].tasks.data(), set.l[k].tasks.size()));
   }
-  CK(dalloc(set.gsplit, (size_t)std::max(1LL, floats)));
+  set.listed = true;
+  return PNFAM_OK;
+}
+
+// and their pre-split ground-state operands, by the first run that takes them
+static int tc_operands(pnfam_ctx* c, int form) {
+  pnfam_ctx::TCSet& set = c->tc32[form];
+  if (set.built) return PNFAM_OK;
+  const int rc = tc_tables(c, form);
+  if (rc) return rc;
+  CK(dalloc(set.gsplit, (size_t)std::max(1LL, set.floats)));
   for (const TaskListTC& tl : set.l) {
     int mc = 0;
     for (const GemmTaskTC& t : tl.tasks) mc = std::max(mc, t.nterm * ((t.K + GTC_K - 1) / GTC_K));
@@ -1886,7 +1897,7 @@ static int ensure_buffers32(pnfam_ctx* c, int P, bool pair, bool run) {
     c->have_hphi = true;
   }
   if (run) {
-    const int rc = tc_tables(c, c->form);
+    const int rc = tc_operands(c, c->form);
     if (rc) return rc;
   }
   if (!general || !run) return PNFAM_OK;
@@ -2179,7 +2190,11 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
     if (rcs) return rcs;
   }
   c->pg_ready = c->pg_on = c->pg_built = c->have_general = c->have_k1 = false;
-  c->tc32[0].built = c->tc32[1].built = false;
+  for (pnfam_ctx::TCSet& s : c->tc32) s.listed = s.built = false;
+  {
+    const int rct = tc_tables(c, c->shared ? 1 : 0);
+    if (rct) return rct;
+  }
   CK(c->k2a.finalize()); CK(c->k2b.finalize());
   if (c->shared) { CK(c->s1a.finalize()); CK(c->s1b.finalize()); CK(c->s2a.finalize()); CK(c->s2b.finalize()); }
   if (!c->sep || !c->sep32) {

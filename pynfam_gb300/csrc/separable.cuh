@@ -79,8 +79,9 @@ SEP_HD double sep_value(int q, const double* z, const double* r, double v, doubl
 // functions are plainly not of the product form (sep_value still has to be compared).
 // Blocks nb / 2 ... are the time-reversed partners of the first half: their states are tried
 // with the factors of the partner's (same functions, spins exchanged) before a search, and
-// the others' searches look at one value before they compare whole functions. Host time,
-// Grace: 0.11 ms at N_sh = 6 and 1.6 at 16 (0.33 and 4.3 with a full search for every state)
+// the others' searches look at one value before they compare whole functions; the values are
+// those of the full search. Host time,
+// Grace: 0.12 ms at N_sh = 6 and 1.6 at 16 (0.33 and 4.3 with a full search for every state)
 inline bool sep_factors(int nb, const int* db, const int* st, const int* nup, int dqp, int nghl, int ngh,
                         const double* phi, SepBasis& B) {
   const int ngl = nghl / ngh;
@@ -93,7 +94,7 @@ inline bool sep_factors(int nb, const int* db, const int* st, const int* nup, in
   std::vector<int> zstar;               // ih of the largest |Z| of each z function
   std::vector<double> ztop;             // and Z there
   std::vector<std::vector<double>> lseg(2 * nb);
-  std::vector<double> row(ngl * 2), wbest(ngl);
+  std::vector<double> row(ngl * 2), wbest(ngl), tops(dqp, 0.0);
   std::vector<int> peer(dqp, -1);       // the state whose factors a state was found to share
   for (int i = 0; i < nb; ++i)
     for (int s = 0; s < 2; ++s) {
@@ -108,11 +109,11 @@ inline bool sep_factors(int nb, const int* db, const int* st, const int* nup, in
       double rtop = 0.0, dtop = 0.0;
       int rmax = 0;
       auto radial = [&](const double* f, int c0) {
-        const double *fd = f + ps, inv = 1.0 / ztop[c0];
+        const double* fd = f + ps;
         rtop = dtop = 0.0;
         for (int l = 0; l < ngl; ++l) {
-          row[2 * l] = f[(size_t)l * ngh + zstar[c0]] * inv;
-          row[2 * l + 1] = fd[(size_t)l * ngh + zstar[c0]] * inv;
+          row[2 * l] = f[(size_t)l * ngh + zstar[c0]] / ztop[c0];
+          row[2 * l + 1] = fd[(size_t)l * ngh + zstar[c0]] / ztop[c0];
           if (fabs(row[2 * l]) > rtop) { rtop = fabs(row[2 * l]); rmax = l; }
           if (fabs(row[2 * l + 1]) > dtop) dtop = fabs(row[2 * l + 1]);
         }
@@ -157,6 +158,7 @@ inline bool sep_factors(int nb, const int* db, const int* st, const int* nup, in
           for (; q < nghl; ++q) { const double x = fabs(f[q]); m4[0] = x > m4[0] ? x : m4[0]; }
           const double top = std::max(std::max(m4[0], m4[1]), std::max(m4[2], m4[3]));
           if (!(top > 0.0) || !std::isfinite(top)) return false;
+          tops[a] = top;
           int m = 0;
           while (fabs(f[m]) != top) ++m;
           const int ls = m / ngh, hs = m % ngh;
@@ -224,27 +226,22 @@ inline bool sep_factors(int nb, const int* db, const int* st, const int* nup, in
       B.lam[k] = d / big;
     }
   }
-  // V and e: phi_4 = (V - e_a) phi_0; e by least squares over the points where V is known, V
-  // from the state that is largest there
+  // V and e: phi_4 / phi_0 = V - e_a, each taken where the state is large
   std::vector<double> w(nghl, 0.0);
   for (int pass = 0; pass < 2; ++pass)
     for (int a = 0; a < dqp; ++a) {
       if (peer[a] >= 0) { B.e[a] = B.e[peer[a]]; continue; }
       const double *f = phi + (size_t)a * nghl, *g = phi + 4 * ps + (size_t)a * nghl;
-      double s0[4] = {0.0, 0.0, 0.0, 0.0}, s1[4] = {0.0, 0.0, 0.0, 0.0};   // four chains
-      auto add = [&](int k, int u) {
-        const double x = w[k] > 0.0 ? f[k] : 0.0;
-        s0[u] += x * x;
-        s1[u] += x * (B.v[k] * x - g[k]);
-      };
-      int k = 0;
-      for (; k + 4 <= nghl; k += 4)
-        for (int u = 0; u < 4; ++u) add(k + u, u);
-      for (; k < nghl; ++k) add(k, 0);
-      const double d = (s0[0] + s0[1]) + (s0[2] + s0[3]);
-      if (d > 0.0) B.e[a] = ((s1[0] + s1[1]) + (s1[2] + s1[3])) / d;
+      double s0 = 0.0, s1 = 0.0;
+      for (int k = 0; k < nghl; ++k) {
+        const double x = fabs(f[k]);
+        if (x < 1e-2 * tops[a] || w[k] == 0.0) continue;
+        s0 += x * w[k];
+        s1 += x * w[k] * (B.v[k] - g[k] / f[k]);
+      }
+      if (s0 > 0.0) B.e[a] = s1 / s0;
       if (pass == 0)
-        for (k = 0; k < nghl; ++k)
+        for (int k = 0; k < nghl; ++k)
           if (fabs(f[k]) > w[k]) { w[k] = fabs(f[k]); B.v[k] = g[k] / f[k] + B.e[a]; }
     }
   return true;
