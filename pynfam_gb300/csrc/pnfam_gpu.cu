@@ -2348,7 +2348,7 @@ static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver
   e->nxy = c->qn(); e->N = (int)(2 * c->nq * e->nxy); e->nops = c->nops;
   if ((rc = ensure_buffers(c, std::max(P, c->cap_P), std::max(std::max(e->M, 1), c->cap_M)))) return rc;
   c->cap_P = std::max(P, c->cap_P); c->cap_M = std::max(std::max(e->M, 1), c->cap_M);
-  if (e->mixed && (rc = ensure_buffers32(c, c->cap_P, c->pair32, true))) return rc;
+  if (e->mixed && (rc = ensure_buffers32(c, c->cap_P, c->pair32 && c->pg_on, true))) return rc;
   // Mixed form (precision 1): one Broyden iteration per evaluation, as in the FP64
   // form, but the residual interaction is evaluated in FP32 on the increment
   // d = X - X_a from an anchor X_a whose image g(X_a) is known in FP64:
