@@ -182,6 +182,9 @@ long long pnfam_gpu_state_size(const pnfam_ctx_t* ctx);
  * others keep iterating.  Engines of different contexts run on their own
  * streams and overlap on the GPU.  One engine per context at a time; the
  * context's solve buffers belong to the engine until pnfam_gpu_engine_free.
+ * pnfam_gpu_set_operator on such a context: an operator of the same block structure
+ * between two evaluations, any other one while the engine has no points (PNFAM_ESTATE
+ * otherwise, or when it has fewer cross terms than the engine returns).
  *
  *   create   slots and solver options (as for pnfam_gpu_solve)
  *   admit    up to n points into free slots; returns the number admitted

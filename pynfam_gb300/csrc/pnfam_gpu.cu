@@ -2131,16 +2131,30 @@ static void set_chunks(pnfam_ctx* c) {
   c->nchunk_c = (int)std::min<long long>(64, std::max<long long>(1, (n + 511) / 512));
 }
 
+// a context's engine under a change of operator: whether it may take it, and its form,
+// buffers and sizes afterwards
+static int engine_accepts(pnfam_ctx* c, int beta_minus, const int* fcols, int nops);
+static int engine_form(pnfam_engine* e, pnfam_ctx* c, bool active);
+static int engine_nactive(const pnfam_engine* e);
+
 extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int* fcols, const double* Fsp,
                                       int n_xterms, const double* const* Gsp) {
   g_err.clear();
   if (!c || !fcols || !Fsp || n_xterms < 0 || (n_xterms > 0 && !Gsp))
     return fail(PNFAM_EINVAL, "pnfam_gpu_set_operator: bad argument");
   const int nb = c->nb;
+  if (c->engine) {
+    const int rce = engine_accepts(c, beta_minus, fcols, 1 + n_xterms);
+    if (rce) return rce;
+  }
   {
     const int rcs = host_structure(c, beta_minus, fcols);
     if (rcs) return rcs;
   }
+  struct Guard {   // an engine does not go on with tables that were not finished
+    pnfam_ctx* c;
+    ~Guard() { if (c) c->detach_engine(); }
+  } guard{c};
   const long long nf = c->nxy;
   c->nops = 1 + n_xterms;
   CK(upload(c->d_fc, c->fc.data(), nb));
@@ -2232,6 +2246,8 @@ extern "C" int pnfam_gpu_set_operator(pnfam_ctx_t* c, int beta_minus, const int*
     CK(cudaGetLastError());
   }
   CK(cudaStreamSynchronize(c->stream));
+  if (c->engine && (rc = engine_form(c->engine, c, true))) return rc;
+  guard.c = nullptr;
   return PNFAM_OK;
 }
 
@@ -2318,20 +2334,10 @@ void pnfam_ctx::detach_engine() {
   }
 }
 
-// active: a start vector, if there is one, vanishes outside the active quasiparticles
-static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver_opts_t* o, bool active = true) {
-  if (!c->have_op) return fail(PNFAM_ESTATE, "call pnfam_gpu_set_operator first");
-  if (o->max_iter < 0) return fail(PNFAM_EINVAL, "max_iter < 0");
-  if (o->precision != 0 && o->precision != 1)
-    return fail(PNFAM_EINVAL, "precision must be 0 (FP64) or 1 (mixed FP32/FP64)");
-  e->c = c; e->o = *o; e->P = P;
-  e->no_res = std::fabs(o->quench_residual_int) < 1e-10;
-  e->M = e->no_res ? -1 : o->broyden_history_size;
-  if (e->M > 64) return fail(PNFAM_EINVAL, "broyden_history_size > 64 is not supported");
-  e->bmode = e->M < 0 ? BRO_NOMIX : e->M == 0 ? BRO_LINEAR : BRO_BROYDEN;
-  e->mixed = o->precision == 1 && !e->no_res;
+// the form of an engine's evaluations on the context's operator, and its buffers
+static int engine_form(pnfam_engine* e, pnfam_ctx* c, bool active) {
   c->sep64 = c->sep && (e->mixed || e->M <= 0 || e->M >= SEP_MIN_HISTORY);
-  c->pair32 = e->mixed && o->reserved[3] <= 0;
+  c->pair32 = e->mixed && e->o.reserved[3] <= 0;
   bool general = !c->shared || !active || (!e->mixed && e->M > 0 && e->M < SEP_MIN_HISTORY);
   if (c->pair32 && c->sep32) {
     pg_prepare(c);
@@ -2345,10 +2351,46 @@ static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver
     CK(c->k1a.finalize()); CK(c->k1b.finalize());
     c->have_k1 = true;
   }
-  e->nxy = c->qn(); e->N = (int)(2 * c->nq * e->nxy); e->nops = c->nops;
-  if ((rc = ensure_buffers(c, std::max(P, c->cap_P), std::max(std::max(e->M, 1), c->cap_M)))) return rc;
-  c->cap_P = std::max(P, c->cap_P); c->cap_M = std::max(std::max(e->M, 1), c->cap_M);
+  e->nxy = c->qn(); e->N = (int)(2 * c->nq * e->nxy);
+  if ((rc = ensure_buffers(c, std::max(e->P, c->cap_P), std::max(std::max(e->M, 1), c->cap_M)))) return rc;
+  c->cap_P = std::max(e->P, c->cap_P); c->cap_M = std::max(std::max(e->M, 1), c->cap_M);
   if (e->mixed && (rc = ensure_buffers32(c, c->cap_P, c->pair32 && c->pg_on, true))) return rc;
+  e->cpart.assign((size_t)e->P * c->nchunk_c * 2 * e->nops, 0.0);
+  CK(e->pin_d.ensure((size_t)3 * e->P + e->cpart.size()));
+  e->dirty_w = true;
+  return PNFAM_OK;
+}
+
+// An operator of another block structure may come while no point is in the engine; one of
+// the same structure at any time between its evaluations. The engine keeps its number of
+// strength values.
+static int engine_accepts(pnfam_ctx* c, int beta_minus, const int* fcols, int nops) {
+  const pnfam_engine* e = c->engine;
+  if (nops < e->nops)
+    return fail(PNFAM_ESTATE, "pnfam_gpu_set_operator: the context's engine has more cross terms");
+  const bool same = c->beta_minus == (beta_minus ? 1 : 0) && std::equal(c->fc.begin(), c->fc.end(), fcols);
+  if (!same && (engine_nactive(e) > 0 || e->pending))
+    return fail(PNFAM_ESTATE, "pnfam_gpu_set_operator: the context's engine has points of another block structure");
+  CK(cudaStreamSynchronize(c->stream64));
+  CK(cudaStreamSynchronize(c->stream));
+  return PNFAM_OK;
+}
+
+// active: a start vector, if there is one, vanishes outside the active quasiparticles
+static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver_opts_t* o, bool active = true) {
+  if (!c->have_op) return fail(PNFAM_ESTATE, "call pnfam_gpu_set_operator first");
+  if (o->max_iter < 0) return fail(PNFAM_EINVAL, "max_iter < 0");
+  if (o->precision != 0 && o->precision != 1)
+    return fail(PNFAM_EINVAL, "precision must be 0 (FP64) or 1 (mixed FP32/FP64)");
+  e->c = c; e->o = *o; e->P = P;
+  e->no_res = std::fabs(o->quench_residual_int) < 1e-10;
+  e->M = e->no_res ? -1 : o->broyden_history_size;
+  if (e->M > 64) return fail(PNFAM_EINVAL, "broyden_history_size > 64 is not supported");
+  e->bmode = e->M < 0 ? BRO_NOMIX : e->M == 0 ? BRO_LINEAR : BRO_BROYDEN;
+  e->mixed = o->precision == 1 && !e->no_res;
+  e->nops = c->nops;
+  int rc = engine_form(e, c, active);
+  if (rc) return rc;
   // Mixed form (precision 1): one Broyden iteration per evaluation, as in the FP64
   // form, but the residual interaction is evaluated in FP32 on the increment
   // d = X - X_a from an anchor X_a whose image g(X_a) is known in FP64:
@@ -2382,9 +2424,8 @@ static int engine_setup(pnfam_engine* e, pnfam_ctx* c, int P, const pnfam_solver
   for (cudaEvent_t& ev : e->aev)
     if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   CK(e->pin_a.ensure((size_t)ANCH_RING * P));
-  e->hsi.assign(P, 0.0); e->cpart.assign((size_t)P * c->nchunk_c * 2 * nops, 0.0);
+  e->hsi.assign(P, 0.0);
   CK(e->pin_i.ensure((size_t)10 * P + 1));
-  CK(e->pin_d.ensure((size_t)3 * P + e->cpart.size()));
   CK(e->pin_u.ensure((size_t)P));
   for (int k = 0; k < 8; ++k) c->stage_ms[k] = 0.0;
   for (int k = 0; k < 5; ++k) c->stage32_ms[k] = 0.0;
