@@ -1305,7 +1305,8 @@ static int ensure_buffers(pnfam_ctx* c, int P, int M) {
 }
 
 static int launch_gemm(pnfam_ctx* c, TaskList& tl, int P, const int* active, cudaStream_t st) {
-  if (tl.ntiles == 0) return PNFAM_OK;
+  if (tl.tasks.empty()) return PNFAM_OK;
+  if (tl.ntiles == 0) return fail(PNFAM_ESTATE, "block GEMMs without their tables");
   k_gemm<<<dim3(tl.ntiles, P), GT_THREADS, 0, st>>>(tl.d_tasks.p, tl.d_tile2task.p, c->d_bufs.p, active);
   c->launches++;
   CK(cudaGetLastError());
