@@ -27,3 +27,31 @@ def test_partner_blocks_of_another_kind(host, change):  # noqa: F811
     assert ngh == 20
     assert np.max(np.abs(s - ws)) <= 1e-12 * np.max(np.abs(ws))
     assert np.max(np.abs(x - wx)) <= 1e-12 * np.max(np.abs(wx))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", ["component", "value", "nan"])
+def test_other_bases_keep_the_general_kernels(monkeypatch, change):
+    """A basis that is a product but for one state's z derivative, one value or a NaN: the field is that
+    of the kernels over the mesh, to the last bit, and not that of the unit sums."""
+    import copy
+    import dataclasses
+    from test_separable import _fields
+    c = _case("S40", 6, "GT-K0")
+    h, k = c.hfb, c.hfb.dqp // 2 + 3
+    wf, wfdz, wfd2 = h.wf.copy(), h.wfdz.copy(), h.wfd2_all.copy()
+    if change == "component":
+        wfdz[k] *= 1.0 + 1e-9
+    elif change == "value":
+        wf[k, 37] += 1e-9
+    else:
+        wfd2[k, 5] = np.nan
+    c = copy.copy(c)
+    c.hfb = dataclasses.replace(h, wf=wf, wfdz=wfdz, wfd2_all=wfd2)
+    got = _fields(c, 4, False)
+    monkeypatch.setenv("PNFAM_GB300_SEPARABLE", "0")
+    want = _fields(c, 4, False)
+    assert all(np.array_equal(g, w, equal_nan=True) for g, w in zip(got, want))
+    monkeypatch.delenv("PNFAM_GB300_SEPARABLE")
+    units = _fields(_case("S40", 6, "GT-K0"), 4, False)
+    assert any(not np.array_equal(g, w) for g, w in zip(got, units))
